@@ -446,13 +446,13 @@ static int run_gemm(const GemmArgs& g, int variant, cudaStream_t stream, void* w
 }
 
 template <typename RoundT, bool kGather>
-static int launch_gate_up_tc(const CUtensorMap& map_x, const CUtensorMap& map_w,
-                             const GateUpParams& p, int grid, cudaStream_t stream) {
+static int launch_gate_up_tc(const CUtensorMap& map_x, const CUtensorMap& map_gate,
+                             const CUtensorMap& map_up, const GateUpParams& p, int grid, cudaStream_t stream) {
   auto kernel = moe_gate_up_tc_kernel<RoundT, kGather>;
   const cudaError_t error = cudaFuncSetAttribute(
       kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GateUpShape::kSmemBytes);
   if (error != cudaSuccess) return static_cast<int>(error);
-  kernel<<<grid, 384, GateUpShape::kSmemBytes, stream>>>(map_x, map_w, p);
+  kernel<<<grid, 384, GateUpShape::kSmemBytes, stream>>>(map_x, map_gate, map_up, p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -737,7 +737,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     }
     uint8_t* scratch = static_cast<uint8_t*>(gate_up_scratch);
     gg::GateUpParams p = {};
-    CUtensorMap map_x, map_w;
+    CUtensorMap map_x, map_gate, map_up;
     int status;
     if (row_gather) {
       p.silu_table = reinterpret_cast<float*>(scratch);
@@ -765,8 +765,17 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     if (status) return status;
     status = gg_moe_silu_table(const_cast<float*>(p.silu_table), out_dtype, stream_ptr);
     if (status) return status;
-    status = gg::encode_int8_rows(&map_w, w1, static_cast<long long>(experts) * 2 * intermediate,
-                                  hidden, hidden, 128);
+    const long long weight_rows = static_cast<long long>(experts) * 2 * intermediate;
+    if (interleaved) {
+      // Every other row: gate rows from the first, up rows from the second.
+      const int8_t* rows = static_cast<const int8_t*>(w1);
+      status = gg::encode_int8_rows(&map_gate, rows, weight_rows / 2, hidden, 2ll * hidden, 128);
+      if (status) return status;
+      status = gg::encode_int8_rows(&map_up, rows + hidden, weight_rows / 2, hidden, 2ll * hidden, 128);
+    } else {
+      status = gg::encode_int8_rows(&map_gate, w1, weight_rows, hidden, hidden, 128);
+      map_up = map_gate;
+    }
     if (status) return status;
     p.order = static_cast<const long long*>(order);
     p.top_k = top_k;
@@ -782,14 +791,14 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     const int grid = static_cast<int>(items < gg::sm_count() ? items : gg::sm_count());
     if (row_gather) {
       if (out_dtype == GG_OUT_BF16) {
-        return gg::launch_gate_up_tc<__nv_bfloat16, true>(map_x, map_w, p, grid, stream);
+        return gg::launch_gate_up_tc<__nv_bfloat16, true>(map_x, map_gate, map_up, p, grid, stream);
       }
-      return gg::launch_gate_up_tc<__half, true>(map_x, map_w, p, grid, stream);
+      return gg::launch_gate_up_tc<__half, true>(map_x, map_gate, map_up, p, grid, stream);
     }
     if (out_dtype == GG_OUT_BF16) {
-      return gg::launch_gate_up_tc<__nv_bfloat16, false>(map_x, map_w, p, grid, stream);
+      return gg::launch_gate_up_tc<__nv_bfloat16, false>(map_x, map_gate, map_up, p, grid, stream);
     }
-    return gg::launch_gate_up_tc<__half, false>(map_x, map_w, p, grid, stream);
+    return gg::launch_gate_up_tc<__half, false>(map_x, map_gate, map_up, p, grid, stream);
   }
   if (tile_rows != gg::kSimtTile || !gate_up_scratch) return static_cast<int>(cudaErrorInvalidValue);
   // CUDA-core path: ragged gathered GEMM into the scratch matrix, then SwiGLU + requantisation.

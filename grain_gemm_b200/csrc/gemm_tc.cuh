@@ -23,6 +23,15 @@
 // 128 rows of A and its own half of B, the leader CTA issues cta_group::2 MMAs that read both
 // CTAs' shared memory and write both CTAs' TMEM.
 //
+// What bounds it: the promotion warps' issue slots.  Per K group of a 128 x 256 tile a scheduler
+// issues 256 conversions, 128 packed multiplies and 128 packed multiply-adds (two slots each);
+// that arithmetic alone, on TMEM contents with no barrier in sight, takes 900 cycles, the MMAs
+// of a 256-deep group 1024.  So everything else in the loop is kept out of the way: waits vote
+// before they branch, the scale ring changes hands four groups at a time, no accumulator is
+// modified inside a branch, and waiting warps poll without a software loop around the probe.
+// That took a group of the G = 32 kernel from 1780 to 1500 cycles (M = 1024, N = K = 8192:
+// 464 to 408 us) and 8192^3 at G = 256 from 479 to 455 us in a short burst.
+//
 // Any M and N (rows/columns beyond the edge are zero-filled by TMA and never stored), any
 // K that is a multiple of 16 (TMA row pitch), G in {32, 64, 128, 256}; a partial last group
 // is zero-filled by TMA and uses scale index Q-1.
@@ -84,6 +93,11 @@ struct TileWork {
   bool whole_g256;           // G = 256 and the range is whole groups: fast issue path
 };
 
+// K groups per hand-over of staged scales: the scale ring is filled and released in chunks of
+// this many groups, so that a promotion warp passes the ring's two barriers once per chunk and
+// not once per group.
+constexpr int kScaleChunkGroups = 4;
+
 template <int kCtaGroup, int BN, int kStages, int kPromoWarps = 8, int kARows = 128>
 struct GemmTcShape {
   static constexpr int kBM = 128;                       // rows per CTA
@@ -101,9 +115,10 @@ struct GemmTcShape {
   // Ring of per-group scale vectors (the short-A shape is the split-K dump kernel, which
   // stages no scales and needs the room for its operand stages).
   static constexpr int kScaleSlots = kARows == 128 ? 8 : 4;
+  static constexpr int kScaleChunks = kScaleSlots / kScaleChunkGroups;
   static constexpr int kScaleSlotFloats = BN + 128;     // scale_b columns, then scale_a rows
   static constexpr int kScaleBytes = kScaleSlots * kScaleSlotFloats * 4;
-  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleSlots) * 8 + 16;
+  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks) * 8 + 16;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleBytes + kBarrierBytes;
   static constexpr int kThreads = (kPromoWarps + 4) * 32;   // + producer, MMA, two spares
   static constexpr int kColumnsPerThread = BN / (kPromoWarps / 4);
@@ -156,26 +171,19 @@ __device__ __forceinline__ TileWork decode_tile(const GemmTcParams& p, int tile,
   return w;
 }
 
-// TMEM drain layouts.  A promotion warp reads its 32 lanes x 32 columns of a block as two
-// fragments of 16 lanes; with r = lane / 4 and q = lane % 4 a thread receives rows r, r + 8
-// (and r + 16, r + 24 from the second fragment) and eight columns of the block:
-//   kFragmentPairs (tcgen05.ld.16x256b.x4): the pairs 8j + 2q, 8j + 2q + 1   (j = 0..3)
-//   kFragmentQuads (tcgen05.ld.16x128b.x8): the columns 4k + q               (k = 0..7)
-// Both need the same scales per thread (4 row scales, 8 column scales per block), far fewer
-// than the row-per-thread 32x32b shape, whose broadcast scale loads saturate the shared-memory
-// return path.  Measured on B200 with eight warps draining 128 lanes x 256 columns: 16x256b
-// delivers 256 B/clk/SM, 16x128b 507 B/clk/SM (32x32b 940 B/clk/SM), so the quad layout halves
-// the time the drain keeps TMEM's read port busy.
-enum FragmentLayout { kFragmentPairs = 0, kFragmentQuads = 1 };
-
-// The accumulator pair j (j = 0..3) of a thread holds the block's columns
-//   pairs layout: 8j + 2q, 8j + 2q + 1        quads layout: 8j + q, 8j + 4 + q.
+// TMEM drain layout.  A promotion warp reads its 32 lanes x 32 columns of a block as two
+// fragments of 16 lanes (tcgen05.ld.16x128b.x8); with r = lane / 4 and q = lane % 4 a thread
+// receives rows r, r + 8 (and r + 16, r + 24 from the second fragment) and the block's columns
+// 4k + q (k = 0..7): accumulator pair j (j = 0..3) holds columns 8j + q and 8j + 4 + q.  A thread
+// needs 4 row scales, and 8 column scales per block, far fewer than in the row-per-thread 32x32b
+// shape, whose broadcast scale loads saturate the shared-memory return path.  Measured on B200
+// with eight warps draining 128 lanes x 256 columns: 16x128b delivers 507 B/clk/SM, 32x32b 940,
+// and 16x256b, which would give adjacent column pairs, 256.
+//
 // Position of block column `c` (0..31) in the scale ring: thread q reads its eight column
 // scales, in accumulator-pair order, as two 16-byte vectors at q * 8.
-template <FragmentLayout kLayout>
 __device__ __forceinline__ int ring_column_position(int c) {
-  if constexpr (kLayout == kFragmentPairs) return ((c >> 1) & 3) * 8 + (c >> 3) * 2 + (c & 1);
-  else return (c & 3) * 8 + (c >> 3) * 2 + ((c >> 2) & 1);
+  return (c & 3) * 8 + (c >> 3) * 2 + ((c >> 2) & 1);
 }
 // Position of row `r` (0..31 within its warp's 32 rows): the thread with row index
 // lane / 4 = r % 8 reads its four rows r % 8 + 8j as one 16-byte vector.
@@ -203,27 +211,18 @@ __device__ __forceinline__ void load_row_scales(const float* warp_rows_base, int
   sa[3] = make_float2(v.w, v.w);
 }
 
-template <FragmentLayout kLayout>
-__device__ __forceinline__ void tmem_ld_fragment(uint32_t taddr, uint32_t (&r)[16]) {
-  if constexpr (kLayout == kFragmentPairs) tmem_ld_16x256b_x4(taddr, r);
-  else tmem_ld_16x128b_x8(taddr, r);
-}
-
 // Promotion of one 16-row x 32-column fragment: this thread holds rows r ("low") and r + 8
 // ("high") and four column pairs; `sb` are the scales of those pairs, read once per 32-column
-// block and used for both 16-row fragments.  Registers: pairs layout 4j + {0,1} = low pair j,
-// 4j + {2,3} = high pair j; quads layout 4j + {0,2} = low pair j, 4j + {1,3} = high pair j.
-template <FragmentLayout kLayout>
+// block and used for both 16-row fragments.  Registers 4j + {0,2} are low pair j, 4j + {1,3}
+// high pair j.
 __device__ __forceinline__ void promote_fragment(const uint32_t (&partial)[16], float2 sa_low2,
                                                  float2 sa_high2, const float2 (&sb)[4],
                                                  float2* acc_low, float2* acc_high) {
-  constexpr int kLowY = kLayout == kFragmentPairs ? 1 : 2;
-  constexpr int kHighX = kLayout == kFragmentPairs ? 2 : 1;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const float2 low = make_float2(__int2float_rn(static_cast<int>(partial[4 * j + 0])),
-                                   __int2float_rn(static_cast<int>(partial[4 * j + kLowY])));
-    const float2 high = make_float2(__int2float_rn(static_cast<int>(partial[4 * j + kHighX])),
+                                   __int2float_rn(static_cast<int>(partial[4 * j + 2])));
+    const float2 high = make_float2(__int2float_rn(static_cast<int>(partial[4 * j + 1])),
                                     __int2float_rn(static_cast<int>(partial[4 * j + 3])));
     acc_low[j] = __ffma2_rn(low, __fmul2_rn(sa_low2, sb[j]), acc_low[j]);
     acc_high[j] = __ffma2_rn(high, __fmul2_rn(sa_high2, sb[j]), acc_high[j]);
@@ -268,7 +267,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   constexpr int kNC = Shape::kColumnsPerThread;   // columns owned by one promotion thread
   constexpr int kProducerWarp = kPromoWarps, kMmaWarp = kPromoWarps + 1;
   constexpr int kScaleWarp = kPromoWarps + 2;
-  constexpr FragmentLayout kLayout = kFragmentQuads;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -281,11 +279,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint64_t* tmem_full_bar = empty_bar + kStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint64_t* scale_full_bar = tmem_empty_bar + 2;
-  uint64_t* scale_empty_bar = scale_full_bar + Shape::kScaleSlots;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(scale_empty_bar + Shape::kScaleSlots);
+  uint64_t* scale_empty_bar = scale_full_bar + Shape::kScaleChunks;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(scale_empty_bar + Shape::kScaleChunks);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5;
+  // The same in every lane, and known to be: addresses built from it stay in uniform registers.
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const uint32_t cta_rank = kCtaGroup == 2 ? cluster_ctarank() : 0u;
   const int worker = blockIdx.x / kCtaGroup;
@@ -303,7 +302,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       mbar_init(&tmem_full_bar[i], 1);
       mbar_init(&tmem_empty_bar[i], kPromoWarps * kCtaGroup);
     }
-    for (int i = 0; i < Shape::kScaleSlots; ++i) {
+    for (int i = 0; i < Shape::kScaleChunks; ++i) {
       mbar_init(&scale_full_bar[i], 32);            // every lane of the scale warp
       mbar_init(&scale_empty_bar[i], kPromoWarps);  // one arrival per promotion warp
     }
@@ -504,7 +503,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // warps and a global-memory latency of several K groups stays hidden (a version that
     // held one group in registers left the promotion warps waiting for scales).
     constexpr int kColumnsPerLane = BN / 32;
-    uint32_t slot = 0, phase = 0;
+    // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
+    const uint32_t column_position = 4 * ring_column_position(lane);
+    const uint32_t row_position = 4 * ring_row_position(lane);
+    const uint32_t ring_base = smem_u32(scale_ring);
+    uint32_t chunk = 0, phase = 0;
     bool ok = true;
     for (int tile = worker; tile < total_tiles && ok; tile += workers) {
       const TileWork work = decode_tile(p, tile, tiles_m);
@@ -521,46 +524,39 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         row_limit = p.m;
       }
       const int n0 = work.tn * BN;
-      // Per-lane sources and destinations do not change within the tile.
-      const float* sb_source[kColumnsPerLane];
-      const float* sa_source[4];
-      bool sb_valid[kColumnsPerLane], sa_valid[4];
-#pragma unroll
-      for (int i = 0; i < kColumnsPerLane; ++i) {
-        const int col = n0 + lane + 32 * i;
-        sb_valid[i] = col < p.n;
-        sb_source[i] = sb_base + (sb_valid[i] ? col * p.sb_sn : 0);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = row0 + lane + 32 * i;
-        sa_valid[i] = r < row_limit;
-        sa_source[i] = p.scale_a + (sa_valid[i] ? r * p.sa_sm : 0);
-      }
-      const int column_position = ring_column_position<kLayout>(lane);
-      const int row_position = ring_row_position(lane);
-      for (int g = 0; g < work.groups; ++g) {
-        const bool got = mbar_test(&scale_empty_bar[slot], phase ^ 1u) ||
-                         mbar_wait(&scale_empty_bar[slot], phase ^ 1u, kSiteScaleEmpty, abort_flag);
-        if (!__all_sync(0xffffffffu, got)) {
+      // The lane's first column and row; the others follow at steps of 32.  One pointer per
+      // operand advances through a group's copies and on to the next group, which keeps the
+      // warp within its registers.  A copy that is not valid writes zero and reads nothing.
+      const float* sb_source = sb_base + static_cast<long long>(n0 + lane) * p.sb_sn +
+                               static_cast<long long>(work.group_begin) * p.sb_sg;
+      const float* sa_source = p.scale_a + static_cast<long long>(row0 + lane) * p.sa_sm +
+                               static_cast<long long>(work.group_begin) * p.sa_sg;
+      const int columns_left = p.n - n0 - lane, rows_left = row_limit - row0 - lane;
+      const long long sb_step = 32 * p.sb_sn, sb_next = p.sb_sg - kColumnsPerLane * sb_step;
+      const long long sa_step = 32 * p.sa_sm, sa_next = p.sa_sg - 4 * sa_step;
+      for (int g = 0; g < work.groups; g += kScaleChunkGroups) {
+        if (!mbar_wait_warp(&scale_empty_bar[chunk], phase ^ 1u, kSiteScaleEmpty, abort_flag)) {
           ok = false;
           break;
         }
-        const long long group = work.group_begin + g;
-        float* destination = scale_ring + slot * Shape::kScaleSlotFloats;
+        const int in_chunk = min(kScaleChunkGroups, work.groups - g);
+        uint32_t destination = ring_base + chunk * (kScaleChunkGroups * Shape::kScaleSlotFloats * 4);
+        for (int i = 0; i < in_chunk; ++i) {
 #pragma unroll
-        for (int i = 0; i < kColumnsPerLane; ++i) {
-          cp_async_f32(destination + 32 * i + column_position, sb_source[i] + group * p.sb_sg,
-                       sb_valid[i]);
-        }
+          for (int j = 0; j < kColumnsPerLane; ++j, sb_source += sb_step) {
+            cp_async_f32(destination + 128 * j + column_position, sb_source, 32 * j < columns_left);
+          }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          cp_async_f32(destination + BN + 32 * i + row_position, sa_source[i] + group * p.sa_sg,
-                       sa_valid[i]);
+          for (int j = 0; j < 4; ++j, sa_source += sa_step) {
+            cp_async_f32(destination + 4 * BN + 128 * j + row_position, sa_source, 32 * j < rows_left);
+          }
+          sb_source += sb_next;
+          sa_source += sa_next;
+          destination += Shape::kScaleSlotFloats * 4;
         }
-        cp_async_arrive(&scale_full_bar[slot]);
-        if (++slot == Shape::kScaleSlots) {
-          slot = 0;
+        cp_async_arrive(&scale_full_bar[chunk]);
+        if (++chunk == Shape::kScaleChunks) {
+          chunk = 0;
           phase ^= 1u;
         }
       }
@@ -575,7 +571,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int row_in_cta = quarter * 32 + lane;
     const int col_base = half * kNC;
     uint32_t group_sequence = 0;
-    uint32_t scale_slot = 0, scale_phase = 0;
+    uint32_t scale_chunk = 0, scale_phase = 0;
     bool ok = true;
     OutT* c = reinterpret_cast<OutT*>(p.c);
     // A failed wait clears `ok` but the loops keep their shape, so that every thread still
@@ -657,14 +653,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       static_assert(!kDump || kCtaGroup == 1, "split-K dump runs on single CTAs");
       const int fragment_row = lane >> 2;
 
-      // `ok` is the same in every lane (mbar_wait_warp votes), so the .sync.aligned TMEM
-      // instructions below always see a converged warp, also after a wait has run out.
-      for (int g = 0; g < groups; ++g, ++group_sequence) {
-        // This group's scales, staged by the scale warp.
-        if (ok) {
-          ok = mbar_wait_warp(&scale_full_bar[scale_slot], scale_phase, kSiteScaleFull, abort_flag);
+      if (!warp_has_rows) {
+        // None of this warp's 32 rows exists (a skinny problem, the ragged end of an expert):
+        // nothing to promote, scales and buffers go straight back.
+        for (int g = 0; g < groups; ++g, ++group_sequence) {
+          const int in_chunk = g & (kScaleChunkGroups - 1);
+          const uint32_t buffer = group_sequence & 1u;
+          if (ok) {
+            ok = mbar_wait_warp(&tmem_full_bar[buffer], (group_sequence >> 1) & 1u,
+                                kSiteEpilogueTmemFull, abort_flag);
+          }
+          if (ok && in_chunk == 0) {
+            ok = mbar_wait_warp(&scale_full_bar[scale_chunk], scale_phase, kSiteScaleFull, abort_flag);
+          }
+          if (lane == 0) {
+            if constexpr (kCtaGroup == 1) mbar_arrive(&tmem_empty_bar[buffer]);
+            else mbar_arrive_cluster(&tmem_empty_bar[buffer], 0);
+          }
+          if (in_chunk == kScaleChunkGroups - 1 || g == groups - 1) {
+            if (lane == 0) mbar_arrive(&scale_empty_bar[scale_chunk]);
+            if (++scale_chunk == Shape::kScaleChunks) {
+              scale_chunk = 0;
+              scale_phase ^= 1u;
+            }
+          }
         }
-        const float* scale_slot_base = scale_ring + scale_slot * Shape::kScaleSlotFloats;
+        continue;
+      }
+      // `ok` is the same in every lane (mbar_wait_warp votes), so the .sync.aligned TMEM
+      // instructions below always see a converged warp, also after a wait has run out.  The
+      // arithmetic itself is not conditional on it (a tile with a failed wait is not stored):
+      // inside a branch the compiler copies half of the accumulators around every group.
+      for (int g = 0; g < groups; ++g, ++group_sequence) {
+        // This group's scales, staged by the scale warp a chunk of groups at a time.
+        const int in_chunk = g & (kScaleChunkGroups - 1);
+        if (in_chunk == 0 && ok) {
+          ok = mbar_wait_warp(&scale_full_bar[scale_chunk], scale_phase, kSiteScaleFull, abort_flag);
+        }
+        const float* scale_slot_base =
+            scale_ring + (scale_chunk * kScaleChunkGroups + in_chunk) * Shape::kScaleSlotFloats;
         float2 sa[4];
         load_row_scales(scale_slot_base + BN + quarter * 32, fragment_row, sa);
         const uint32_t buffer = group_sequence & 1u;
@@ -681,17 +708,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         // of the next fragment is in flight while the current one is promoted.
         uint32_t partial_a[16], partial_b[16];
         float2 sb[4];
-        if (ok && !warp_has_rows) {
-          // None of this warp's 32 rows exists (a skinny problem, the ragged end of an expert):
-          // nothing to promote, the buffer goes straight back.
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if constexpr (kCtaGroup == 1) mbar_arrive(&tmem_empty_bar[buffer]);
-            else mbar_arrive_cluster(&tmem_empty_bar[buffer], 0);
-          }
-        } else if (ok) {
-          tmem_ld_fragment<kLayout>(taddr_low, partial_a);
+        {
+          tmem_ld_16x128b_x8(taddr_low, partial_a);
 #pragma unroll
           for (int fragment = 0; fragment < 2 * kBlocks; ++fragment) {
             const int block = fragment >> 1;
@@ -701,8 +719,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             if (fragment + 1 < 2 * kBlocks) {
               const uint32_t next = ((fragment + 1) & 1 ? taddr_high : taddr_low) +
                                     ((fragment + 1) >> 1) * 32;
-              if (fragment & 1) tmem_ld_fragment<kLayout>(next, partial_a);
-              else tmem_ld_fragment<kLayout>(next, partial_b);
+              if (fragment & 1) tmem_ld_16x128b_x8(next, partial_a);
+              else tmem_ld_16x128b_x8(next, partial_b);
             } else {
               // All of this warp's TMEM accesses for the buffer are done: hand it back.
               tcgen05_fence_before();
@@ -713,26 +731,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               }
             }
             if (fragment & 1) {
-              promote_fragment<kLayout>(partial_b, sa[2], sa[3], sb, &acc[2][block * 4],
-                                      &acc[3][block * 4]);
+              promote_fragment(partial_b, sa[2], sa[3], sb, &acc[2][block * 4],
+                               &acc[3][block * 4]);
             } else {
-              promote_fragment<kLayout>(partial_a, sa[0], sa[1], sb, &acc[0][block * 4],
-                                      &acc[1][block * 4]);
+              promote_fragment(partial_a, sa[0], sa[1], sb, &acc[0][block * 4],
+                               &acc[1][block * 4]);
             }
           }
         }
-        // Every lane has consumed the slot's values (they fed the arithmetic above).
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&scale_empty_bar[scale_slot]);
-        if (++scale_slot == Shape::kScaleSlots) {
-          scale_slot = 0;
-          scale_phase ^= 1u;
+        if (in_chunk == kScaleChunkGroups - 1 || g == groups - 1) {
+          // Every lane has consumed the chunk's values (they fed the arithmetic above).
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&scale_empty_bar[scale_chunk]);
+          if (++scale_chunk == Shape::kScaleChunks) {
+            scale_chunk = 0;
+            scale_phase ^= 1u;
+          }
         }
       }
       // The fragment layout leaves each lane with columns spread over the block.  A 4x4
       // exchange inside every quad gives lane q the eight consecutive columns 8q..8q+7 of each
-      // 32-column block (after it, accumulator pair i of the quads layout holds columns
-      // 8q + i and 8q + 4 + i), so that a row leaves as 16-byte stores: a quarter of the store
+      // 32-column block (after it, accumulator pair i holds columns 8q + i and 8q + 4 + i), so that a row leaves as 16-byte stores: a quarter of the store
       // instructions and of the memory-pipe wavefronts of pair stores.
       if (ok) {
         const int quad = lane & 3;
@@ -783,13 +802,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                   for (int i = 0; i < 4; ++i) w[half][i] = pack_pair<OutT>(acc[r][(block + half) * 4 + i]);
                   quad_transpose(w[half], quad);
-                  if constexpr (kLayout == kFragmentQuads) {
-                    const uint32_t v0 = w[half][0], v1 = w[half][1], v2 = w[half][2], v3 = w[half][3];
-                    w[half][0] = __byte_perm(v0, v1, 0x5410);
-                    w[half][1] = __byte_perm(v2, v3, 0x5410);
-                    w[half][2] = __byte_perm(v0, v1, 0x7632);
-                    w[half][3] = __byte_perm(v2, v3, 0x7632);
-                  }
+                  const uint32_t v0 = w[half][0], v1 = w[half][1], v2 = w[half][2], v3 = w[half][3];
+                  w[half][0] = __byte_perm(v0, v1, 0x5410);
+                  w[half][1] = __byte_perm(v2, v3, 0x5410);
+                  w[half][2] = __byte_perm(v0, v1, 0x7632);
+                  w[half][3] = __byte_perm(v2, v3, 0x7632);
                 }
                 // Low lanes keep block `block` and give away the next one, high lanes the reverse.
                 uint32_t received[4];
@@ -826,13 +843,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
               for (int i = 0; i < 4; ++i) w[i] = pack_pair<OutT>(acc[r][block * 4 + i]);
               quad_transpose(w, quad);
-              if constexpr (kLayout == kFragmentQuads) {
-                const uint32_t v0 = w[0], v1 = w[1], v2 = w[2], v3 = w[3];
-                w[0] = __byte_perm(v0, v1, 0x5410);
-                w[1] = __byte_perm(v2, v3, 0x5410);
-                w[2] = __byte_perm(v0, v1, 0x7632);
-                w[3] = __byte_perm(v2, v3, 0x7632);
-              }
+              const uint32_t v0 = w[0], v1 = w[1], v2 = w[2], v3 = w[3];
+              w[0] = __byte_perm(v0, v1, 0x5410);
+              w[1] = __byte_perm(v2, v3, 0x5410);
+              w[2] = __byte_perm(v0, v1, 0x7632);
+              w[3] = __byte_perm(v2, v3, 0x7632);
               if (row_stored) {
                 if (aligned && col + 8 <= p.n) {
                   *reinterpret_cast<uint4*>(c_row + col) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -857,21 +872,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               if (row_stored) {
                 if (aligned && col + 8 <= p.n) {
                   uint4* out = reinterpret_cast<uint4*>(c_row + col);
-                  if constexpr (kLayout == kFragmentQuads) {
-                    out[0] = make_uint4(wx[0], wx[1], wx[2], wx[3]);
-                    out[1] = make_uint4(wy[0], wy[1], wy[2], wy[3]);
-                  } else {
-                    out[0] = make_uint4(wx[0], wy[0], wx[1], wy[1]);
-                    out[1] = make_uint4(wx[2], wy[2], wx[3], wy[3]);
-                  }
+                  out[0] = make_uint4(wx[0], wx[1], wx[2], wx[3]);
+                  out[1] = make_uint4(wy[0], wy[1], wy[2], wy[3]);
                 } else {
                   uint32_t* out = reinterpret_cast<uint32_t*>(c_row);
-                  constexpr int kStepX = kLayout == kFragmentQuads ? 1 : 2;
-                  constexpr int kOffsetY = kLayout == kFragmentQuads ? 4 : 1;
 #pragma unroll
                   for (int j = 0; j < 4; ++j) {
-                    if (col + kStepX * j < p.n) out[col + kStepX * j] = wx[j];
-                    if (col + kStepX * j + kOffsetY < p.n) out[col + kStepX * j + kOffsetY] = wy[j];
+                    if (col + j < p.n) out[col + j] = wx[j];
+                    if (col + 4 + j < p.n) out[col + 4 + j] = wy[j];
                   }
                 }
               }

@@ -56,9 +56,10 @@ struct GateUpShape {
   static constexpr int kStashBytes = 256 * 64 * 4;   // 64 parked FP32 values per promotion thread
   static constexpr int kRingFloats = 256 + 128;   // column scales then row scales of one group
   static constexpr int kScaleSlots = 8;
+  static constexpr int kScaleChunks = kScaleSlots / kScaleChunkGroups;
   static constexpr int kScaleBytes = kScaleSlots * kRingFloats * 4;
   static constexpr int kAmaxBytes = 2 * 4 * 128 * 4;   // two item parities x (sub, half) x 128 rows
-  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleSlots) * 8 + 16;
+  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks) * 8 + 16;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStashBytes + kScaleBytes +
                                     kAmaxBytes + kBarrierBytes;
 };
@@ -101,10 +102,16 @@ __device__ __forceinline__ int gate_up_source_row(const GateUpParams& p, int row
 // kGather: map_x covers the original activations x[T, H] and the producer fetches each tile's
 // rows by token index with TMA row gathers (no copy of the rows in sorted order exists);
 // otherwise map_x covers a pre-sorted copy [S, H] and the tile is one tiled box.
+// map_gate and map_up cover the weight rows.  For the split layout both are the whole weight and
+// a channel's up row lies I rows behind its gate row; for the interleaved layout each covers every
+// other row (twice the row pitch, map_up starting one row later), so that the accumulator has
+// 128 gate columns and then 128 up columns in either case and nothing behind the loads
+// depends on the layout.
 template <typename RoundT, bool kGather>
 __global__ void __launch_bounds__(384, 1)
 moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
-                      const __grid_constant__ CUtensorMap map_w, const GateUpParams p) {
+                      const __grid_constant__ CUtensorMap map_gate,
+                      const __grid_constant__ CUtensorMap map_up, const GateUpParams p) {
   using Shape = GateUpShape;
   constexpr int kStages = Shape::kStages;
   constexpr int BN = 256;
@@ -122,11 +129,12 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   uint64_t* tmem_full_bar = empty_bar + kStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint64_t* scale_full_bar = tmem_empty_bar + 2;
-  uint64_t* scale_empty_bar = scale_full_bar + Shape::kScaleSlots;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(scale_empty_bar + Shape::kScaleSlots);
+  uint64_t* scale_empty_bar = scale_full_bar + Shape::kScaleChunks;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(scale_empty_bar + Shape::kScaleChunks);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5;
+  // The same in every lane, and known to be: addresses built from it stay in uniform registers.
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int channel_groups = p.intermediate / 256;
   const int groups = p.hidden / 256;
@@ -141,7 +149,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       mbar_init(&tmem_full_bar[i], 1);
       mbar_init(&tmem_empty_bar[i], 8);
     }
-    for (int i = 0; i < Shape::kScaleSlots; ++i) {
+    for (int i = 0; i < Shape::kScaleChunks; ++i) {
       mbar_init(&scale_full_bar[i], 32);   // every lane of the scale warp
       mbar_init(&scale_empty_bar[i], 8);   // one arrival per promotion warp
     }
@@ -150,7 +158,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   }
   if (warp == 8 && lane == 0) {
     prefetch_tensormap(&map_x);
-    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_gate);
+    prefetch_tensormap(&map_up);
   }
   // The row-tile list has room for the worst case and its used entries come first; the kernel
   // walks only those.  (An expert-parallel rank's list is sized for every row it could
@@ -171,7 +180,6 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   const int total_items = used_row_tiles * channel_groups;
-  constexpr FragmentLayout kLayout = kFragmentPairs;
 
   // Warps 8-11 (producer, MMA issuer, two spares) give registers to the promotion warps.
   if (warp >= 8) {
@@ -196,9 +204,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
         for (int sub = 0; sub < 2 && ok; ++sub) {
           const int channel0 = jg * 256 + sub * 128;
-          const int w_base = expert * 2 * p.intermediate;
-          const int row_gate = p.interleaved ? w_base + 2 * channel0 : w_base + channel0;
-          const int row_up = p.interleaved ? row_gate + 128 : w_base + p.intermediate + channel0;
+          const int row_gate = expert * (p.interleaved ? 1 : 2) * p.intermediate + channel0;
+          const int row_up = p.interleaved ? row_gate : row_gate + p.intermediate;
           for (int slab = 0, x = 0; slab < slabs; ++slab, x += 128) {
             if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, kSiteProducerEmpty, abort_flag)) {
               ok = false;
@@ -209,8 +216,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             if (leader) {
               mbar_expect_tx(&full_bar[stage], Shape::kStageBytes);
               if constexpr (!kGather) tma_load_2d(a_dst, &map_x, &full_bar[stage], x, row0);
-              tma_load_2d(b_dst, &map_w, &full_bar[stage], x, row_gate);
-              tma_load_2d(b_dst + 128 * 128, &map_w, &full_bar[stage], x, row_up);
+              tma_load_2d(b_dst, &map_gate, &full_bar[stage], x, row_gate);
+              tma_load_2d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, row_up);
             }
             if constexpr (kGather) {
               // Every lane fetches its four rows: 32 gathers of 512 bytes fill the A tile.
@@ -230,10 +237,14 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       // shared-memory ring with asynchronous 4-byte copies that land in the order the
       // promotion threads read; the copies themselves signal the slot's barrier, so the warp
       // runs a whole ring ahead and global-memory latency stays hidden.
-      uint32_t slot = 0, phase = 0;
+      uint32_t chunk = 0, phase = 0;
       bool ok = true;
-      const int column_position = ring_column_position<kLayout>(lane);
-      const int row_position = ring_row_position(lane);
+      // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
+      const uint32_t column_position = 4 * ring_column_position(lane);
+      const uint32_t row_position = 4 * ring_row_position(lane);
+      const uint32_t ring_base = smem_u32(sb_ring);
+      const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale
+      const int sb_step = p.interleaved ? 64 : 32;                // 32 channels further
       for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
         int tile, jg, expert;
         if (!gate_up_item(p, item, channel_groups, tile, jg, expert)) continue;
@@ -250,35 +261,32 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           sa_source[i] = p.row_scale + source_row * groups;
         }
         for (int sub = 0; sub < 2 && ok; ++sub) {
-          const int channel0 = jg * 256 + sub * 128;
-          const float* sb_source[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int c = lane + 32 * i;   // accumulator column
-            const int sb_col = p.interleaved ? 2 * channel0 + c
-                                             : (i < 4 ? channel0 + c : p.intermediate + channel0 + c - 128);
-            sb_source[i] = sb_base + sb_col;
-          }
-          for (int g = 0; g < groups; ++g) {
-            const bool got = mbar_test(&scale_empty_bar[slot], phase ^ 1u) ||
-                             mbar_wait(&scale_empty_bar[slot], phase ^ 1u, kSiteScaleEmpty, abort_flag);
-            if (!__all_sync(0xffffffffu, got)) {
+          const int channel = jg * 256 + sub * 128 + lane;
+          const float* sb_source = sb_base + (p.interleaved ? 2 * channel : channel);
+          for (int g = 0; g < groups; g += kScaleChunkGroups) {
+            if (!mbar_wait_warp(&scale_empty_bar[chunk], phase ^ 1u, kSiteScaleEmpty, abort_flag)) {
               ok = false;
               break;
             }
-            float* destination = sb_ring + slot * Shape::kRingFloats;
+            const int in_chunk = min(kScaleChunkGroups, groups - g);
+            uint32_t destination = ring_base + chunk * (kScaleChunkGroups * Shape::kRingFloats * 4);
+            for (int i = 0; i < in_chunk; ++i) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              cp_async_f32(destination + 32 * i + column_position,
-                           sb_source[i] + static_cast<long long>(g) * 2 * p.intermediate, true);
-            }
+              for (int j = 0; j < 8; ++j) {
+                cp_async_f32(destination + 128 * j + column_position,
+                             sb_source + (j & 3) * sb_step + (j < 4 ? 0 : up_offset), true);
+              }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              cp_async_f32(destination + BN + 32 * i + row_position, sa_source[i] + g, sa_valid[i]);
+              for (int j = 0; j < 4; ++j) {
+                cp_async_f32(destination + 4 * BN + 128 * j + row_position, sa_source[j] + (g + i),
+                             sa_valid[j]);
+              }
+              sb_source += 2 * p.intermediate;
+              destination += Shape::kRingFloats * 4;
             }
-            cp_async_arrive(&scale_full_bar[slot]);
-            if (++slot == Shape::kScaleSlots) {
-              slot = 0;
+            cp_async_arrive(&scale_full_bar[chunk]);
+            if (++chunk == Shape::kScaleChunks) {
+              chunk = 0;
               phase ^= 1u;
             }
           }
@@ -342,19 +350,18 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   } else {
     setmaxnreg_inc<GG_PROMO_REGS>();
     // ------------------------------------------------------------ promotion + SwiGLU warps
-    // Fragment layout (tmem_ld_16x256b_x4): warp (quarter, half) drains TMEM lanes
+    // Fragment layout (tmem_ld_16x128b_x8): warp (quarter, half) drains TMEM lanes
     // 32*quarter.. of four 32-column blocks; a thread owns tile rows
     // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, the column pairs
-    // 8i + 2*(lane%4), +1 (i = 0..3).  Split layout: blocks 0,1 are 64 gate columns of this
-    // half, blocks 2,3 the matching up columns; interleaved: each pair is (gate, up) of one
-    // channel.
+    // 8i + lane%4, +4 (i = 0..3).  Blocks 0,1 are 64 gate columns of this half, blocks 2,3 the
+    // matching up columns.
     const int half = warp >> 2;
     const int quarter = warp & 3;
     const int tid = threadIdx.x;
     const int fragment_row = lane >> 2;
     const int quad = lane & 3;
     uint32_t group_sequence = 0;
-    uint32_t scale_slot = 0, scale_phase = 0;
+    uint32_t scale_chunk = 0, scale_phase = 0;
     bool ok = true;
     float4* stash4 = reinterpret_cast<float4*>(stash) + tid;   // element j at stash4[j * 256]
     // The row-maximum exchange buffer alternates between two copies from one work item to the
@@ -362,12 +369,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     // half is still reading this item's; the barrier of the next item keeps it from getting
     // two items ahead.
     uint32_t item_parity = 0;
-    int block_column[4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      block_column[b] = p.interleaved ? half * 128 + 32 * b
-                                      : (b < 2 ? half * 64 + 32 * b : 128 + half * 64 + 32 * (b - 2));
-    }
+    // First accumulator column of block b: gate columns of this half, then the up columns.
+    const auto block_column = [half](int b) { return half * 64 + 32 * (b & 1) + (b < 2 ? 0 : 128); };
     for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
       int tile, jg, expert;
       if (!gate_up_item(p, item, channel_groups, tile, jg, expert)) continue;
@@ -384,13 +387,16 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           for (int i = 0; i < 16; ++i) acc[r][i] = make_float2(0.0f, 0.0f);
         }
         for (int g = 0; g < groups; ++g, ++group_sequence) {
-          // This group's scales, staged by the scale warp: [0, 256) column scales by
-          // accumulator column, [256, 384) row scales by tile row (both in the order the
-          // promotion threads read them).  `ok` is the same in every lane.
-          if (ok) {
-            ok = mbar_wait_warp(&scale_full_bar[scale_slot], scale_phase, kSiteScaleFull, abort_flag);
+          // This group's scales, staged by the scale warp a chunk of groups at a time: [0, 256)
+          // column scales by accumulator column, [256, 384) row scales by tile row (both in the
+          // order the promotion threads read them).  `ok` is the same in every lane; the
+          // arithmetic is not conditional on it (an item with a failed wait is not stored):
+          // inside a branch the compiler copies half of the accumulators around every group.
+          const int in_chunk = g & (kScaleChunkGroups - 1);
+          if (in_chunk == 0 && ok) {
+            ok = mbar_wait_warp(&scale_full_bar[scale_chunk], scale_phase, kSiteScaleFull, abort_flag);
           }
-          const float* slot = sb_ring + scale_slot * Shape::kRingFloats;
+          const float* slot = sb_ring + (scale_chunk * kScaleChunkGroups + in_chunk) * Shape::kRingFloats;
           float2 sa[4];
           load_row_scales(slot + BN + quarter * 32, fragment_row, sa);
           const uint32_t buffer = group_sequence & 1u;
@@ -404,45 +410,42 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           const uint32_t taddr_high = taddr_low + (16u << 16);
           uint32_t partial_a[16], partial_b[16];
           float2 sb[4];
-          if (ok) {
-            tmem_ld_16x256b_x4(taddr_low + block_column[0], partial_a);
+          tmem_ld_16x128b_x8(taddr_low + block_column(0), partial_a);
 #pragma unroll
-            for (int fragment = 0; fragment < 8; ++fragment) {
-              const int block = fragment >> 1;
-              if ((fragment & 1) == 0) load_column_scales(slot + block_column[block], quad, sb);
-              tmem_ld_wait();
-              if (fragment + 1 < 8) {
-                const uint32_t next = ((fragment + 1) & 1 ? taddr_high : taddr_low) +
-                                      block_column[(fragment + 1) >> 1];
-                if (fragment & 1) tmem_ld_16x256b_x4(next, partial_a);
-                else tmem_ld_16x256b_x4(next, partial_b);
-              } else {
-                // All of this warp's TMEM accesses for the buffer are done: hand it back.
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tmem_empty_bar[buffer]);
-              }
-              if (fragment & 1) {
-                promote_fragment<kLayout>(partial_b, sa[2], sa[3], sb, &acc[2][block * 4],
-                                        &acc[3][block * 4]);
-              } else {
-                promote_fragment<kLayout>(partial_a, sa[0], sa[1], sb, &acc[0][block * 4],
-                                        &acc[1][block * 4]);
-              }
+          for (int fragment = 0; fragment < 8; ++fragment) {
+            const int block = fragment >> 1;
+            if ((fragment & 1) == 0) load_column_scales(slot + block_column(block), quad, sb);
+            tmem_ld_wait();
+            if (fragment + 1 < 8) {
+              const uint32_t next = ((fragment + 1) & 1 ? taddr_high : taddr_low) +
+                                    block_column((fragment + 1) >> 1);
+              if (fragment & 1) tmem_ld_16x128b_x8(next, partial_a);
+              else tmem_ld_16x128b_x8(next, partial_b);
+            } else {
+              // All of this warp's TMEM accesses for the buffer are done: hand it back.
+              tcgen05_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&tmem_empty_bar[buffer]);
+            }
+            if (fragment & 1) {
+              promote_fragment(partial_b, sa[2], sa[3], sb, &acc[2][block * 4], &acc[3][block * 4]);
+            } else {
+              promote_fragment(partial_a, sa[0], sa[1], sb, &acc[0][block * 4], &acc[1][block * 4]);
             }
           }
-          // Every lane has consumed the slot's values (they fed the arithmetic above).
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&scale_empty_bar[scale_slot]);
-          if (++scale_slot == Shape::kScaleSlots) {
-            scale_slot = 0;
-            scale_phase ^= 1u;
+          if (in_chunk == kScaleChunkGroups - 1 || g == groups - 1) {
+            // Every lane has consumed the chunk's values (they fed the arithmetic above).
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&scale_empty_bar[scale_chunk]);
+            if (++scale_chunk == Shape::kScaleChunks) {
+              scale_chunk = 0;
+              scale_phase ^= 1u;
+            }
           }
         }
 
-        // SwiGLU on the rounded gate/up values.  h[r][k] is channel (of this sub-tile's 128)
-        //   split:       half*64 + (k/8)*32 + 8*((k%8)/2) + 2*quad + k%2
-        //   interleaved: half*64 + (k/4)*16 + 4*(k%4) + quad
+        // SwiGLU on the rounded gate/up values.  h[r][8b + 2i] and h[r][8b + 2i + 1] are channels
+        // half*64 + 32b + 8i + quad and +4 of this sub-tile's 128.
         // gate and up are rounded to the output type first (pack_pair), so silu(gate) is a
         // lookup by the gate's 16-bit pattern in a table built with the formula itself.
         float h[4][16];
@@ -450,22 +453,14 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           float row_amax = 0.0f;
-          if (p.interleaved) {
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const uint32_t pair = pack_pair<RoundT>(acc[r][k]);   // (gate, up) of one channel
-              h[r][k] = __fmul_rn(__ldg(p.silu_table + (pair & 0xffffu)), unpack_pair<RoundT>(pair).y);
-            }
-          } else {
+          for (int b = 0; b < 2; ++b) {
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const uint32_t gate = pack_pair<RoundT>(acc[r][b * 4 + i]);
-                const float2 up = unpack_pair<RoundT>(pack_pair<RoundT>(acc[r][(2 + b) * 4 + i]));
-                h[r][b * 8 + 2 * i] = __fmul_rn(__ldg(p.silu_table + (gate & 0xffffu)), up.x);
-                h[r][b * 8 + 2 * i + 1] = __fmul_rn(__ldg(p.silu_table + (gate >> 16)), up.y);
-              }
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t gate = pack_pair<RoundT>(acc[r][b * 4 + i]);
+              const float2 up = unpack_pair<RoundT>(pack_pair<RoundT>(acc[r][(2 + b) * 4 + i]));
+              h[r][b * 8 + 2 * i] = __fmul_rn(__ldg(p.silu_table + (gate & 0xffffu)), up.x);
+              h[r][b * 8 + 2 * i + 1] = __fmul_rn(__ldg(p.silu_table + (gate >> 16)), up.y);
             }
           }
 #pragma unroll
@@ -526,31 +521,19 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                   code[k] = static_cast<uint32_t>(quantize_value(v[k], scale)) & 0xffu;
               }
               int8_t* q_piece = q_row + piece * 128 + half * 64;
-              if (p.interleaved) {
-                // Lane `quad` holds channels 16*blk + 4i + quad; after the exchange it holds the
-                // four consecutive channels 16*blk + 4*quad .. +3.
+              // Lane `quad` holds channels 32*b + 8i + quad and +4; after the exchange it holds the
+              // eight channels 32*b + 8*quad .. +7, the first four in the low bytes.
 #pragma unroll
-                for (int blk = 0; blk < 4; ++blk) {
-                  uint32_t w[4] = {code[blk * 4], code[blk * 4 + 1], code[blk * 4 + 2], code[blk * 4 + 3]};
-                  quad_transpose(w, quad);
-                  if (row_stored) {
-                    *reinterpret_cast<uint32_t*>(q_piece + blk * 16 + 4 * quad) =
-                        w[0] | (w[1] << 8) | (w[2] << 16) | (w[3] << 24);
-                  }
-                }
-              } else {
-                // Lane `quad` holds channel pairs 32*b + 8i + 2*quad, +1; after the exchange it
-                // holds the eight consecutive channels 32*b + 8*quad .. +7.
+              for (int b = 0; b < 2; ++b) {
+                uint32_t w[4];
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                  uint32_t w[4];
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) w[i] = code[b * 8 + 2 * i] | (code[b * 8 + 2 * i + 1] << 8);
-                  quad_transpose(w, quad);
-                  if (row_stored) {
-                    *reinterpret_cast<uint2*>(q_piece + b * 32 + 8 * quad) =
-                        make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
-                  }
+                for (int i = 0; i < 4; ++i) w[i] = code[b * 8 + 2 * i] | (code[b * 8 + 2 * i + 1] << 8);
+                quad_transpose(w, quad);
+                if (row_stored) {
+                  const uint32_t front = __byte_perm(w[0], w[1], 0x5140);
+                  const uint32_t back = __byte_perm(w[2], w[3], 0x5140);
+                  *reinterpret_cast<uint2*>(q_piece + b * 32 + 8 * quad) =
+                      make_uint2(__byte_perm(front, back, 0x5410), __byte_perm(front, back, 0x7632));
                 }
               }
             }

@@ -95,21 +95,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
                : "memory");
 }
 
-// Upper bound, in nanoseconds, for which one try_wait may keep the thread suspended before it
-// reports "not yet"; keeps waiting warps from burning issue slots on polling.
-#ifndef GG_TRY_WAIT_SUSPEND_NS
-#define GG_TRY_WAIT_SUSPEND_NS 20000
-#endif
-constexpr uint32_t kTryWaitSuspendNs = GG_TRY_WAIT_SUSPEND_NS;
+// Longest time a wait may take before the kernel gives up (nanoseconds of %globaltimer).
+constexpr uint64_t kWaitLimitNs = 2000000000ull;
 
-// Single non-blocking probe of a phase parity.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+// One probe by the whole warp: true when every lane sees the phase complete.  The hardware may
+// keep the warp suspended for a while before it answers "not yet", so a waiting warp takes few
+// issue slots.  (The form with an explicit suspension limit is not used: the compiler expands it
+// into a loop of some ten instructions around a sleep, which the other warps of the scheduler
+// pay for.)
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
+      ".reg .pred p, q;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
+      "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
       "}"
       : "=r"(done)
       : "r"(smem_u32(bar)), "r"(parity)
@@ -117,55 +118,34 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
-// Longest time a wait may take before the kernel gives up (nanoseconds of %globaltimer).
-constexpr uint64_t kWaitLimitNs = 2000000000ull;
-
-// Bounded wait on a phase parity.  Returns false (after reporting `site`) when the
-// barrier has not flipped within `limit_ns`, or when another thread of the CTA has already
-// given up (*abort_flag != 0).  The clock is read only after a probe has failed and come
-// back from its suspension, every 64 such failures, so a wait that succeeds costs nothing.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned int site,
-                                          volatile int* abort_flag,
-                                          uint64_t limit_ns = kWaitLimitNs) {
-  const uint32_t addr = smem_u32(bar);
+// Warp-collective bounded wait: every lane probes and the verdict is voted on before any lane
+// branches, so that it is the same in all lanes and the loop never diverges.  Issuing warps
+// stay converged this way, so that descriptor and address arithmetic around their
+// tcgen05.mma / TMA instructions runs in the uniform datapath; only the issue itself is left to
+// one elected lane.  The promotion warps use it too: their tcgen05.ld / tcgen05.wait are
+// .sync.aligned and must see the whole warp take one path, also after a wait has run out.
+// A wait that finds its phase complete costs 25 cycles, against 73 with a per-lane branch into
+// the waiting loop in front of the vote (measured on one warp with the phase always complete),
+// and a wait that has to poll takes no issue slots for reconvergence.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned int site,
+                                               volatile int* abort_flag,
+                                               uint64_t limit_ns = kWaitLimitNs) {
   uint64_t start = 0;
   for (uint32_t spin = 0;; ++spin) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t"
-        "}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity), "r"(kTryWaitSuspendNs)
-        : "memory");
-    if (done) return true;
-    if ((spin & 0x3fu) == 0x3fu) {
-      if (*abort_flag) return false;
+    if (mbar_test_warp(bar, parity)) return true;
+    if ((spin & 0xfu) == 0xfu) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
       const uint64_t now = global_timer_ns();
-      if (start == 0) {
-        start = now;
-      } else if (now - start > limit_ns) {
-        *abort_flag = 1;
-        report_timeout(site);
+      if (start == 0) start = now;
+      if (__any_sync(0xffffffffu, now - start > limit_ns)) {
+        if (lane_id() == 0) {
+          *abort_flag = 1;
+          report_timeout(site);
+        }
         return false;
       }
     }
   }
-}
-
-// Warp-collective wait: every lane probes, then waits if needed; the verdict is the same in
-// all lanes.  Issuing warps stay converged this way, so that descriptor and address
-// arithmetic around their tcgen05.mma / TMA instructions runs in the uniform datapath; only
-// the issue itself is left to one elected lane.  The promotion warps use it too: their
-// tcgen05.ld / tcgen05.wait are .sync.aligned and must see the whole warp take one path,
-// also after a wait has run out.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned int site,
-                                               volatile int* abort_flag,
-                                               uint64_t limit_ns = kWaitLimitNs) {
-  const bool got = mbar_test(bar, parity) || mbar_wait(bar, parity, site, abort_flag, limit_ns);
-  return __all_sync(0xffffffffu, got);
 }
 
 // 16-byte shared-memory load by 32-bit shared address (a pointer that went through integer
@@ -181,8 +161,8 @@ __device__ __forceinline__ float4 lds_f32x4(uint32_t smem_address) {
 // ---------------------------------------------------------------- cp.async (scale staging)
 
 // Asynchronous 4-byte copy global -> shared; `valid == false` writes zero without reading.
-__device__ __forceinline__ void cp_async_f32(float* smem_dst, const float* src, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem_dst)), "l"(src),
+__device__ __forceinline__ void cp_async_f32(uint32_t smem_dst, const float* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_dst), "l"(src),
                "r"(valid ? 4 : 0)
                : "memory");
 }
@@ -360,28 +340,12 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)
 }
 
 
-// 16 TMEM lanes x 32 columns in the matrix-fragment layout: with q = lane % 4 and
-// r = lane / 4, register 4i+0/4i+1 hold row r, columns 8i+2q and 8i+2q+1; registers 4i+2/4i+3
-// hold row r+8, same columns (i = 0..3).  taddr.lane selects the first of the 16 lanes.
-__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
-
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 // 16 TMEM lanes x 32 columns as 4-column groups: with q = lane % 4 and r = lane / 4, register
 // 2k holds row r, column 4k + q and register 2k + 1 holds row r + 8, same column (k = 0..7).
-// Drains TMEM at twice the rate of the 16x256b shape (507 against 256 B/clk/SM measured).
 __device__ __forceinline__ void tmem_ld_16x128b_x8(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.16x128b.x8.b32 "
