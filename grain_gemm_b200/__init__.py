@@ -11,13 +11,13 @@ __all__ = ["__version__", "get_kernel_config", "int8_gemm", "moe_ffn", "quantize
 
 def __getattr__(name):
     if name in ("int8_gemm", "get_kernel_config"):
-        from . import gemm
-        return getattr(gemm, name)
-    if name == "moe_ffn":
-        from .moe import moe_ffn
-        return moe_ffn
-    if name in ("quantize_rows", "prepare_weight", "interleave_gate_up", "route_topk",
-                "route_topk_routes"):
-        from . import quantize
-        return getattr(quantize, name)
-    raise AttributeError(f"module 'grain_gemm_b200' has no attribute '{name}'")
+        from . import gemm as module
+    elif name == "moe_ffn":
+        from . import moe as module
+    elif name in ("quantize_rows", "prepare_weight", "interleave_gate_up", "route_topk",
+                  "route_topk_routes"):
+        from . import quantize as module
+    else:
+        raise AttributeError(f"module 'grain_gemm_b200' has no attribute '{name}'")
+    value = globals()[name] = getattr(module, name)   # found directly from the next use on
+    return value

@@ -10,6 +10,8 @@ is no fallback: a missing or stale library is an error.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 from functools import lru_cache
 
 import torch
@@ -88,6 +90,28 @@ def library():
     if lib.gg_abi_version() != _build.ABI_VERSION:
         raise RuntimeError("libgrain_b200.so reports a different ABI version than this package")
     return lib
+
+
+@lru_cache(maxsize=1)
+def host():
+    """The native host path (``csrc/host.cpp``) bound to the library's entry points.
+
+    Its functions run a public call whose arguments are what the documentation asks for and
+    return ``None`` for every other call, which then takes the Python path."""
+    from .gemm import _variant_table
+    lib = library()
+    loader = importlib.machinery.ExtensionFileLoader("grain_gemm_b200._host",
+                                                     str(_build.HOST_MODULE))
+    module = importlib.util.module_from_spec(
+        importlib.util.spec_from_file_location(loader.name, loader.path, loader=loader))
+    loader.exec_module(module)
+    addresses = {name: ctypes.cast(getattr(lib, name), _VOID).value for name in _SIGNATURES}
+    table = {}
+    for key, rows in _variant_table().items():
+        table[tuple(int(part) for part in key.split(":"))] = [
+            (bound, VARIANTS[name]) for bound, name in rows]
+    module.bind(addresses, table)
+    return module
 
 
 def is_available():

@@ -1,0 +1,627 @@
+// The host side of the hot calls: argument checks, output allocation and launches in one native
+// call per public entry point.
+//
+// A call of a decode step launches kernels of 3-15 us; the Python path around the C ABI (checks
+// attribute by attribute, a ctypes conversion per argument, stream and device look-ups) took
+// 40 us for a GEMM and 200 us for a MoE layer and was what such a step waited for.  Each function
+// here accepts exactly the calls that the Python path accepts AND whose tensors are plain dense
+// CUDA tensors, and returns None for everything else (wrong arguments, tensor subclasses, modes,
+// functorch levels, tracing, stream capture, operands that need a copy first): the caller
+// then takes the Python path, which raises the documented errors or does the rare work.
+// The kernels are reached through the C ABI of libgrain_b200.so; bind() receives its entry points,
+// so this module links against torch only.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <climits>
+#include <map>
+#include <string>
+#include <tuple>
+#include <utility>
+#include <vector>
+
+#include "../../include/grain_gemm_b200.h"
+
+namespace {
+
+// ---------------------------------------------------------------- the library's entry points
+
+struct Library {
+  decltype(&gg_error_string) error_string;
+  decltype(&gg_int8_gemm_ws) int8_gemm_ws;
+  decltype(&gg_int8_gemm_workspace_bytes) int8_gemm_workspace_bytes;
+  decltype(&gg_quantize_rows) quantize_rows;
+  decltype(&gg_moe_route_topk) moe_route_topk;
+  decltype(&gg_moe_route_workspace_bytes) moe_route_workspace_bytes;
+  decltype(&gg_moe_route) moe_route;
+  decltype(&gg_moe_tile_capacity) moe_tile_capacity;
+  decltype(&gg_moe_tiles) moe_tiles;
+  decltype(&gg_moe_gate_up_scratch_bytes) moe_gate_up_scratch_bytes;
+  decltype(&gg_moe_gate_up) moe_gate_up;
+  decltype(&gg_moe_down) moe_down;
+  decltype(&gg_moe_combine) moe_combine;
+  decltype(&gg_report_to_host) report_to_host;
+};
+Library lib;
+
+// Measured shape -> variant table: (group, n, k) -> ascending (bound on m, variant).
+std::map<std::tuple<int64_t, int64_t, int64_t>, std::vector<std::pair<int64_t, int>>> variant_table;
+
+struct Status {   // a status other than zero, to be raised once the GIL is held again
+  int code = 0;
+  const char* what = "";
+  bool set(int status, const char* name) {
+    if (status != 0 && code == 0) { code = status; what = name; }
+    return status != 0;
+  }
+};
+
+PyObject* raise_status(const Status& s) {
+  PyErr_Format(PyExc_RuntimeError, "%s failed: %s (status %d)", s.what, lib.error_string(s.code), s.code);
+  return nullptr;
+}
+
+class ReleasedGil {
+ public:
+  ReleasedGil() : state_(PyEval_SaveThread()) {}
+  ~ReleasedGil() { PyEval_RestoreThread(state_); }
+  ReleasedGil(const ReleasedGil&) = delete;
+ private:
+  PyThreadState* state_;
+};
+
+// ---------------------------------------------------------------- what this path may take
+
+// Nothing that wants to see the Python path's torch calls (function or dispatch modes, functorch,
+// tracing) is active.
+bool plain_context() {
+  return !at::impl::torch_function_mode_enabled() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Tracer);
+}
+
+const c10::DispatchKeySet kForeignKeys({
+    c10::DispatchKey::Python, c10::DispatchKey::PythonTLSSnapshot, c10::DispatchKey::FuncTorchBatched,
+    c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Batched, c10::DispatchKey::Functionalize,
+    c10::DispatchKey::Negative, c10::DispatchKey::Conjugate, c10::DispatchKey::ZeroTensor});
+
+// A torch.Tensor (no subclass) that is an ordinary dense CUDA tensor.
+bool plain_cuda(PyObject* object) {
+  if (!THPVariable_CheckExact(object)) return false;
+  const at::Tensor& t = THPVariable_Unpack(object);
+  return t.defined() && t.layout() == at::kStrided && t.is_cuda() && !t.key_set().has_any(kForeignKeys);
+}
+
+const at::Tensor& tensor(PyObject* object) { return THPVariable_Unpack(object); }
+
+bool b200(c10::DeviceIndex device) {
+  const cudaDeviceProp* properties = at::cuda::getDeviceProperties(device);
+  return properties->major == 10 && properties->minor == 0;
+}
+
+// out-dtype code of the C ABI; -1 for any other object.
+int out_code(PyObject* dtype) {
+  if (!THPDtype_Check(dtype)) return -1;
+  switch (reinterpret_cast<THPDtype*>(dtype)->scalar_type) {
+    case at::kFloat: return GG_OUT_FP32;
+    case at::kBFloat16: return GG_OUT_BF16;
+    case at::kHalf: return GG_OUT_FP16;
+    default: return -1;
+  }
+}
+
+int out_code(at::ScalarType type) {
+  return type == at::kFloat ? GG_OUT_FP32 : type == at::kBFloat16 ? GG_OUT_BF16
+         : type == at::kHalf ? GG_OUT_FP16 : -1;
+}
+
+at::ScalarType out_type(int code) {
+  return code == GG_OUT_FP32 ? at::kFloat : code == GG_OUT_BF16 ? at::kBFloat16 : at::kHalf;
+}
+
+bool group_ok(int64_t g) { return g == 32 || g == 64 || g == 128 || g == 256; }
+
+// The value of an exact Python int (not a bool) that fits; -1 otherwise.
+int64_t small_int(PyObject* object) {
+  if (!PyLong_CheckExact(object)) return -1;
+  int overflow = 0;
+  const long long value = PyLong_AsLongLongAndOverflow(object, &overflow);
+  return overflow == 0 && value >= 0 && value <= INT_MAX ? value : -1;
+}
+
+at::Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& device) {
+  return at::empty(sizes, at::TensorOptions().dtype(type).device(device));
+}
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// ---------------------------------------------------------------- int8_gemm
+
+// Two-dimensional, positive strides, relative offsets within 31 bits.
+bool gemm_operand(const at::Tensor& t, at::ScalarType type, int64_t rows, int64_t columns) {
+  if (t.dim() != 2 || t.scalar_type() != type || t.size(0) != rows || t.size(1) != columns) return false;
+  const int64_t s0 = t.stride(0), s1 = t.stride(1);
+  return s0 > 0 && s1 > 0 && (rows - 1) * s0 + (columns - 1) * s1 <= INT_MAX;
+}
+
+// int8_gemm(a, b, scale_a, scale_b, group_size, output_dtype)
+PyObject* int8_gemm(PyObject*, PyObject* const* args, Py_ssize_t count) {
+  HANDLE_TH_ERRORS
+  if (count != 6 || !plain_context()) Py_RETURN_NONE;
+  for (int i = 0; i < 4; ++i) {
+    if (!plain_cuda(args[i])) Py_RETURN_NONE;
+  }
+  const at::Tensor &a = tensor(args[0]), &b = tensor(args[1]), &sa = tensor(args[2]), &sb = tensor(args[3]);
+  const int64_t group = small_int(args[4]);
+  const int out_dtype = out_code(args[5]);
+  if (!group_ok(group) || out_dtype < 0 || a.dim() != 2 || b.dim() != 2) Py_RETURN_NONE;
+  const int64_t m = a.size(0), k = a.size(1), n = b.size(1);
+  if (m <= 0 || n <= 0 || k <= 0 || m > INT_MAX || n > INT_MAX || k > INT_MAX || m * n > (1ll << 31)) {
+    Py_RETURN_NONE;
+  }
+  const int64_t groups = (k + group - 1) / group;
+  if (!gemm_operand(a, at::kChar, m, k) || !gemm_operand(b, at::kChar, k, n) ||
+      !gemm_operand(sa, at::kFloat, m, groups) || !gemm_operand(sb, at::kFloat, groups, n) ||
+      b.device() != a.device() || sa.device() != a.device() || sb.device() != a.device() ||
+      !b200(a.device().index())) {
+    Py_RETURN_NONE;
+  }
+  // Large problems whose operands want a copy into K-contiguous storage first.
+  if (2.0 * m * n * k >= 4294967296.0 && k % 16 == 0 &&
+      (a.stride(1) != 1 || a.stride(0) % 16 != 0 || !aligned16(a.data_ptr()) || b.stride(0) != 1 ||
+       b.stride(1) % 16 != 0 || !aligned16(b.data_ptr()))) {
+    Py_RETURN_NONE;
+  }
+  // A dimension of size one is never stepped through: any stride the tensor cores accept will do.
+  int64_t a_sm = a.stride(0), a_sk = a.stride(1), b_sk = b.stride(0), b_sn = b.stride(1);
+  if (k == 1) a_sk = b_sk = 1;
+  if (m == 1) a_sm = (k * a_sk + 15) / 16 * 16;
+  if (n == 1) b_sn = (k * b_sk + 15) / 16 * 16;
+  int variant = GG_VARIANT_AUTO;
+  if (a_sk == 1 && b_sk == 1 && a_sm % 16 == 0 && b_sn % 16 == 0 && a_sm >= k && b_sn >= k &&
+      aligned16(a.data_ptr()) && aligned16(b.data_ptr())) {
+    const auto rows = variant_table.find({group, n, k});
+    if (rows != variant_table.end()) {
+      variant = rows->second.back().second;
+      for (const auto& row : rows->second) {
+        if (m <= row.first) { variant = row.second; break; }
+      }
+    }
+  }
+  Status status;
+  at::Tensor c;
+  {
+    ReleasedGil released;
+    const c10::cuda::CUDAGuard guard(a.device());
+    c = empty({m, n}, out_type(out_dtype), a.device());
+    // Skinny problems split K over the SMs through a workspace of INT32 group dots.
+    at::Tensor workspace;
+    size_t bytes = 0;
+    if (variant == GG_VARIANT_AUTO || variant == GG_VARIANT_TC_SPLITK) {
+      bytes = lib.int8_gemm_workspace_bytes(m, n, k, group);
+      if (bytes) workspace = empty({static_cast<int64_t>(bytes)}, at::kByte, a.device());
+    }
+    status.set(lib.int8_gemm_ws(a.data_ptr(), b.data_ptr(), sa.data_ptr(), sb.data_ptr(), c.data_ptr(), m,
+                                n, k, a_sm, a_sk, b_sk, b_sn, sa.stride(0), sa.stride(1), sb.stride(0),
+                                sb.stride(1), n, group, out_dtype, variant,
+                                bytes ? workspace.data_ptr() : nullptr, bytes,
+                                c10::cuda::getCurrentCUDAStream(a.device().index())),
+               "gg_int8_gemm");
+  }
+  if (status.code) return raise_status(status);
+  return THPVariable_Wrap(c);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- quantize_rows, routing
+
+PyObject* pair(const at::Tensor& first, const at::Tensor& second) {
+  PyObject* result = PyTuple_New(2);
+  if (!result) return nullptr;
+  PyTuple_SET_ITEM(result, 0, THPVariable_Wrap(first));
+  PyTuple_SET_ITEM(result, 1, THPVariable_Wrap(second));
+  return result;
+}
+
+// quantize_rows(x, group_size)
+PyObject* quantize_rows(PyObject*, PyObject* const* args, Py_ssize_t count) {
+  HANDLE_TH_ERRORS
+  if (count != 2 || !plain_context() || !plain_cuda(args[0])) Py_RETURN_NONE;
+  const at::Tensor& x = tensor(args[0]);
+  const int64_t group = small_int(args[1]);
+  const int in_dtype = out_code(x.scalar_type());
+  if (!group_ok(group) || in_dtype < 0 || x.dim() < 1 || !x.is_contiguous() || x.numel() == 0) Py_RETURN_NONE;
+  const int64_t width = x.size(-1);
+  if (width % 256 || width > INT_MAX || !b200(x.device().index())) Py_RETURN_NONE;
+  Status status;
+  at::Tensor q, scales;
+  {
+    ReleasedGil released;
+    const c10::cuda::CUDAGuard guard(x.device());
+    q = empty(x.sizes(), at::kChar, x.device());
+    auto sizes = x.sizes().vec();
+    sizes.back() = width / group;
+    scales = empty(sizes, at::kFloat, x.device());
+    status.set(lib.quantize_rows(x.data_ptr(), in_dtype, x.numel() / width, width, group, q.data_ptr(),
+                                 scales.data_ptr(), c10::cuda::getCurrentCUDAStream(x.device().index())),
+               "gg_quantize_rows");
+  }
+  if (status.code) return raise_status(status);
+  return pair(q, scales);
+  END_HANDLE_TH_ERRORS
+}
+
+// Buffers of one routing: the fields of moe.Routes.
+struct Routing {
+  at::Tensor effective_ids, order, inverse, counts, offsets, statistics, tiles, scratch;
+};
+
+constexpr int kTileRows = 128;
+
+// route_topk_routes(logits, top_k, token_mask or None, 64-bit ids?): the fused decode-sized call
+// with its row-tile list.  Returns (weights, ids, order, counts, offsets, inverse, effective_ids,
+// statistics, tile_expert, tile_row).
+PyObject* route_topk_routes(PyObject*, PyObject* const* args, Py_ssize_t count) {
+  HANDLE_TH_ERRORS
+  if (count != 4 || !plain_context() || !plain_cuda(args[0])) Py_RETURN_NONE;
+  const at::Tensor& logits = tensor(args[0]);
+  const int64_t top_k = small_int(args[1]);
+  const bool wide = args[3] == Py_True;
+  if (logits.dim() != 2 || !logits.is_contiguous()) Py_RETURN_NONE;
+  const int64_t tokens = logits.size(0), experts = logits.size(1);
+  const int in_dtype = out_code(logits.scalar_type());
+  if (in_dtype < 0 || top_k <= 0 || top_k > experts || experts > 1024 || tokens <= 0 || tokens > 1024 ||
+      tokens * top_k > 1024) {
+    Py_RETURN_NONE;
+  }
+  const at::Tensor* mask = nullptr;
+  if (args[2] != Py_None) {
+    if (!plain_cuda(args[2])) Py_RETURN_NONE;
+    mask = &tensor(args[2]);
+    if (!mask->is_contiguous() || mask->element_size() != 1 || mask->numel() != tokens ||
+        mask->device() != logits.device()) {
+      Py_RETURN_NONE;
+    }
+  }
+  Status status;
+  const at::Device device = logits.device();
+  at::Tensor weights, ids, tile_expert, tile_row;
+  Routing r;
+  {
+    ReleasedGil released;
+    const c10::cuda::CUDAGuard guard(device);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index());
+    const int64_t slots = tokens * top_k;
+    const at::ScalarType id_type = wide ? at::kLong : at::kInt;
+    weights = empty({tokens, top_k}, at::kFloat, device);
+    ids = empty({tokens, top_k}, id_type, device);
+    r.effective_ids = empty({slots}, id_type, device);
+    r.order = empty({slots}, at::kLong, device);
+    r.inverse = empty({slots}, at::kInt, device);
+    r.counts = empty({experts}, at::kInt, device);
+    r.offsets = empty({experts + 1}, at::kInt, device);
+    r.statistics = empty({3}, at::kInt, device);
+    const int capacity = lib.moe_tile_capacity(slots, experts, kTileRows);
+    tile_expert = empty({capacity}, at::kInt, device);
+    tile_row = empty({capacity}, at::kInt, device);
+    if (!status.set(lib.moe_route_topk(logits.data_ptr(), in_dtype, mask ? mask->data_ptr() : nullptr, tokens,
+                                       experts, top_k, weights.data_ptr(), ids.data_ptr(), wide,
+                                       r.effective_ids.data_ptr(), r.order.data_ptr(), r.inverse.data_ptr(),
+                                       r.counts.data_ptr(), r.offsets.data_ptr(), r.statistics.data_ptr(), stream),
+                    "gg_moe_route_topk")) {
+      status.set(lib.moe_tiles(r.offsets.data_ptr(), experts, kTileRows, capacity, tile_expert.data_ptr(),
+                               tile_row.data_ptr(), stream),
+                 "gg_moe_tiles");
+    }
+  }
+  if (status.code) return raise_status(status);
+  const at::Tensor* parts[] = {&weights, &ids, &r.order, &r.counts, &r.offsets, &r.inverse, &r.effective_ids,
+                               &r.statistics, &tile_expert, &tile_row};
+  PyObject* result = PyTuple_New(10);
+  if (!result) return nullptr;
+  for (int i = 0; i < 10; ++i) PyTuple_SET_ITEM(result, i, THPVariable_Wrap(*parts[i]));
+  return result;
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- moe_ffn
+
+// Shape, dtype and strides as moe_ffn documents them: contiguous, or the transposed view of
+// contiguous Linear storage (a dimension of size one may have any positive stride).
+bool moe_operand(const at::Tensor& t, at::IntArrayRef shape, bool transposed) {
+  if (t.sizes() != shape || t.requires_grad()) return false;
+  int64_t wanted = 1;
+  for (int i = static_cast<int>(shape.size()) - 1; i >= 0; --i) {
+    const int d = transposed && i >= 1 ? 3 - i : i;     // the last two dimensions change places
+    if (t.stride(d) <= 0 || (shape[d] > 1 && t.stride(d) != wanted)) return false;
+    wanted *= shape[d];
+  }
+  return true;
+}
+
+// A buffer of the caller's workspace dictionary (or a new one without a workspace); a buffer is
+// replaced when its shape, dtype or device changes.  Needs the GIL.
+at::Tensor buffer(PyObject* workspace, const char* name, at::IntArrayRef sizes, at::ScalarType type,
+                  const at::Device& device) {
+  if (!workspace) return empty(sizes, type, device);
+  PyObject* held = PyDict_GetItemString(workspace, name);
+  if (held && THPVariable_Check(held)) {
+    const at::Tensor& t = THPVariable_Unpack(held);
+    if (t.sizes() == sizes && t.scalar_type() == type && t.device() == device) return t;
+  }
+  at::Tensor fresh = empty(sizes, type, device);
+  PyObject* wrapped = THPVariable_Wrap(fresh);
+  if (!wrapped || PyDict_SetItemString(workspace, name, wrapped) != 0) {
+    Py_XDECREF(wrapped);
+    throw python_error();
+  }
+  Py_DECREF(wrapped);
+  return fresh;
+}
+
+// moe_ffn(hidden_states, w_gate_up, w_down, topk_weights, topk_ids, scale_x, scale_gate_up,
+//         scale_down, token_mask or None, output_dtype, interleaved, workspace dict or None,
+//         routes or None, pinned words of a device index)
+// routes = (order, inverse, offsets, statistics, tile_expert, tile_row, tokens, top_k, experts).
+PyObject* moe_ffn(PyObject*, PyObject* const* args, Py_ssize_t count) {
+  HANDLE_TH_ERRORS
+  if (count != 14 || !plain_context()) Py_RETURN_NONE;
+  for (int i = 0; i < 8; ++i) {
+    if (!plain_cuda(args[i])) Py_RETURN_NONE;
+  }
+  const at::Tensor &x = tensor(args[0]), &w1 = tensor(args[1]), &w2 = tensor(args[2]);
+  const at::Tensor &weights = tensor(args[3]), &ids = tensor(args[4]), &scale_x = tensor(args[5]);
+  const at::Tensor &scale_w1 = tensor(args[6]), &scale_w2 = tensor(args[7]);
+  const int out_dtype = out_code(args[9]);
+  const int interleaved = args[10] == Py_True;
+  if (x.dim() != 2 || w1.dim() != 3 || w2.dim() != 3 || ids.dim() != 2 ||
+      (out_dtype != GG_OUT_BF16 && out_dtype != GG_OUT_FP16)) {
+    Py_RETURN_NONE;
+  }
+  const int64_t tokens = x.size(0), hidden = x.size(1), experts = w1.size(0), inter = w1.size(2) / 2;
+  const int64_t top_k = ids.size(1);
+  if (tokens <= 0 || experts <= 0 || hidden <= 0 || inter <= 0 || hidden % 256 || inter % 256 || top_k < 1 ||
+      top_k > experts || experts > INT_MAX || tokens > INT_MAX) {
+    Py_RETURN_NONE;
+  }
+  const int64_t limit = INT_MAX;
+  const int64_t slots = tokens * top_k;
+  if (slots > limit || slots * std::max(hidden, 2 * inter) > limit || tokens * hidden > limit) Py_RETURN_NONE;
+  if (x.scalar_type() != at::kChar || w1.scalar_type() != at::kChar || w2.scalar_type() != at::kChar ||
+      weights.scalar_type() != at::kFloat || scale_x.scalar_type() != at::kFloat ||
+      scale_w1.scalar_type() != at::kFloat || scale_w2.scalar_type() != at::kFloat ||
+      (ids.scalar_type() != at::kLong && ids.scalar_type() != at::kInt)) {
+    Py_RETURN_NONE;
+  }
+  if (!moe_operand(x, {tokens, hidden}, false) || !moe_operand(w1, {experts, hidden, 2 * inter}, true) ||
+      !moe_operand(w2, {experts, inter, hidden}, true) || !moe_operand(weights, {tokens, top_k}, false) ||
+      !moe_operand(ids, {tokens, top_k}, false) || !moe_operand(scale_x, {tokens, hidden / 256}, false) ||
+      !moe_operand(scale_w1, {experts, hidden / 256, 2 * inter}, false) ||
+      !moe_operand(scale_w2, {experts, inter / 256, hidden}, false) ||
+      // Weights and their scales: rows within 31 bits (elements may exceed them).
+      experts * std::max(hidden, 2 * inter) > limit ||
+      experts * std::max(hidden, inter) > limit) {
+    Py_RETURN_NONE;
+  }
+  const at::Device device = x.device();
+  for (int i = 1; i < 8; ++i) {
+    if (tensor(args[i]).device() != device) Py_RETURN_NONE;
+  }
+  const at::Tensor* mask = nullptr;
+  if (args[8] != Py_None) {
+    if (!plain_cuda(args[8])) Py_RETURN_NONE;
+    mask = &tensor(args[8]);
+    if (mask->scalar_type() != at::kBool || !moe_operand(*mask, {tokens}, false) || mask->device() != device) {
+      Py_RETURN_NONE;
+    }
+  }
+  if (!aligned16(x.data_ptr()) || !aligned16(w1.data_ptr()) || !aligned16(w2.data_ptr()) ||
+      !b200(device.index())) {
+    Py_RETURN_NONE;
+  }
+  PyObject* workspace = args[11] == Py_None ? nullptr : args[11];
+  PyObject* given = args[12] == Py_None ? nullptr : args[12];
+  if ((workspace && !PyDict_CheckExact(workspace)) || !PyCallable_Check(args[13])) Py_RETURN_NONE;
+  if (given) {
+    if (!PyTuple_CheckExact(given) || PyTuple_GET_SIZE(given) != 9) Py_RETURN_NONE;
+    for (int i = 0; i < 6; ++i) {
+      PyObject* part = PyTuple_GET_ITEM(given, i);
+      if (!plain_cuda(part) || tensor(part).device() != device || !tensor(part).is_contiguous()) Py_RETURN_NONE;
+    }
+    if (small_int(PyTuple_GET_ITEM(given, 6)) != tokens || small_int(PyTuple_GET_ITEM(given, 7)) != top_k ||
+        small_int(PyTuple_GET_ITEM(given, 8)) != experts) {
+      Py_RETURN_NONE;
+    }
+  }
+  const c10::cuda::CUDAGuard guard(device);
+  const c10::cuda::CUDAStream torch_stream = c10::cuda::getCurrentCUDAStream(device.index());
+  const cudaStream_t stream = torch_stream;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    Py_RETURN_NONE;
+  }
+
+  // Buffers (the workspace dictionary needs the GIL).
+  Routing r;
+  at::Tensor tile_expert, tile_row;
+  const int capacity = std::max(1, lib.moe_tile_capacity(slots, experts, kTileRows));
+  size_t route_bytes = 0;
+  if (given) {
+    r.order = tensor(PyTuple_GET_ITEM(given, 0));
+    r.inverse = tensor(PyTuple_GET_ITEM(given, 1));
+    r.offsets = tensor(PyTuple_GET_ITEM(given, 2));
+    r.statistics = tensor(PyTuple_GET_ITEM(given, 3));
+    tile_expert = tensor(PyTuple_GET_ITEM(given, 4));
+    tile_row = tensor(PyTuple_GET_ITEM(given, 5));
+  } else {
+    r.effective_ids = buffer(workspace, "effective_ids", {slots}, ids.scalar_type(), device);
+    r.order = buffer(workspace, "order", {slots}, at::kLong, device);
+    r.inverse = buffer(workspace, "inverse", {slots}, at::kInt, device);
+    r.counts = buffer(workspace, "counts", {experts}, at::kInt, device);
+    r.offsets = buffer(workspace, "offsets", {experts + 1}, at::kInt, device);
+    r.statistics = buffer(workspace, "statistics", {3}, at::kInt, device);
+    route_bytes = lib.moe_route_workspace_bytes(tokens, top_k, experts);
+    if (route_bytes) {
+      r.scratch = buffer(workspace, "route_scratch", {static_cast<int64_t>(route_bytes)}, at::kByte, device);
+    }
+    r.tiles = buffer(workspace, "tiles", {2, capacity}, at::kInt, device);
+  }
+  const at::Tensor qh = buffer(workspace, "qh", {slots, inter}, at::kChar, device);
+  const at::Tensor sh = buffer(workspace, "sh", {slots, inter / 256}, at::kFloat, device);
+  const int64_t scratch_bytes = std::max<int64_t>(16, lib.moe_gate_up_scratch_bytes(slots, hidden, inter, kTileRows, 0));
+  const at::Tensor scratch = buffer(workspace, "gate_up_scratch", {scratch_bytes}, at::kByte, device);
+  const at::Tensor expert_out = buffer(workspace, "expert_output", {slots, hidden}, out_type(out_dtype), device);
+  // This thread's page-locked words; asked for only now, since an allocation of page-locked memory
+  // does not go with a capture.
+  PyObject* held_words = PyObject_CallFunction(args[13], "i", static_cast<int>(device.index()));
+  if (!held_words) return nullptr;
+  if (!THPVariable_Check(held_words)) {
+    Py_DECREF(held_words);
+    Py_RETURN_NONE;
+  }
+  const at::Tensor words = tensor(held_words);
+  Py_DECREF(held_words);
+
+  Status status;
+  at::Tensor out;
+  bool invalid_ids = false;
+  {
+    ReleasedGil released;
+    out = empty({tokens, hidden}, out_type(out_dtype), device);
+    const int* experts_of = given ? tile_expert.data_ptr<int>() : r.tiles.data_ptr<int>();
+    const int* rows_of = given ? tile_row.data_ptr<int>() : r.tiles.data_ptr<int>() + capacity;
+    const int tiles = given ? static_cast<int>(tile_expert.numel()) : capacity;
+    if (!given) {
+      status.set(lib.moe_route(ids.data_ptr(), ids.scalar_type() == at::kLong, mask ? mask->data_ptr() : nullptr,
+                               tokens, top_k, experts, r.effective_ids.data_ptr(), r.order.data_ptr(),
+                               r.inverse.data_ptr(), r.counts.data_ptr(), r.offsets.data_ptr(),
+                               r.statistics.data_ptr(), route_bytes ? r.scratch.data_ptr() : nullptr,
+                               route_bytes, stream),
+                 "gg_moe_route");
+      if (!status.code) {
+        status.set(lib.moe_tiles(r.offsets.data_ptr(), experts, kTileRows, capacity, const_cast<int*>(experts_of),
+                                 const_cast<int*>(rows_of), stream),
+                   "gg_moe_tiles");
+      }
+    }
+    // The check for unmasked ids outside [0, E): three integers are stored into page-locked host
+    // memory by a kernel and looked at after the remaining stages are in the stream.
+    at::cuda::CUDAEvent event;
+    if (!status.code) {
+      if (lib.report_to_host(r.statistics.data_ptr(), 3, words.data_ptr(), stream) != 0) {
+        words.copy_(r.statistics, /*non_blocking=*/true);
+      }
+      event.record(torch_stream);
+      status.set(lib.moe_gate_up(x.data_ptr(), scale_x.data_ptr(), w1.data_ptr(), scale_w1.data_ptr(),
+                                 r.order.data_ptr(), r.offsets.data_ptr(), experts_of, rows_of, tiles, kTileRows,
+                                 qh.data_ptr(), sh.data_ptr(), scratch.data_ptr(), tokens, top_k, experts, hidden,
+                                 inter, interleaved, out_dtype, 0, stream),
+                 "gg_moe_gate_up");
+    }
+    if (!status.code) {
+      status.set(lib.moe_down(qh.data_ptr(), sh.data_ptr(), w2.data_ptr(), scale_w2.data_ptr(), r.offsets.data_ptr(),
+                              experts_of, rows_of, tiles, kTileRows, expert_out.data_ptr(), nullptr, slots, experts,
+                              hidden, inter, out_dtype, stream),
+                 "gg_moe_down");
+    }
+    if (!status.code) {
+      status.set(lib.moe_combine(expert_out.data_ptr(), weights.data_ptr(), r.inverse.data_ptr(), out.data_ptr(),
+                                 tokens, top_k, hidden, out_dtype, stream),
+                 "gg_moe_combine");
+    }
+    if (!status.code) {
+      event.synchronize();
+      invalid_ids = words.data_ptr<int>()[0] != 0;
+    }
+  }
+  if (status.code) return raise_status(status);
+  if (invalid_ids) {
+    PyErr_SetString(PyExc_ValueError, "unmasked topk_ids must be in [0, E)");
+    return nullptr;
+  }
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// ---------------------------------------------------------------- module
+
+// bind({"gg_...": address}, {(group, n, k): [(bound, variant code)]})
+PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t count) {
+  HANDLE_TH_ERRORS
+  if (count != 2 || !PyDict_Check(args[0]) || !PyDict_Check(args[1])) {
+    PyErr_SetString(PyExc_TypeError, "bind(entry points, variant table)");
+    return nullptr;
+  }
+  Library fresh = {};
+  const auto entry = [&](const char* name, auto& slot) {
+    PyObject* address = PyDict_GetItemString(args[0], name);
+    if (!address) {
+      PyErr_SetString(PyExc_KeyError, name);
+      throw python_error();
+    }
+    slot = reinterpret_cast<std::remove_reference_t<decltype(slot)>>(PyLong_AsVoidPtr(address));
+    if (!slot) throw python_error();
+  };
+  entry("gg_error_string", fresh.error_string);
+  entry("gg_int8_gemm_ws", fresh.int8_gemm_ws);
+  entry("gg_int8_gemm_workspace_bytes", fresh.int8_gemm_workspace_bytes);
+  entry("gg_quantize_rows", fresh.quantize_rows);
+  entry("gg_moe_route_topk", fresh.moe_route_topk);
+  entry("gg_moe_route_workspace_bytes", fresh.moe_route_workspace_bytes);
+  entry("gg_moe_route", fresh.moe_route);
+  entry("gg_moe_tile_capacity", fresh.moe_tile_capacity);
+  entry("gg_moe_tiles", fresh.moe_tiles);
+  entry("gg_moe_gate_up_scratch_bytes", fresh.moe_gate_up_scratch_bytes);
+  entry("gg_moe_gate_up", fresh.moe_gate_up);
+  entry("gg_moe_down", fresh.moe_down);
+  entry("gg_moe_combine", fresh.moe_combine);
+  entry("gg_report_to_host", fresh.report_to_host);
+  decltype(variant_table) table;
+  PyObject *key, *rows;
+  Py_ssize_t position = 0;
+  while (PyDict_Next(args[1], &position, &key, &rows)) {
+    long long g, n, k;
+    if (!PyArg_ParseTuple(key, "LLL", &g, &n, &k)) return nullptr;
+    auto& entries = table[{g, n, k}];
+    for (Py_ssize_t i = 0; i < PyList_Size(rows); ++i) {
+      long long bound;
+      int variant;
+      if (!PyArg_ParseTuple(PyList_GET_ITEM(rows, i), "Li", &bound, &variant)) return nullptr;
+      entries.emplace_back(bound, variant);
+    }
+    if (entries.empty()) table.erase({g, n, k});
+  }
+  lib = fresh;
+  variant_table = std::move(table);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(bind)), METH_FASTCALL, nullptr},
+    {"int8_gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(int8_gemm)), METH_FASTCALL, nullptr},
+    {"quantize_rows", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(quantize_rows)), METH_FASTCALL, nullptr},
+    {"route_topk_routes", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(route_topk_routes)), METH_FASTCALL,
+     nullptr},
+    {"moe_ffn", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(moe_ffn)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "grain_gemm_b200._host", nullptr, -1, methods,
+                      nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }

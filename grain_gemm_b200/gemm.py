@@ -241,6 +241,11 @@ def int8_gemm(a, b, scale_a, scale_b, *, group_size=256,
     kernel variant (see ``_loader.VARIANTS``) and is meant for tests and benchmarks.
     """
     _check_backend(backend)
+    if variant == "auto" and isinstance(a, torch.Tensor) and a.is_cuda:
+        # The whole call natively; None for anything but plain CUDA operands it can take as they are.
+        result = _loader.host().int8_gemm(a, b, scale_a, scale_b, group_size, output_dtype)
+        if result is not None:
+            return result
     m, n, k = _validate(a, b, scale_a, scale_b, group_size, output_dtype)
     with torch.cuda.device(a.device):
         if m == 0 or n == 0 or k == 0:

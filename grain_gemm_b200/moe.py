@@ -308,6 +308,22 @@ def combine(expert_output, topk_weights, routes, *, output_dtype=torch.bfloat16)
 _HOST = threading.local()
 
 
+def _pinned_words(device_index, count, slot):
+    """``count`` page-locked INT32 words of this thread, one buffer per device and ``slot``."""
+    buffers = getattr(_HOST, "buffers", None)
+    if buffers is None:
+        buffers = _HOST.buffers = {}
+    key = (device_index, slot, count)
+    words = buffers.get(key)
+    if words is None:
+        words = buffers[key] = torch.empty((count,), dtype=torch.int32, pin_memory=True)
+    return words
+
+
+def _statistics_words(device_index):
+    return _pinned_words(device_index, 3, "statistics")
+
+
 def _statistics_readback(statistics, count=3, slot="statistics"):
     """Start handing ``count`` integers of ``statistics`` to pinned host memory.
 
@@ -320,14 +336,7 @@ def _statistics_readback(statistics, count=3, slot="statistics"):
     device and ``slot`` is reused: a call's readback is consumed before the same thread can
     start another call.
     """
-    from . import _loader
-    buffers = getattr(_HOST, "buffers", None)
-    if buffers is None:
-        buffers = _HOST.buffers = {}
-    key = (statistics.device.index, slot, count)
-    if key not in buffers:
-        buffers[key] = torch.empty((count,), dtype=torch.int32, pin_memory=True)
-    host = buffers[key]
+    host = _pinned_words(statistics.device.index, count, slot)
     status = _loader.library().gg_report_to_host(
         _loader.pointer(statistics), count, host.data_ptr(), _loader.stream_pointer(statistics.device))
     if status != 0:
@@ -367,6 +376,23 @@ def moe_ffn(hidden_states, w_gate_up, w_down, topk_weights, topk_ids, *,
     (a ``MoEWorkspace``) makes repeated calls reuse their intermediate buffers.  ``routes``
     (from ``prepare_routes`` or ``route_topk_routes`` on the same ids and mask) skips stage 1.
     """
+    if (variant == "auto" and type(group_size) is int and group_size == 256 and activation == "swiglu"
+            and backend in ("auto", "cuda") and gate_up_layout in ("split", "interleaved")
+            and (workspace is None or type(workspace) is MoEWorkspace)
+            and (routes is None or (type(routes) is Routes and routes.tile_rows == TENSOR_CORE_TILE_ROWS
+                                    and routes.tile_expert is not None))
+            and isinstance(hidden_states, torch.Tensor) and hidden_states.is_cuda):
+        # The whole call natively; None for anything but plain CUDA operands outside a capture.
+        out = _loader.host().moe_ffn(
+            hidden_states, w_gate_up, w_down, topk_weights, topk_ids, scale_x, scale_gate_up, scale_down,
+            token_mask, output_dtype, gate_up_layout == "interleaved",
+            None if workspace is None else workspace._buffers,
+            None if routes is None else (routes.order, routes.inverse, routes.offsets, routes.statistics,
+                                         routes.tile_expert, routes.tile_row, routes.tokens,
+                                         routes.top_k, routes.experts),
+            _statistics_words)
+        if out is not None:
+            return out
     tokens, hidden, intermediate, experts, top_k = _validate(
         hidden_states, w_gate_up, w_down, topk_weights, topk_ids,
         scale_x, scale_gate_up, scale_down, token_mask, group_size, activation, backend,

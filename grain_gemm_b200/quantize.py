@@ -28,6 +28,10 @@ def quantize_rows(x, group_size=256, *, rows_per_program=4):
     ``rows_per_program`` is accepted for signature compatibility and ignored.
     """
     del rows_per_program
+    if isinstance(x, torch.Tensor) and x.is_cuda:
+        result = _loader.host().quantize_rows(x, group_size)
+        if result is not None:
+            return result
     if not isinstance(x, torch.Tensor) or x.dim() < 1:
         raise ValueError("x must be a tensor with at least one dimension")
     if x.dtype not in _loader.OUT_DTYPE:
@@ -96,6 +100,13 @@ def route_topk_routes(logits, top_k, *, token_mask=None, ids_dtype=torch.int64, 
     ``moe_ffn(..., routes=routes)`` to skip its own routing.  Results are identical either way.
     """
     from . import moe
+    if (tile_rows == 128 and isinstance(logits, torch.Tensor) and logits.is_cuda
+            and (ids_dtype is torch.int64 or ids_dtype is torch.int32)):
+        parts = _loader.host().route_topk_routes(logits, top_k, token_mask, ids_dtype is torch.int64)
+        if parts is not None:
+            weights, ids, order, counts, offsets, inverse, effective_ids, statistics, expert, row = parts
+            return weights, ids, moe.Routes(order, counts, offsets, inverse, effective_ids, statistics,
+                                            *ids.shape, logits.shape[1], tile_rows, expert, row)
     if not isinstance(logits, torch.Tensor) or logits.dim() != 2:
         raise ValueError("logits must be a [T, E] tensor")
     tokens, experts = logits.shape

@@ -1,0 +1,159 @@
+"""The native host path (``csrc/host.cpp``) against the Python path behind the same entry points.
+
+The native functions either run a call or return ``None``; whatever they accept has to give the
+Python path's result bit for bit (both launch the same kernels), and what the Python path
+refuses has to stay refused with the same error.
+"""
+
+import pytest
+import torch
+
+from grain_gemm_b200 import _loader, int8_gemm, moe, moe_ffn, quantize_rows, route_topk_routes
+
+
+class _PythonOnly:
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+@pytest.fixture
+def python_path(monkeypatch):
+    """A function that runs a call with the native path switched off."""
+    def run(function, *args, **kwargs):
+        with monkeypatch.context() as patch:
+            patch.setattr(_loader, "host", _PythonOnly)
+            return function(*args, **kwargs)
+    return run
+
+
+def test_native_path_leaves_everything_but_plain_cuda_tensors_to_python():
+    host = _loader.host()
+    a = torch.zeros((4, 256), dtype=torch.int8)
+    one = torch.ones((4, 1))
+    assert host.int8_gemm(a, a.t(), one, one.t().contiguous(), 256, torch.bfloat16) is None
+    assert host.int8_gemm(None, 1, "x", a, 256, torch.bfloat16) is None
+    assert host.int8_gemm() is None
+    assert host.quantize_rows(torch.zeros((2, 256)), 256) is None
+    assert host.quantize_rows(3, 256) is None
+    assert host.route_topk_routes(torch.zeros((2, 8)), 2, None, True) is None
+    assert host.moe_ffn(*([None] * 14)) is None
+    with pytest.raises(TypeError):
+        host.bind(1, 2)
+    with pytest.raises(KeyError):
+        host.bind({}, {})
+
+
+def _gemm_case(form, m, n, k, group):
+    generator = torch.Generator().manual_seed(m * 7 + n * 3 + k + group)
+    a = torch.randint(-127, 128, (m, k), dtype=torch.int8, generator=generator).cuda()
+    w = torch.randint(-127, 128, (n, k), dtype=torch.int8, generator=generator).cuda()
+    groups = -(-k // group)
+    sa = torch.rand((m, groups), generator=generator).cuda()
+    sb = torch.rand((groups, n), generator=generator).cuda()
+    b = w.t()
+    if form == "row_major_b":
+        b = b.contiguous()
+    elif form == "wide_rows":
+        a = torch.nn.functional.pad(a, (0, 48))[:, :k]
+    elif form == "odd_rows":
+        a = torch.nn.functional.pad(a, (0, 3))[:, :k]
+    elif form == "scale_views":
+        sa, sb = sa.t().contiguous().t(), sb.t().contiguous().t()
+    elif form == "strided_a":
+        a = a.repeat_interleave(2, dim=1)[:, ::2]
+    return a, b, sa, sb
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["plain", "row_major_b", "wide_rows", "odd_rows", "scale_views", "strided_a"])
+@pytest.mark.parametrize("m,n,k,group", [(1, 64, 256, 256), (1, 1, 48, 32), (17, 200, 272, 128),
+                                         (33, 1, 1, 32), (700, 520, 4112, 256)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gemm_equals_python_path(python_path, form, m, n, k, group, dtype):
+    a, b, sa, sb = _gemm_case(form, m, n, k, group)
+    kwargs = dict(group_size=group, output_dtype=dtype)
+    expected = python_path(int8_gemm, a, b, sa, sb, **kwargs)
+    actual = int8_gemm(a, b, sa, sb, **kwargs)
+    assert actual.dtype == dtype and actual.is_contiguous() and torch.equal(actual, expected)
+
+
+@pytest.mark.gpu
+def test_refused_and_special_calls_take_the_python_path():
+    host = _loader.host()
+    a, b, sa, sb = _gemm_case("plain", 16, 64, 256, 256)
+    good = (a, b, sa, sb, 256, torch.bfloat16)
+    assert host.int8_gemm(*good) is not None
+    for bad in ((a.float(), *good[1:]), (a, b, sa[:, :0], *good[3:]), (*good[:4], 48, good[5]),
+                (*good[:4], True, good[5]), (*good[:5], torch.float64), (a, b[:, :32], *good[2:]),
+                (a.cpu(), *good[1:]), (a[:0], b, sa[:0], *good[3:]),
+                (a, b, sa.expand(16, 1)[:1].expand(16, 1), *good[3:])):
+        assert host.int8_gemm(*bad) is None
+    with torch.overrides.BaseTorchFunctionMode():
+        assert host.int8_gemm(*good) is None
+    class Sub(torch.Tensor):
+        pass
+    assert host.int8_gemm(a.as_subclass(Sub), *good[1:]) is None
+    seen = []
+    torch.vmap(lambda x: (seen.append(host.int8_gemm(x, *good[1:])), x)[1])(a.unsqueeze(0))
+    assert seen == [None]
+    with pytest.raises(ValueError, match="scale_a must have shape"):
+        int8_gemm(a, b, sa[:, :0], sb)
+
+
+def _moe_case(tokens, experts, top_k, layout, mask):
+    generator = torch.Generator(device="cuda").manual_seed(tokens + experts)
+    hidden, inter = 512, 256
+    def weights(n, k):
+        w = torch.randint(-127, 128, (experts, n, k), dtype=torch.int8, device="cuda", generator=generator)
+        return w.transpose(-2, -1), torch.rand((experts, k // 256, n), device="cuda", generator=generator) / 2000
+    w1, s1 = weights(2 * inter, hidden)
+    w2, s2 = weights(hidden, inter)
+    x, sx = quantize_rows(torch.randn((tokens, hidden), device="cuda", generator=generator))
+    logits = torch.randn((tokens, experts), device="cuda", generator=generator)
+    token_mask = torch.rand((tokens,), device="cuda", generator=generator) > 0.3 if mask else None
+    return logits, dict(hidden_states=x, w_gate_up=w1, w_down=w2, scale_x=sx, scale_gate_up=s1, scale_down=s2,
+                        gate_up_layout=layout, token_mask=token_mask)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,experts,top_k,layout,mask", [
+    (1, 8, 2, "split", False), (37, 4, 4, "interleaved", True), (300, 16, 4, "interleaved", False),
+    (1500, 8, 1, "split", True)])
+@pytest.mark.parametrize("use_workspace", [False, True])
+@pytest.mark.parametrize("use_routes", [False, True])
+def test_moe_equals_python_path(python_path, tokens, experts, top_k, layout, mask, use_workspace, use_routes):
+    logits, ffn = _moe_case(tokens, experts, top_k, layout, mask)
+    weights, ids, routes = route_topk_routes(logits, top_k, token_mask=ffn["token_mask"])
+    other = python_path(route_topk_routes, logits, top_k, token_mask=ffn["token_mask"])
+    assert torch.equal(weights, other[0]) and torch.equal(ids, other[1])
+    valid = int(routes.offsets[-1])
+    for name in ("counts", "offsets", "inverse", "effective_ids", "statistics", "tile_expert"):
+        assert torch.equal(getattr(routes, name), getattr(other[2], name)), name
+    assert torch.equal(routes.order[:valid], other[2].order[:valid])
+    call = dict(ffn, topk_weights=weights, topk_ids=ids, routes=routes if use_routes else None)
+    workspace = moe.MoEWorkspace() if use_workspace else None
+    expected = python_path(moe_ffn, **call)
+    for _ in range(2):
+        assert torch.equal(moe_ffn(**call, workspace=workspace), expected)
+    if use_workspace:
+        held = {name: (tuple(t.shape), t.dtype) for name, t in workspace._buffers.items()}
+        again = moe.MoEWorkspace()
+        python_path(moe_ffn, **call, workspace=again)
+        assert held == {name: (tuple(t.shape), t.dtype) for name, t in again._buffers.items()}
+
+
+@pytest.mark.gpu
+def test_moe_bad_ids_raise_and_capture_takes_the_python_path():
+    logits, ffn = _moe_case(8, 4, 2, "split", False)
+    weights, ids, _ = route_topk_routes(logits, 2)
+    bad = ids.clone()
+    bad[3, 1] = 4
+    with pytest.raises(ValueError, match=r"unmasked topk_ids must be in \[0, E\)"):
+        moe_ffn(**ffn, topk_weights=weights, topk_ids=bad)
+    expected = moe_ffn(**ffn, topk_weights=weights, topk_ids=ids)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = moe_ffn(**ffn, topk_weights=weights, topk_ids=ids)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, expected)
