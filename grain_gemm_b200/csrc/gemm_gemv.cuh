@@ -17,6 +17,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace gg {
 
 constexpr int kGemvThreads = 256;
@@ -91,6 +93,8 @@ __global__ void __launch_bounds__(kGemvThreads, kRows <= 2 ? 4 : 2) gemm_gemv_ke
   const int warp_columns = max(0, min(p.columns_per_warp, p.n - warp_first));
   const int blocks = warp_columns * blocks_per_column;
 
+  dependents_may_launch();
+  previous_kernel_done();
   // The first eight loads of weights are requested before anything else.
   const int8_t* weights = p.b + static_cast<long long>(warp_first) * p.b_sn;
   uint4 w[8];

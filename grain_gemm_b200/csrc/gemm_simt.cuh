@@ -166,6 +166,8 @@ fold_partials_kernel(const int* __restrict__ partials, const float* __restrict__
                      const float* __restrict__ scale_b, OutT* __restrict__ c, int m, int n,
                      int groups, long long sa_sm, long long sa_sg, long long sb_sg, long long sb_sn,
                      long long ldc) {
+  dependents_may_launch();
+  previous_kernel_done();
   const int col = blockIdx.x * 256 + threadIdx.x;
   const int row = blockIdx.y;
   if (col >= n) return;

@@ -330,6 +330,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   if constexpr (kCtaGroup == 2) cluster_sync_all();
   if (warp == kMmaWarp) tmem_alloc<kCtaGroup>(tmem_holder, Shape::kTmemColumns);
+  if constexpr (!kGrouped) previous_kernel_done();
   tcgen05_fence_before();
   __syncthreads();
   if constexpr (kCtaGroup == 2) cluster_sync_all();
@@ -385,6 +386,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
     }
+    dependents_may_launch();   // the CTA's last loads are on their way
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer
     // The warp of the pair's leader CTA walks the loop converged; one elected lane issues every

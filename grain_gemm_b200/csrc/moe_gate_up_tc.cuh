@@ -231,6 +231,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           }
         }
       }
+      dependents_may_launch();   // the CTA's last loads are on their way
     } else if (warp == 10) {
       // ---------------------------------------------------------- scale staging warp
       // Copies each group's 256 column scales (by accumulator column) and 128 row scales into a

@@ -44,11 +44,12 @@ __device__ __forceinline__ int route_key(const RouteParams& p, long long s, bool
 }
 
 // Stable placement of one chunk: `cursor[key]` holds the next free slot of each key for this
-// chunk; warps take turns in index order, lanes of a warp rank themselves among equal keys.
+// chunk; the first `turns` warps (those that have assignments) take turns in index order, lanes
+// of a warp rank themselves among equal keys.
 __device__ __forceinline__ void route_place_chunk(const RouteParams& p, long long s, bool present,
-                                                  int key, int* cursor) {
+                                                  int key, int* cursor, int turns) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int turn = 0; turn < kRouteChunk / 32; ++turn) {
+  for (int turn = 0; turn < turns; ++turn) {
     if (warp == turn) {
       const unsigned active = __ballot_sync(0xffffffffu, present);
       if (present) {
@@ -71,23 +72,41 @@ __device__ __forceinline__ void route_place_chunk(const RouteParams& p, long lon
 }
 
 // Scan of the per-key totals held in bins[0..E]; leaves bins[key] = first slot of the key and
-// writes counts, offsets and statistics.  Called by one thread.
+// writes counts, offsets and statistics.  Called by one whole warp, 32 keys at a time (a single
+// thread took 2 us of a decode step for 128 experts).
 __device__ __forceinline__ void route_finish_totals(const RouteParams& p, int* bins, int invalid) {
-  int running = 0, maximum = 0;
-  p.offsets[0] = 0;
-  for (int e = 0; e <= p.experts; ++e) {
-    const int count = bins[e];
-    bins[e] = running;
-    running += count;
+  const int lane = threadIdx.x & 31;
+  int running = 0, maximum = 0, valid = 0;
+  for (int base = 0; base <= p.experts; base += 32) {
+    const int e = base + lane;
+    const int count = e <= p.experts ? bins[e] : 0;
+    int inclusive = count;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
+      if (lane >= offset) inclusive += other;
+    }
+    const int first = running + inclusive - count;
+    if (e <= p.experts) bins[e] = first;
     if (e < p.experts) {
       p.counts[e] = count;
-      p.offsets[e + 1] = running;
+      p.offsets[e + 1] = first + count;
       maximum = max(maximum, count);
+      valid = first + count;
     }
+    running += __shfl_sync(0xffffffffu, inclusive, 31);
   }
-  p.statistics[0] = invalid;
-  p.statistics[1] = maximum;
-  p.statistics[2] = p.offsets[p.experts];
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1) {
+    maximum = max(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
+    valid = max(valid, __shfl_xor_sync(0xffffffffu, valid, offset));
+  }
+  if (lane == 0) {
+    p.offsets[0] = 0;
+    p.statistics[0] = invalid;
+    p.statistics[1] = maximum;
+    p.statistics[2] = valid;
+  }
 }
 
 // Whole routing problem in one CTA (S <= 1024): keys, histogram, scan and placement.
@@ -105,12 +124,14 @@ __device__ __forceinline__ void route_single_body(const RouteParams& p, int* bin
     if (invalid) atomicAdd(&bins[p.experts + 1], 1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) route_finish_totals(p, bins, bins[p.experts + 1]);
+  if (threadIdx.x < 32) route_finish_totals(p, bins, bins[p.experts + 1]);
   __syncthreads();
-  route_place_chunk(p, s, present, key, bins);
+  route_place_chunk(p, s, present, key, bins, static_cast<int>((slots + 31) / 32));
 }
 
 __global__ void __launch_bounds__(kRouteChunk) route_single_kernel(const RouteParams p) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int bins[];  // [E + 2]; the last entry counts invalid ids
   route_single_body(p, bins);
 }
@@ -129,6 +150,8 @@ constexpr int kRouteMediumSlots = 32 * 32 * kRouteMediumRounds;   // 8192 assign
 constexpr int kRouteMediumKeys = 512;                              // experts + 1 at most
 
 __global__ void __launch_bounds__(1024) route_medium_kernel(const RouteParams p) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int medium_smem[];     // [32][keys] per-warp histograms / bases, then scratch
   const int keys = p.experts + 1;
   int* warp_bins = medium_smem;
@@ -248,6 +271,8 @@ __global__ void __launch_bounds__(1024) route_medium_kernel(const RouteParams p)
 }
 
 __global__ void __launch_bounds__(kRouteChunk) route_histogram_kernel(const RouteParams p) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int bins[];
   const long long slots = static_cast<long long>(p.tokens) * p.top_k;
   const int chunks = gridDim.x;
@@ -269,6 +294,8 @@ __global__ void __launch_bounds__(kRouteChunk) route_histogram_kernel(const Rout
 
 // One CTA: turns the per-chunk histograms into per-chunk first slots (in place).
 __global__ void __launch_bounds__(1024) route_scan_kernel(const RouteParams p, int chunks) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int bins[];  // [E + 1]
   const int stride = p.experts + 1;
   for (int key = threadIdx.x; key <= p.experts; key += blockDim.x) {
@@ -277,10 +304,14 @@ __global__ void __launch_bounds__(1024) route_scan_kernel(const RouteParams p, i
     bins[key] = total;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     int invalid = 0;
     const int* invalid_counts = p.workspace + static_cast<long long>(chunks) * stride;
-    for (int c = 0; c < chunks; ++c) invalid += invalid_counts[c];
+    for (int c = threadIdx.x; c < chunks; c += 32) invalid += invalid_counts[c];
+#pragma unroll
+    for (int offset = 16; offset > 0; offset >>= 1) {
+      invalid += __shfl_xor_sync(0xffffffffu, invalid, offset);
+    }
     route_finish_totals(p, bins, invalid);
   }
   __syncthreads();
@@ -296,6 +327,8 @@ __global__ void __launch_bounds__(1024) route_scan_kernel(const RouteParams p, i
 }
 
 __global__ void __launch_bounds__(kRouteChunk) route_place_kernel(const RouteParams p) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int bins[];
   const long long slots = static_cast<long long>(p.tokens) * p.top_k;
   const int* first = p.workspace + static_cast<long long>(blockIdx.x) * (p.experts + 1);
@@ -308,7 +341,7 @@ __global__ void __launch_bounds__(kRouteChunk) route_place_kernel(const RoutePar
     key = p.ids_are_i64 ? static_cast<int>(reinterpret_cast<const long long*>(p.effective_ids)[s])
                         : reinterpret_cast<const int*>(p.effective_ids)[s];
   }
-  route_place_chunk(p, s, present, key, bins);
+  route_place_chunk(p, s, present, key, bins, kRouteChunk / 32);
 }
 
 // Hands a few integers (routing statistics, error flags) to the host by storing them into
@@ -318,6 +351,8 @@ __global__ void __launch_bounds__(kRouteChunk) route_place_kernel(const RoutePar
 // and the stream does not wait for the copy engine either.
 __global__ void __launch_bounds__(32)
 report_to_host_kernel(const int* __restrict__ values, int count, int* host_words) {
+  dependents_may_launch();
+  previous_kernel_done();
   for (int i = threadIdx.x; i < count; i += 32) host_words[i] = values[i];
   __threadfence_system();
 }
@@ -329,6 +364,8 @@ report_to_host_kernel(const int* __restrict__ values, int count, int* host_words
 __global__ void __launch_bounds__(1024)
 moe_tiles_kernel(const int* __restrict__ offsets, int experts, int tile_rows, int max_tiles,
                  int* __restrict__ tile_expert, int* __restrict__ tile_row) {
+  dependents_may_launch();
+  previous_kernel_done();
   __shared__ int warp_total[32];
   __shared__ int carry;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -380,36 +417,69 @@ moe_tiles_kernel(const int* __restrict__ offsets, int experts, int tile_rows, in
 // arguments.  Entry b holds the result for the value whose bit pattern is b, computed here with
 // exactly the operations of swiglu_value, hence bit-identical to evaluating the formula
 // (the idea of the reference's experiments/thor_interleaved_mega/exact_silu_lut.cuh:1-36).
-__global__ void __launch_bounds__(256)
-silu_table_kernel(float* __restrict__ silu_table, int half_output) {
-  const int bits = blockIdx.x * 256 + threadIdx.x;
-  if (bits >= 65536) return;
+__device__ __forceinline__ float silu_of_bits(int bits, int half_output) {
   const float gate = half_output ? __half2float(__ushort_as_half(static_cast<unsigned short>(bits)))
                                  : __uint_as_float(static_cast<uint32_t>(bits) << 16);
-  silu_table[bits] = __fdiv_rn(gate, __fadd_rn(1.0f, expf(-gate)));
+  return __fdiv_rn(gate, __fadd_rn(1.0f, expf(-gate)));
+}
+
+__global__ void __launch_bounds__(256)
+silu_table_kernel(float* __restrict__ silu_table, int half_output) {
+  dependents_may_launch();
+  previous_kernel_done();
+  const int bits = blockIdx.x * 256 + threadIdx.x;
+  if (bits < 65536) silu_table[bits] = silu_of_bits(bits, half_output);
 }
 
 // Activation rows and their scales in sorted-slot order, for the valid slots only:
 // sorted_x[slot, :] = x[order[slot] / top_k, :] and likewise for the row scales (the
 // pre-sorted mode of the fused Gate/Up kernel, kept for measurements against the row-gather
 // mode).  One warp per slot; a row is `hidden` bytes (a multiple of 256) moved as 16-byte vectors.
+// Bound by HBM (S * H bytes written; the reads repeat top_k times and hit L2).  A lane keeps
+// eight loads in flight, and the token of the warp's next slot is fetched ahead: with one load
+// at a time the copy of 131072 rows of 7168 bytes took 301 us, a little under half the copy rate.
+// The first kSiluBlocks blocks also fill the SiLU table that the same Gate/Up call reads (a launch
+// of its own cost 1.7 us).
+constexpr int kSiluBlocks = 64;
+
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const int8_t* __restrict__ x, const float* __restrict__ scale_x,
                    const long long* __restrict__ order, const int* __restrict__ offsets,
                    int experts, int top_k, int hidden, int8_t* __restrict__ sorted_x,
-                   float* __restrict__ sorted_scale) {
+                   float* __restrict__ sorted_scale, float* __restrict__ silu_table,
+                   int half_output) {
+  dependents_may_launch();
+  previous_kernel_done();
   const int valid = offsets[experts];
   const int lane = threadIdx.x & 31;
   const int groups = hidden / 256;
   const int vectors = hidden / 16;
-  for (long long slot = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5); slot < valid;
-       slot += static_cast<long long>(gridDim.x) * 8) {
-    const long long token = order[slot] / top_k;
+  const int stride = gridDim.x * 8;
+  int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
+  long long next = slot < valid ? order[slot] : 0;
+  for (; slot < valid; slot += stride) {
+    const long long token = next / top_k;
+    if (slot + stride < valid) next = order[slot + stride];
     const uint4* source = reinterpret_cast<const uint4*>(x + token * hidden);
-    uint4* destination = reinterpret_cast<uint4*>(sorted_x + slot * hidden);
-    for (int i = lane; i < vectors; i += 32) destination[i] = source[i];
+    uint4* destination = reinterpret_cast<uint4*>(sorted_x + static_cast<long long>(slot) * hidden);
+    for (int i = lane; i < vectors; i += 256) {
+      uint4 held[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (i + 32 * j < vectors) held[j] = __ldg(source + i + 32 * j);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (i + 32 * j < vectors) destination[i + 32 * j] = held[j];
+      }
+    }
     for (int g = lane; g < groups; g += 32) {
-      sorted_scale[slot * groups + g] = scale_x[token * groups + g];
+      sorted_scale[static_cast<long long>(slot) * groups + g] = scale_x[token * groups + g];
+    }
+  }
+  if (blockIdx.x < kSiluBlocks) {
+    for (int bits = blockIdx.x * 256 + threadIdx.x; bits < 65536; bits += kSiluBlocks * 256) {
+      silu_table[bits] = silu_of_bits(bits, half_output);
     }
   }
 }
@@ -529,6 +599,8 @@ template <typename InT>
 __global__ void __launch_bounds__(256)
 router_topk_kernel(const InT* __restrict__ logits, int tokens, int experts, int top_k,
                    float* __restrict__ weights, void* __restrict__ ids, int ids_are_i64) {
+  dependents_may_launch();
+  previous_kernel_done();
   const int lane = threadIdx.x & 31;
   const int token = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (token >= tokens) return;
@@ -545,6 +617,8 @@ template <typename InT>
 __global__ void __launch_bounds__(kRouteChunk)
 route_topk_single_kernel(const InT* __restrict__ logits, float* __restrict__ weights,
                          const RouteParams p) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int bins[];  // [E + 2]
   const int lane = threadIdx.x & 31;
   for (int token = threadIdx.x >> 5; token < p.tokens; token += kRouteChunk / 32) {
@@ -560,43 +634,62 @@ route_topk_single_kernel(const InT* __restrict__ logits, float* __restrict__ wei
 //   scale = div_rn(max(amax, 1e-12), 127);  q = clamp(nearbyint(div_rn(v, scale)), +-127).
 // Eight consecutive values per lane (16 bytes of BF16/FP16, 32 of FP32); a group of G values
 // is G/8 neighbouring lanes, so a warp covers 256/G groups of one row at a time.  HBM bound:
-// sizeof(InT) bytes read and one byte (+ 4/G) written per element.
-template <typename InT>
+// sizeof(InT) bytes read and one byte (+ 4/G) written per element.  A warp requests kItems
+// 256-value chunks before it works on the first, and the codes divide by the guarded FMA
+// sequence: with one chunk per warp and library divisions (a branch each) 16384 rows of 7168
+// BF16 values took 190 us, 1.9 TB/s.
+template <typename InT, int kItems>
 __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const InT* __restrict__ x, long long rows, int width, int group,
                      int8_t* __restrict__ q, float* __restrict__ s) {
+  dependents_may_launch();
+  previous_kernel_done();
   const int lane = threadIdx.x & 31;
-  const int chunks = width / 256;                 // 256-value chunks per row (width % 256 == 0)
-  const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  if (item >= rows * chunks) return;
-  const long long row = item / chunks;
-  const int column = static_cast<int>(item - row * chunks) * 256 + lane * 8;
-  const InT* source = x + row * width + column;
-  float v[8];
-  if constexpr (sizeof(InT) == 4) {
-    const float4 a = *reinterpret_cast<const float4*>(source);
-    const float4 b = *reinterpret_cast<const float4*>(source + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-    const uint4 raw = *reinterpret_cast<const uint4*>(source);
-    const InT* values = reinterpret_cast<const InT*>(&raw);
+  // Rows are contiguous and hold whole 256-value chunks, so item i is simply the i-th chunk of x
+  // and its groups are consecutive in s.
+  const long long items = rows * (width / 256);
+  const long long first = (static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * kItems;
+  constexpr int kWords = sizeof(InT) / 2;        // 16-byte words per lane and chunk
+  uint4 raw[kItems][kWords];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = static_cast<float>(values[i]);
-  }
-  float amax = 0.0f;
+  for (int i = 0; i < kItems; ++i) {
+    if (first + i < items) {
+      const uint4* source = reinterpret_cast<const uint4*>(x + (first + i) * 256 + lane * 8);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-  for (int offset = group / 16; offset > 0; offset >>= 1) {
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
+      for (int w = 0; w < kWords; ++w) raw[i][w] = __ldg(source + w);
+    }
   }
-  const float scale = quantize_scale(amax);
-  uint32_t packed[2] = {0u, 0u};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    packed[i >> 2] |= (static_cast<uint32_t>(quantize_value(v[i], scale)) & 0xffu) << (8 * (i & 3));
+  for (int i = 0; i < kItems; ++i) {
+    if (first + i >= items) return;              // the same for the whole warp
+    float v[8];
+    const InT* values = reinterpret_cast<const InT*>(raw[i]);
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = static_cast<float>(values[j]);
+      amax = fmaxf(amax, fabsf(v[j]));
+    }
+    for (int offset = group / 16; offset > 0; offset >>= 1) {
+      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
+    }
+    const float scale = quantize_scale(amax);
+    uint32_t packed[2] = {0u, 0u};
+    if (quantize_division_is_safe(amax)) {
+      const float y = __frcp_rn(scale);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        packed[j >> 2] |= (static_cast<uint32_t>(quantize_value_by_fma(v[j], scale, y)) & 0xffu) << (8 * (j & 3));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        packed[j >> 2] |= (static_cast<uint32_t>(quantize_value(v[j], scale)) & 0xffu) << (8 * (j & 3));
+      }
+    }
+    *reinterpret_cast<uint2*>(q + (first + i) * 256 + lane * 8) = make_uint2(packed[0], packed[1]);
+    if ((lane & (group / 8 - 1)) == 0) s[((first + i) * 256 + lane * 8) / group] = scale;
   }
-  *reinterpret_cast<uint2*>(q + row * width + column) = make_uint2(packed[0], packed[1]);
-  if ((lane & (group / 8 - 1)) == 0) s[row * (width / group) + column / group] = scale;
 }
 
 // Stand-alone SwiGLU + G256 requantisation over a [rows, 2I] gate/up matrix (the unfused
@@ -651,6 +744,8 @@ __global__ void __launch_bounds__(256)
 combine_kernel(const T* __restrict__ expert_out, const float* __restrict__ weights,
                const int* __restrict__ inverse, T* __restrict__ out, int top_k, int hidden,
                int vector_ok) {
+  dependents_may_launch();
+  previous_kernel_done();
   extern __shared__ int slot_smem[];  // [R] slots then [R] weights
   float* weight_smem = reinterpret_cast<float*>(slot_smem + top_k);
   const long long token = blockIdx.x;

@@ -63,6 +63,21 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ---------------------------------------------------------------- programmatic launches
+
+// The kernels of the call chains are launched with programmatic stream serialisation (the two
+// grouped tensor-core kernels excepted): their blocks may become resident while the previous kernel of the stream still runs, and do their set-up
+// there.  dependents_may_launch() lets the NEXT kernel do the same; previous_kernel_done() returns
+// when the previous kernel has completed and its writes are visible, and stands before the first
+// access to global memory, reads included (nothing is known about who wrote the operands).
+// Since every kernel waits for its predecessor, a completed kernel implies all earlier ones.
+__device__ __forceinline__ void dependents_may_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void previous_kernel_done() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- mbarrier
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
