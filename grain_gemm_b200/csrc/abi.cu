@@ -60,6 +60,31 @@ static int encode_int8_rows(CUtensorMap* map, const void* base, long long rows, 
   return result == CUDA_SUCCESS ? 0 : -10000 - static_cast<int>(result);
 }
 
+// Tensor map over the rows of a weight matrix, boxes of 128 bytes x box_rows.  With `permuted` (rows
+// a multiple of 32) every block of 32 rows is delivered in the order the epilogue's fragments
+// want: row 8q + k of the block lands in row 4k + q of the tile (see gemm_tc.cuh).  The kernels
+// load with coordinates (x, 0, 0, row / 32) then, with (x, row, 0, 0) otherwise.
+static int weight_row_map(CUtensorMap* map, const void* base, long long rows, long long cols,
+                          long long pitch, int box_rows, bool permuted) {
+  EncodeTiledFn encode = encode_tiled_fn();
+  if (encode == nullptr) return static_cast<int>(cudaErrorNotSupported);
+  const cuuint64_t columns = static_cast<cuuint64_t>(cols), step = static_cast<cuuint64_t>(pitch);
+  const cuuint32_t box = static_cast<cuuint32_t>(box_rows);
+  const cuuint64_t own_dims[4] = {columns, static_cast<cuuint64_t>(rows), 1, 1};
+  const cuuint64_t own_strides[3] = {step, step, step};
+  const cuuint32_t own_box[4] = {128u, box, 1u, 1u};
+  const cuuint64_t permuted_dims[4] = {columns, 4, 8, static_cast<cuuint64_t>(rows / 32)};
+  const cuuint64_t permuted_strides[3] = {8 * step, step, 32 * step};
+  const cuuint32_t permuted_box[4] = {128u, 4u, 8u, box / 32};
+  const cuuint32_t element_strides[4] = {1u, 1u, 1u, 1u};
+  const CUresult result = encode(
+      map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), permuted ? permuted_dims : own_dims,
+      permuted ? permuted_strides : own_strides, permuted ? permuted_box : own_box, element_strides,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return result == CUDA_SUCCESS ? 0 : -10000 - static_cast<int>(result);
+}
+
 static int sm_count() {
   // Immutable device property, cached per device.
   static int cached[64] = {0};
@@ -361,7 +386,8 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   CUtensorMap map_a, map_b;
   int status = encode_int8_rows(&map_a, g.a, g.m, g.k, g.a_sm, 128);
   if (status) return status;
-  status = encode_int8_rows(&map_b, g.b, g.n, g.k, g.b_sn, pair ? bn / 2 : bn);
+  const bool permuted = g.n % 32 == 0;
+  status = weight_row_map(&map_b, g.b, g.n, g.k, g.b_sn, pair ? bn / 2 : bn, permuted);
   if (status) return status;
   GemmTcParams p = {};
   p.scale_a = static_cast<const float*>(g.scale_a);
@@ -373,6 +399,8 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   p.group_size = g.group_size;
   p.k_splits = 1;
   p.band_rows = 16;
+  p.permuted_columns = permuted;
+  p.sb_vectors = permuted && g.sb_sn == 1 && g.sb_sg % 4 == 0 && aligned16(g.scale_b);
   p.tiles_m = (g.m + (pair ? 255 : 127)) / (pair ? 256 : 128);
   p.tiles_n = (g.n + bn - 1) / bn;
   const int out_bytes = g.out_dtype == GG_OUT_FP32 ? 4 : 2;
@@ -397,7 +425,8 @@ static int launch_gemm_splitk(const GemmArgs& g, void* workspace, size_t workspa
   CUtensorMap map_a, map_b;
   int status = encode_int8_rows(&map_a, g.a, g.m, g.k, g.a_sm, 32);
   if (status) return status;
-  status = encode_int8_rows(&map_b, g.b, g.n, g.k, g.b_sn, 256);
+  // The dots leave in column order (a thread stores consecutive TMEM columns of one row).
+  status = weight_row_map(&map_b, g.b, g.n, g.k, g.b_sn, 256, false);
   if (status) return status;
   GemmTcParams p = {};
   p.m = g.m; p.n = g.n; p.k = g.k;
@@ -811,11 +840,11 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     if (interleaved) {
       // Every other row: gate rows from the first, up rows from the second.
       const int8_t* rows = static_cast<const int8_t*>(w1);
-      status = gg::encode_int8_rows(&map_gate, rows, weight_rows / 2, hidden, 2ll * hidden, 128);
+      status = gg::weight_row_map(&map_gate, rows, weight_rows / 2, hidden, 2ll * hidden, 128, true);
       if (status) return status;
-      status = gg::encode_int8_rows(&map_up, rows + hidden, weight_rows / 2, hidden, 2ll * hidden, 128);
+      status = gg::weight_row_map(&map_up, rows + hidden, weight_rows / 2, hidden, 2ll * hidden, 128, true);
     } else {
-      status = gg::encode_int8_rows(&map_gate, w1, weight_rows, hidden, hidden, 128);
+      status = gg::weight_row_map(&map_gate, w1, weight_rows, hidden, hidden, 128, true);
       map_up = map_gate;
     }
     if (status) return status;
@@ -829,6 +858,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     p.s = static_cast<float*>(s);
     p.hidden = hidden; p.intermediate = intermediate;
     p.max_tiles = tile_capacity; p.interleaved = interleaved;
+    p.sw_vectors = !interleaved && gg::aligned16(scale_w1);
     const long long items = static_cast<long long>(tile_capacity) * (intermediate / 256);
     const int grid = static_cast<int>(items < gg::sm_count() ? items : gg::sm_count());
     if (row_gather) {
@@ -901,8 +931,9 @@ int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_
     int status = gg::encode_int8_rows(&map_a, q, assignments, intermediate, intermediate, 128);
     if (status) return status;
     const int bn = hidden >= 256 ? 256 : hidden >= 128 ? 128 : 64;
-    status = gg::encode_int8_rows(&map_b, w2, static_cast<long long>(experts) * hidden, intermediate,
-                                  intermediate, bn);
+    const bool permuted = hidden % 32 == 0;
+    status = gg::weight_row_map(&map_b, w2, static_cast<long long>(experts) * hidden, intermediate,
+                                intermediate, bn, permuted);
     if (status) return status;
     gg::GemmTcParams p = {};
     p.scale_a = static_cast<const float*>(s);
@@ -914,6 +945,8 @@ int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_
     p.group_size = 256;
     p.k_splits = 1;
     p.band_rows = 8;
+    p.permuted_columns = permuted;
+    p.sb_vectors = permuted && gg::aligned16(scale_w2);
     p.tiles_m = tile_capacity;
     p.tiles_n = (hidden + bn - 1) / bn;
     p.c_vector_ok = 1;

@@ -79,6 +79,10 @@ struct GemmTcParams {
   // the INT32 group dots go to partials[Q][M][N] instead of being promoted (a second kernel
   // then folds them in group order).  k_splits == 1 and partials == null otherwise.
   int band_rows;               // row tiles per scheduling band
+  // N is a multiple of 32 and map_b delivers every block of 32 weight rows in fragment order
+  // (weight_row_map); otherwise the rows arrive in their own order.
+  int permuted_columns;
+  int sb_vectors;              // permuted_columns, and scale_b may be read 16 bytes at a time
   int k_splits;
   int groups_per_split;
   int* partials;
@@ -180,8 +184,17 @@ __device__ __forceinline__ TileWork decode_tile(const GemmTcParams& p, int tile,
 // with eight warps draining 128 lanes x 256 columns: 16x128b delivers 507 B/clk/SM, 32x32b 940,
 // and 16x256b, which would give adjacent column pairs, 256.
 //
-// Position of block column `c` (0..31) in the scale ring: thread q reads its eight column
-// scales, in accumulator-pair order, as two 16-byte vectors at q * 8.
+// A row leaves as 16-byte stores of consecutive columns, so thread q wants the outputs
+// 8q .. 8q + 7 of a block in its eight columns 4k + q.  Weight row 8q + k therefore has to sit in
+// row 4k + q of the B tile's block, and the tensor map does that on the way in: it presents the
+// weight as [N/32][k = 8][q = 4][K] (weight_row_map in abi.cu), and accumulator pair j holds the
+// outputs 8q + 2j and 8q + 2j + 1.  Nothing is exchanged between lanes and the scales are used in
+// their own order.  (With rows in their own order, pair j holds outputs 8j + q and 8j + 4 + q and a
+// 4x4 exchange inside every quad precedes the stores: 64 shuffles and 600 instructions a
+// warp and tile.  Only widths that are not a multiple of 32 still do that.)
+//
+// Position of block column `c` (0..31) in the scale ring for rows in their own order: thread q
+// reads its eight column scales, in accumulator-pair order, as two 16-byte vectors at q * 8.
 __device__ __forceinline__ int ring_column_position(int c) {
   return (c & 3) * 8 + (c >> 3) * 2 + ((c >> 2) & 1);
 }
@@ -256,6 +269,17 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int q) {
   t0 = __shfl_xor_sync(0xffffffffu, t0, 2);
   t1 = __shfl_xor_sync(0xffffffffu, t1, 2);
   if (upper) { w[0] = t0; w[1] = t1; } else { w[2] = t0; w[3] = t1; }
+}
+
+// Packed output pairs of a block whose weight rows came in their own order: lane q enters with the
+// columns 8i + q (low halves) and 8i + 4 + q and leaves with columns 8q .. 8q + 7.
+__device__ __forceinline__ void own_order_exchange(uint32_t (&w)[4], int q) {
+  quad_transpose(w, q);
+  const uint32_t v0 = w[0], v1 = w[1], v2 = w[2], v3 = w[3];
+  w[0] = __byte_perm(v0, v1, 0x5410);
+  w[1] = __byte_perm(v2, v3, 0x5410);
+  w[2] = __byte_perm(v0, v1, 0x7632);
+  w[3] = __byte_perm(v2, v3, 0x7632);
 }
 
 template <int kCtaGroup, int BN, int kStages, typename OutT, bool kGrouped, int kPromoWarps,
@@ -362,6 +386,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         row_a = (tm * kCtaGroup + static_cast<int>(cta_rank)) * Shape::kBM;
         row_b = tn * BN + static_cast<int>(cta_rank) * Shape::kBRows;
       }
+      const int b_c1 = p.permuted_columns ? 0 : row_b, b_c3 = p.permuted_columns ? row_b >> 5 : 0;
       for (int slab = 0, x = work.k_begin; slab < work.slabs; ++slab, x += Shape::kBK) {
         if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, kSiteProducerEmpty, abort_flag)) {
           ok = false;
@@ -373,11 +398,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if constexpr (kCtaGroup == 1) {
             mbar_expect_tx(&full_bar[stage], Shape::kStageBytes);
             tma_load_2d(a_dst, &map_a, &full_bar[stage], x, row_a);
-            tma_load_2d(b_dst, &map_b, &full_bar[stage], x, row_b);
+            tma_load_4d(b_dst, &map_b, &full_bar[stage], x, b_c1, b_c3);
           } else {
             if (cta_rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Shape::kStageBytes);
             tma_load_2d_pair(a_dst, &map_a, &full_bar[stage], x, row_a);
-            tma_load_2d_pair(b_dst, &map_b, &full_bar[stage], x, row_b);
+            tma_load_4d_pair(b_dst, &map_b, &full_bar[stage], x, b_c1, b_c3);
           }
         }
         if (++stage == kStages) {
@@ -506,7 +531,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // held one group in registers left the promotion warps waiting for scales).
     constexpr int kColumnsPerLane = BN / 32;
     // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-    const uint32_t column_position = 4 * ring_column_position(lane);
+    const uint32_t column_position = 4 * (p.permuted_columns ? lane : ring_column_position(lane));
     const uint32_t row_position = 4 * ring_row_position(lane);
     const uint32_t ring_base = smem_u32(scale_ring);
     uint32_t chunk = 0, phase = 0;
@@ -531,6 +556,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       // warp within its registers.  A copy that is not valid writes zero and reads nothing.
       const float* sb_source = sb_base + static_cast<long long>(n0 + lane) * p.sb_sn +
                                static_cast<long long>(work.group_begin) * p.sb_sg;
+      const float* vector_source = sb_base + n0 + 4 * lane + static_cast<long long>(work.group_begin) * p.sb_sg;
       const float* sa_source = p.scale_a + static_cast<long long>(row0 + lane) * p.sa_sm +
                                static_cast<long long>(work.group_begin) * p.sa_sg;
       const int columns_left = p.n - n0 - lane, rows_left = row_limit - row0 - lane;
@@ -544,15 +570,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int in_chunk = min(kScaleChunkGroups, work.groups - g);
         uint32_t destination = ring_base + chunk * (kScaleChunkGroups * Shape::kScaleSlotFloats * 4);
         for (int i = 0; i < in_chunk; ++i) {
+          if (p.sb_vectors) {
+            // Four consecutive columns per copy; a block of 32 columns exists as a whole or not.
+            const float* source = vector_source;
 #pragma unroll
-          for (int j = 0; j < kColumnsPerLane; ++j, sb_source += sb_step) {
-            cp_async_f32(destination + 128 * j + column_position, sb_source, 32 * j < columns_left);
+            for (int j = 0; j < (BN + 127) / 128; ++j, source += 128) {
+              if (BN >= 128 || lane < BN / 4) {
+                cp_async_f32x4(destination + 512 * j + 16 * lane, source, n0 + 128 * j + 4 * lane < p.n);
+              }
+            }
+            vector_source += p.sb_sg;
+          } else {
+#pragma unroll
+            for (int j = 0; j < kColumnsPerLane; ++j, sb_source += sb_step) {
+              cp_async_f32(destination + 128 * j + column_position, sb_source, 32 * j < columns_left);
+            }
+            sb_source += sb_next;
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j, sa_source += sa_step) {
             cp_async_f32(destination + 4 * BN + 128 * j + row_position, sa_source, 32 * j < rows_left);
           }
-          sb_source += sb_next;
           sa_source += sa_next;
           destination += Shape::kScaleSlotFloats * 4;
         }
@@ -751,11 +789,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
-      // The fragment layout leaves each lane with columns spread over the block.  A 4x4
-      // exchange inside every quad gives lane q the eight consecutive columns 8q..8q+7 of each
-      // 32-column block (after it, accumulator pair i holds columns 8q + i and 8q + 4 + i), so that a row leaves as 16-byte stores: a quarter of the store
-      // instructions and of the memory-pipe wavefronts of pair stores.
+      // Lane q stores the eight consecutive columns 8q..8q+7 of each 32-column block: a quarter of
+      // the store instructions and of the memory-pipe wavefronts of pair stores.
       if (ok) {
+        const bool exchange = p.permuted_columns == 0;
         const int quad = lane & 3;
         const int first_row = row - row_in_cta + quarter * 32 + fragment_row;
         const bool aligned = p.c_vector_ok != 0;
@@ -803,12 +840,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 for (int half = 0; half < 2; ++half) {
 #pragma unroll
                   for (int i = 0; i < 4; ++i) w[half][i] = pack_pair<OutT>(acc[r][(block + half) * 4 + i]);
-                  quad_transpose(w[half], quad);
-                  const uint32_t v0 = w[half][0], v1 = w[half][1], v2 = w[half][2], v3 = w[half][3];
-                  w[half][0] = __byte_perm(v0, v1, 0x5410);
-                  w[half][1] = __byte_perm(v2, v3, 0x5410);
-                  w[half][2] = __byte_perm(v0, v1, 0x7632);
-                  w[half][3] = __byte_perm(v2, v3, 0x7632);
+                  if (exchange) own_order_exchange(w[half], quad);
                 }
                 // Low lanes keep block `block` and give away the next one, high lanes the reverse.
                 uint32_t received[4];
@@ -844,12 +876,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               uint32_t w[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) w[i] = pack_pair<OutT>(acc[r][block * 4 + i]);
-              quad_transpose(w, quad);
-              const uint32_t v0 = w[0], v1 = w[1], v2 = w[2], v3 = w[3];
-              w[0] = __byte_perm(v0, v1, 0x5410);
-              w[1] = __byte_perm(v2, v3, 0x5410);
-              w[2] = __byte_perm(v0, v1, 0x7632);
-              w[3] = __byte_perm(v2, v3, 0x7632);
+              if (exchange) own_order_exchange(w, quad);
               if (row_stored) {
                 if (aligned && col + 8 <= p.n) {
                   *reinterpret_cast<uint4*>(c_row + col) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -869,8 +896,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 wx[i] = __float_as_uint(acc[r][block * 4 + i].x);
                 wy[i] = __float_as_uint(acc[r][block * 4 + i].y);
               }
-              quad_transpose(wx, quad);
-              quad_transpose(wy, quad);
+              if (exchange) {
+                quad_transpose(wx, quad);
+                quad_transpose(wy, quad);
+              } else {
+                const uint32_t x1 = wx[1], x2 = wx[2], x3 = wx[3], y0 = wy[0], y1 = wy[1], y2 = wy[2];
+                wx[1] = y0; wx[2] = x1; wx[3] = y1;
+                wy[0] = x2; wy[1] = y2; wy[2] = x3;
+              }
               if (row_stored) {
                 if (aligned && col + 8 <= p.n) {
                   uint4* out = reinterpret_cast<uint4*>(c_row + col);

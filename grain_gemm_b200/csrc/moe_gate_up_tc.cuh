@@ -46,6 +46,7 @@ struct GateUpParams {
   int8_t* q;                  // [S, I]
   float* s;                   // [S, I/256]
   int hidden, intermediate, max_tiles, interleaved;
+  int sw_vectors;             // scale_w may be read 16 bytes at a time (split layout, aligned)
 };
 
 struct GateUpShape {
@@ -216,8 +217,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             if (leader) {
               mbar_expect_tx(&full_bar[stage], Shape::kStageBytes);
               if constexpr (!kGather) tma_load_2d(a_dst, &map_x, &full_bar[stage], x, row0);
-              tma_load_2d(b_dst, &map_gate, &full_bar[stage], x, row_gate);
-              tma_load_2d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, row_up);
+              tma_load_4d(b_dst, &map_gate, &full_bar[stage], x, 0, row_gate >> 5);
+              tma_load_4d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, 0, row_up >> 5);
             }
             if constexpr (kGather) {
               // Every lane fetches its four rows: 32 gathers of 512 bytes fill the A tile.
@@ -240,8 +241,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       // runs a whole ring ahead and global-memory latency stays hidden.
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
-      // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-      const uint32_t column_position = 4 * ring_column_position(lane);
+      // Byte offset of this lane's row within a 32-float block of a ring slot.
       const uint32_t row_position = 4 * ring_row_position(lane);
       const uint32_t ring_base = smem_u32(sb_ring);
       const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale
@@ -262,7 +262,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           sa_source[i] = p.row_scale + source_row * groups;
         }
         for (int sub = 0; sub < 2 && ok; ++sub) {
-          const int channel = jg * 256 + sub * 128 + lane;
+          const int channel = jg * 256 + sub * 128 + (p.sw_vectors ? 4 * lane : lane);
           const float* sb_source = sb_base + (p.interleaved ? 2 * channel : channel);
           for (int g = 0; g < groups; g += kScaleChunkGroups) {
             if (!mbar_wait_warp(&scale_empty_bar[chunk], phase ^ 1u, kSiteScaleEmpty, abort_flag)) {
@@ -272,10 +272,15 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const int in_chunk = min(kScaleChunkGroups, groups - g);
             uint32_t destination = ring_base + chunk * (kScaleChunkGroups * Shape::kRingFloats * 4);
             for (int i = 0; i < in_chunk; ++i) {
+              if (p.sw_vectors) {
+                cp_async_f32x4(destination + 16 * lane, sb_source, true);
+                cp_async_f32x4(destination + 512 + 16 * lane, sb_source + up_offset, true);
+              } else {
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                cp_async_f32(destination + 128 * j + column_position,
-                             sb_source + (j & 3) * sb_step + (j < 4 ? 0 : up_offset), true);
+                for (int j = 0; j < 8; ++j) {
+                  cp_async_f32(destination + 128 * j + 4 * lane,
+                               sb_source + (j & 3) * sb_step + (j < 4 ? 0 : up_offset), true);
+                }
               }
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -353,9 +358,9 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     // ------------------------------------------------------------ promotion + SwiGLU warps
     // Fragment layout (tmem_ld_16x128b_x8): warp (quarter, half) drains TMEM lanes
     // 32*quarter.. of four 32-column blocks; a thread owns tile rows
-    // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, the column pairs
-    // 8i + lane%4, +4 (i = 0..3).  Blocks 0,1 are 64 gate columns of this half, blocks 2,3 the
-    // matching up columns.
+    // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, the channel pairs
+    // 8*(lane%4) + 2i, +1 (i = 0..3; the weight rows arrive in fragment order).  Blocks 0,1 are 64
+    // gate columns of this half, blocks 2,3 the matching up columns.
     const int half = warp >> 2;
     const int quarter = warp & 3;
     const int tid = threadIdx.x;
@@ -446,7 +451,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
 
         // SwiGLU on the rounded gate/up values.  h[r][8b + 2i] and h[r][8b + 2i + 1] are channels
-        // half*64 + 32b + 8i + quad and +4 of this sub-tile's 128.
+        // half*64 + 32b + 8*quad + 2i and +1 of this sub-tile's 128.
         // gate and up are rounded to the output type first (pack_pair), so silu(gate) is a
         // lookup by the gate's 16-bit pattern in a table built with the formula itself.
         float h[4][16];
@@ -522,19 +527,14 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                   code[k] = static_cast<uint32_t>(quantize_value(v[k], scale)) & 0xffu;
               }
               int8_t* q_piece = q_row + piece * 128 + half * 64;
-              // Lane `quad` holds channels 32*b + 8i + quad and +4; after the exchange it holds the
-              // eight channels 32*b + 8*quad .. +7, the first four in the low bytes.
+              // Lane `quad` holds the eight channels 32*b + 8*quad .. +7.
+              if (row_stored) {
 #pragma unroll
-              for (int b = 0; b < 2; ++b) {
-                uint32_t w[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = code[b * 8 + 2 * i] | (code[b * 8 + 2 * i + 1] << 8);
-                quad_transpose(w, quad);
-                if (row_stored) {
-                  const uint32_t front = __byte_perm(w[0], w[1], 0x5140);
-                  const uint32_t back = __byte_perm(w[2], w[3], 0x5140);
+                for (int b = 0; b < 2; ++b) {
+                  const uint32_t* w = code + b * 8;
                   *reinterpret_cast<uint2*>(q_piece + b * 32 + 8 * quad) =
-                      make_uint2(__byte_perm(front, back, 0x5410), __byte_perm(front, back, 0x7632));
+                      make_uint2(w[0] | (w[1] << 8) | (w[2] << 16) | (w[3] << 24),
+                                 w[4] | (w[5] << 8) | (w[6] << 16) | (w[7] << 24));
                 }
               }
             }
