@@ -312,6 +312,22 @@ static GemmSimtParams simt_params(const GemmArgs& g) {
   return p;
 }
 
+// Clusters of this launch that are resident at once, at most `most`; asked once per device.
+template <typename Kernel>
+static int resident_clusters(Kernel kernel, const cudaLaunchConfig_t& config, int (&cached)[64], int most) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return most;
+  if (cached[device] == 0) {
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess || clusters <= 0) {
+      (void)cudaGetLastError();
+      clusters = most;
+    }
+    cached[device] = clusters;
+  }
+  return cached[device] < most ? cached[device] : most;
+}
+
 template <int kCtaGroup, int BN, int kStages, typename OutT, bool kGrouped, int kPromoWarps,
           int kARows = 128>
 static int launch_tc_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b,
@@ -343,17 +359,7 @@ static int launch_tc_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b,
   int workers_max = sm_count() / kCtaGroup;
   if constexpr (kCtaGroup > 1) {
     static int cached[64] = {0};
-    int device = 0;
-    if (cudaGetDevice(&device) == cudaSuccess && device >= 0 && device < 64) {
-      if (cached[device] == 0) {
-        int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess || clusters <= 0) {
-          clusters = workers_max;
-        }
-        cached[device] = clusters;
-      }
-      if (cached[device] < workers_max) workers_max = cached[device];
-    }
+    workers_max = resident_clusters(kernel, config, cached, workers_max);
   }
   const long long tiles = static_cast<long long>(p.tiles_m) * p.tiles_n;
   const int workers = static_cast<int>(tiles < workers_max ? tiles : workers_max);
@@ -514,15 +520,68 @@ static int launch_quantize(const InT* x, long long rows, int width, int group, l
   return launch(quantize_rows_kernel<InT, 1>, grid, 256, 0, stream, x, rows, width, group, q, s);
 }
 
-template <typename RoundT, bool kGather>
-static int launch_gate_up_tc(const CUtensorMap& map_x, const CUtensorMap& map_gate,
-                             const CUtensorMap& map_up, const GateUpParams& p, int grid, cudaStream_t stream) {
-  auto kernel = moe_gate_up_tc_kernel<RoundT, kGather>;
+template <typename RoundT, bool kGather, bool kPair>
+static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& map_gate,
+                                 const CUtensorMap& map_up, const GateUpParams& p, long long items,
+                                 cudaStream_t stream) {
+  auto kernel = moe_gate_up_tc_kernel<RoundT, kGather, kPair>;
   const cudaError_t error = cudaFuncSetAttribute(
       kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GateUpShape::kSmemBytes);
   if (error != cudaSuccess) return static_cast<int>(error);
-  kernel<<<grid, 384, GateUpShape::kSmemBytes, stream>>>(map_x, map_gate, map_up, p);
-  return static_cast<int>(cudaGetLastError());
+  constexpr int kCtas = kPair ? 2 : 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(sm_count() / kCtas * kCtas);
+  config.blockDim = dim3(384);
+  config.dynamicSmemBytes = GateUpShape::kSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = kCtas;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  int workers = sm_count() / kCtas;
+  if constexpr (kPair) {
+    static int cached[64] = {0};   // pairs that are resident at once: immutable per device
+    workers = resident_clusters(kernel, config, cached, workers);
+  }
+  if (items < workers) workers = static_cast<int>(items);
+  config.gridDim = dim3(workers * kCtas);
+  return static_cast<int>(cudaLaunchKernelEx(&config, kernel, map_x, map_gate, map_up, p));
+}
+
+// Whole items go to single CTAs, or half an item to each CTA of a pair.  A pair finishes in half the
+// time but exchanges row maxima between its CTAs (4 % of an item), so it pays where whole items
+// fill their last wave badly: `tiles` (an estimate; the exact number is on the device) times the
+// channel groups, over the SMs.  Measured, Gate/Up with the rest of the call, single against pair:
+// 1 token over 8 of 128 experts (24 items) 52 and 46 us, 8 tokens, H = 4096, I = 14336, 8 experts
+// (448 items, 4 against 3.5 waves) 260 and 251 us, 256 tokens, I = 1536, 32 experts (192 items,
+// 2 against 1.5) 184 and 170 us, but 512 tokens, I = 768, 128 experts (384 items, 3 waves either
+// way) 176 and 188 us.
+static bool gate_up_pairs(long long tiles, int channel_groups) {
+  const long long items = tiles * channel_groups;
+  const int sms = sm_count(), pairs = sms / 2;
+  const long long single_waves = (items + sms - 1) / sms, pair_waves = (items + pairs - 1) / pairs;
+  return pair_waves * 52 < single_waves * 100;
+}
+
+template <typename RoundT>
+static int launch_gate_up_tc(const CUtensorMap& map_x, const CUtensorMap& map_gate,
+                             const CUtensorMap& map_up, const GateUpParams& p, long long slots, int experts,
+                             bool row_gather, cudaStream_t stream) {
+  // Row tiles in use: bounded by the list and by the slots; estimated as one per expert while an
+  // expert has few rows, as full tiles and half a tile of remainder per expert beyond.
+  const int channel_groups = p.intermediate / 256;
+  const long long bound = slots < p.max_tiles ? slots : p.max_tiles;
+  const long long spread = slots < experts ? slots : experts;
+  const long long estimate = slots <= 64ll * experts ? spread : slots / 128 + experts / 2;
+  const long long items = bound * channel_groups;
+  if (row_gather) return launch_gate_up_kernel<RoundT, true, false>(map_x, map_gate, map_up, p, items, stream);
+  if (gate_up_pairs(estimate, channel_groups)) {
+    return launch_gate_up_kernel<RoundT, false, true>(map_x, map_gate, map_up, p, items, stream);
+  }
+  return launch_gate_up_kernel<RoundT, false, false>(map_x, map_gate, map_up, p, items, stream);
 }
 
 // One warp waits, with the kernels' own bounded wait, on a barrier that nothing ever
@@ -859,18 +918,10 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     p.hidden = hidden; p.intermediate = intermediate;
     p.max_tiles = tile_capacity; p.interleaved = interleaved;
     p.sw_vectors = !interleaved && gg::aligned16(scale_w1);
-    const long long items = static_cast<long long>(tile_capacity) * (intermediate / 256);
-    const int grid = static_cast<int>(items < gg::sm_count() ? items : gg::sm_count());
-    if (row_gather) {
-      if (out_dtype == GG_OUT_BF16) {
-        return gg::launch_gate_up_tc<__nv_bfloat16, true>(map_x, map_gate, map_up, p, grid, stream);
-      }
-      return gg::launch_gate_up_tc<__half, true>(map_x, map_gate, map_up, p, grid, stream);
-    }
     if (out_dtype == GG_OUT_BF16) {
-      return gg::launch_gate_up_tc<__nv_bfloat16, false>(map_x, map_gate, map_up, p, grid, stream);
+      return gg::launch_gate_up_tc<__nv_bfloat16>(map_x, map_gate, map_up, p, slots, experts, row_gather, stream);
     }
-    return gg::launch_gate_up_tc<__half, false>(map_x, map_gate, map_up, p, grid, stream);
+    return gg::launch_gate_up_tc<__half>(map_x, map_gate, map_up, p, slots, experts, row_gather, stream);
   }
   if (tile_rows != gg::kSimtTile || !gate_up_scratch) return static_cast<int>(cudaErrorInvalidValue);
   // CUDA-core path: ragged gathered GEMM into the scratch matrix, then SwiGLU + requantisation.
@@ -930,7 +981,11 @@ int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_
     CUtensorMap map_a, map_b;
     int status = gg::encode_int8_rows(&map_a, q, assignments, intermediate, intermediate, 128);
     if (status) return status;
-    const int bn = hidden >= 256 ? 256 : hidden >= 128 ? 128 : 64;
+    // Narrower column tiles as long as all tiles still fit one wave (a layer of one token has a
+    // handful of row tiles and would leave most SMs idle); slots bound the row tiles in use.
+    const long long used_tiles = assignments < tile_capacity ? assignments : tile_capacity;
+    int bn = hidden >= 256 ? 256 : hidden >= 128 ? 128 : 64;
+    while (bn > 64 && used_tiles * ((hidden + bn / 2 - 1) / (bn / 2)) <= gg::sm_count()) bn /= 2;
     const bool permuted = hidden % 32 == 0;
     status = gg::weight_row_map(&map_b, w2, static_cast<long long>(experts) * hidden, intermediate,
                                 intermediate, bn, permuted);

@@ -16,13 +16,20 @@
 // whole box), so it is what the Python layer picks by default.
 //
 // Work item = (128-row tile of one expert, 256-channel group), processed as two sub-tiles of
-// 128 channels; a sub-tile is one N = 256 accumulator (128 gate + 128 up columns) in TMEM.
+// 128 channels, one after the other or by a pair of CTAs; a sub-tile is one N = 256 accumulator
+// (128 gate + 128 up columns) in TMEM.
 //   warp 8    TMA producer: per stage the activation rows (one box, or 32 row gathers) and two weight boxes
 //   warp 9    MMA issuer (tcgen05.mma kind::i8, two TMEM buffers)
 //   warp 10   scale staging (cp.async of each K group's column and row scales into a shared-memory ring)
 //   warps 0-7 promotion per K group, then SwiGLU (silu by table lookup); the first sub-tile's h
 //             is parked in shared memory until the second sub-tile supplies the other half of
 //             the row maximum.
+// What bounds it: for many rows the promotion warps' issue slots (see gemm_tc.cuh; the same loop
+// took 4096 tokens over 8 experts, H = 4096, I = 14336, from 996 to 886 us and 16384 tokens over
+// 256 experts, H = 7168, I = 2048, from 4650 to 4270 us), for few rows the weights' way from HBM:
+// 16 tokens over 8 experts read 0.94 GB in 195 us (4.8 TB/s), held back by the last wave of items
+// (see gate_up_pairs in abi.cu), one token over 8 of 128 experts 25 MB in 19 us, 34 with whole
+// items on 24 CTAs.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -60,7 +67,7 @@ struct GateUpShape {
   static constexpr int kScaleChunks = kScaleSlots / kScaleChunkGroups;
   static constexpr int kScaleBytes = kScaleSlots * kRingFloats * 4;
   static constexpr int kAmaxBytes = 2 * 4 * 128 * 4;   // two item parities x (sub, half) x 128 rows
-  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks) * 8 + 16;
+  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks + 8) * 8 + 16;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStashBytes + kScaleBytes +
                                     kAmaxBytes + kBarrierBytes;
 };
@@ -108,7 +115,11 @@ __device__ __forceinline__ int gate_up_source_row(const GateUpParams& p, int row
 // other row (twice the row pitch, map_up starting one row later), so that the accumulator has
 // 128 gate columns and then 128 up columns in either case and nothing behind the loads
 // depends on the layout.
-template <typename RoundT, bool kGather>
+//
+// kPair: a work item goes to a cluster of two CTAs, one sub-tile each, which exchange their row
+// maxima through distributed shared memory instead of parking the first sub-tile's h.  For calls
+// with so few items that whole items leave SMs idle: see the rule at the launch.
+template <typename RoundT, bool kGather, bool kPair>
 __global__ void __launch_bounds__(384, 1)
 moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                       const __grid_constant__ CUtensorMap map_gate,
@@ -131,7 +142,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint64_t* scale_full_bar = tmem_empty_bar + 2;
   uint64_t* scale_empty_bar = scale_full_bar + Shape::kScaleChunks;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(scale_empty_bar + Shape::kScaleChunks);
+  uint64_t* amax_bar = scale_empty_bar + Shape::kScaleChunks;   // kPair: [item parity][lane quarter]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(amax_bar + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   // The same in every lane, and known to be: addresses built from it stay in uniform registers.
@@ -154,6 +166,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       mbar_init(&scale_full_bar[i], 32);   // every lane of the scale warp
       mbar_init(&scale_empty_bar[i], 8);   // one arrival per promotion warp
     }
+    for (int i = 0; i < 8; ++i) mbar_init(&amax_bar[i], 4);   // two warps of each CTA
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -178,9 +191,15 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   if (warp == 9) tmem_alloc<1>(tmem_holder, 512);
   tcgen05_fence_before();
   __syncthreads();
+  if constexpr (kPair) cluster_sync_all();   // the peer's barriers exist from here on
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   const int total_items = used_row_tiles * channel_groups;
+  const uint32_t cta_rank = kPair ? cluster_ctarank() : 0u;
+  const int first_item = kPair ? blockIdx.x / 2 : blockIdx.x;
+  const int item_step = kPair ? gridDim.x / 2 : gridDim.x;
+  const int sub_begin = kPair ? static_cast<int>(cta_rank) : 0;
+  const int sub_end = kPair ? sub_begin + 1 : 2;
 
   // Warps 8-11 (producer, MMA issuer, two spares) give registers to the promotion warps.
   if (warp >= 8) {
@@ -193,7 +212,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       const bool leader = elect_one();
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+      for (int item = first_item; item < total_items && ok; item += item_step) {
         int tile, jg, expert;
         if (!gate_up_item(p, item, channel_groups, tile, jg, expert)) continue;
         const int row0 = p.tile_row[tile];
@@ -203,7 +222,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 #pragma unroll
           for (int i = 0; i < 4; ++i) source[i] = gate_up_source_row(p, row0 + 4 * lane + i, row_end);
         }
-        for (int sub = 0; sub < 2 && ok; ++sub) {
+        for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
           const int channel0 = jg * 256 + sub * 128;
           const int row_gate = expert * (p.interleaved ? 1 : 2) * p.intermediate + channel0;
           const int row_up = p.interleaved ? row_gate : row_gate + p.intermediate;
@@ -246,7 +265,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       const uint32_t ring_base = smem_u32(sb_ring);
       const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale
       const int sb_step = p.interleaved ? 64 : 32;                // 32 channels further
-      for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+      for (int item = first_item; item < total_items && ok; item += item_step) {
         int tile, jg, expert;
         if (!gate_up_item(p, item, channel_groups, tile, jg, expert)) continue;
         const int row0 = p.tile_row[tile];
@@ -261,7 +280,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           const long long source_row = kGather ? gate_up_source_row(p, r, row_end) : (sa_valid[i] ? r : 0);
           sa_source[i] = p.row_scale + source_row * groups;
         }
-        for (int sub = 0; sub < 2 && ok; ++sub) {
+        for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
           const int channel = jg * 256 + sub * 128 + (p.sw_vectors ? 4 * lane : lane);
           const float* sb_source = sb_base + (p.interleaved ? 2 * channel : channel);
           for (int g = 0; g < groups; g += kScaleChunkGroups) {
@@ -311,9 +330,9 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       uint32_t stage = 0, phase = 0;
       uint32_t buffer = 0, empty_parity = 1;
       bool ok = true;
-      for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+      for (int item = first_item; item < total_items && ok; item += item_step) {
         if (p.tile_expert[item / channel_groups] < 0) continue;
-        for (int sub = 0; sub < 2 && ok; ++sub) {
+        for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
           for (int slab = 0; slab < slabs; ++slab) {
             if (!mbar_wait_warp(&full_bar[stage], phase, kSiteMmaFull, abort_flag)) {
               ok = false;
@@ -374,10 +393,10 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     // next: a warp may start the next item (and write its sub-tile 0 maxima) while its partner
     // half is still reading this item's; the barrier of the next item keeps it from getting
     // two items ahead.
-    uint32_t item_parity = 0;
+    uint32_t item_parity = 0, item_phase = 0;
     // First accumulator column of block b: gate columns of this half, then the up columns.
     const auto block_column = [half](int b) { return half * 64 + 32 * (b & 1) + (b < 2 ? 0 : 128); };
-    for (int item = blockIdx.x; item < total_items; item += gridDim.x) {
+    for (int item = first_item; item < total_items; item += item_step) {
       int tile, jg, expert;
       if (!gate_up_item(p, item, channel_groups, tile, jg, expert)) continue;
       const int row0 = p.tile_row[tile];
@@ -385,7 +404,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       const int first_row = row0 + quarter * 32 + fragment_row;   // + 8r
       float amax_first[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 
-      for (int sub = 0; sub < 2; ++sub) {
+      for (int sub = sub_begin; sub < sub_end; ++sub) {
         float2 acc[4][16];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -476,10 +495,12 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           row_amax = fmaxf(row_amax, __shfl_xor_sync(0xffffffffu, row_amax, 2));
           amax[r] = row_amax;
           if (quad == 0) {
-            amax_part[((item_parity * 2 + sub) * 2 + half) * 128 + quarter * 32 + fragment_row + 8 * r] = row_amax;
+            float* mine = &amax_part[((item_parity * 2 + sub) * 2 + half) * 128 + quarter * 32 + fragment_row + 8 * r];
+            *mine = row_amax;
+            if constexpr (kPair) store_cluster_f32(mine, cta_rank ^ 1u, row_amax);
           }
         }
-        if (sub == 0) {
+        if (!kPair && sub == 0) {
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
 #pragma unroll
@@ -489,7 +510,22 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             amax_first[r] = amax[r];
           }
         } else {
-          named_barrier_sync(1, 256);
+          if constexpr (kPair) {
+            // The row maxima of this lane quarter from all four warps that hold its rows' channels
+            // (two here, two in the peer CTA).  A warp that has failed arrives all the same.
+            // Maxima and barriers alternate between two sets: a warp that arrives for item n + 2
+            // has seen the arrivals for n + 1, which the other warps make after their waits for
+            // n, so that neither an arrival nor a store runs ahead into a set still in use.
+            uint64_t* exchange = &amax_bar[item_parity * 4 + quarter];
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(exchange);
+              mbar_arrive_cluster_release(exchange, cta_rank ^ 1u);
+            }
+            if (ok) ok = mbar_wait_warp<true>(exchange, item_phase, kSiteDrain, abort_flag);
+          } else {
+            named_barrier_sync(1, 256);
+          }
           const bool all_ok = ok;
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
@@ -497,6 +533,9 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             float row_max = fmaxf(amax[r], amax_first[r]);
             row_max = fmaxf(row_max, amax_part[((item_parity * 2 + 0) * 2 + (half ^ 1)) * 128 + tile_row]);
             row_max = fmaxf(row_max, amax_part[((item_parity * 2 + 1) * 2 + (half ^ 1)) * 128 + tile_row]);
+            if constexpr (kPair) {
+              row_max = fmaxf(row_max, amax_part[((item_parity * 2 + (sub ^ 1)) * 2 + half) * 128 + tile_row]);
+            }
             const float scale = quantize_scale(row_max);
             const bool by_fma = quantize_division_is_safe(row_max);
             const float y = __frcp_rn(scale);
@@ -504,8 +543,9 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const bool row_stored = all_ok && row < row_end;
             int8_t* q_row = p.q + static_cast<long long>(row) * p.intermediate + jg * 256;
 #pragma unroll
-            for (int piece = 0; piece < 2; ++piece) {
-              // piece 0: parked first sub-tile (channels 0..127), piece 1: registers.
+            for (int piece = kPair ? 1 : 0; piece < 2; ++piece) {
+              // piece 0: parked first sub-tile (channels 0..127), piece 1: registers (with kPair
+              // this CTA's only sub-tile).
               float v[16];
 #pragma unroll
               for (int k = 0; k < 16; k += 4) {
@@ -526,7 +566,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 for (int k = 0; k < 16; ++k)
                   code[k] = static_cast<uint32_t>(quantize_value(v[k], scale)) & 0xffu;
               }
-              int8_t* q_piece = q_row + piece * 128 + half * 64;
+              int8_t* q_piece = q_row + (kPair ? sub : piece) * 128 + half * 64;
               // Lane `quad` holds the eight channels 32*b + 8*quad .. +7.
               if (row_stored) {
 #pragma unroll
@@ -538,18 +578,20 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 }
               }
             }
-            if (row_stored && half == 0 && quad == 0) {
+            if (row_stored && half == 0 && quad == 0 && (!kPair || sub == 0)) {
               p.s[static_cast<long long>(row) * channel_groups + jg] = scale;
             }
           }
         }
       }
       item_parity ^= 1u;
+      if (item_parity == 0) item_phase ^= 1u;
     }
   }
 
   tcgen05_fence_before();
   __syncthreads();
+  if constexpr (kPair) cluster_sync_all();   // no CTA leaves while its peer may still write here
   if (warp == 9) tmem_dealloc<1>(tmem_base, 512);
 }
 

@@ -104,6 +104,29 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t cta)
       : "memory");
 }
 
+// The same with release semantics at cluster scope: stores to that CTA's shared memory that this
+// warp made before are visible to a thread that acquires the phase at cluster scope.
+__device__ __forceinline__ void mbar_arrive_cluster_release(uint64_t* bar, uint32_t cta) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remote];\n\t"
+      "}" ::"r"(smem_u32(bar)), "r"(cta)
+      : "memory");
+}
+
+// Store to the same shared-memory offset in CTA `cta` of the cluster.
+__device__ __forceinline__ void store_cluster_f32(float* p, uint32_t cta, float value) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
+      "st.shared::cluster.f32 [remote], %2;\n\t"
+      "}" ::"r"(smem_u32(p)), "r"(cta), "f"(value)
+      : "memory");
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                "r"(bytes)
@@ -118,18 +141,33 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;
 // issue slots.  (The form with an explicit suspension limit is not used: the compiler expands it
 // into a loop of some ten instructions around a sleep, which the other warps of the scheduler
 // pay for.)
+// kClusterScope: the probe acquires what other CTAs of the cluster released.
+template <bool kClusterScope = false>
 __device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
   uint32_t done;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p, q;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "vote.sync.all.pred q, p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t"
-      "}"
-      : "=r"(done)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
+  if constexpr (kClusterScope) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t"
+        "}"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  }
   return done != 0;
 }
 
@@ -142,12 +180,13 @@ __device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
 // A wait that finds its phase complete costs 25 cycles, against 73 with a per-lane branch into
 // the waiting loop in front of the vote (measured on one warp with the phase always complete),
 // and a wait that has to poll takes no issue slots for reconvergence.
+template <bool kClusterScope = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned int site,
                                                volatile int* abort_flag,
                                                uint64_t limit_ns = kWaitLimitNs) {
   uint64_t start = 0;
   for (uint32_t spin = 0;; ++spin) {
-    if (mbar_test_warp(bar, parity)) return true;
+    if (mbar_test_warp<kClusterScope>(bar, parity)) return true;
     if ((spin & 0xfu) == 0xfu) {
       if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
       const uint64_t now = global_timer_ns();
