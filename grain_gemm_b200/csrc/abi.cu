@@ -540,7 +540,9 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
   attribute[0].val.clusterDim.y = 1;
   attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
-  config.numAttrs = 1;
+  // No cluster attribute for single CTAs: even a cluster of one changes how they are placed (16384
+  // tokens over 256 experts 8.32 to 8.49 ms a layer, 4096 over 8 1.56 to 1.58 ms).
+  config.numAttrs = kPair ? 1 : 0;
   int workers = sm_count() / kCtas;
   if constexpr (kPair) {
     static int cached[64] = {0};   // pairs that are resident at once: immutable per device
@@ -559,7 +561,13 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
 // (448 items, 4 against 3.5 waves) 260 and 251 us, 256 tokens, I = 1536, 32 experts (192 items,
 // 2 against 1.5) 184 and 170 us, but 512 tokens, I = 768, 128 experts (384 items, 3 waves either
 // way) 176 and 188 us.
-static bool gate_up_pairs(long long tiles, int channel_groups) {
+// Row tiles are estimated as one per expert while an expert has few rows, as full tiles and half a
+// tile of remainder per expert beyond.
+// Only pairs take their weight rows in fragment order; for single CTAs, which amortise the
+// exchange over a whole item, it made no difference beyond the spread of the runs.
+static bool gate_up_pairs(long long slots, int experts, int channel_groups) {
+  const long long spread = slots < experts ? slots : experts;
+  const long long tiles = slots <= 64ll * experts ? spread : slots / 128 + experts / 2;
   const long long items = tiles * channel_groups;
   const int sms = sm_count(), pairs = sms / 2;
   const long long single_waves = (items + sms - 1) / sms, pair_waves = (items + pairs - 1) / pairs;
@@ -568,17 +576,12 @@ static bool gate_up_pairs(long long tiles, int channel_groups) {
 
 template <typename RoundT>
 static int launch_gate_up_tc(const CUtensorMap& map_x, const CUtensorMap& map_gate,
-                             const CUtensorMap& map_up, const GateUpParams& p, long long slots, int experts,
+                             const CUtensorMap& map_up, const GateUpParams& p, long long slots, bool pairs,
                              bool row_gather, cudaStream_t stream) {
-  // Row tiles in use: bounded by the list and by the slots; estimated as one per expert while an
-  // expert has few rows, as full tiles and half a tile of remainder per expert beyond.
-  const int channel_groups = p.intermediate / 256;
-  const long long bound = slots < p.max_tiles ? slots : p.max_tiles;
-  const long long spread = slots < experts ? slots : experts;
-  const long long estimate = slots <= 64ll * experts ? spread : slots / 128 + experts / 2;
-  const long long items = bound * channel_groups;
+  const long long bound = slots < p.max_tiles ? slots : p.max_tiles;   // row tiles in use
+  const long long items = bound * (p.intermediate / 256);
   if (row_gather) return launch_gate_up_kernel<RoundT, true, false>(map_x, map_gate, map_up, p, items, stream);
-  if (gate_up_pairs(estimate, channel_groups)) {
+  if (pairs) {
     return launch_gate_up_kernel<RoundT, false, true>(map_x, map_gate, map_up, p, items, stream);
   }
   return launch_gate_up_kernel<RoundT, false, false>(map_x, map_gate, map_up, p, items, stream);
@@ -895,15 +898,16 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
       status = gg_moe_silu_table(const_cast<float*>(p.silu_table), out_dtype, stream_ptr);
       if (status) return status;
     }
+    const bool pairs = !row_gather && gg::gate_up_pairs(slots, experts, intermediate / 256);
     const long long weight_rows = static_cast<long long>(experts) * 2 * intermediate;
     if (interleaved) {
       // Every other row: gate rows from the first, up rows from the second.
       const int8_t* rows = static_cast<const int8_t*>(w1);
-      status = gg::weight_row_map(&map_gate, rows, weight_rows / 2, hidden, 2ll * hidden, 128, true);
+      status = gg::weight_row_map(&map_gate, rows, weight_rows / 2, hidden, 2ll * hidden, 128, pairs);
       if (status) return status;
-      status = gg::weight_row_map(&map_up, rows + hidden, weight_rows / 2, hidden, 2ll * hidden, 128, true);
+      status = gg::weight_row_map(&map_up, rows + hidden, weight_rows / 2, hidden, 2ll * hidden, 128, pairs);
     } else {
-      status = gg::weight_row_map(&map_gate, w1, weight_rows, hidden, hidden, 128, true);
+      status = gg::weight_row_map(&map_gate, w1, weight_rows, hidden, hidden, 128, pairs);
       map_up = map_gate;
     }
     if (status) return status;
@@ -919,9 +923,9 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     p.max_tiles = tile_capacity; p.interleaved = interleaved;
     p.sw_vectors = !interleaved && gg::aligned16(scale_w1);
     if (out_dtype == GG_OUT_BF16) {
-      return gg::launch_gate_up_tc<__nv_bfloat16>(map_x, map_gate, map_up, p, slots, experts, row_gather, stream);
+      return gg::launch_gate_up_tc<__nv_bfloat16>(map_x, map_gate, map_up, p, slots, pairs, row_gather, stream);
     }
-    return gg::launch_gate_up_tc<__half>(map_x, map_gate, map_up, p, slots, experts, row_gather, stream);
+    return gg::launch_gate_up_tc<__half>(map_x, map_gate, map_up, p, slots, pairs, row_gather, stream);
   }
   if (tile_rows != gg::kSimtTile || !gate_up_scratch) return static_cast<int>(cudaErrorInvalidValue);
   // CUDA-core path: ragged gathered GEMM into the scratch matrix, then SwiGLU + requantisation.

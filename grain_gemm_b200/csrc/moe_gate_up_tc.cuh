@@ -236,8 +236,10 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             if (leader) {
               mbar_expect_tx(&full_bar[stage], Shape::kStageBytes);
               if constexpr (!kGather) tma_load_2d(a_dst, &map_x, &full_bar[stage], x, row0);
-              tma_load_4d(b_dst, &map_gate, &full_bar[stage], x, 0, row_gate >> 5);
-              tma_load_4d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, 0, row_up >> 5);
+              tma_load_4d(b_dst, &map_gate, &full_bar[stage], x, kPair ? 0 : row_gate,
+                          kPair ? row_gate >> 5 : 0);
+              tma_load_4d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, kPair ? 0 : row_up,
+                          kPair ? row_up >> 5 : 0);
             }
             if constexpr (kGather) {
               // Every lane fetches its four rows: 32 gathers of 512 bytes fill the A tile.
@@ -260,7 +262,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       // runs a whole ring ahead and global-memory latency stays hidden.
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
-      // Byte offset of this lane's row within a 32-float block of a ring slot.
+      // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
+      const uint32_t column_position = 4 * (kPair ? lane : ring_column_position(lane));
       const uint32_t row_position = 4 * ring_row_position(lane);
       const uint32_t ring_base = smem_u32(sb_ring);
       const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale
@@ -281,7 +284,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           sa_source[i] = p.row_scale + source_row * groups;
         }
         for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
-          const int channel = jg * 256 + sub * 128 + (p.sw_vectors ? 4 * lane : lane);
+          const int channel = jg * 256 + sub * 128 + (kPair && p.sw_vectors ? 4 * lane : lane);
           const float* sb_source = sb_base + (p.interleaved ? 2 * channel : channel);
           for (int g = 0; g < groups; g += kScaleChunkGroups) {
             if (!mbar_wait_warp(&scale_empty_bar[chunk], phase ^ 1u, kSiteScaleEmpty, abort_flag)) {
@@ -291,13 +294,13 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const int in_chunk = min(kScaleChunkGroups, groups - g);
             uint32_t destination = ring_base + chunk * (kScaleChunkGroups * Shape::kRingFloats * 4);
             for (int i = 0; i < in_chunk; ++i) {
-              if (p.sw_vectors) {
+              if (kPair && p.sw_vectors) {
                 cp_async_f32x4(destination + 16 * lane, sb_source, true);
                 cp_async_f32x4(destination + 512 + 16 * lane, sb_source + up_offset, true);
               } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                  cp_async_f32(destination + 128 * j + 4 * lane,
+                  cp_async_f32(destination + 128 * j + column_position,
                                sb_source + (j & 3) * sb_step + (j < 4 ? 0 : up_offset), true);
                 }
               }
@@ -377,9 +380,9 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     // ------------------------------------------------------------ promotion + SwiGLU warps
     // Fragment layout (tmem_ld_16x128b_x8): warp (quarter, half) drains TMEM lanes
     // 32*quarter.. of four 32-column blocks; a thread owns tile rows
-    // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, the channel pairs
-    // 8*(lane%4) + 2i, +1 (i = 0..3; the weight rows arrive in fragment order).  Blocks 0,1 are 64
-    // gate columns of this half, blocks 2,3 the matching up columns.
+    // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, four channel pairs i: with kPair
+    // 8*(lane%4) + 2i, +1 (the weight rows arrive in fragment order), else 8i + lane%4, +4.  Blocks
+    // 0,1 are 64 gate columns of this half, blocks 2,3 the matching up columns.
     const int half = warp >> 2;
     const int quarter = warp & 3;
     const int tid = threadIdx.x;
@@ -470,7 +473,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
 
         // SwiGLU on the rounded gate/up values.  h[r][8b + 2i] and h[r][8b + 2i + 1] are channels
-        // half*64 + 32b + 8*quad + 2i and +1 of this sub-tile's 128.
+        // half*64 + 32b + 8*quad + 2i and +1 of this sub-tile's 128 (kPair), else
+        // half*64 + 32b + 8i + quad and +4.
         // gate and up are rounded to the output type first (pack_pair), so silu(gate) is a
         // lookup by the gate's 16-bit pattern in a table built with the formula itself.
         float h[4][16];
@@ -567,15 +571,23 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                   code[k] = static_cast<uint32_t>(quantize_value(v[k], scale)) & 0xffu;
               }
               int8_t* q_piece = q_row + (kPair ? sub : piece) * 128 + half * 64;
-              // Lane `quad` holds the eight channels 32*b + 8*quad .. +7.
-              if (row_stored) {
+              // Lane `quad` stores the eight channels 32*b + 8*quad .. +7: with kPair it holds them,
+              // else an exchange inside the quad brings them, the first four in the low bytes.
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                  const uint32_t* w = code + b * 8;
-                  *reinterpret_cast<uint2*>(q_piece + b * 32 + 8 * quad) =
-                      make_uint2(w[0] | (w[1] << 8) | (w[2] << 16) | (w[3] << 24),
-                                 w[4] | (w[5] << 8) | (w[6] << 16) | (w[7] << 24));
+              for (int b = 0; b < 2; ++b) {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = code[b * 8 + 2 * i] | (code[b * 8 + 2 * i + 1] << 8);
+                uint2 packed;
+                if constexpr (kPair) {
+                  packed = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+                } else {
+                  quad_transpose(w, quad);
+                  const uint32_t front = __byte_perm(w[0], w[1], 0x5140);
+                  const uint32_t back = __byte_perm(w[2], w[3], 0x5140);
+                  packed = make_uint2(__byte_perm(front, back, 0x5410), __byte_perm(front, back, 0x7632));
                 }
+                if (row_stored) *reinterpret_cast<uint2*>(q_piece + b * 32 + 8 * quad) = packed;
               }
             }
             if (row_stored && half == 0 && quad == 0 && (!kPair || sub == 0)) {
