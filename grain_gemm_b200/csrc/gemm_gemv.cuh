@@ -37,9 +37,10 @@ struct GemvParams {
   int columns_per_warp;     // 1 .. kGemvMaxColumnsPerWarp; a CTA owns 8 times as many columns
 };
 
-__device__ __forceinline__ uint4 ldg_stream_16(const void* address) {
+// 16 bytes of the weights, read once.  Volatile, so it stays behind previous_kernel_done().
+__device__ __forceinline__ uint4 ld_stream_16(const void* address) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(address));
   return v;
@@ -65,7 +66,7 @@ __device__ __forceinline__ void gemv_step(const GemvParams& p, const uint4& w, i
   for (int r = 0; r < kRows; ++r) {
     // Rows at or beyond M repeat the last row (their results are never stored).
     const int row = r < p.m ? r : p.m - 1;
-    const uint4 x = __ldg(reinterpret_cast<const uint4*>(p.a + static_cast<long long>(row) * p.a_sm + offset));
+    const uint4 x = *reinterpret_cast<const uint4*>(p.a + static_cast<long long>(row) * p.a_sm + offset);
     sum[r] = valid ? dot16(w, x) : 0;
   }
 #pragma unroll
@@ -101,7 +102,7 @@ __global__ void __launch_bounds__(kGemvThreads, kRows <= 2 ? 4 : 2) gemm_gemv_ke
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int chunk = j * 32 + lane;
-    w[j] = blocks > 0 && chunk < chunks ? ldg_stream_16(weights + (static_cast<long long>(chunk) << 4))
+    w[j] = blocks > 0 && chunk < chunks ? ld_stream_16(weights + (static_cast<long long>(chunk) << 4))
                                         : make_uint4(0u, 0u, 0u, 0u);
   }
 
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(kGemvThreads, kRows <= 2 ? 4 : 2) gemm_gemv_ke
       // The register is free again: its next load goes out at once, so that eight loads stay
       // in flight per lane throughout.
       const int chunk = next_base + j * 32;
-      w[j] = more && chunk < chunks ? ldg_stream_16(next + (static_cast<long long>(chunk) << 4))
+      w[j] = more && chunk < chunks ? ld_stream_16(next + (static_cast<long long>(chunk) << 4))
                                     : make_uint4(0u, 0u, 0u, 0u);
     }
   }

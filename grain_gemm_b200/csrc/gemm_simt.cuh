@@ -162,9 +162,8 @@ gemm_simt_kernel(const GemmSimtParams p) {
 // order, C[m,n] = cast(fold_g fmaf(float(p_g), sa[m,g]*sb[g,n], total)); one thread per output.
 template <typename OutT>
 __global__ void __launch_bounds__(256)
-fold_partials_kernel(const int* __restrict__ partials, const float* __restrict__ scale_a,
-                     const float* __restrict__ scale_b, OutT* __restrict__ c, int m, int n,
-                     int groups, long long sa_sm, long long sa_sg, long long sb_sg, long long sb_sn,
+fold_partials_kernel(const int* partials, const float* scale_a, const float* scale_b, OutT* c, int m,
+                     int n, int groups, long long sa_sm, long long sa_sg, long long sb_sg, long long sb_sn,
                      long long ldc) {
   dependents_may_launch();
   previous_kernel_done();

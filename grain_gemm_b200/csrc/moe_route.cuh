@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kRouteChunk) route_place_kernel(const RoutePar
 // the host at the same time still learns the values as soon as the producing kernel is done,
 // and the stream does not wait for the copy engine either.
 __global__ void __launch_bounds__(32)
-report_to_host_kernel(const int* __restrict__ values, int count, int* host_words) {
+report_to_host_kernel(const int* values, int count, int* host_words) {
   dependents_may_launch();
   previous_kernel_done();
   for (int i = threadIdx.x; i < count; i += 32) host_words[i] = values[i];
@@ -362,8 +362,8 @@ report_to_host_kernel(const int* __restrict__ values, int count, int* host_words
 // entries get expert -1.  One CTA: a block-wide exclusive scan of the experts' tile counts,
 // 1024 experts at a time.
 __global__ void __launch_bounds__(1024)
-moe_tiles_kernel(const int* __restrict__ offsets, int experts, int tile_rows, int max_tiles,
-                 int* __restrict__ tile_expert, int* __restrict__ tile_row) {
+moe_tiles_kernel(const int* offsets, int experts, int tile_rows, int max_tiles, int* tile_expert,
+                 int* tile_row) {
   dependents_may_launch();
   previous_kernel_done();
   __shared__ int warp_total[32];
@@ -424,7 +424,7 @@ __device__ __forceinline__ float silu_of_bits(int bits, int half_output) {
 }
 
 __global__ void __launch_bounds__(256)
-silu_table_kernel(float* __restrict__ silu_table, int half_output) {
+silu_table_kernel(float* silu_table, int half_output) {
   dependents_may_launch();
   previous_kernel_done();
   const int bits = blockIdx.x * 256 + threadIdx.x;
@@ -443,11 +443,9 @@ silu_table_kernel(float* __restrict__ silu_table, int half_output) {
 constexpr int kSiluBlocks = 64;
 
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const int8_t* __restrict__ x, const float* __restrict__ scale_x,
-                   const long long* __restrict__ order, const int* __restrict__ offsets,
-                   int experts, int top_k, int hidden, int8_t* __restrict__ sorted_x,
-                   float* __restrict__ sorted_scale, float* __restrict__ silu_table,
-                   int half_output) {
+gather_rows_kernel(const int8_t* x, const float* scale_x, const long long* order, const int* offsets,
+                   int experts, int top_k, int hidden, int8_t* sorted_x, float* sorted_scale,
+                   float* silu_table, int half_output) {
   dependents_may_launch();
   previous_kernel_done();
   const int valid = offsets[experts];
@@ -466,7 +464,7 @@ gather_rows_kernel(const int8_t* __restrict__ x, const float* __restrict__ scale
       uint4 held[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        if (i + 32 * j < vectors) held[j] = __ldg(source + i + 32 * j);
+        if (i + 32 * j < vectors) held[j] = source[i + 32 * j];
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -532,10 +530,8 @@ __device__ __forceinline__ int quantize_value_by_fma(float h, float scale, float
 // it to the caller: benchmarks/bench_moe_ffn.py:283-285, docs/moe_ffn.md:5-7).  One warp per
 // token; expert e lives in lane e % 32, slot e / 32 (E <= 1024).  Logits must be finite.
 template <typename InT>
-__device__ __forceinline__ void router_topk_token(const InT* __restrict__ row, int experts, int top_k,
-                                                  float* __restrict__ weights,
-                                                  void* __restrict__ ids, int ids_are_i64,
-                                                  long long token, int lane) {
+__device__ __forceinline__ void router_topk_token(const InT* row, int experts, int top_k, float* weights,
+                                                  void* ids, int ids_are_i64, long long token, int lane) {
   constexpr float kLowest = -3.402823466e+38f;
   float value[32];
 #pragma unroll
@@ -597,8 +593,8 @@ __device__ __forceinline__ void router_topk_token(const InT* __restrict__ row, i
 
 template <typename InT>
 __global__ void __launch_bounds__(256)
-router_topk_kernel(const InT* __restrict__ logits, int tokens, int experts, int top_k,
-                   float* __restrict__ weights, void* __restrict__ ids, int ids_are_i64) {
+router_topk_kernel(const InT* logits, int tokens, int experts, int top_k, float* weights, void* ids,
+                   int ids_are_i64) {
   dependents_may_launch();
   previous_kernel_done();
   const int lane = threadIdx.x & 31;
@@ -615,8 +611,7 @@ router_topk_kernel(const InT* __restrict__ logits, int tokens, int experts, int 
 // the input of the second.
 template <typename InT>
 __global__ void __launch_bounds__(kRouteChunk)
-route_topk_single_kernel(const InT* __restrict__ logits, float* __restrict__ weights,
-                         const RouteParams p) {
+route_topk_single_kernel(const InT* logits, float* weights, const RouteParams p) {
   dependents_may_launch();
   previous_kernel_done();
   extern __shared__ int bins[];  // [E + 2]
@@ -640,8 +635,7 @@ route_topk_single_kernel(const InT* __restrict__ logits, float* __restrict__ wei
 // BF16 values took 190 us, 1.9 TB/s.
 template <typename InT, int kItems>
 __global__ void __launch_bounds__(256)
-quantize_rows_kernel(const InT* __restrict__ x, long long rows, int width, int group,
-                     int8_t* __restrict__ q, float* __restrict__ s) {
+quantize_rows_kernel(const InT* x, long long rows, int width, int group, int8_t* q, float* s) {
   dependents_may_launch();
   previous_kernel_done();
   const int lane = threadIdx.x & 31;
@@ -656,7 +650,7 @@ quantize_rows_kernel(const InT* __restrict__ x, long long rows, int width, int g
     if (first + i < items) {
       const uint4* source = reinterpret_cast<const uint4*>(x + (first + i) * 256 + lane * 8);
 #pragma unroll
-      for (int w = 0; w < kWords; ++w) raw[i][w] = __ldg(source + w);
+      for (int w = 0; w < kWords; ++w) raw[i][w] = source[w];
     }
   }
 #pragma unroll
@@ -741,9 +735,8 @@ swiglu_quantize_kernel(const InT* __restrict__ gate_up, long long rows,
 // One CTA per token, 8 columns per thread per step.
 template <typename T>
 __global__ void __launch_bounds__(256)
-combine_kernel(const T* __restrict__ expert_out, const float* __restrict__ weights,
-               const int* __restrict__ inverse, T* __restrict__ out, int top_k, int hidden,
-               int vector_ok) {
+combine_kernel(const T* expert_out, const float* weights, const int* inverse, T* out, int top_k,
+               int hidden, int vector_ok) {
   dependents_may_launch();
   previous_kernel_done();
   extern __shared__ int slot_smem[];  // [R] slots then [R] weights

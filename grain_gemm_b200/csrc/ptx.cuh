@@ -66,11 +66,16 @@ __device__ __forceinline__ bool elect_one() {
 // ---------------------------------------------------------------- programmatic launches
 
 // The kernels of the call chains are launched with programmatic stream serialisation (the two
-// grouped tensor-core kernels excepted): their blocks may become resident while the previous kernel of the stream still runs, and do their set-up
-// there.  dependents_may_launch() lets the NEXT kernel do the same; previous_kernel_done() returns
-// when the previous kernel has completed and its writes are visible, and stands before the first
-// access to global memory, reads included (nothing is known about who wrote the operands).
+// grouped tensor-core kernels excepted): their blocks may become resident while the previous
+// kernel of the stream still runs, and do their set-up there.  dependents_may_launch() lets the
+// NEXT kernel do the same; previous_kernel_done() returns when the previous kernel has completed
+// and its writes are visible, and stands before the first access to global memory, reads included
+// (nothing is known about who wrote the operands).
 // Since every kernel waits for its predecessor, a completed kernel implies all earlier ones.
+// What such a kernel reads may be written after its blocks have started, so it reads with
+// ordinary loads: no __ldg, no ld.global.nc, and no __restrict__ pointer, from which the compiler
+// makes the same.  The read-only path is defined only for memory that stays constant from a
+// kernel's start to its end, and neither the wait nor its memory clobber orders it.
 __device__ __forceinline__ void dependents_may_launch() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
