@@ -97,14 +97,27 @@ def host():
     """The native host path (``csrc/host.cpp``) bound to the library's entry points.
 
     Its functions run a public call whose arguments are what the documentation asks for and
-    return ``None`` for every other call, which then takes the Python path."""
+    return ``None`` for every other call, which then takes the Python path.  A host path that
+    is absent, built for another torch or Python, or that does not load is a ``RuntimeError``."""
     from .gemm import _variant_table
     lib = library()
+    if not _build.host_module_is_current():
+        built, here = _build.manifest().get("host_module"), _build.host_environment()
+        differs = ([f"{key} {built.get(key)}, not {value}" for key, value in here.items()
+                    if built.get(key) != value] if isinstance(built, dict) else [])
+        raise RuntimeError(
+            f"{_build.HOST_MODULE.name} is "
+            + (f"built for {'; '.join(differs)}" if differs else "not built")
+            + "; rebuild with `python -m grain_gemm_b200.build`")
     loader = importlib.machinery.ExtensionFileLoader("grain_gemm_b200._host",
                                                      str(_build.HOST_MODULE))
-    module = importlib.util.module_from_spec(
-        importlib.util.spec_from_file_location(loader.name, loader.path, loader=loader))
-    loader.exec_module(module)
+    try:
+        module = importlib.util.module_from_spec(
+            importlib.util.spec_from_file_location(loader.name, loader.path, loader=loader))
+        loader.exec_module(module)
+    except ImportError as error:
+        raise RuntimeError(f"{_build.HOST_MODULE.name} does not load ({error}); "
+                           "rebuild with `python -m grain_gemm_b200.build`") from error
     addresses = {name: ctypes.cast(getattr(lib, name), _VOID).value for name in _SIGNATURES}
     table = {}
     for key, rows in _variant_table().items():
@@ -115,8 +128,10 @@ def host():
 
 
 def is_available():
+    """Whether public calls can run: the library and the host path load."""
     try:
         library()
+        host()
     except (OSError, RuntimeError, AttributeError):
         return False
     return True

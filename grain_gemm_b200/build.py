@@ -2,11 +2,13 @@
 public calls, against this interpreter's torch) and record what they were built from.
 
 Both are built in-tree, next to this file, together with ``build.json`` (compiler
-target, ABI version and the SHA-256 of every source file).  The loader refuses a library
-whose manifest does not match the sources beside it, the same provenance rule as the
-reference's native bridges (``src/grain_gemm/kernels/moe_gather.py:29-55`` there).
+target, ABI version, the SHA-256 of every source file and, for the host path, the torch and
+Python it was compiled against).  The loader refuses a library whose manifest does not match
+the sources beside it, the same provenance rule as the reference's native bridges
+(``src/grain_gemm/kernels/moe_gather.py:29-55`` there), and a host path built for another torch
+or Python than the running one.
 
-    python -m grain_gemm_b200.build
+    python -m grain_gemm_b200.build [--force] [--verbose]
 """
 
 from __future__ import annotations
@@ -51,15 +53,35 @@ def find_nvcc():
     raise RuntimeError("nvcc not found; set NVCC or add the CUDA toolkit to PATH")
 
 
-def is_current():
-    if not (LIBRARY.is_file() and HOST_MODULE.is_file() and MANIFEST.is_file()):
-        return False
+def manifest():
+    """What is recorded about the built files; empty when nothing readable is."""
     try:
-        manifest = json.loads(MANIFEST.read_text())
+        recorded = json.loads(MANIFEST.read_text())
     except (OSError, ValueError):
-        return False
-    return (manifest.get("abi_version") == ABI_VERSION
-            and manifest.get("source_sha256") == source_hashes())
+        return {}
+    return recorded if isinstance(recorded, dict) else {}
+
+
+def is_current():
+    """Whether the library was built from the sources beside it."""
+    recorded = manifest()
+    return (LIBRARY.is_file() and recorded.get("abi_version") == ABI_VERSION
+            and recorded.get("source_sha256") == source_hashes())
+
+
+def host_environment():
+    """What the host path's machine code depends on besides its source: it uses the layouts and
+    inline functions of torch's headers and Python's C API."""
+    import torch
+    return {"torch": str(torch.__version__), "torch_git": torch.version.git_version,
+            "cuda": torch.version.cuda, "python": sysconfig.get_config_var("SOABI"),
+            "cxx11_abi": bool(torch._C._GLIBCXX_USE_CXX11_ABI), "flags": HOST_FLAGS}
+
+
+def host_module_is_current():
+    """Whether the host path was built from these sources, for this torch and this Python."""
+    return (HOST_MODULE.is_file() and is_current()
+            and manifest().get("host_module") == host_environment())
 
 
 def _build_host_module(output):
@@ -80,8 +102,8 @@ def _build_host_module(output):
 
 
 def build_library(force=False, verbose=False):
-    """Compile the library unless an up-to-date one is already in place."""
-    if not force and is_current():
+    """Compile the library and the host path unless up-to-date ones are already in place."""
+    if not force and is_current() and host_module_is_current():
         return LIBRARY
     nvcc = find_nvcc()
     with tempfile.TemporaryDirectory(dir=PACKAGE) as scratch:
@@ -104,6 +126,7 @@ def build_library(force=False, verbose=False):
         "abi_version": ABI_VERSION,
         "flags": ARCH_FLAGS + FLAGS,
         "source_sha256": source_hashes(),
+        "host_module": host_environment(),
     }, indent=1) + "\n")
     return LIBRARY
 
