@@ -92,15 +92,28 @@ def library():
     return lib
 
 
+class _PythonPath:
+    """Stands in for the host path where the build left it out: every call is declined."""
+
+    @staticmethod
+    def _decline(*arguments):
+        return None
+
+    int8_gemm = quantize_rows = route_topk_routes = moe_ffn = _decline
+
+
 @lru_cache(maxsize=1)
 def host():
     """The native host path (``csrc/host.cpp``) bound to the library's entry points.
 
     Its functions run a public call whose arguments are what the documentation asks for and
-    return ``None`` for every other call, which then takes the Python path.  A host path that
-    is absent, built for another torch or Python, or that does not load is a ``RuntimeError``."""
+    return ``None`` for every other call, which then takes the Python path.  A build without the
+    host path answers ``None`` to every call; a host path that is absent, built for another torch
+    or Python, or that does not load is a ``RuntimeError``."""
     from .gemm import _variant_table
     lib = library()
+    if _build.library_only():
+        return _PythonPath()
     if not _build.host_module_is_current():
         built, here = _build.manifest().get("host_module"), _build.host_environment()
         differs = ([f"{key} {built.get(key)}, not {value}" for key, value in here.items()

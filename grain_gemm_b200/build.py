@@ -8,7 +8,11 @@ the sources beside it, the same provenance rule as the reference's native bridge
 (``src/grain_gemm/kernels/moe_gather.py:29-55`` there), and a host path built for another torch
 or Python than the running one.
 
-    python -m grain_gemm_b200.build [--force] [--verbose]
+The library does not depend on the host path.  ``--library-only`` builds it alone, for a binding
+of the C ABI or where torch's headers or a C++ compiler for them are missing; the public
+Python functions then run all calls through their Python path.
+
+    python -m grain_gemm_b200.build [--library-only] [--force] [--verbose]
 """
 
 from __future__ import annotations
@@ -84,6 +88,11 @@ def host_module_is_current():
             and manifest().get("host_module") == host_environment())
 
 
+def library_only():
+    """Whether the build was asked to leave the host path out."""
+    return manifest().get("host_module") is False
+
+
 def _build_host_module(output):
     """Compile the native host path against the torch of this interpreter."""
     import torch
@@ -101,10 +110,8 @@ def _build_host_module(output):
         raise RuntimeError(f"{command[0]} failed:\n{result.stdout}\n{result.stderr}")
 
 
-def build_library(force=False, verbose=False):
-    """Compile the library and the host path unless up-to-date ones are already in place."""
-    if not force and is_current() and host_module_is_current():
-        return LIBRARY
+def _build_library(verbose):
+    """Compile the library, put it in place and record it, without a host path so far."""
     nvcc = find_nvcc()
     with tempfile.TemporaryDirectory(dir=PACKAGE) as scratch:
         output = Path(scratch) / LIBRARY.name
@@ -116,21 +123,47 @@ def build_library(force=False, verbose=False):
             raise RuntimeError(f"nvcc failed:\n{result.stdout}\n{result.stderr}")
         if verbose:
             print(result.stderr)
-        host = Path(scratch) / HOST_MODULE.name
-        _build_host_module(host)
-        os.replace(host, HOST_MODULE)
         os.replace(output, LIBRARY)
-    MANIFEST.write_text(json.dumps({
+    _record({
         "architecture": "sm_100",
         "compiler_architecture": "sm_100a",
         "abi_version": ABI_VERSION,
         "flags": ARCH_FLAGS + FLAGS,
         "source_sha256": source_hashes(),
-        "host_module": host_environment(),
-    }, indent=1) + "\n")
+    })
+
+
+def _record(values):
+    MANIFEST.write_text(json.dumps(values, indent=1) + "\n")
+
+
+def build_library(force=False, verbose=False, host_module=True):
+    """Compile the library and the host path unless up-to-date ones are already in place.
+
+    ``host_module=False`` leaves the host path out.  When only the host path cannot be built the
+    library is in place all the same, and the error says so."""
+    if force or not is_current():
+        _build_library(verbose)
+    if not host_module:
+        if not library_only():
+            _record({**manifest(), "host_module": False})
+            HOST_MODULE.unlink(missing_ok=True)
+        return LIBRARY
+    if force or not host_module_is_current():
+        with tempfile.TemporaryDirectory(dir=PACKAGE) as scratch:
+            output = Path(scratch) / HOST_MODULE.name
+            try:
+                _build_host_module(output)
+            except Exception as error:
+                raise RuntimeError(
+                    f"{LIBRARY.name} is built, the native host path is not ({error}); "
+                    "`python -m grain_gemm_b200.build --library-only` does without it") from error
+            os.replace(output, HOST_MODULE)
+        _record({**manifest(), "host_module": host_environment()})
     return LIBRARY
 
 
 if __name__ == "__main__":
-    build_library(force="--force" in sys.argv, verbose="--verbose" in sys.argv)
+    build_library(force="--force" in sys.argv, verbose="--verbose" in sys.argv,
+                  host_module="--library-only" not in sys.argv)
     print(LIBRARY)

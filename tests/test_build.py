@@ -2,6 +2,7 @@
 the torch and Python it was compiled against."""
 
 import json
+import subprocess
 
 import pytest
 import torch
@@ -21,6 +22,15 @@ def loader():
     clear()
     yield clear
     clear()
+
+
+@pytest.fixture
+def elsewhere(tmp_path, monkeypatch, loader):
+    """The built files' places in an empty folder."""
+    for name in ("LIBRARY", "HOST_MODULE", "MANIFEST"):
+        monkeypatch.setattr(build, name, tmp_path / getattr(build, name).name)
+    monkeypatch.setattr(build, "PACKAGE", tmp_path)
+    return tmp_path
 
 
 def test_the_host_path_records_what_it_was_built_for(loader):
@@ -52,3 +62,58 @@ def test_a_host_path_that_does_not_load_is_refused(loader, tmp_path, monkeypatch
     with pytest.raises(RuntimeError, match="does not load .*rebuild"):
         _loader.host()
     assert not _loader.is_available()
+
+
+def _fake_nvcc(monkeypatch):
+    commands = []
+
+    def run(command, **kwargs):
+        commands.append(command)
+        output = command[command.index("-o") + 1]
+        open(output, "wb").close()
+        return subprocess.CompletedProcess(command, 0, "", "")
+
+    monkeypatch.setattr(build.subprocess, "run", run)
+    monkeypatch.setattr(build, "find_nvcc", lambda: "/usr/local/cuda/bin/nvcc")
+    return commands
+
+
+def test_the_library_is_built_where_the_host_path_cannot_be(elsewhere, monkeypatch):
+    commands = _fake_nvcc(monkeypatch)
+
+    def without_headers(output):
+        raise RuntimeError("no such file: ATen/ATen.h")
+
+    monkeypatch.setattr(build, "_build_host_module", without_headers)
+    with pytest.raises(RuntimeError, match="libgrain_b200.so is built.*ATen.h.*--library-only"):
+        build.build_library()
+    assert build.is_current() and not build.host_module_is_current() and not build.library_only()
+    assert len(commands) == 1
+    build.build_library(host_module=False)
+    assert len(commands) == 1                      # the library was already there
+    assert build.is_current() and build.library_only()
+
+
+def test_only_the_part_that_is_out_of_date_is_built(elsewhere, monkeypatch):
+    commands = _fake_nvcc(monkeypatch)
+    build.build_library()
+    assert len(commands) == 2 and build.host_module_is_current()
+    build.build_library()
+    assert len(commands) == 2
+    recorded = build.manifest()
+    recorded["host_module"]["torch"] = "1.0.0"
+    build.MANIFEST.write_text(json.dumps(recorded))
+    build.build_library()
+    assert len(commands) == 3 and commands[2][-1] == "-ltorch_python"
+    assert build.host_module_is_current()
+
+
+def test_without_the_host_path_every_call_takes_the_python_path(loader, tmp_path, monkeypatch):
+    recorded = {**json.loads(build.MANIFEST.read_text()), "host_module": False}
+    altered = tmp_path / "build.json"
+    altered.write_text(json.dumps(recorded))
+    monkeypatch.setattr(build, "MANIFEST", altered)
+    assert _loader.is_available()
+    host = _loader.host()
+    assert host.int8_gemm(1, 2, 3) is None and host.quantize_rows(1, 2) is None
+    assert host.route_topk_routes(1) is None and host.moe_ffn() is None
