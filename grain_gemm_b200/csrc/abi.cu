@@ -24,6 +24,13 @@ constexpr int kAbiVersion = 4;
 
 // ---------------------------------------------------------------- host helpers
 
+// Status of a runtime call.  The runtime also keeps the error of a failed call for this thread until
+// somebody asks; it is taken away here, or the next good launch of this library would report it.
+static int finished(cudaError_t error) {
+  if (error != cudaSuccess) (void)cudaGetLastError();
+  return static_cast<int>(error);
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                    const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -33,8 +40,7 @@ static EncodeTiledFn encode_tiled_fn() {
   static EncodeTiledFn fn = [] {
     void* ptr = nullptr;
     cudaDriverEntryPointQueryResult query;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &query) !=
-            cudaSuccess ||
+    if (finished(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &query)) != 0 ||
         query != cudaDriverEntryPointSuccess) {
       ptr = nullptr;
     }
@@ -89,10 +95,10 @@ static int sm_count() {
   // Immutable device property, cached per device.
   static int cached[64] = {0};
   int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return 148;
+  if (finished(cudaGetDevice(&device)) != 0 || device < 0 || device >= 64) return 148;
   if (cached[device] == 0) {
     int count = 0;
-    if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+    if (finished(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device)) != 0 ||
         count <= 0) {
       count = 148;
     }
@@ -120,7 +126,7 @@ static int launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
   config.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
+  return finished(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...));
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -208,8 +214,7 @@ static int gemv_ctas_per_sm(int rows) {
     int blocks = 0;
     const cudaError_t error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &blocks, gemv_kernel(rows, 256), kGemvThreads, 4096);
-    if (error != cudaSuccess) (void)cudaGetLastError();
-    cached[index] = error == cudaSuccess && blocks > 0 ? blocks : 2;
+    cached[index] = finished(error) == 0 && blocks > 0 ? blocks : 2;
   }
   return cached[index];
 }
@@ -253,10 +258,9 @@ static int launch_gemv(const GemmArgs& g, cudaStream_t stream) {
   if (smem > 48 * 1024) {
     const cudaError_t error = cudaFuncSetAttribute(
         kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (error != cudaSuccess) return static_cast<int>(error);
+    if (error != cudaSuccess) return finished(error);
   }
-  launch(kernel, grid, kGemvThreads, smem, stream, p);
-  return static_cast<int>(cudaGetLastError());
+  return launch(kernel, grid, kGemvThreads, smem, stream, p);
 }
 
 static int select_variant(const GemmArgs& g) {
@@ -316,11 +320,10 @@ static GemmSimtParams simt_params(const GemmArgs& g) {
 template <typename Kernel>
 static int resident_clusters(Kernel kernel, const cudaLaunchConfig_t& config, int (&cached)[64], int most) {
   int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return most;
+  if (finished(cudaGetDevice(&device)) != 0 || device < 0 || device >= 64) return most;
   if (cached[device] == 0) {
     int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess || clusters <= 0) {
-      (void)cudaGetLastError();
+    if (finished(cudaOccupancyMaxActiveClusters(&clusters, kernel, &config)) != 0 || clusters <= 0) {
       clusters = most;
     }
     cached[device] = clusters;
@@ -336,7 +339,7 @@ static int launch_tc_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b,
   auto kernel = gemm_tc_kernel<kCtaGroup, BN, kStages, OutT, kGrouped, kPromoWarps, false, kARows>;
   cudaError_t error =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kSmemBytes);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return finished(error);
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(sm_count() / kCtaGroup * kCtaGroup);
   config.blockDim = dim3(Shape::kThreads);
@@ -365,8 +368,7 @@ static int launch_tc_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b,
   const int workers = static_cast<int>(tiles < workers_max ? tiles : workers_max);
   if (workers <= 0) return 0;
   config.gridDim = dim3(workers * kCtaGroup);
-  error = cudaLaunchKernelEx(&config, kernel, map_a, map_b, p);
-  return static_cast<int>(error);
+  return finished(cudaLaunchKernelEx(&config, kernel, map_a, map_b, p));
 }
 
 template <int kCtaGroup, int BN, int kStages, bool kGrouped, int kPromoWarps = 8, int kARows = 128>
@@ -447,12 +449,11 @@ static int launch_gemm_splitk(const GemmArgs& g, void* workspace, size_t workspa
   auto kernel = gemm_tc_kernel<1, 256, 6, float, false, 8, true, 32>;
   cudaError_t error =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kSmemBytes);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return finished(error);
   const int items = p.tiles_n * p.k_splits;
   const int grid = items < sm_count() ? items : sm_count();
-  launch(kernel, grid, Shape::kThreads, Shape::kSmemBytes, stream, map_a, map_b, p);
-  error = cudaGetLastError();
-  if (error != cudaSuccess) return static_cast<int>(error);
+  status = launch(kernel, grid, Shape::kThreads, Shape::kSmemBytes, stream, map_a, map_b, p);
+  if (status) return status;
   const int groups = (g.k + g.group_size - 1) / g.group_size;
   const dim3 fold_grid((g.n + 255) / 256, g.m);
   const int* partials = static_cast<const int*>(workspace);
@@ -460,22 +461,18 @@ static int launch_gemm_splitk(const GemmArgs& g, void* workspace, size_t workspa
   const float* sb = static_cast<const float*>(g.scale_b);
   switch (g.out_dtype) {
     case GG_OUT_FP32:
-      launch(fold_partials_kernel<float>, fold_grid, 256, 0, stream,
+      return launch(fold_partials_kernel<float>, fold_grid, 256, 0, stream,
           partials, sa, sb, static_cast<float*>(g.c), g.m, g.n, groups, g.sa_sm, g.sa_sg, g.sb_sg,
           g.sb_sn, g.ldc);
-      break;
     case GG_OUT_BF16:
-      launch(fold_partials_kernel<__nv_bfloat16>, fold_grid, 256, 0, stream,
+      return launch(fold_partials_kernel<__nv_bfloat16>, fold_grid, 256, 0, stream,
           partials, sa, sb, static_cast<__nv_bfloat16*>(g.c), g.m, g.n, groups, g.sa_sm, g.sa_sg,
           g.sb_sg, g.sb_sn, g.ldc);
-      break;
     default:
-      launch(fold_partials_kernel<__half>, fold_grid, 256, 0, stream,
+      return launch(fold_partials_kernel<__half>, fold_grid, 256, 0, stream,
           partials, sa, sb, static_cast<__half*>(g.c), g.m, g.n, groups, g.sa_sm, g.sa_sg, g.sb_sg,
           g.sb_sn, g.ldc);
-      break;
   }
-  return static_cast<int>(cudaGetLastError());
 }
 
 static int run_gemm(const GemmArgs& g, int variant, cudaStream_t stream, void* workspace = nullptr,
@@ -527,7 +524,7 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
   auto kernel = moe_gate_up_tc_kernel<RoundT, kGather, kPair>;
   const cudaError_t error = cudaFuncSetAttribute(
       kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GateUpShape::kSmemBytes);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return finished(error);
   constexpr int kCtas = kPair ? 2 : 1;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(sm_count() / kCtas * kCtas);
@@ -550,7 +547,7 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
   }
   if (items < workers) workers = static_cast<int>(items);
   config.gridDim = dim3(workers * kCtas);
-  return static_cast<int>(cudaLaunchKernelEx(&config, kernel, map_x, map_gate, map_up, p));
+  return finished(cudaLaunchKernelEx(&config, kernel, map_x, map_gate, map_up, p));
 }
 
 // Whole items go to single CTAs, or half an item to each CTA of a pair.  A pair finishes in half the
@@ -726,20 +723,18 @@ int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens,
     if (smem > 48 * 1024) {
       error = cudaFuncSetAttribute(gg::route_single_kernel,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-      if (error != cudaSuccess) return static_cast<int>(error);
+      if (error != cudaSuccess) return gg::finished(error);
     }
-    gg::launch(gg::route_single_kernel, 1, gg::kRouteChunk, smem, stream, p);
-    return static_cast<int>(cudaGetLastError());
+    return gg::launch(gg::route_single_kernel, 1, gg::kRouteChunk, smem, stream, p);
   }
   if (slots <= gg::kRouteMediumSlots && experts + 1 <= gg::kRouteMediumKeys) {
     const size_t medium = (static_cast<size_t>(33) * (experts + 1) + 33) * sizeof(int);
     if (medium > 48 * 1024) {
       error = cudaFuncSetAttribute(gg::route_medium_kernel,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(medium));
-      if (error != cudaSuccess) return static_cast<int>(error);
+      if (error != cudaSuccess) return gg::finished(error);
     }
-    gg::launch(gg::route_medium_kernel, 1, 1024, medium, stream, p);
-    return static_cast<int>(cudaGetLastError());
+    return gg::launch(gg::route_medium_kernel, 1, 1024, medium, stream, p);
   }
   if (workspace_bytes < gg_moe_route_workspace_bytes(tokens, top_k, experts) || !workspace) {
     return static_cast<int>(cudaErrorInvalidValue);
@@ -751,13 +746,13 @@ int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens,
                                reinterpret_cast<const void*>(gg::route_place_kernel)}) {
       error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(smem));
-      if (error != cudaSuccess) return static_cast<int>(error);
+      if (error != cudaSuccess) return gg::finished(error);
     }
   }
-  gg::launch(gg::route_histogram_kernel, chunks, gg::kRouteChunk, smem, stream, p);
-  gg::launch(gg::route_scan_kernel, 1, 1024, smem, stream, p, chunks);
-  gg::launch(gg::route_place_kernel, chunks, gg::kRouteChunk, smem, stream, p);
-  return static_cast<int>(cudaGetLastError());
+  int status = gg::launch(gg::route_histogram_kernel, chunks, gg::kRouteChunk, smem, stream, p);
+  if (!status) status = gg::launch(gg::route_scan_kernel, 1, 1024, smem, stream, p, chunks);
+  if (!status) status = gg::launch(gg::route_place_kernel, chunks, gg::kRouteChunk, smem, stream, p);
+  return status;
 }
 
 // ---- routing without any allocation -----------------------------------------------------
@@ -775,13 +770,13 @@ static int static_route_scratch(int** out) {
   static std::mutex guard;
   int device = 0;
   cudaError_t error = cudaGetDevice(&device);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return gg::finished(error);
   if (device < 0 || device >= 64) return static_cast<int>(cudaErrorInvalidDevice);
   std::lock_guard<std::mutex> lock(guard);
   if (address[device] == nullptr) {
     void* pointer = nullptr;
     error = cudaGetSymbolAddress(&pointer, g_static_route_scratch);
-    if (error != cudaSuccess) return static_cast<int>(error);
+    if (error != cudaSuccess) return gg::finished(error);
     address[device] = static_cast<int*>(pointer);
   }
   *out = address[device];
@@ -818,10 +813,9 @@ int gg_moe_tiles(const void* offsets, int experts, int tile_rows, int capacity, 
   if (!offsets || !tile_expert || !tile_row || experts <= 0 || tile_rows <= 0 || capacity <= 0) {
     return static_cast<int>(cudaErrorInvalidValue);
   }
-  gg::launch(gg::moe_tiles_kernel, 1, 1024, 0, static_cast<cudaStream_t>(stream),
-      static_cast<const int*>(offsets), experts, tile_rows, capacity, static_cast<int*>(tile_expert),
-      static_cast<int*>(tile_row));
-  return static_cast<int>(cudaGetLastError());
+  return gg::launch(gg::moe_tiles_kernel, 1, 1024, 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const int*>(offsets), experts, tile_rows, capacity,
+                    static_cast<int*>(tile_expert), static_cast<int*>(tile_row));
 }
 
 size_t gg_moe_gate_up_scratch_bytes(int assignments, int hidden, int intermediate, int tile_rows,
@@ -842,9 +836,8 @@ int gg_moe_silu_table(void* table, int out_dtype, void* stream_ptr) {
   if (!table || (out_dtype != GG_OUT_BF16 && out_dtype != GG_OUT_FP16)) {
     return static_cast<int>(cudaErrorInvalidValue);
   }
-  gg::launch(gg::silu_table_kernel, 256, 256, 0, static_cast<cudaStream_t>(stream_ptr),
-      static_cast<float*>(table), out_dtype == GG_OUT_FP16 ? 1 : 0);
-  return static_cast<int>(cudaGetLastError());
+  return gg::launch(gg::silu_table_kernel, 256, 256, 0, static_cast<cudaStream_t>(stream_ptr),
+                    static_cast<float*>(table), out_dtype == GG_OUT_FP16 ? 1 : 0);
 }
 
 int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const void* scale_w1,
@@ -885,12 +878,11 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
       p.row_scale = sorted_scale;
       const long long blocks = (slots + 7) / 8 > gg::kSiluBlocks ? (slots + 7) / 8 : gg::kSiluBlocks;
       const int limit = gg::sm_count() * 8;
-      gg::launch(gg::gather_rows_kernel, static_cast<int>(blocks < limit ? blocks : limit), 256, 0, stream,
+      status = gg::launch(gg::gather_rows_kernel, static_cast<int>(blocks < limit ? blocks : limit), 256, 0, stream,
           static_cast<const int8_t*>(x), static_cast<const float*>(scale_x),
           static_cast<const long long*>(order), static_cast<const int*>(offsets), experts, top_k,
           hidden, sorted_x, sorted_scale, const_cast<float*>(p.silu_table), out_dtype == GG_OUT_FP16 ? 1 : 0);
-      const cudaError_t error = cudaGetLastError();
-      if (error != cudaSuccess) return static_cast<int>(error);
+      if (status) return status;
       status = gg::encode_int8_rows(&map_x, sorted_x, slots, hidden, hidden, 128);
     }
     if (status) return status;
@@ -1138,32 +1130,33 @@ int gg_peer_alloc(size_t bytes, void** pointer) {
   if (!pointer || bytes == 0) return static_cast<int>(cudaErrorInvalidValue);
   void* memory = nullptr;
   cudaError_t error = cudaMalloc(&memory, bytes);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return gg::finished(error);
   error = cudaMemset(memory, 0, bytes);
   if (error != cudaSuccess) {
-    cudaFree(memory);
-    return static_cast<int>(error);
+    const int status = gg::finished(error);
+    (void)gg::finished(cudaFree(memory));
+    return status;
   }
   *pointer = memory;
   return 0;
 }
 
-int gg_peer_free(void* pointer) { return static_cast<int>(cudaFree(pointer)); }
+int gg_peer_free(void* pointer) { return gg::finished(cudaFree(pointer)); }
 
 int gg_peer_export(void* pointer, void* handle) {
   if (!pointer || !handle) return static_cast<int>(cudaErrorInvalidValue);
   static_assert(sizeof(cudaIpcMemHandle_t) == 64, "the handle travels as 64 bytes");
-  return static_cast<int>(cudaIpcGetMemHandle(static_cast<cudaIpcMemHandle_t*>(handle), pointer));
+  return gg::finished(cudaIpcGetMemHandle(static_cast<cudaIpcMemHandle_t*>(handle), pointer));
 }
 
 int gg_peer_import(const void* handle, void** pointer) {
   if (!handle || !pointer) return static_cast<int>(cudaErrorInvalidValue);
   cudaIpcMemHandle_t copy;
   memcpy(&copy, handle, sizeof(copy));
-  return static_cast<int>(cudaIpcOpenMemHandle(pointer, copy, cudaIpcMemLazyEnablePeerAccess));
+  return gg::finished(cudaIpcOpenMemHandle(pointer, copy, cudaIpcMemLazyEnablePeerAccess));
 }
 
-int gg_peer_release(void* pointer) { return static_cast<int>(cudaIpcCloseMemHandle(pointer)); }
+int gg_peer_release(void* pointer) { return gg::finished(cudaIpcCloseMemHandle(pointer)); }
 
 int gg_moe_topk(const void* logits, int in_dtype, int tokens, int experts, int top_k, void* weights,
                 void* ids, int ids_are_i64, void* stream_ptr) {
@@ -1176,18 +1169,19 @@ int gg_moe_topk(const void* logits, int in_dtype, int tokens, int experts, int t
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   const int grid = (tokens + 7) / 8;
   float* w = static_cast<float*>(weights);
+  int status;
   if (in_dtype == GG_OUT_FP32) {
-    gg::launch(gg::router_topk_kernel<float>, grid, 256, 0, stream, static_cast<const float*>(logits), tokens,
+    status = gg::launch(gg::router_topk_kernel<float>, grid, 256, 0, stream, static_cast<const float*>(logits), tokens,
                                                              experts, top_k, w, ids, ids_are_i64);
   } else if (in_dtype == GG_OUT_BF16) {
-    gg::launch(gg::router_topk_kernel<__nv_bfloat16>, grid, 256, 0, stream,
+    status = gg::launch(gg::router_topk_kernel<__nv_bfloat16>, grid, 256, 0, stream,
         static_cast<const __nv_bfloat16*>(logits), tokens, experts, top_k, w, ids, ids_are_i64);
   } else {
-    gg::launch(gg::router_topk_kernel<__half>, grid, 256, 0, stream, static_cast<const __half*>(logits),
+    status = gg::launch(gg::router_topk_kernel<__half>, grid, 256, 0, stream, static_cast<const __half*>(logits),
                                                               tokens, experts, top_k, w, ids,
                                                               ids_are_i64);
   }
-  return static_cast<int>(cudaGetLastError());
+  return status;
 }
 
 int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int tokens, int experts,
@@ -1215,17 +1209,18 @@ int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int to
   p.statistics = static_cast<int*>(statistics);
   const size_t smem = static_cast<size_t>(experts + 2) * sizeof(int);
   float* w = static_cast<float*>(weights);
+  int status;
   if (in_dtype == GG_OUT_FP32) {
-    gg::launch(gg::route_topk_single_kernel<float>, 1, gg::kRouteChunk, smem, stream,
+    status = gg::launch(gg::route_topk_single_kernel<float>, 1, gg::kRouteChunk, smem, stream,
         static_cast<const float*>(logits), w, p);
   } else if (in_dtype == GG_OUT_BF16) {
-    gg::launch(gg::route_topk_single_kernel<__nv_bfloat16>, 1, gg::kRouteChunk, smem, stream,
+    status = gg::launch(gg::route_topk_single_kernel<__nv_bfloat16>, 1, gg::kRouteChunk, smem, stream,
         static_cast<const __nv_bfloat16*>(logits), w, p);
   } else {
-    gg::launch(gg::route_topk_single_kernel<__half>, 1, gg::kRouteChunk, smem, stream,
+    status = gg::launch(gg::route_topk_single_kernel<__half>, 1, gg::kRouteChunk, smem, stream,
         static_cast<const __half*>(logits), w, p);
   }
-  return static_cast<int>(cudaGetLastError());
+  return status;
 }
 
 int gg_quantize_rows(const void* x, int in_dtype, long long rows, int width, int group_size,
@@ -1253,8 +1248,7 @@ int gg_quantize_rows(const void* x, int in_dtype, long long rows, int width, int
     status = gg::launch_quantize(static_cast<const __half*>(x), rows, width, group_size, items, codes, scales,
                                  stream);
   }
-  if (status) return status;
-  return static_cast<int>(cudaGetLastError());
+  return status;
 }
 
 int gg_moe_combine(const void* expert_out, const void* weights, const void* inverse, void* out,
@@ -1278,16 +1272,17 @@ int gg_moe_combine(const void* expert_out, const void* weights, const void* inve
   int threads = ((chunks + passes - 1) / passes + 31) / 32 * 32;
   if (threads > 256) threads = 256;
   if (threads < 32) threads = 32;
+  int status;
   if (out_dtype == GG_OUT_BF16) {
-    gg::launch(gg::combine_kernel<__nv_bfloat16>, tokens, threads, smem, stream,
+    status = gg::launch(gg::combine_kernel<__nv_bfloat16>, tokens, threads, smem, stream,
         static_cast<const __nv_bfloat16*>(expert_out), static_cast<const float*>(weights),
         static_cast<const int*>(inverse), static_cast<__nv_bfloat16*>(out), top_k, hidden, vector_ok);
   } else {
-    gg::launch(gg::combine_kernel<__half>, tokens, threads, smem, stream,
+    status = gg::launch(gg::combine_kernel<__half>, tokens, threads, smem, stream,
         static_cast<const __half*>(expert_out), static_cast<const float*>(weights),
         static_cast<const int*>(inverse), static_cast<__half*>(out), top_k, hidden, vector_ok);
   }
-  return static_cast<int>(cudaGetLastError());
+  return status;
 }
 
 int gg_report_to_host(const void* values, int count, void* host_words, void* stream_ptr) {
@@ -1297,13 +1292,9 @@ int gg_report_to_host(const void* values, int count, void* host_words, void* str
   // address is asked for rather than assumed.
   void* mapped = nullptr;
   cudaError_t error = cudaHostGetDevicePointer(&mapped, host_words, 0);
-  if (error != cudaSuccess) {
-    (void)cudaGetLastError();
-    return static_cast<int>(error);
-  }
-  gg::launch(gg::report_to_host_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream_ptr),
-      static_cast<const int*>(values), count, static_cast<int*>(mapped));
-  return static_cast<int>(cudaGetLastError());
+  if (error != cudaSuccess) return gg::finished(error);
+  return gg::launch(gg::report_to_host_kernel, 1, 32, 0, static_cast<cudaStream_t>(stream_ptr),
+                    static_cast<const int*>(values), count, static_cast<int*>(mapped));
 }
 
 int gg_selftest_wait_timeout(long long limit_ns, void* result, void* stream_ptr) {
@@ -1321,18 +1312,18 @@ int gg_device_status(int* status, void* stream_ptr) {
   unsigned int words[4] = {0, 0, 0, 0};
   cudaError_t error = cudaMemcpyFromSymbolAsync(words, gg::g_device_status, sizeof(words), 0,
                                                 cudaMemcpyDeviceToHost, stream);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return gg::finished(error);
   error = cudaStreamSynchronize(stream);
-  if (error != cudaSuccess) return static_cast<int>(error);
+  if (error != cudaSuccess) return gg::finished(error);
   *status = static_cast<int>(words[0]);
   if (words[0] != 0) {
     const unsigned int zeros[4] = {0, 0, 0, 0};
     error = cudaMemcpyToSymbolAsync(gg::g_device_status, zeros, sizeof(zeros), 0,
                                     cudaMemcpyHostToDevice, stream);
-    if (error != cudaSuccess) return static_cast<int>(error);
+    if (error != cudaSuccess) return gg::finished(error);
     error = cudaStreamSynchronize(stream);
   }
-  return static_cast<int>(error);
+  return gg::finished(error);
 }
 
 }  // extern "C"
