@@ -17,6 +17,7 @@
 #include "moe_ep.cuh"
 #include "moe_gate_up_tc.cuh"
 #include "moe_route.cuh"
+#include "tensor_map.cuh"
 
 namespace gg {
 
@@ -31,11 +32,6 @@ static int finished(cudaError_t error) {
   return static_cast<int>(error);
 }
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 static EncodeTiledFn encode_tiled_fn() {
   static EncodeTiledFn fn = [] {
     void* ptr = nullptr;
@@ -47,48 +43,6 @@ static EncodeTiledFn encode_tiled_fn() {
     return reinterpret_cast<EncodeTiledFn>(ptr);
   }();
   return fn;
-}
-
-// Tensor map over a row-major int8 matrix [rows, cols] with row pitch `pitch` bytes; boxes of
-// 128 bytes x box_rows with the 128-byte swizzle; out-of-range elements read as zero.
-static int encode_int8_rows(CUtensorMap* map, const void* base, long long rows, long long cols,
-                            long long pitch, int box_rows) {
-  EncodeTiledFn encode = encode_tiled_fn();
-  if (encode == nullptr) return static_cast<int>(cudaErrorNotSupported);
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch)};
-  const cuuint32_t box[2] = {128u, static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t element_strides[2] = {1u, 1u};
-  const CUresult result = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base),
-                                 dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return result == CUDA_SUCCESS ? 0 : -10000 - static_cast<int>(result);
-}
-
-// Tensor map over the rows of a weight matrix, boxes of 128 bytes x box_rows.  With `permuted` (rows
-// a multiple of 32) every block of 32 rows is delivered in the order the epilogue's fragments
-// want: row 8q + k of the block lands in row 4k + q of the tile (see gemm_tc.cuh).  The kernels
-// load with coordinates (x, 0, 0, row / 32) then, with (x, row, 0, 0) otherwise.
-static int weight_row_map(CUtensorMap* map, const void* base, long long rows, long long cols,
-                          long long pitch, int box_rows, bool permuted) {
-  EncodeTiledFn encode = encode_tiled_fn();
-  if (encode == nullptr) return static_cast<int>(cudaErrorNotSupported);
-  const cuuint64_t columns = static_cast<cuuint64_t>(cols), step = static_cast<cuuint64_t>(pitch);
-  const cuuint32_t box = static_cast<cuuint32_t>(box_rows);
-  const cuuint64_t own_dims[4] = {columns, static_cast<cuuint64_t>(rows), 1, 1};
-  const cuuint64_t own_strides[3] = {step, step, step};
-  const cuuint32_t own_box[4] = {128u, box, 1u, 1u};
-  const cuuint64_t permuted_dims[4] = {columns, 4, 8, static_cast<cuuint64_t>(rows / 32)};
-  const cuuint64_t permuted_strides[3] = {8 * step, step, 32 * step};
-  const cuuint32_t permuted_box[4] = {128u, 4u, 8u, box / 32};
-  const cuuint32_t element_strides[4] = {1u, 1u, 1u, 1u};
-  const CUresult result = encode(
-      map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), permuted ? permuted_dims : own_dims,
-      permuted ? permuted_strides : own_strides, permuted ? permuted_box : own_box, element_strides,
-      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return result == CUDA_SUCCESS ? 0 : -10000 - static_cast<int>(result);
 }
 
 static int sm_count() {
@@ -392,10 +346,10 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
                  : (variant == GG_VARIANT_TC_N128 || variant == GG_VARIANT_TC_PAIR_N128) ? 128
                                                                                          : 64;
   CUtensorMap map_a, map_b;
-  int status = encode_int8_rows(&map_a, g.a, g.m, g.k, g.a_sm, 128);
+  int status = row_map(encode_tiled_fn(), &map_a, g.a, g.m, g.k, g.a_sm, 128);
   if (status) return status;
-  const bool permuted = g.n % 32 == 0;
-  status = weight_row_map(&map_b, g.b, g.n, g.k, g.b_sn, pair ? bn / 2 : bn, permuted);
+  bool permuted = g.n % 32 == 0;
+  status = weight_row_map(encode_tiled_fn(), &map_b, g.b, g.n, g.k, g.b_sn, pair ? bn / 2 : bn, &permuted);
   if (status) return status;
   GemmTcParams p = {};
   p.scale_a = static_cast<const float*>(g.scale_a);
@@ -431,10 +385,11 @@ static int launch_gemm_splitk(const GemmArgs& g, void* workspace, size_t workspa
     return static_cast<int>(cudaErrorInvalidValue);
   }
   CUtensorMap map_a, map_b;
-  int status = encode_int8_rows(&map_a, g.a, g.m, g.k, g.a_sm, 32);
+  int status = row_map(encode_tiled_fn(), &map_a, g.a, g.m, g.k, g.a_sm, 32);
   if (status) return status;
   // The dots leave in column order (a thread stores consecutive TMEM columns of one row).
-  status = weight_row_map(&map_b, g.b, g.n, g.k, g.b_sn, 256, false);
+  bool permuted = false;
+  status = weight_row_map(encode_tiled_fn(), &map_b, g.b, g.n, g.k, g.b_sn, 256, &permuted);
   if (status) return status;
   GemmTcParams p = {};
   p.m = g.m; p.n = g.n; p.k = g.k;
@@ -866,7 +821,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     if (row_gather) {
       p.silu_table = reinterpret_cast<float*>(scratch);
       p.row_scale = static_cast<const float*>(scale_x);
-      status = gg::encode_int8_rows(&map_x, x, tokens, hidden, hidden, 1);
+      status = gg::row_map(gg::encode_tiled_fn(), &map_x, x, tokens, hidden, hidden, 1);
     } else {
       // Activation rows and their scales in sorted-slot order first.
       int8_t* sorted_x = reinterpret_cast<int8_t*>(scratch);
@@ -883,25 +838,18 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
           static_cast<const long long*>(order), static_cast<const int*>(offsets), experts, top_k,
           hidden, sorted_x, sorted_scale, const_cast<float*>(p.silu_table), out_dtype == GG_OUT_FP16 ? 1 : 0);
       if (status) return status;
-      status = gg::encode_int8_rows(&map_x, sorted_x, slots, hidden, hidden, 128);
+      status = gg::row_map(gg::encode_tiled_fn(), &map_x, sorted_x, slots, hidden, hidden, 128);
     }
     if (status) return status;
     if (row_gather) {
       status = gg_moe_silu_table(const_cast<float*>(p.silu_table), out_dtype, stream_ptr);
       if (status) return status;
     }
-    const bool pairs = !row_gather && gg::gate_up_pairs(slots, experts, intermediate / 256);
-    const long long weight_rows = static_cast<long long>(experts) * 2 * intermediate;
-    if (interleaved) {
-      // Every other row: gate rows from the first, up rows from the second.
-      const int8_t* rows = static_cast<const int8_t*>(w1);
-      status = gg::weight_row_map(&map_gate, rows, weight_rows / 2, hidden, 2ll * hidden, 128, pairs);
-      if (status) return status;
-      status = gg::weight_row_map(&map_up, rows + hidden, weight_rows / 2, hidden, 2ll * hidden, 128, pairs);
-    } else {
-      status = gg::weight_row_map(&map_gate, w1, weight_rows, hidden, hidden, 128, pairs);
-      map_up = map_gate;
-    }
+    // Pairs need their weight rows in fragment order; without such a map the item stays on one CTA.
+    bool pairs = !row_gather && gg::gate_up_pairs(slots, experts, intermediate / 256);
+    status = gg::gate_up_row_maps(gg::encode_tiled_fn(), &map_gate, &map_up, w1,
+                                  static_cast<long long>(experts) * 2 * intermediate, hidden, interleaved != 0,
+                                  &pairs);
     if (status) return status;
     p.order = static_cast<const long long*>(order);
     p.top_k = top_k;
@@ -975,16 +923,16 @@ int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_
     }
     const unsigned long long* destinations = static_cast<const unsigned long long*>(row_destination);
     CUtensorMap map_a, map_b;
-    int status = gg::encode_int8_rows(&map_a, q, assignments, intermediate, intermediate, 128);
+    int status = gg::row_map(gg::encode_tiled_fn(), &map_a, q, assignments, intermediate, intermediate, 128);
     if (status) return status;
     // Narrower column tiles as long as all tiles still fit one wave (a layer of one token has a
     // handful of row tiles and would leave most SMs idle); slots bound the row tiles in use.
     const long long used_tiles = assignments < tile_capacity ? assignments : tile_capacity;
     int bn = hidden >= 256 ? 256 : hidden >= 128 ? 128 : 64;
     while (bn > 64 && used_tiles * ((hidden + bn / 2 - 1) / (bn / 2)) <= gg::sm_count()) bn /= 2;
-    const bool permuted = hidden % 32 == 0;
-    status = gg::weight_row_map(&map_b, w2, static_cast<long long>(experts) * hidden, intermediate,
-                                intermediate, bn, permuted);
+    bool permuted = hidden % 32 == 0;
+    status = gg::weight_row_map(gg::encode_tiled_fn(), &map_b, w2, static_cast<long long>(experts) * hidden,
+                                intermediate, intermediate, bn, &permuted);
     if (status) return status;
     gg::GemmTcParams p = {};
     p.scale_a = static_cast<const float*>(s);

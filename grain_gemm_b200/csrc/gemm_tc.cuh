@@ -187,7 +187,7 @@ __device__ __forceinline__ TileWork decode_tile(const GemmTcParams& p, int tile,
 // A row leaves as 16-byte stores of consecutive columns, so thread q wants the outputs
 // 8q .. 8q + 7 of a block in its eight columns 4k + q.  Weight row 8q + k therefore has to sit in
 // row 4k + q of the B tile's block, and the tensor map does that on the way in: it presents the
-// weight as [N/32][k = 8][q = 4][K] (weight_row_map in abi.cu), and accumulator pair j holds the
+// weight as [N/32][k = 8][q = 4][K] (weight_row_map in tensor_map.cuh), and accumulator pair j holds the
 // outputs 8q + 2j and 8q + 2j + 1.  Nothing is exchanged between lanes and the scales are used in
 // their own order.  (With rows in their own order, pair j holds outputs 8j + q and 8j + 4 + q and a
 // 4x4 exchange inside every quad precedes the stores: 64 shuffles and 600 instructions a

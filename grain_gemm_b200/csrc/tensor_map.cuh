@@ -1,0 +1,87 @@
+// Tensor maps of the operands, encoded on the host.  The driver's encoder is an argument, so that the
+// choices made here can be tested without a GPU.
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime_api.h>
+
+namespace gg {
+
+using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// Boxes with the 128-byte swizzle over bytes; out-of-range elements read as zero.
+static inline int encode_bytes(EncodeTiledFn encode, CUtensorMap* map, const void* base, int rank,
+                               const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+  if (encode == nullptr) return static_cast<int>(cudaErrorNotSupported);
+  const cuuint32_t element_strides[4] = {1u, 1u, 1u, 1u};
+  const CUresult result = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, static_cast<cuuint32_t>(rank),
+                                 const_cast<void*>(base), dims, strides, box, element_strides,
+                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return result == CUDA_SUCCESS ? 0 : -10000 - static_cast<int>(result);
+}
+
+// Tensor map over a row-major int8 matrix [rows, cols] with row pitch `pitch` bytes; boxes of
+// 128 bytes x box_rows.
+static inline int row_map(EncodeTiledFn encode, CUtensorMap* map, const void* base, long long rows,
+                          long long cols, long long pitch, int box_rows) {
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch)};
+  const cuuint32_t box[2] = {128u, static_cast<cuuint32_t>(box_rows)};
+  return encode_bytes(encode, map, base, 2, dims, strides, box);
+}
+
+// Tensor map over the rows of a weight matrix, boxes of 128 bytes x box_rows.  With `permuted` (asked for
+// only where rows and box_rows are multiples of 32) every block of 32 rows is delivered in the
+// order the epilogue's fragments want: row 8q + k of the block lands in row 4k + q of the tile (see
+// gemm_tc.cuh).  The kernels load with coordinates (x, 0, 0, row / 32) then, with (x, row, 0, 0)
+// otherwise.
+//
+// The permuted map steps 8 rows in its second dimension and 1 row in its third.  The driver API's
+// documentation asks that each stride be a multiple of the one before; the encoder of driver 580.159
+// does not enforce that and the copies deliver what the strides say (every bit-for-bit GEMM test
+// depends on it).  Because it is not promised, an encoder that refuses the map is answered with the
+// rows in their own order: `permuted` tells which of the two `map` is, and the kernels do the
+// exchange between lanes themselves then.
+static inline int weight_row_map(EncodeTiledFn encode, CUtensorMap* map, const void* base, long long rows,
+                                 long long cols, long long pitch, int box_rows, bool* permuted) {
+  const cuuint64_t columns = static_cast<cuuint64_t>(cols), step = static_cast<cuuint64_t>(pitch);
+  const cuuint32_t box = static_cast<cuuint32_t>(box_rows);
+  if (*permuted) {
+    const cuuint64_t dims[4] = {columns, 4, 8, static_cast<cuuint64_t>(rows / 32)};
+    const cuuint64_t strides[3] = {8 * step, step, 32 * step};
+    const cuuint32_t boxes[4] = {128u, 4u, 8u, box / 32};
+    const int status = encode_bytes(encode, map, base, 4, dims, strides, boxes);
+    if (status == 0) return 0;
+    *permuted = false;
+  }
+  const cuuint64_t dims[4] = {columns, static_cast<cuuint64_t>(rows), 1, 1};
+  const cuuint64_t strides[3] = {step, step, step};
+  const cuuint32_t boxes[4] = {128u, box, 1u, 1u};
+  return encode_bytes(encode, map, base, 4, dims, strides, boxes);
+}
+
+// Maps of the gate and the up rows of [experts * 2I, hidden] weights: for the split layout both are
+// the whole weight, for the interleaved one each covers every other row.  One order for both.
+static inline int gate_up_row_maps(EncodeTiledFn encode, CUtensorMap* gate, CUtensorMap* up, const void* weights,
+                                   long long rows, int hidden, bool interleaved, bool* permuted) {
+  if (!interleaved) {
+    const int status = weight_row_map(encode, gate, weights, rows, hidden, hidden, 128, permuted);
+    *up = *gate;
+    return status;
+  }
+  const signed char* first = static_cast<const signed char*>(weights);
+  int status = weight_row_map(encode, gate, first, rows / 2, hidden, 2ll * hidden, 128, permuted);
+  if (status) return status;
+  const bool gate_permuted = *permuted;
+  status = weight_row_map(encode, up, first + hidden, rows / 2, hidden, 2ll * hidden, 128, permuted);
+  if (status == 0 && gate_permuted != *permuted) {
+    status = weight_row_map(encode, gate, first, rows / 2, hidden, 2ll * hidden, 128, permuted);
+  }
+  return status;
+}
+
+}  // namespace gg

@@ -1,0 +1,115 @@
+"""The weight's tensor map: rows in the epilogue's order, or in their own where the driver's encoder
+refuses that map.  The choice is host code; a small program runs it against encoders of its own."""
+
+import os
+import subprocess
+
+import pytest
+
+from grain_gemm_b200 import build
+
+PROGRAM = r"""
+#include <cstdio>
+#include <vector>
+#include "tensor_map.cuh"
+
+struct Encoded {
+  const char* base;
+  std::vector<unsigned long long> dims, strides, box;
+};
+static std::vector<Encoded> calls;
+static int refuse;             // 0 nothing, 1 strides that are not multiples of the one before, 2 everything,
+                               // 3 such strides from the second map on
+
+static CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t rank, void* base, const cuuint64_t* dims,
+                       const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t*, CUtensorMapInterleave,
+                       CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
+  Encoded e;
+  e.base = static_cast<const char*>(base);
+  e.dims.assign(dims, dims + rank);
+  e.strides.assign(strides, strides + rank - 1);
+  e.box.assign(box, box + rank);
+  calls.push_back(e);
+  bool ascending = true;
+  for (cuuint32_t i = 1; i + 1 < rank; ++i) ascending = ascending && strides[i] % strides[i - 1] == 0;
+  if (refuse == 2 || (refuse == 1 && !ascending) || (refuse == 3 && !ascending && calls.size() > 1)) {
+    return CUDA_ERROR_INVALID_VALUE;
+  }
+  return CUDA_SUCCESS;
+}
+
+// Rows of the matrix in the order in which the last map's box at block 0 delivers them.
+static void print_rows(const Encoded& e, long long pitch) {
+  for (unsigned long long c = 0; c < e.box[3]; ++c)
+    for (unsigned long long b = 0; b < e.box[2]; ++b)
+      for (unsigned long long a = 0; a < e.box[1]; ++a)
+        std::printf(" %lld", static_cast<long long>(a * e.strides[0] + b * e.strides[1] + c * e.strides[2]) / pitch);
+  std::printf("\n");
+}
+
+int main() {
+  char memory[1];
+  CUtensorMap map, up;
+  for (refuse = 0; refuse < 3; ++refuse) {
+    for (bool permuted : {true, false}) {
+      calls.clear();
+      bool order = permuted;
+      const int status = gg::weight_row_map(encode, &map, memory, 320, 512, 528, 64, &order);
+      std::printf("weight %d %d: status %d order %d encoded %zu rows", refuse, permuted, status, order, calls.size());
+      print_rows(calls.back(), 528);
+    }
+  }
+  for (int interleaved : {0, 1}) {
+    for (int which : {0, 1, 3}) {
+      refuse = which;
+      calls.clear();
+      bool order = true;
+      const int status = gg::gate_up_row_maps(encode, &map, &up, memory, 1024, 256, interleaved, &order);
+      std::printf("gate_up %d %d: status %d order %d", interleaved, refuse, status, order);
+      for (const Encoded& e : calls) std::printf(" (%d,%llu)", static_cast<int>(e.base - memory), e.dims[1]);
+      std::printf("\n");
+    }
+  }
+  bool order = true;
+  std::printf("none %d\n", gg::weight_row_map(nullptr, &map, memory, 320, 512, 528, 64, &order));
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def lines(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("tensor_map")
+    (folder / "program.cpp").write_text(PROGRAM)
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.find_nvcc()))), "include")
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-x", "c++", f"-I{build.CSRC}", f"-I{include}",
+                    "-o", str(folder / "program"), str(folder / "program.cpp")], check=True)
+    output = subprocess.run([str(folder / "program")], check=True, capture_output=True, text=True).stdout
+    return dict(line.split(":", 1) if ":" in line else line.split(" ", 1) for line in output.splitlines())
+
+
+OWN = " ".join(str(r) for r in range(64))
+FRAGMENT = " ".join(str(32 * block + 8 * q + k) for block in range(2) for k in range(8) for q in range(4))
+
+
+def test_rows_land_where_the_fragments_want_them(lines):
+    assert lines["weight 0 1"] == f" status 0 order 1 encoded 1 rows {FRAGMENT}"
+    assert lines["weight 0 0"] == f" status 0 order 0 encoded 1 rows {OWN}"
+
+
+def test_a_refused_map_is_answered_with_the_rows_own_order(lines):
+    assert lines["weight 1 1"] == f" status 0 order 0 encoded 2 rows {OWN}"
+    assert lines["weight 1 0"] == f" status 0 order 0 encoded 1 rows {OWN}"
+
+
+def test_an_encoder_that_refuses_both_is_an_error(lines):
+    assert lines["weight 2 1"].startswith(" status -10001 order 0 encoded 2")
+    assert lines["none"].strip() == "801"        # cudaErrorNotSupported
+
+
+def test_gate_and_up_rows_come_in_one_order(lines):
+    # Base offset and first row dimension of every map that was encoded: 4 in fragment order.
+    assert lines["gate_up 0 0"] == " status 0 order 1 (0,4)"
+    assert lines["gate_up 0 1"] == " status 0 order 0 (0,4) (0,1024)"
+    assert lines["gate_up 1 0"] == " status 0 order 1 (0,4) (256,4)"
+    assert lines["gate_up 1 1"] == " status 0 order 0 (0,4) (0,512) (256,512)"
+    assert lines["gate_up 1 3"] == " status 0 order 0 (0,4) (256,4) (256,512) (0,512)"
