@@ -44,18 +44,28 @@ def test_widths_in_both_weight_orders(variant, n, dtype):
 @pytest.mark.parametrize("group", [32, 256])
 @pytest.mark.parametrize("groups", [1, 3, 4, 5, 8, 9])
 def test_group_counts_around_the_scale_chunks(variant, group, groups):
-    # Several tiles per CTA (pair), so that the ring's position is carried from tile to tile.
+    # One tile per CTA (pair): the ring's chunks and slots within a tile.
     case = _case(300, 320, group * groups, group, groups)
     actual = _run([t.cuda() for t in case], group, torch.float32, variant)
     assert torch.equal(actual.cpu(), oracle.int8_gemm(*case, group, torch.float32))
 
 
-def test_many_tiles_per_cta_carry_the_ring():
-    case = _case(2600, 4128, 96, 32, 7)     # 17 x 21 tiles of 128 x 256, three groups each
-    actual = _run([t.cuda() for t in case], 32, torch.bfloat16, "tc_n128")
-    rows = torch.arange(0, 2600, 37)
-    expected = oracle.int8_gemm(case[0][rows], case[1], case[2][rows], case[3], 32, torch.bfloat16)
-    assert torch.equal(actual.cpu()[rows], expected)
+@pytest.mark.parametrize("variant", VARIANTS)
+@pytest.mark.parametrize("groups", [1, 3, 5, 9])
+def test_many_tiles_per_cta_carry_the_ring(variant, groups):
+    # More than two tiles for every CTA (pair), so that a chunk that was only partly used and the
+    # ring's position are carried from tile to tile.
+    rows, columns, ctas = {"tc_n256": (128, 256, 1), "tc_n128": (128, 128, 1), "tc_n64": (128, 64, 1),
+                           "tc_pair_n256": (256, 256, 2), "tc_pair_n128": (256, 128, 2)}[variant]
+    m, n = 2600, 19 * columns + 32
+    tiles = -(-m // rows) * -(-n // columns)
+    workers = torch.cuda.get_device_properties(0).multi_processor_count // ctas
+    assert tiles > 2 * workers
+    case = _case(m, n, 32 * groups, 32, 7 + groups)
+    actual = _run([t.cuda() for t in case], 32, torch.bfloat16, variant)
+    take = torch.arange(0, m, 37)
+    expected = oracle.int8_gemm(case[0][take], case[1], case[2][take], case[3], 32, torch.bfloat16)
+    assert torch.equal(actual.cpu()[take], expected)
 
 
 @pytest.mark.parametrize("form", ["offset", "odd_pitch", "strided", "transposed"])
