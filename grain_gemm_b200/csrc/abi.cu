@@ -512,9 +512,13 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
 // 1 token over 8 of 128 experts (24 items) 52 and 46 us, 8 tokens, H = 4096, I = 14336, 8 experts
 // (448 items, 4 against 3.5 waves) 260 and 251 us, 256 tokens, I = 1536, 32 experts (192 items,
 // 2 against 1.5) 184 and 170 us, but 512 tokens, I = 768, 128 experts (384 items, 3 waves either
-// way) 176 and 188 us.
+// way) 176 and 188 us.  None of these lies near the line itself, which follows from the 4 %: a pair's
+// item counts 0.52 of a whole one.
 // Row tiles are estimated as one per expert while an expert has few rows, as full tiles and half a
-// tile of remainder per expert beyond.
+// tile of remainder per expert beyond; a call sized for a capacity (a rank of an expert-parallel step) is
+// estimated at that capacity, not at the rows it received.  Half the SMs is an upper bound on
+// the pairs that are resident at once (see resident_clusters), so on a part that holds fewer a size
+// near a wave's edge may go to pairs that need one wave more than counted here.
 // Only pairs take their weight rows in fragment order; for single CTAs, which amortise the
 // exchange over a whole item, it made no difference beyond the spread of the runs.
 static bool gate_up_pairs(long long slots, int experts, int channel_groups) {

@@ -14,11 +14,12 @@
 //               TMEM, two accumulator buffers of BN columns.  The first MMA of every K group
 //               overwrites the buffer, the last one commits it to the promotion warps.
 //   scale warp  cp.async of each group's scale_b columns and scale_a rows into a shared-memory
-//               ring, a whole ring ahead of the promotion warps
+//               ring, up to a whole ring ahead of the promotion warps
 //   warps 0-7   promotion: drain the group's INT32 tile with tcgen05.ld in a matrix-fragment
 //               layout (a thread owns 4 rows x 32 columns of its warp's 32 x 128 region),
 //               multiply by sa*sb, add into FP32 registers while the tensor core works on the
-//               next group; at the end of the tile cast, exchange inside quads and store.
+//               next group; at the end of the tile cast and store (weight rows that came in their
+//               own order are exchanged inside quads of lanes first).
 // kCtaGroup == 2 pairs two CTAs (a 2-CTA cluster) on a 256 x BN tile: each CTA loads its own
 // 128 rows of A and its own half of B, the leader CTA issues cta_group::2 MMAs that read both
 // CTAs' shared memory and write both CTAs' TMEM.
@@ -28,9 +29,12 @@
 // that arithmetic alone, on TMEM contents with no barrier in sight, takes 900 cycles, the MMAs
 // of a 256-deep group 1024.  So everything else in the loop is kept out of the way: waits vote
 // before they branch, the scale ring changes hands four groups at a time, no accumulator is
-// modified inside a branch, and waiting warps poll without a software loop around the probe.
-// That took a group of the G = 32 kernel from 1780 to 1500 cycles (M = 1024, N = K = 8192:
-// 464 to 408 us) and 8192^3 at G = 256 from 479 to 455 us in a short burst.
+// modified inside a branch, the probe of a wait carries no suspension limit, and the finished tile
+// needs no exchange between lanes.  That took a group of the G = 32 kernel, everything included, from
+// 1780 to 1500 cycles (M = 1024, N = K = 8192: 464 to 391 us, two waves of 256 groups) and 8192^3 at
+// G = 256 from 479 to 450 us in a short burst.  There a group takes 1710 to 1770 cycles at the 1.70
+// to 1.76 GHz that the part holds inside the launch: more than the loop's 1500, the rest is not
+// accounted for.
 //
 // Any M and N (rows/columns beyond the edge are zero-filled by TMA and never stored), any
 // K that is a multiple of 16 (TMA row pitch), G in {32, 64, 128, 256}; a partial last group
@@ -191,7 +195,7 @@ __device__ __forceinline__ TileWork decode_tile(const GemmTcParams& p, int tile,
 // outputs 8q + 2j and 8q + 2j + 1.  Nothing is exchanged between lanes and the scales are used in
 // their own order.  (With rows in their own order, pair j holds outputs 8j + q and 8j + 4 + q and a
 // 4x4 exchange inside every quad precedes the stores: 64 shuffles and 600 instructions a
-// warp and tile.  Only widths that are not a multiple of 32 still do that.)
+// warp and tile.  Widths that are not a multiple of 32 do that.)
 //
 // Position of block column `c` (0..31) in the scale ring for rows in their own order: thread q
 // reads its eight column scales, in accumulator-pair order, as two 16-byte vectors at q * 8.
@@ -523,12 +527,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (warp == kScaleWarp && !kDump) {
     // ------------------------------------------------------------ scale staging warp
-    // Copies each group's scale_b columns and scale_a rows into a shared-memory ring with
-    // asynchronous 4-byte copies (cp.async) that land directly in the order the promotion
-    // threads read; each lane's copies signal the slot's barrier when they have arrived.
-    // Nothing passes through registers, so the warp runs a whole ring ahead of the promotion
-    // warps and a global-memory latency of several K groups stays hidden (a version that
-    // held one group in registers left the promotion warps waiting for scales).
+    // Copies each group's scale_b columns (16 bytes at a time with sb_vectors, else 4) and scale_a
+    // rows (4 bytes) into a shared-memory ring with asynchronous copies (cp.async) that land
+    // directly in the order the promotion threads read; each lane's copies signal the chunk's
+    // barrier when they have arrived.  Nothing passes through registers, so the warp runs up to
+    // a ring ahead of the promotion warps and a global-memory latency of several K groups
+    // stays hidden (a version that held one group in registers left the promotion warps
+    // waiting for scales).
     constexpr int kColumnsPerLane = BN / 32;
     // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
     const uint32_t column_position = 4 * (p.permuted_columns ? lane : ring_column_position(lane));
@@ -680,8 +685,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         continue;
       }
-      // Fragment layout: this thread owns rows (lane / 4) + 8 * s, s = 0..3, of its warp's 32
-      // rows, and in every 8-column group the two columns 2 * (lane % 4), +1.
+      // This thread owns rows lane / 4 + 8 * s, s = 0..3, of its warp's 32 rows and, in every block
+      // of 32 columns, the eight outputs of its quad position (see the drain layout above).
       constexpr int kBlocks = kNC / 32;          // 32-column blocks in this warp's columns
       constexpr int kPairs = kNC / 8;            // column pairs per owned row
       float2 acc[4][kPairs];

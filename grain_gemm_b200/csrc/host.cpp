@@ -6,8 +6,9 @@
 // 40 us for a GEMM and 200 us for a MoE layer and was what such a step waited for.  Each function
 // here accepts exactly the calls that the Python path accepts AND whose tensors are plain dense
 // CUDA tensors, and returns None for everything else (wrong arguments, tensor subclasses, modes,
-// functorch levels, tracing, stream capture, operands that need a copy first): the caller
-// then takes the Python path, which raises the documented errors or does the rare work.
+// functorch levels, tracing, operands that need a copy first, and moe_ffn, which reads words back,
+// under stream capture): the caller then takes the Python path, which raises the documented
+// errors or does the rare work.
 // The kernels are reached through the C ABI of libgrain_b200.so; bind() receives its entry points,
 // so this module links against torch only.
 #define PY_SSIZE_T_CLEAN

@@ -256,10 +256,11 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       dependents_may_launch();   // the CTA's last loads are on their way
     } else if (warp == 10) {
       // ---------------------------------------------------------- scale staging warp
-      // Copies each group's 256 column scales (by accumulator column) and 128 row scales into a
-      // shared-memory ring with asynchronous 4-byte copies that land in the order the
-      // promotion threads read; the copies themselves signal the slot's barrier, so the warp
-      // runs a whole ring ahead and global-memory latency stays hidden.
+      // Copies each group's 256 column scales (by accumulator column; 16 bytes at a time for pairs
+      // with sw_vectors, else 4) and 128 row scales (4 bytes) into a shared-memory ring with
+      // asynchronous copies that land in the order the promotion threads read; the copies
+      // themselves signal the chunk's barrier, so the warp runs up to a ring ahead and
+      // global-memory latency stays hidden.
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
       // Byte offsets of this lane's column and row within a 32-float block of a ring slot.

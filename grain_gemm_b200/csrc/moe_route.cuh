@@ -432,9 +432,9 @@ silu_table_kernel(float* silu_table, int half_output) {
 }
 
 // Activation rows and their scales in sorted-slot order, for the valid slots only:
-// sorted_x[slot, :] = x[order[slot] / top_k, :] and likewise for the row scales (the
-// pre-sorted mode of the fused Gate/Up kernel, kept for measurements against the row-gather
-// mode).  One warp per slot; a row is `hidden` bytes (a multiple of 256) moved as 16-byte vectors.
+// sorted_x[slot, :] = x[order[slot] / top_k, :] and likewise for the row scales (what the fused
+// Gate/Up kernel reads unless it fetches the rows by index itself).  One warp per slot; a row is
+// `hidden` bytes (a multiple of 256) moved as 16-byte vectors.
 // Bound by HBM (S * H bytes written; the reads repeat top_k times and hit L2).  A lane keeps
 // eight loads in flight, and the token of the warp's next slot is fetched ahead: with one load
 // at a time the copy of 131072 rows of 7168 bytes took 301 us, a little under half the copy rate.
