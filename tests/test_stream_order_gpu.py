@@ -143,3 +143,51 @@ def test_moe_stages_without_any_wait(tokens, experts, top_k):
         return call
 
     _compare(_chained(inputs, stages(moe.MoEWorkspace())), _alone(inputs, stages(None)))
+
+
+# The predecessor in time is on another stream: an event stands between the two, in eager calls and
+# as a second dependency of the first captured kernel.
+@pytest.mark.parametrize("captured", [False, True])
+def test_operands_written_on_another_stream(captured):
+    from grain_gemm_b200 import int8_gemm, quantize_rows
+    rows, n, k = 200, 1056, 2304
+    generator = torch.Generator(device="cuda").manual_seed(5)
+    b = _weights((n, k), generator).t()
+    scale_b = torch.rand((k // 256, n), device="cuda", generator=generator)
+    inputs = [torch.randn((rows, k), device="cuda", generator=generator) * (1 + i) for i in range(8)]
+    big = torch.randn((4096, 4096), device="cuda", generator=generator)
+    x, source, early = torch.empty_like(inputs[0]), torch.empty_like(inputs[0]), torch.empty_like(inputs[0])
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def step():
+        side.wait_stream(main)
+        quantize_rows(early)                       # a kernel of this package right before the join
+        with torch.cuda.stream(side):
+            product = big @ big                    # keeps the side stream busy for a while
+            torch.add(source, product[0, 0] * 0, out=x)
+        main.wait_stream(side)
+        q, scale = quantize_rows(x)
+        return q, scale, int8_gemm(q, b, scale, scale_b)
+
+    expected = []
+    for value in inputs:
+        q, scale = quantize_rows(value)
+        expected.append([q, scale, int8_gemm(q, b, scale, scale_b)])
+    early.copy_(inputs[0])
+    source.copy_(inputs[0])
+    torch.cuda.synchronize()
+    results = []
+    with torch.cuda.stream(main):
+        step()
+        main.synchronize()
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=main):
+                outputs = step()
+        for value in inputs:
+            source.copy_(value)
+            if captured:
+                graph.replay()
+            results.append([t.clone() for t in (outputs if captured else step())])
+    torch.cuda.synchronize()
+    _compare(results, expected)
