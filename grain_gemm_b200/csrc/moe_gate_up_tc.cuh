@@ -24,6 +24,9 @@
 //   warps 0-7 promotion per K group, then SwiGLU (silu by table lookup); the first sub-tile's h
 //             is parked in shared memory until the second sub-tile supplies the other half of
 //             the row maximum.
+// After the K loops of an item the promotion warps apply SwiGLU and requantise, 9000 cycles a sub-tile
+// when every code took two conversion instructions (loop: 25 700 cycles at H = 4096), 6700 with the
+// sequence of RowQuantizer (512 tokens over 128 experts, H = 2048, I = 768: 95.7 to 88.0 us a launch).
 // What bounds it: for many rows the promotion warps' issue slots (see gemm_tc.cuh; the same loop
 // took 4096 tokens over 8 experts, H = 4096, I = 14336, from 996 to 886 us and 16384 tokens over
 // 256 experts, H = 7168, I = 2048, from 4650 to 4270 us), for few rows the weights' way from HBM:
@@ -541,9 +544,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             if constexpr (kPair) {
               row_max = fmaxf(row_max, amax_part[((item_parity * 2 + (sub ^ 1)) * 2 + half) * 128 + tile_row]);
             }
-            const float scale = quantize_scale(row_max);
-            const bool by_fma = quantize_division_is_safe(row_max);
-            const float y = __frcp_rn(scale);
+            const RowQuantizer quantizer(row_max);
             const int row = first_row + 8 * r;
             const bool row_stored = all_ok && row < row_end;
             int8_t* q_row = p.q + static_cast<long long>(row) * p.intermediate + jg * 256;
@@ -562,15 +563,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 }
               }
               uint32_t code[16];
-              if (by_fma) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k)
-                  code[k] = static_cast<uint32_t>(quantize_value_by_fma(v[k], scale, y)) & 0xffu;
-              } else {
-#pragma unroll
-                for (int k = 0; k < 16; ++k)
-                  code[k] = static_cast<uint32_t>(quantize_value(v[k], scale)) & 0xffu;
-              }
+              quantizer.codes(v, code);
               int8_t* q_piece = q_row + (kPair ? sub : piece) * 128 + half * 64;
               // Lane `quad` stores the eight channels 32*b + 8*quad .. +7: with kPair it holds them,
               // else an exchange inside the quad brings them, the first four in the low bytes.
@@ -578,10 +571,10 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
               for (int b = 0; b < 2; ++b) {
                 uint32_t w[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = code[b * 8 + 2 * i] | (code[b * 8 + 2 * i + 1] << 8);
+                for (int i = 0; i < 4; ++i) w[i] = __byte_perm(code[b * 8 + 2 * i], code[b * 8 + 2 * i + 1], 0x0040);
                 uint2 packed;
                 if constexpr (kPair) {
-                  packed = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+                  packed = make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
                 } else {
                   quad_transpose(w, quad);
                   const uint32_t front = __byte_perm(w[0], w[1], 0x5140);
@@ -592,7 +585,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
               }
             }
             if (row_stored && half == 0 && quad == 0 && (!kPair || sub == 0)) {
-              p.s[static_cast<long long>(row) * channel_groups + jg] = scale;
+              p.s[static_cast<long long>(row) * channel_groups + jg] = quantizer.scale;
             }
           }
         }

@@ -507,20 +507,54 @@ __device__ __forceinline__ int quantize_value(float h, float scale) {
 // correctly rounded quotient.  It needs every intermediate to stay normal; the caller tests
 // the row's range and falls back to the library division outside it, so codes always equal
 // those of __fdiv_rn.
-__device__ __forceinline__ float divide_by_fma(float n, float d, float y) {
-  float q = __fmul_rn(n, y);
-  q = __fmaf_rn(__fmaf_rn(-d, q, n), y, q);  // now within 1 ulp
-  return __fmaf_rn(__fmaf_rn(-d, q, n), y, q);
+//
+// Rounding to an integer needs no conversion instruction either (two a value, on a unit of 16 lanes a
+// clock, were what the requantisation waited for): adding 1.5 * 2^23 rounds to nearest even at units
+// and leaves the integer in the low bits.  |h| <= row maximum and scale >= (1 - 2^-24) max / 127 bound
+// the quotient by 127.00001, so the upper clamp has nothing to do; the lower one turns NaN into
+// -127, as it does in quantize_value.
+//
+// Two values at a time; the codes are the low bytes of the returned words.
+__device__ __forceinline__ float2 quantize_pair_by_fma(float2 h, float2 minus_scale, float2 y) {
+  float2 q = __fmul2_rn(h, y);
+  q = __ffma2_rn(__ffma2_rn(minus_scale, q, h), y, q);  // now within 1 ulp
+  q = __ffma2_rn(__ffma2_rn(minus_scale, q, h), y, q);
+  q.x = fmaxf(q.x, -127.0f);
+  q.y = fmaxf(q.y, -127.0f);
+  return __fadd2_rn(q, make_float2(12582912.0f, 12582912.0f));
 }
 // Row scales for which h / scale may use the sequence with y = __frcp_rn(scale): quotients
 // of magnitude >= 1/4 then have normal residuals, and smaller ones round to 0 either way.
 __device__ __forceinline__ bool quantize_division_is_safe(float row_max) {
   return row_max < 1.0e30f;  // also false for NaN and infinity
 }
-__device__ __forceinline__ int quantize_value_by_fma(float h, float scale, float y) {
-  const float rounded = nearbyintf(divide_by_fma(h, scale, y));
-  return static_cast<int>(fminf(fmaxf(rounded, -127.0f), 127.0f));
-}
+// Codes of two values of a row (low byte of each word), as quantize_value gives them.
+struct RowQuantizer {
+  float scale;
+  bool by_fma;
+  float2 minus_scale, y;
+  __device__ __forceinline__ explicit RowQuantizer(float row_max) {
+    scale = quantize_scale(row_max);
+    by_fma = quantize_division_is_safe(row_max);
+    const float reciprocal = __frcp_rn(scale);
+    minus_scale = make_float2(-scale, -scale);
+    y = make_float2(reciprocal, reciprocal);
+  }
+  template <int kCount>
+  __device__ __forceinline__ void codes(const float (&v)[kCount], uint32_t (&code)[kCount]) const {
+    if (by_fma) {
+#pragma unroll
+      for (int k = 0; k < kCount; k += 2) {
+        const float2 pair = quantize_pair_by_fma(make_float2(v[k], v[k + 1]), minus_scale, y);
+        code[k] = __float_as_uint(pair.x);
+        code[k + 1] = __float_as_uint(pair.y);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kCount; ++k) code[k] = static_cast<uint32_t>(quantize_value(v[k], scale));
+    }
+  }
+};
 
 // Router front-end: per token, the top_k largest of E logits (ties to the lower expert id,
 // ids in descending order of logit, like torch.topk on distinct values) and their routing
@@ -630,9 +664,9 @@ route_topk_single_kernel(const InT* logits, float* weights, const RouteParams p)
 // Eight consecutive values per lane (16 bytes of BF16/FP16, 32 of FP32); a group of G values
 // is G/8 neighbouring lanes, so a warp covers 256/G groups of one row at a time.  HBM bound:
 // sizeof(InT) bytes read and one byte (+ 4/G) written per element.  A warp requests kItems
-// 256-value chunks before it works on the first, and the codes divide by the guarded FMA
-// sequence: with one chunk per warp and library divisions (a branch each) 16384 rows of 7168
-// BF16 values took 190 us, 1.9 TB/s.
+// 256-value chunks before it works on the first, and the codes come from the guarded FMA
+// sequence (see RowQuantizer).  16384 rows of 7168 BF16 values: 190 us with one chunk per warp and
+// library divisions, 140 us with conversion instructions behind the sequence, 114 us (3.1 TB/s) now.
 template <typename InT, int kItems>
 __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const InT* x, long long rows, int width, int group, int8_t* q, float* s) {
@@ -667,22 +701,16 @@ quantize_rows_kernel(const InT* x, long long rows, int width, int group, int8_t*
     for (int offset = group / 16; offset > 0; offset >>= 1) {
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, offset));
     }
-    const float scale = quantize_scale(amax);
-    uint32_t packed[2] = {0u, 0u};
-    if (quantize_division_is_safe(amax)) {
-      const float y = __frcp_rn(scale);
+    const RowQuantizer quantizer(amax);
+    uint32_t code[8], packed[2];
+    quantizer.codes(v, code);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        packed[j >> 2] |= (static_cast<uint32_t>(quantize_value_by_fma(v[j], scale, y)) & 0xffu) << (8 * (j & 3));
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        packed[j >> 2] |= (static_cast<uint32_t>(quantize_value(v[j], scale)) & 0xffu) << (8 * (j & 3));
-      }
+    for (int j = 0; j < 2; ++j) {
+      packed[j] = __byte_perm(__byte_perm(code[4 * j], code[4 * j + 1], 0x0040),
+                              __byte_perm(code[4 * j + 2], code[4 * j + 3], 0x0040), 0x5410);
     }
     *reinterpret_cast<uint2*>(q + (first + i) * 256 + lane * 8) = make_uint2(packed[0], packed[1]);
-    if ((lane & (group / 8 - 1)) == 0) s[((first + i) * 256 + lane * 8) / group] = scale;
+    if ((lane & (group / 8 - 1)) == 0) s[((first + i) * 256 + lane * 8) / group] = quantizer.scale;
   }
 }
 
