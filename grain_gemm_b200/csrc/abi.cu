@@ -340,6 +340,13 @@ static int launch_tc_dtype(const CUtensorMap& map_a, const CUtensorMap& map_b, c
   }
 }
 
+// Rows of the blocks in which the kernel for tiles of `bn` columns takes the weight.
+static int weight_row_block(int bn, int out_dtype) {
+  const int bytes = out_dtype == GG_OUT_FP32 ? 4 : 2;
+  return bn == 256 ? GemmTcShape<1, 256, 4>::row_block(bytes)
+         : bn == 128 ? GemmTcShape<1, 128, 6>::row_block(bytes) : GemmTcShape<1, 64, 8>::row_block(bytes);
+}
+
 static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   const bool pair = variant == GG_VARIANT_TC_PAIR_N256 || variant == GG_VARIANT_TC_PAIR_N128;
   const int bn = (variant == GG_VARIANT_TC_N256 || variant == GG_VARIANT_TC_PAIR_N256) ? 256
@@ -348,8 +355,10 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   CUtensorMap map_a, map_b;
   int status = row_map(encode_tiled_fn(), &map_a, g.a, g.m, g.k, g.a_sm, 128);
   if (status) return status;
-  bool permuted = g.n % 32 == 0;
-  status = weight_row_map(encode_tiled_fn(), &map_b, g.b, g.n, g.k, g.b_sn, pair ? bn / 2 : bn, &permuted);
+  const int row_block = weight_row_block(bn, g.out_dtype);
+  bool permuted = g.n % row_block == 0;
+  status = weight_row_map(encode_tiled_fn(), &map_b, g.b, g.n, g.k, g.b_sn, pair ? bn / 2 : bn, &permuted,
+                          row_block);
   if (status) return status;
   GemmTcParams p = {};
   p.scale_a = static_cast<const float*>(g.scale_a);
@@ -934,9 +943,10 @@ int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_
     const long long used_tiles = assignments < tile_capacity ? assignments : tile_capacity;
     int bn = hidden >= 256 ? 256 : hidden >= 128 ? 128 : 64;
     while (bn > 64 && used_tiles * ((hidden + bn / 2 - 1) / (bn / 2)) <= gg::sm_count()) bn /= 2;
-    bool permuted = hidden % 32 == 0;
+    const int row_block = gg::weight_row_block(bn, out_dtype);
+    bool permuted = hidden % row_block == 0;
     status = gg::weight_row_map(gg::encode_tiled_fn(), &map_b, w2, static_cast<long long>(experts) * hidden,
-                                intermediate, intermediate, bn, &permuted);
+                                intermediate, intermediate, bn, &permuted, row_block);
     if (status) return status;
     gg::GemmTcParams p = {};
     p.scale_a = static_cast<const float*>(s);

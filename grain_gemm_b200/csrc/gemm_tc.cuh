@@ -83,8 +83,8 @@ struct GemmTcParams {
   // the INT32 group dots go to partials[Q][M][N] instead of being promoted (a second kernel
   // then folds them in group order).  k_splits == 1 and partials == null otherwise.
   int band_rows;               // row tiles per scheduling band
-  // N is a multiple of 32 and map_b delivers every block of 32 weight rows in fragment order
-  // (weight_row_map); otherwise the rows arrive in their own order.
+  // N is a multiple of the row block and map_b delivers the blocks in fragment order (weight_row_map);
+  // otherwise the rows arrive in their own order.
   int permuted_columns;
   int sb_vectors;              // permuted_columns, and scale_b may be read 16 bytes at a time
   int k_splits;
@@ -130,6 +130,8 @@ struct GemmTcShape {
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleBytes + kBarrierBytes;
   static constexpr int kThreads = (kPromoWarps + 4) * 32;   // + producer, MMA, two spares
   static constexpr int kColumnsPerThread = BN / (kPromoWarps / 4);
+  // Weight rows come in blocks of this many for outputs of `bytes` bytes (see the drain layout below).
+  static constexpr int row_block(int bytes) { return bytes == 2 && kColumnsPerThread >= 64 ? 64 : 32; }
   static constexpr int kDrainWidth = kPromoWarps == 16 ? 16 : 32;  // columns per tcgen05.ld
   static constexpr int kPromoRegisters = kPromoWarps == 16 ? 104 : GG_PROMO_REGS;
   static constexpr int kAuxRegisters = kPromoWarps == 16 ? 48 : GG_AUX_REGS;
@@ -188,28 +190,38 @@ __device__ __forceinline__ TileWork decode_tile(const GemmTcParams& p, int tile,
 // with eight warps draining 128 lanes x 256 columns: 16x128b delivers 507 B/clk/SM, 32x32b 940,
 // and 16x256b, which would give adjacent column pairs, 256.
 //
-// A row leaves as 16-byte stores of consecutive columns, so thread q wants the outputs
-// 8q .. 8q + 7 of a block in its eight columns 4k + q.  Weight row 8q + k therefore has to sit in
-// row 4k + q of the B tile's block, and the tensor map does that on the way in: it presents the
-// weight as [N/32][k = 8][q = 4][K] (weight_row_map in tensor_map.cuh), and accumulator pair j holds the
-// outputs 8q + 2j and 8q + 2j + 1.  Nothing is exchanged between lanes and the scales are used in
-// their own order.  (With rows in their own order, pair j holds outputs 8j + q and 8j + 4 + q and a
-// 4x4 exchange inside every quad precedes the stores: 64 shuffles and 600 instructions a
-// warp and tile.  Widths that are not a multiple of 32 do that.)
+// A row leaves as 32-byte stores, four lanes covering 128 consecutive bytes (one cache line) of it:
+// thread q wants 16 consecutive 16-bit outputs, or eight FP32 ones.  So the tensor map permutes the
+// weight's rows on the way in, in blocks of 64 or 32 (weight_row_map in tensor_map.cuh): the block's
+// row 16q + 8b + k (FP32: 8q + k) comes to TMEM column 32b + 4k + q, accumulator pair j of the block's
+// half b holds the outputs 16q + 8b + 2j and + 1, and nothing is exchanged between lanes.
+// The stores are bound by the cache lines that a warp's instruction touches: with 16-byte stores (eight
+// half lines an instruction) the tile of 128 x 256 16-bit outputs took 3100 to 3700 cycles, as long as
+// two or three K groups; the grouped Down projection of 512 tokens over 128 experts (H = 2048, three groups
+// a tile) went from 50.7 to 41.8 us, 256 x 4096 x 4096 with FP32 outputs from 11.5 to 10.9 us.  Widths that are not a multiple of the block take the rows in their own order,
+// where pair j holds the columns 8j + q and 8j + 4 + q of 32 and a 4x4 exchange inside every quad
+// precedes 16-byte stores.
 //
-// Position of block column `c` (0..31) in the scale ring for rows in their own order: thread q
-// reads its eight column scales, in accumulator-pair order, as two 16-byte vectors at q * 8.
-__device__ __forceinline__ int ring_column_position(int c) {
-  return (c & 3) * 8 + (c >> 3) * 2 + ((c >> 2) & 1);
+// Byte offset in a scale slot of thread q's eight column scales, in accumulator-pair order, for the
+// 32-column block `block`, less q times column_quad_bytes: the order in which permuted rows' scales
+// lie in memory anyway.
+template <int kRowBlock>
+__host__ __device__ constexpr int column_block_bytes(int block) {
+  return kRowBlock == 64 ? (block >> 1) * 256 + (block & 1) * 32 : block * 128;
+}
+template <int kRowBlock>
+__host__ __device__ constexpr int column_quad_bytes() { return kRowBlock == 64 ? 64 : 32; }
+// Byte offset of column `c` (0..31) of a 32-column block from column_block_bytes, rows in their own order.
+template <int kRowBlock>
+__device__ __forceinline__ int ring_column_bytes(int c) {
+  return (c & 3) * column_quad_bytes<kRowBlock>() + 4 * ((c >> 3) * 2 + ((c >> 2) & 1));
 }
 // Position of row `r` (0..31 within its warp's 32 rows): the thread with row index
 // lane / 4 = r % 8 reads its four rows r % 8 + 8j as one 16-byte vector.
 __device__ __forceinline__ int ring_row_position(int r) { return (r & 7) * 4 + (r >> 3); }
 
-// The eight column scales (four pairs) of this thread for one 32-column block.
-__device__ __forceinline__ void load_column_scales(const float* block_base, int quad,
-                                                   float2 (&sb)[4]) {
-  const uint32_t address = smem_u32(block_base + quad * 8);
+// The eight column scales (four pairs) of this thread for one 32-column block, by shared address.
+__device__ __forceinline__ void load_column_scales(uint32_t address, float2 (&sb)[4]) {
   const float4 lo = lds_f32x4(address);
   const float4 hi = lds_f32x4(address + 16);
   sb[0] = make_float2(lo.x, lo.y);
@@ -293,6 +305,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                const GemmTcParams p) {
   using Shape = GemmTcShape<kCtaGroup, BN, kStages, kPromoWarps, kARows>;
   constexpr int kNC = Shape::kColumnsPerThread;   // columns owned by one promotion thread
+  constexpr int kRowBlock = Shape::row_block(sizeof(OutT));
   constexpr int kProducerWarp = kPromoWarps, kMmaWarp = kPromoWarps + 1;
   constexpr int kScaleWarp = kPromoWarps + 2;
 
@@ -390,7 +403,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         row_a = (tm * kCtaGroup + static_cast<int>(cta_rank)) * Shape::kBM;
         row_b = tn * BN + static_cast<int>(cta_rank) * Shape::kBRows;
       }
-      const int b_c1 = p.permuted_columns ? 0 : row_b, b_c3 = p.permuted_columns ? row_b >> 5 : 0;
+      const int b_c1 = p.permuted_columns ? 0 : row_b;
+      const int b_c3 = p.permuted_columns ? row_b / kRowBlock : 0;
       for (int slab = 0, x = work.k_begin; slab < work.slabs; ++slab, x += Shape::kBK) {
         if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, kSiteProducerEmpty, abort_flag)) {
           ok = false;
@@ -536,7 +550,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // waiting for scales).
     constexpr int kColumnsPerLane = BN / 32;
     // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-    const uint32_t column_position = 4 * (p.permuted_columns ? lane : ring_column_position(lane));
+    // (Rows in fragment order keep their scales in memory order, otherwise they go to where the
+    // promotion threads look for the columns they hold.)
+    const uint32_t column_position = p.permuted_columns ? 4 * lane : ring_column_bytes<kRowBlock>(lane);
+    const uint32_t odd_block = p.permuted_columns ? 128 : column_block_bytes<kRowBlock>(1);
     const uint32_t row_position = 4 * ring_row_position(lane);
     const uint32_t ring_base = smem_u32(scale_ring);
     uint32_t chunk = 0, phase = 0;
@@ -588,7 +605,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           } else {
 #pragma unroll
             for (int j = 0; j < kColumnsPerLane; ++j, sb_source += sb_step) {
-              cp_async_f32(destination + 128 * j + column_position, sb_source, 32 * j < columns_left);
+              cp_async_f32(destination + 256 * (j >> 1) + (j & 1 ? odd_block : 0) + column_position, sb_source,
+                           32 * j < columns_left);
             }
             sb_source += sb_next;
           }
@@ -745,7 +763,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                               kSiteEpilogueTmemFull, abort_flag);
         }
         tcgen05_fence_after();
-        const float* sb_columns = scale_slot_base + col_base;
+        const uint32_t sb_columns =
+            smem_u32(scale_slot_base + col_base) + (lane & 3) * column_quad_bytes<kRowBlock>();
         const uint32_t taddr_low =
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buffer * BN + col_base;
         const uint32_t taddr_high = taddr_low + (16u << 16);
@@ -759,7 +778,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           for (int fragment = 0; fragment < 2 * kBlocks; ++fragment) {
             const int block = fragment >> 1;
             const int high_half = fragment & 1;
-            if (!high_half) load_column_scales(sb_columns + block * 32, lane & 3, sb);
+            if (!high_half) load_column_scales(sb_columns + column_block_bytes<kRowBlock>(block), sb);
             tmem_ld_wait();
             if (fragment + 1 < 2 * kBlocks) {
               const uint32_t next = ((fragment + 1) & 1 ? taddr_high : taddr_low) +
@@ -794,27 +813,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           }
         }
       }
-      // Lane q stores the eight consecutive columns 8q..8q+7 of each 32-column block: a quarter of
-      // the store instructions and of the memory-pipe wavefronts of pair stores.
+      // Lane q stores 32 consecutive bytes of a block at a time (see the drain layout above).
       if (ok) {
         const bool exchange = p.permuted_columns == 0;
         const int quad = lane & 3;
         const int first_row = row - row_in_cta + quarter * 32 + fragment_row;
         const bool aligned = p.c_vector_ok != 0;
-        // Destination addresses of this thread's four rows and of the four rows of the lane it
-        // exchanges with, fetched in one batch before the first store: a load issued between
-        // the stores would wait behind them (the compiler must assume they alias), one round
-        // trip per row instead of one per tile.
+        // Destination addresses of this thread's four rows, fetched in one batch before the first
+        // store: a load issued between the stores would wait behind them (the compiler must assume
+        // they alias), one round trip per row instead of one per tile.
         [[maybe_unused]] unsigned long long own_destination[4] = {0ull, 0ull, 0ull, 0ull};
-        [[maybe_unused]] unsigned long long other_destination[4] = {0ull, 0ull, 0ull, 0ull};
         if constexpr (kGrouped) {
           if (p.row_destination != nullptr) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
               const int out_row = first_row + 8 * r;
-              const int partner_row = out_row + (fragment_row < 4 ? 4 : -4);
               if (out_row < row_limit) own_destination[r] = __ldg(p.row_destination + out_row);
-              if (partner_row < row_limit) other_destination[r] = __ldg(p.row_destination + partner_row);
             }
           }
         }
@@ -830,58 +844,32 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               c_row = reinterpret_cast<OutT*>(own_destination[r]);
             }
           }
-          if constexpr (kGrouped && sizeof(OutT) == 2 && kBlocks % 2 == 0) {
-            // Rows that leave for another GPU's memory: lanes 16 apart (rows 4 apart) swap one
-            // of two neighbouring blocks, so that a store instruction covers four rows with 128
-            // contiguous bytes each instead of eight rows with 64; a link carries full cache
-            // lines better than halves.  All conditions are the same in every lane.
-            if (p.row_destination != nullptr && aligned && n0 + col_base + kNC <= p.n) {
-              const bool low = fragment_row < 4;
-              const unsigned long long partner_destination = other_destination[r];
+          // Columns are whole 32-byte pieces from the start of the row on (permuted rows: N is a
+          // multiple of the block).
+          const bool wide = aligned && !exchange && (reinterpret_cast<uintptr_t>(c_row) & 31) == 0;
+          if constexpr (sizeof(OutT) == 2) {
+            if constexpr (kRowBlock == 64) {
+              if (wide) {
 #pragma unroll
-              for (int block = 0; block < kBlocks; block += 2) {
-                uint32_t w[2][4];
+                for (int block = 0; block < kBlocks; block += 2) {
+                  const int col = n0 + col_base + block * 32 + 16 * quad;
+                  uint32_t w[8];
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-#pragma unroll
-                  for (int i = 0; i < 4; ++i) w[half][i] = pack_pair<OutT>(acc[r][(block + half) * 4 + i]);
-                  if (exchange) own_order_exchange(w[half], quad);
+                  for (int i = 0; i < 8; ++i) w[i] = pack_pair<OutT>(acc[r][block * 4 + i]);
+                  if (row_stored && col < p.n) store_global_32(c_row + col, w);
                 }
-                // Low lanes keep block `block` and give away the next one, high lanes the reverse.
-                uint32_t received[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  received[i] = __shfl_xor_sync(0xffffffffu, low ? w[1][i] : w[0][i], 16);
-                }
-                const int col = n0 + col_base + (block + (low ? 0 : 1)) * 32 + 8 * quad;
-                // First the rows of the low lanes, then the rows of the high lanes.
-                const unsigned long long first = low ? reinterpret_cast<unsigned long long>(c_row)
-                                                     : partner_destination;
-                const unsigned long long second = low ? partner_destination
-                                                      : reinterpret_cast<unsigned long long>(c_row);
-                const bool first_stored = low ? row_stored : partner_destination != 0ull;
-                const bool second_stored = low ? partner_destination != 0ull : row_stored;
-                const uint4 own = low ? make_uint4(w[0][0], w[0][1], w[0][2], w[0][3])
-                                      : make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
-                const uint4 other = make_uint4(received[0], received[1], received[2], received[3]);
-                if (first_stored) {
-                  *reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(first) + col) = low ? own : other;
-                }
-                if (second_stored) {
-                  *reinterpret_cast<uint4*>(reinterpret_cast<OutT*>(second) + col) = low ? other : own;
-                }
+                continue;
               }
-              continue;
             }
-          }
 #pragma unroll
-          for (int block = 0; block < kBlocks; ++block) {
-            const int col = n0 + col_base + block * 32 + 8 * quad;
-            if constexpr (sizeof(OutT) == 2) {
+            for (int block = 0; block < kBlocks; ++block) {
               uint32_t w[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) w[i] = pack_pair<OutT>(acc[r][block * 4 + i]);
               if (exchange) own_order_exchange(w, quad);
+              const int col = n0 + col_base +
+                              (exchange || kRowBlock == 32 ? block * 32 + 8 * quad
+                                                           : (block & ~1) * 32 + 16 * quad + (block & 1) * 8);
               if (row_stored) {
                 if (aligned && col + 8 <= p.n) {
                   *reinterpret_cast<uint4*>(c_row + col) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -894,32 +882,45 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                   }
                 }
               }
-            } else {
-              uint32_t wx[4], wy[4];
+            }
+          } else {
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                wx[i] = __float_as_uint(acc[r][block * 4 + i].x);
-                wy[i] = __float_as_uint(acc[r][block * 4 + i].y);
-              }
+            for (int block = 0; block < kBlocks; ++block) {
+              const int col = n0 + col_base + block * 32 + 8 * quad;
+              uint32_t w[8];   // columns col .. col + 7
               if (exchange) {
+                uint32_t wx[4], wy[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  wx[i] = __float_as_uint(acc[r][block * 4 + i].x);
+                  wy[i] = __float_as_uint(acc[r][block * 4 + i].y);
+                }
                 quad_transpose(wx, quad);
                 quad_transpose(wy, quad);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  w[i] = wx[i];
+                  w[4 + i] = wy[i];
+                }
               } else {
-                const uint32_t x1 = wx[1], x2 = wx[2], x3 = wx[3], y0 = wy[0], y1 = wy[1], y2 = wy[2];
-                wx[1] = y0; wx[2] = x1; wx[3] = y1;
-                wy[0] = x2; wy[1] = y2; wy[2] = x3;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  w[2 * i] = __float_as_uint(acc[r][block * 4 + i].x);
+                  w[2 * i + 1] = __float_as_uint(acc[r][block * 4 + i].y);
+                }
               }
               if (row_stored) {
-                if (aligned && col + 8 <= p.n) {
+                if (wide) {
+                  if (col < p.n) store_global_32(c_row + col, w);
+                } else if (aligned && col + 8 <= p.n) {
                   uint4* out = reinterpret_cast<uint4*>(c_row + col);
-                  out[0] = make_uint4(wx[0], wx[1], wx[2], wx[3]);
-                  out[1] = make_uint4(wy[0], wy[1], wy[2], wy[3]);
+                  out[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                  out[1] = make_uint4(w[4], w[5], w[6], w[7]);
                 } else {
                   uint32_t* out = reinterpret_cast<uint32_t*>(c_row);
 #pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    if (col + j < p.n) out[col + j] = wx[j];
-                    if (col + 4 + j < p.n) out[col + 4 + j] = wy[j];
+                  for (int j = 0; j < 8; ++j) {
+                    if (col + j < p.n) out[col + j] = w[j];
                   }
                 }
               }

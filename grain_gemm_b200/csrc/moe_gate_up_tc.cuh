@@ -267,7 +267,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
       // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-      const uint32_t column_position = 4 * (kPair ? lane : ring_column_position(lane));
+      const uint32_t column_position = kPair ? 4 * lane : ring_column_bytes<32>(lane);
       const uint32_t row_position = 4 * ring_row_position(lane);
       const uint32_t ring_base = smem_u32(sb_ring);
       const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale
@@ -446,7 +446,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 #pragma unroll
           for (int fragment = 0; fragment < 8; ++fragment) {
             const int block = fragment >> 1;
-            if ((fragment & 1) == 0) load_column_scales(slot + block_column(block), quad, sb);
+            if ((fragment & 1) == 0) load_column_scales(smem_u32(slot + block_column(block) + quad * 8), sb);
             tmem_ld_wait();
             if (fragment + 1 < 8) {
               const uint32_t next = ((fragment + 1) & 1 ? taddr_high : taddr_low) +

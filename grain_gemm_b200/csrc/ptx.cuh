@@ -217,6 +217,13 @@ __device__ __forceinline__ float4 lds_f32x4(uint32_t smem_address) {
   return v;
 }
 
+// 32 bytes to global memory in one instruction (the address is a multiple of 32).
+__device__ __forceinline__ void store_global_32(void* address, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(address), "r"(w[0]),
+               "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
+}
+
 // ---------------------------------------------------------------- cp.async (scale staging)
 
 // Asynchronous 4-byte copy global -> shared; `valid == false` writes zero without reading.

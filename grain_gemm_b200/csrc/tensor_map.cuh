@@ -35,25 +35,27 @@ static inline int row_map(EncodeTiledFn encode, CUtensorMap* map, const void* ba
 }
 
 // Tensor map over the rows of a weight matrix, boxes of 128 bytes x box_rows.  With `permuted` (asked for
-// only where rows and box_rows are multiples of 32) every block of 32 rows is delivered in the
-// order the epilogue's fragments want: row 8q + k of the block lands in row 4k + q of the tile (see
-// gemm_tc.cuh).  The kernels load with coordinates (x, 0, 0, row / 32) then, with (x, row, 0, 0)
-// otherwise.
+// only where rows and box_rows are multiples of `block`, 32 or 64) every block of rows is delivered in
+// the order the epilogue's fragments want: row (block / 4) * q + k of the block lands in row 4k + q of
+// the tile (see gemm_tc.cuh).  The kernels load with coordinates (x, 0, 0, row / block) then, with
+// (x, row, 0, 0) otherwise.
 //
-// The permuted map steps 8 rows in its second dimension and 1 row in its third.  The driver API's
+// The permuted map steps 8 or 16 rows in its second dimension and 1 row in its third.  The driver API's
 // documentation asks that each stride be a multiple of the one before; the encoder of driver 580.159
 // does not enforce that and the copies deliver what the strides say (every bit-for-bit GEMM test
 // depends on it).  Because it is not promised, an encoder that refuses the map is answered with the
 // rows in their own order: `permuted` tells which of the two `map` is, and the kernels do the
 // exchange between lanes themselves then.
 static inline int weight_row_map(EncodeTiledFn encode, CUtensorMap* map, const void* base, long long rows,
-                                 long long cols, long long pitch, int box_rows, bool* permuted) {
+                                 long long cols, long long pitch, int box_rows, bool* permuted,
+                                 int block = 32) {
   const cuuint64_t columns = static_cast<cuuint64_t>(cols), step = static_cast<cuuint64_t>(pitch);
   const cuuint32_t box = static_cast<cuuint32_t>(box_rows);
   if (*permuted) {
-    const cuuint64_t dims[4] = {columns, 4, 8, static_cast<cuuint64_t>(rows / 32)};
-    const cuuint64_t strides[3] = {8 * step, step, 32 * step};
-    const cuuint32_t boxes[4] = {128u, 4u, 8u, box / 32};
+    const cuuint32_t run = static_cast<cuuint32_t>(block) / 4;
+    const cuuint64_t dims[4] = {columns, 4, run, static_cast<cuuint64_t>(rows / block)};
+    const cuuint64_t strides[3] = {run * step, step, 4 * run * step};
+    const cuuint32_t boxes[4] = {128u, 4u, run, box / (4 * run)};
     const int status = encode_bytes(encode, map, base, 4, dims, strides, boxes);
     if (status == 0) return 0;
     *permuted = false;

@@ -1,0 +1,41 @@
+"""How a finished tile leaves: 32-byte stores where columns and addresses allow them, narrower ones
+elsewhere.  Compared bit for bit with the CUDA-core kernel at the edges of the rule: widths that end
+within a tile, within a block of weight rows or within 16 bytes, and outputs that start at any alignment.
+"""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+M, K, G = 133, 272, 128
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("variant", ["tc_n64", "tc_n128", "tc_n256", "tc_pair_n128", "tc_pair_n256"])
+@pytest.mark.parametrize("n", [64, 320, 96, 224, 200, 77])
+def test_widths_and_alignments(n, variant, dtype):
+    from grain_gemm_b200 import _loader, gemm
+    gen = torch.Generator(device="cuda").manual_seed(n)
+
+    def draw(*shape):
+        return torch.randint(-127, 128, shape, dtype=torch.int8, device="cuda", generator=gen)
+
+    a, b = draw(M, K), draw(n, K).t()
+    sa = torch.rand((M, 3), device="cuda", generator=gen) / 127
+    # Column scales contiguous (16-byte copies), or every other one of a wider matrix.
+    wide = torch.rand((3, 2 * n), device="cuda", generator=gen) / 127
+    for sb in (wide[:, :n].contiguous(), wide[:, ::2]):
+        expected = gemm.launch(a, b, sa, sb, torch.empty((M, n), dtype=dtype, device="cuda"), G, "simt")
+        size = expected.element_size()
+        for offset in (0, 16, 8, 4):                        # bytes from a 32-byte boundary
+            for pitch in (0, 16, 4):                        # bytes between rows beyond the columns
+                columns = n + pitch // size
+                memory = torch.full((M * columns + 64,), 7.0, dtype=dtype, device="cuda")
+                first = (-memory.data_ptr() % 32 + offset) // size
+                out = memory[first:first + M * columns].view(M, columns)
+                gemm.launch(a, b, sa, sb, out[:, :n], G, variant)
+                assert torch.equal(out[:, :n], expected), (offset, pitch)
+                assert bool((out[:, n:] == 7.0).all()) and bool((memory[:first] == 7.0).all())
+                assert bool((memory[first + M * columns:] == 7.0).all())
+    assert _loader.device_status() == 0
