@@ -486,14 +486,13 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
                                  const CUtensorMap& map_up, const GateUpParams& p, long long items,
                                  cudaStream_t stream) {
   auto kernel = moe_gate_up_tc_kernel<RoundT, kGather, kPair>;
-  const cudaError_t error = cudaFuncSetAttribute(
-      kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GateUpShape::kSmemBytes);
+  constexpr int kCtas = kPair ? 2 : 1, kSmemBytes = kPair ? GateUpPairShape::kSmemBytes : GateUpShape::kSmemBytes;
+  const cudaError_t error = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (error != cudaSuccess) return finished(error);
-  constexpr int kCtas = kPair ? 2 : 1;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(sm_count() / kCtas * kCtas);
   config.blockDim = dim3(384);
-  config.dynamicSmemBytes = GateUpShape::kSmemBytes;
+  config.dynamicSmemBytes = kSmemBytes;
   config.stream = stream;
   cudaLaunchAttribute attribute[1];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -514,29 +513,30 @@ static int launch_gate_up_kernel(const CUtensorMap& map_x, const CUtensorMap& ma
   return finished(cudaLaunchKernelEx(&config, kernel, map_x, map_gate, map_up, p));
 }
 
-// Whole items go to single CTAs, or half an item to each CTA of a pair.  A pair finishes in half the
-// time but exchanges row maxima between its CTAs (4 % of an item), so it pays where whole items
-// fill their last wave badly: `tiles` (an estimate; the exact number is on the device) times the
-// channel groups, over the SMs.  Measured, Gate/Up with the rest of the call, single against pair:
-// 1 token over 8 of 128 experts (24 items) 52 and 46 us, 8 tokens, H = 4096, I = 14336, 8 experts
-// (448 items, 4 against 3.5 waves) 260 and 251 us, 256 tokens, I = 1536, 32 experts (192 items,
-// 2 against 1.5) 184 and 170 us, but 512 tokens, I = 768, 128 experts (384 items, 3 waves either
-// way) 176 and 188 us.  None of these lies near the line itself, which follows from the 4 %: a pair's
-// item counts 0.52 of a whole one.
-// Row tiles are estimated as one per expert while an expert has few rows, as full tiles and half a
-// tile of remainder per expert beyond; a call sized for a capacity (a rank of an expert-parallel step) is
-// estimated at that capacity, not at the rows it received.  Half the SMs is an upper bound on
-// the pairs that are resident at once (see resident_clusters), so on a part that holds fewer a size
-// near a wave's edge may go to pairs that need one wave more than counted here.
-// Only pairs take their weight rows in fragment order; for single CTAs, which amortise the
-// exchange over a whole item, it made no difference beyond the spread of the runs.
+// Whole items go to single CTAs, token rows on the tensor core's M side, or half an item to each CTA of a
+// pair, weight rows on the M side.  A pair takes half an item's time while the rows are few (one exchange
+// of row maxima against operand stages that hold weights only), and more of it the fuller the tiles
+// are: measured, time of a wave of pairs over one of single CTAs, H = 4096, I = 2048, 32 experts with
+// 8 / 32 / 48 / 64 / 96 rows each: 0.48, 0.50, 0.51, 0.52, 0.56 (93 against 97 us at 8 rows, 120 against 106
+// at 96; two single waves); H = 4096, I = 14336, 8 experts with 900: 0.54; H = 7168, I = 2048, 256 experts with
+// 512: 0.56.  So pairs pay where whole items fill their last wave badly: 1 token over 8 of 128 experts
+// (24 items, one wave either way) 12.0 against 23.2 us, 16 tokens, H = 4096, I = 14336, 8 experts (448 items,
+// 7 waves against 4) 155 against 182 us; 512 tokens, I = 768, 128 experts (384 items, 6 against 3) 86 against 87.
+// `tiles` is an estimate (the exact number is on the device): one row tile per expert while an expert
+// has few rows, full tiles and half a tile of remainder per expert beyond; a call sized for a
+// capacity (a rank of an expert-parallel step) is estimated at that capacity, not at the rows it
+// received.  Half the SMs is an upper bound on the pairs that are resident at once (see
+// resident_clusters), so on a part that holds fewer a size near a wave's edge may go to pairs that need
+// one wave more than counted here.
 static bool gate_up_pairs(long long slots, int experts, int channel_groups) {
   const long long spread = slots < experts ? slots : experts;
   const long long tiles = slots <= 64ll * experts ? spread : slots / 128 + experts / 2;
   const long long items = tiles * channel_groups;
   const int sms = sm_count(), pairs = sms / 2;
   const long long single_waves = (items + sms - 1) / sms, pair_waves = (items + pairs - 1) / pairs;
-  return pair_waves * 52 < single_waves * 100;
+  const long long rows = slots / (spread > 0 ? spread : 1);
+  const int percent = rows <= 8 ? 48 : rows <= 32 ? 50 : rows <= 64 ? 52 : 56;
+  return pair_waves * percent < single_waves * 100;
 }
 
 template <typename RoundT>
@@ -830,6 +830,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     uint8_t* scratch = static_cast<uint8_t*>(gate_up_scratch);
     gg::GateUpParams p = {};
     CUtensorMap map_x, map_gate, map_up;
+    const void* x_rows = x;   // what map_x covers
     int status;
     if (row_gather) {
       p.silu_table = reinterpret_cast<float*>(scratch);
@@ -851,6 +852,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
           static_cast<const long long*>(order), static_cast<const int*>(offsets), experts, top_k,
           hidden, sorted_x, sorted_scale, const_cast<float*>(p.silu_table), out_dtype == GG_OUT_FP16 ? 1 : 0);
       if (status) return status;
+      x_rows = sorted_x;
       status = gg::row_map(gg::encode_tiled_fn(), &map_x, sorted_x, slots, hidden, hidden, 128);
     }
     if (status) return status;
@@ -858,12 +860,25 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
       status = gg_moe_silu_table(const_cast<float*>(p.silu_table), out_dtype, stream_ptr);
       if (status) return status;
     }
-    // Pairs need their weight rows in fragment order; without such a map the item stays on one CTA.
+    // Pairs need their weight rows by channel; without such a map the item stays on one CTA.
     bool pairs = !row_gather && gg::gate_up_pairs(slots, experts, intermediate / 256);
-    status = gg::gate_up_row_maps(gg::encode_tiled_fn(), &map_gate, &map_up, w1,
-                                  static_cast<long long>(experts) * 2 * intermediate, hidden, interleaved != 0,
-                                  &pairs);
-    if (status) return status;
+    if (pairs) {
+      CUtensorMap map_rows;
+      pairs = gg::gate_up_channel_map(gg::encode_tiled_fn(), &map_gate, w1, experts, intermediate, hidden,
+                                      interleaved != 0) == 0 &&
+              gg::row_map(gg::encode_tiled_fn(), &map_rows, x_rows, slots, hidden, hidden, 16) == 0;
+      if (pairs) {
+        map_x = map_rows;
+        map_up = map_gate;
+      }
+    }
+    if (!pairs) {
+      bool permuted = false;
+      status = gg::gate_up_row_maps(gg::encode_tiled_fn(), &map_gate, &map_up, w1,
+                                    static_cast<long long>(experts) * 2 * intermediate, hidden, interleaved != 0,
+                                    &permuted);
+      if (status) return status;
+    }
     p.order = static_cast<const long long*>(order);
     p.top_k = top_k;
     p.scale_w = static_cast<const float*>(scale_w1);
@@ -874,7 +889,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     p.s = static_cast<float*>(s);
     p.hidden = hidden; p.intermediate = intermediate;
     p.max_tiles = tile_capacity; p.interleaved = interleaved;
-    p.sw_vectors = !interleaved && gg::aligned16(scale_w1);
+    p.sw_vectors = gg::aligned16(scale_w1);
     if (out_dtype == GG_OUT_BF16) {
       return gg::launch_gate_up_tc<__nv_bfloat16>(map_x, map_gate, map_up, p, slots, pairs, row_gather, stream);
     }

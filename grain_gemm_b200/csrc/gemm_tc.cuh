@@ -298,6 +298,21 @@ __device__ __forceinline__ void own_order_exchange(uint32_t (&w)[4], int q) {
   w[3] = __byte_perm(v2, v3, 0x7632);
 }
 
+// Entries of a row-tile list that are in use (they come first).  One warp probes 32 places at a time: two
+// rounds for 129 entries, three for 1280, where a binary search by one thread took 8 or 11, each a
+// memory latency in front of the kernel's first load.
+__device__ __forceinline__ int used_tiles(const int* tile_expert, int entries, int lane) {
+  int low = 0, high = entries;   // the first unused entry lies between them
+  while (low < high) {
+    const int step = (high - low + 31) / 32, probe = low + lane * step;
+    const int used = __popc(__ballot_sync(0xffffffffu, probe < high && tile_expert[probe] >= 0));
+    if (used == 0) return low;
+    high = min(high, low + used * step);
+    low += (used - 1) * step + 1;
+  }
+  return low;
+}
+
 template <int kCtaGroup, int BN, int kStages, typename OutT, bool kGrouped, int kPromoWarps,
           bool kDump = false, int kARows = 128>
 __global__ void __launch_bounds__((kPromoWarps + 4) * 32, 1)
@@ -359,14 +374,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // row it could receive, several times what it does receive.)
   __shared__ int used_row_tiles;
   if constexpr (kGrouped) {
-    if (threadIdx.x == 32) {
-      int low = 0, high = p.tiles_m;
-      while (low < high) {
-        const int middle = (low + high) >> 1;
-        if (p.tile_expert[middle] >= 0) low = middle + 1;
-        else high = middle;
-      }
-      used_row_tiles = low;
+    if (warp == 1) {
+      const int used = used_tiles(p.tile_expert, p.tiles_m, lane);
+      if (lane == 0) used_row_tiles = used;
     }
   }
   if constexpr (kCtaGroup == 2) cluster_sync_all();

@@ -16,48 +16,31 @@
 // whole box), so it is what the Python layer picks by default.
 //
 // Work item = (128-row tile of one expert, 256-channel group), processed as two sub-tiles of
-// 128 channels, one after the other or by a pair of CTAs; a sub-tile is one N = 256 accumulator
-// (128 gate + 128 up columns) in TMEM.
+// 128 channels, one after the other; a sub-tile is one N = 256 accumulator (128 gate + 128 up columns)
+// in TMEM.  Calls with few rows an expert take the form in moe_gate_up_pair.cuh where that is faster.
 //   warp 8    TMA producer: per stage the activation rows (one box, or 32 row gathers) and two weight boxes
 //   warp 9    MMA issuer (tcgen05.mma kind::i8, two TMEM buffers)
 //   warp 10   scale staging (cp.async of each K group's column and row scales into a shared-memory ring)
 //   warps 0-7 promotion per K group, then SwiGLU (silu by table lookup); the first sub-tile's h
 //             is parked in shared memory until the second sub-tile supplies the other half of
 //             the row maximum.
-// After the K loops of an item the promotion warps apply SwiGLU and requantise, 9000 cycles a sub-tile
-// when every code took two conversion instructions (loop: 25 700 cycles at H = 4096), 6700 with the
-// sequence of RowQuantizer (512 tokens over 128 experts, H = 2048, I = 768: 95.7 to 88.0 us a launch).
-// What bounds it: for many rows the promotion warps' issue slots (see gemm_tc.cuh; the same loop
-// took 4096 tokens over 8 experts, H = 4096, I = 14336, from 996 to 886 us and 16384 tokens over
-// 256 experts, H = 7168, I = 2048, from 4650 to 4270 us), for few rows the weights' way from HBM:
-// 16 tokens over 8 experts read 0.94 GB in 195 us (4.8 TB/s), held back by the last wave of items
-// (see gate_up_pairs in abi.cu), one token over 8 of 128 experts 25 MB in 19 us, 34 with whole
-// items on 24 CTAs.
+// What bounds it: the promotion warps.  A K group takes 1600 cycles (see gemm_tc.cuh), and after the K loops
+// of a sub-tile they leave it for SwiGLU (4400 cycles, the table look-ups) and the requantisation, which
+// took 4500 when every code cost two conversion instructions and takes 2200 with the sequence of
+// RowQuantizer (4096 tokens over 8 experts, H = 4096, I = 14336: 898 to 862 us; 512 over 128, H = 2048,
+// I = 768: 95.7 to 88.0 us; 16384 over 256, H = 7168, I = 2048: 4490 to 4420 us).
 #pragma once
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "gemm_tc.cuh"
+#include "moe_gate_up.cuh"
+#include "moe_gate_up_pair.cuh"
 #include "moe_route.cuh"
 #include "ptx.cuh"
 
 namespace gg {
-
-struct GateUpParams {
-  const float* row_scale;     // gathered: scale_x [T, H/256]; pre-sorted: [S, H/256] by sorted slot
-  const long long* order;     // [S] sorted slot -> flattened assignment (gathered mode)
-  int top_k;                  // assignment / top_k = token
-  const float* silu_table;    // [65536] silu of every value of the output type, by bit pattern
-  const float* scale_w;       // [E, H/256, 2I]
-  const int* expert_offsets;  // [E+1]
-  const int* tile_expert;     // [max_tiles]
-  const int* tile_row;        // [max_tiles]
-  int8_t* q;                  // [S, I]
-  float* s;                   // [S, I/256]
-  int hidden, intermediate, max_tiles, interleaved;
-  int sw_vectors;             // scale_w may be read 16 bytes at a time (split layout, aligned)
-};
 
 struct GateUpShape {
   static constexpr int kStages = 3;
@@ -70,39 +53,10 @@ struct GateUpShape {
   static constexpr int kScaleChunks = kScaleSlots / kScaleChunkGroups;
   static constexpr int kScaleBytes = kScaleSlots * kRingFloats * 4;
   static constexpr int kAmaxBytes = 2 * 4 * 128 * 4;   // two item parities x (sub, half) x 128 rows
-  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks + 8) * 8 + 16;
+  static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks) * 8 + 16;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kStashBytes + kScaleBytes +
                                     kAmaxBytes + kBarrierBytes;
 };
-
-// Work item -> (row tile, channel group).  Items of one expert are consecutive and ordered
-// channel-group-major: neighbouring CTAs work on different row tiles of the same expert
-// against the same 256-channel weight block, so that block is read from DRAM once and served
-// from L2 to the other row tiles.  Returns false for items past the last used tile.
-__device__ __forceinline__ bool gate_up_item(const GateUpParams& p, int item, int channel_groups,
-                                             int& tile, int& jg, int& expert) {
-  const int probe = item / channel_groups;
-  expert = p.tile_expert[probe];
-  if (expert < 0) return false;
-  const int begin = p.expert_offsets[expert];
-  const int rows = p.expert_offsets[expert + 1] - begin;
-  const int first = probe - (p.tile_row[probe] - begin) / 128;
-  const int span = (rows + 127) / 128;
-  const int local = item - first * channel_groups;
-  jg = local / span;
-  tile = first + local - jg * span;
-  return true;
-}
-
-// The two 16-bit floats of a packed pair as FP32 (exact).
-template <typename T>
-__device__ __forceinline__ float2 unpack_pair(uint32_t packed) {
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    return make_float2(__uint_as_float(packed << 16), __uint_as_float(packed & 0xffff0000u));
-  } else {
-    return __half22float2(*reinterpret_cast<const __half2*>(&packed));
-  }
-}
 
 // Token row of the tile row `row` (gathered mode); rows past the expert's last one read token 0,
 // whose data only feeds accumulator rows that are never stored.
@@ -119,14 +73,17 @@ __device__ __forceinline__ int gate_up_source_row(const GateUpParams& p, int row
 // 128 gate columns and then 128 up columns in either case and nothing behind the loads
 // depends on the layout.
 //
-// kPair: a work item goes to a cluster of two CTAs, one sub-tile each, which exchange their row
-// maxima through distributed shared memory instead of parking the first sub-tile's h.  For calls
-// with so few items that whole items leave SMs idle: see the rule at the launch.
+// kPair: the form for few rows an expert, on clusters of two CTAs (moe_gate_up_pair.cuh); map_x covers the
+// pre-sorted copy in boxes of 16 rows, map_gate the weight rows by channel.
 template <typename RoundT, bool kGather, bool kPair>
 __global__ void __launch_bounds__(384, 1)
 moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                       const __grid_constant__ CUtensorMap map_gate,
                       const __grid_constant__ CUtensorMap map_up, const GateUpParams p) {
+  if constexpr (kPair) {
+    gate_up_pair_body<RoundT>(map_x, map_gate, p);
+    return;
+  }
   using Shape = GateUpShape;
   constexpr int kStages = Shape::kStages;
   constexpr int BN = 256;
@@ -145,8 +102,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
   uint64_t* scale_full_bar = tmem_empty_bar + 2;
   uint64_t* scale_empty_bar = scale_full_bar + Shape::kScaleChunks;
-  uint64_t* amax_bar = scale_empty_bar + Shape::kScaleChunks;   // kPair: [item parity][lane quarter]
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(amax_bar + 8);
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(scale_empty_bar + Shape::kScaleChunks);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
   // The same in every lane, and known to be: addresses built from it stay in uniform registers.
@@ -169,7 +125,6 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       mbar_init(&scale_full_bar[i], 32);   // every lane of the scale warp
       mbar_init(&scale_empty_bar[i], 8);   // one arrival per promotion warp
     }
-    for (int i = 0; i < 8; ++i) mbar_init(&amax_bar[i], 4);   // two warps of each CTA
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -182,27 +137,17 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   // walks only those.  (An expert-parallel rank's list is sized for every row it could
   // receive, several times what it does receive.)
   __shared__ int used_row_tiles;
-  if (threadIdx.x == 32) {
-    int low = 0, high = p.max_tiles;
-    while (low < high) {
-      const int middle = (low + high) >> 1;
-      if (p.tile_expert[middle] >= 0) low = middle + 1;
-      else high = middle;
-    }
-    used_row_tiles = low;
+  if (warp == 1) {
+    const int used = used_tiles(p.tile_expert, p.max_tiles, lane);
+    if (lane == 0) used_row_tiles = used;
   }
   if (warp == 9) tmem_alloc<1>(tmem_holder, 512);
   tcgen05_fence_before();
   __syncthreads();
-  if constexpr (kPair) cluster_sync_all();   // the peer's barriers exist from here on
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   const int total_items = used_row_tiles * channel_groups;
-  const uint32_t cta_rank = kPair ? cluster_ctarank() : 0u;
-  const int first_item = kPair ? blockIdx.x / 2 : blockIdx.x;
-  const int item_step = kPair ? gridDim.x / 2 : gridDim.x;
-  const int sub_begin = kPair ? static_cast<int>(cta_rank) : 0;
-  const int sub_end = kPair ? sub_begin + 1 : 2;
+  const int first_item = blockIdx.x, item_step = gridDim.x;
 
   // Warps 8-11 (producer, MMA issuer, two spares) give registers to the promotion warps.
   if (warp >= 8) {
@@ -225,7 +170,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 #pragma unroll
           for (int i = 0; i < 4; ++i) source[i] = gate_up_source_row(p, row0 + 4 * lane + i, row_end);
         }
-        for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
+        for (int sub = 0; sub < 2 && ok; ++sub) {
           const int channel0 = jg * 256 + sub * 128;
           const int row_gate = expert * (p.interleaved ? 1 : 2) * p.intermediate + channel0;
           const int row_up = p.interleaved ? row_gate : row_gate + p.intermediate;
@@ -239,10 +184,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             if (leader) {
               mbar_expect_tx(&full_bar[stage], Shape::kStageBytes);
               if constexpr (!kGather) tma_load_2d(a_dst, &map_x, &full_bar[stage], x, row0);
-              tma_load_4d(b_dst, &map_gate, &full_bar[stage], x, kPair ? 0 : row_gate,
-                          kPair ? row_gate >> 5 : 0);
-              tma_load_4d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, kPair ? 0 : row_up,
-                          kPair ? row_up >> 5 : 0);
+              tma_load_4d(b_dst, &map_gate, &full_bar[stage], x, row_gate, 0);
+              tma_load_4d(b_dst + 128 * 128, &map_up, &full_bar[stage], x, row_up, 0);
             }
             if constexpr (kGather) {
               // Every lane fetches its four rows: 32 gathers of 512 bytes fill the A tile.
@@ -259,15 +202,14 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       dependents_may_launch();   // the CTA's last loads are on their way
     } else if (warp == 10) {
       // ---------------------------------------------------------- scale staging warp
-      // Copies each group's 256 column scales (by accumulator column; 16 bytes at a time for pairs
-      // with sw_vectors, else 4) and 128 row scales (4 bytes) into a shared-memory ring with
-      // asynchronous copies that land in the order the promotion threads read; the copies
-      // themselves signal the chunk's barrier, so the warp runs up to a ring ahead and
-      // global-memory latency stays hidden.
+      // Copies each group's 256 column scales (by accumulator column) and 128 row scales into a
+      // shared-memory ring with asynchronous 4-byte copies that land in the order the promotion
+      // threads read; the copies themselves signal the chunk's barrier, so the warp runs up to a
+      // ring ahead and global-memory latency stays hidden.
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
       // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-      const uint32_t column_position = kPair ? 4 * lane : ring_column_bytes<32>(lane);
+      const uint32_t column_position = ring_column_bytes<32>(lane);
       const uint32_t row_position = 4 * ring_row_position(lane);
       const uint32_t ring_base = smem_u32(sb_ring);
       const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale
@@ -287,8 +229,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           const long long source_row = kGather ? gate_up_source_row(p, r, row_end) : (sa_valid[i] ? r : 0);
           sa_source[i] = p.row_scale + source_row * groups;
         }
-        for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
-          const int channel = jg * 256 + sub * 128 + (kPair && p.sw_vectors ? 4 * lane : lane);
+        for (int sub = 0; sub < 2 && ok; ++sub) {
+          const int channel = jg * 256 + sub * 128 + lane;
           const float* sb_source = sb_base + (p.interleaved ? 2 * channel : channel);
           for (int g = 0; g < groups; g += kScaleChunkGroups) {
             if (!mbar_wait_warp(&scale_empty_bar[chunk], phase ^ 1u, kSiteScaleEmpty, abort_flag)) {
@@ -298,15 +240,10 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const int in_chunk = min(kScaleChunkGroups, groups - g);
             uint32_t destination = ring_base + chunk * (kScaleChunkGroups * Shape::kRingFloats * 4);
             for (int i = 0; i < in_chunk; ++i) {
-              if (kPair && p.sw_vectors) {
-                cp_async_f32x4(destination + 16 * lane, sb_source, true);
-                cp_async_f32x4(destination + 512 + 16 * lane, sb_source + up_offset, true);
-              } else {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  cp_async_f32(destination + 128 * j + column_position,
-                               sb_source + (j & 3) * sb_step + (j < 4 ? 0 : up_offset), true);
-                }
+              for (int j = 0; j < 8; ++j) {
+                cp_async_f32(destination + 128 * j + column_position,
+                             sb_source + (j & 3) * sb_step + (j < 4 ? 0 : up_offset), true);
               }
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -339,7 +276,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       bool ok = true;
       for (int item = first_item; item < total_items && ok; item += item_step) {
         if (p.tile_expert[item / channel_groups] < 0) continue;
-        for (int sub = sub_begin; sub < sub_end && ok; ++sub) {
+        for (int sub = 0; sub < 2 && ok; ++sub) {
           for (int slab = 0; slab < slabs; ++slab) {
             if (!mbar_wait_warp(&full_bar[stage], phase, kSiteMmaFull, abort_flag)) {
               ok = false;
@@ -384,9 +321,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     // ------------------------------------------------------------ promotion + SwiGLU warps
     // Fragment layout (tmem_ld_16x128b_x8): warp (quarter, half) drains TMEM lanes
     // 32*quarter.. of four 32-column blocks; a thread owns tile rows
-    // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, four channel pairs i: with kPair
-    // 8*(lane%4) + 2i, +1 (the weight rows arrive in fragment order), else 8i + lane%4, +4.  Blocks
-    // 0,1 are 64 gate columns of this half, blocks 2,3 the matching up columns.
+    // 32*quarter + lane/4 + 8r (r = 0..3) and, in every block, four channel pairs i: 8i + lane%4, +4.
+    // Blocks 0,1 are 64 gate columns of this half, blocks 2,3 the matching up columns.
     const int half = warp >> 2;
     const int quarter = warp & 3;
     const int tid = threadIdx.x;
@@ -400,7 +336,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     // next: a warp may start the next item (and write its sub-tile 0 maxima) while its partner
     // half is still reading this item's; the barrier of the next item keeps it from getting
     // two items ahead.
-    uint32_t item_parity = 0, item_phase = 0;
+    uint32_t item_parity = 0;
     // First accumulator column of block b: gate columns of this half, then the up columns.
     const auto block_column = [half](int b) { return half * 64 + 32 * (b & 1) + (b < 2 ? 0 : 128); };
     for (int item = first_item; item < total_items; item += item_step) {
@@ -411,7 +347,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       const int first_row = row0 + quarter * 32 + fragment_row;   // + 8r
       float amax_first[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 
-      for (int sub = sub_begin; sub < sub_end; ++sub) {
+      for (int sub = 0; sub < 2; ++sub) {
         float2 acc[4][16];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -477,8 +413,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
 
         // SwiGLU on the rounded gate/up values.  h[r][8b + 2i] and h[r][8b + 2i + 1] are channels
-        // half*64 + 32b + 8*quad + 2i and +1 of this sub-tile's 128 (kPair), else
-        // half*64 + 32b + 8i + quad and +4.
+        // half*64 + 32b + 8i + quad and +4 of this sub-tile's 128.
         // gate and up are rounded to the output type first (pack_pair), so silu(gate) is a
         // lookup by the gate's 16-bit pattern in a table built with the formula itself.
         float h[4][16];
@@ -503,12 +438,10 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
           row_amax = fmaxf(row_amax, __shfl_xor_sync(0xffffffffu, row_amax, 2));
           amax[r] = row_amax;
           if (quad == 0) {
-            float* mine = &amax_part[((item_parity * 2 + sub) * 2 + half) * 128 + quarter * 32 + fragment_row + 8 * r];
-            *mine = row_amax;
-            if constexpr (kPair) store_cluster_f32(mine, cta_rank ^ 1u, row_amax);
+            amax_part[((item_parity * 2 + sub) * 2 + half) * 128 + quarter * 32 + fragment_row + 8 * r] = row_amax;
           }
         }
-        if (!kPair && sub == 0) {
+        if (sub == 0) {
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
 #pragma unroll
@@ -518,22 +451,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             amax_first[r] = amax[r];
           }
         } else {
-          if constexpr (kPair) {
-            // The row maxima of this lane quarter from all four warps that hold its rows' channels
-            // (two here, two in the peer CTA).  A warp that has failed arrives all the same.
-            // Maxima and barriers alternate between two sets: a warp that arrives for item n + 2
-            // has seen the arrivals for n + 1, which the other warps make after their waits for
-            // n, so that neither an arrival nor a store runs ahead into a set still in use.
-            uint64_t* exchange = &amax_bar[item_parity * 4 + quarter];
-            __syncwarp();
-            if (lane == 0) {
-              mbar_arrive(exchange);
-              mbar_arrive_cluster_release(exchange, cta_rank ^ 1u);
-            }
-            if (ok) ok = mbar_wait_warp<true>(exchange, item_phase, kSiteDrain, abort_flag);
-          } else {
-            named_barrier_sync(1, 256);
-          }
+          named_barrier_sync(1, 256);
           const bool all_ok = ok;
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
@@ -541,17 +459,13 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             float row_max = fmaxf(amax[r], amax_first[r]);
             row_max = fmaxf(row_max, amax_part[((item_parity * 2 + 0) * 2 + (half ^ 1)) * 128 + tile_row]);
             row_max = fmaxf(row_max, amax_part[((item_parity * 2 + 1) * 2 + (half ^ 1)) * 128 + tile_row]);
-            if constexpr (kPair) {
-              row_max = fmaxf(row_max, amax_part[((item_parity * 2 + (sub ^ 1)) * 2 + half) * 128 + tile_row]);
-            }
             const RowQuantizer quantizer(row_max);
             const int row = first_row + 8 * r;
             const bool row_stored = all_ok && row < row_end;
             int8_t* q_row = p.q + static_cast<long long>(row) * p.intermediate + jg * 256;
 #pragma unroll
-            for (int piece = kPair ? 1 : 0; piece < 2; ++piece) {
-              // piece 0: parked first sub-tile (channels 0..127), piece 1: registers (with kPair
-              // this CTA's only sub-tile).
+            for (int piece = 0; piece < 2; ++piece) {
+              // piece 0: parked first sub-tile (channels 0..127), piece 1: registers.
               float v[16];
 #pragma unroll
               for (int k = 0; k < 16; k += 4) {
@@ -564,40 +478,34 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
               }
               uint32_t code[16];
               quantizer.codes(v, code);
-              int8_t* q_piece = q_row + (kPair ? sub : piece) * 128 + half * 64;
-              // Lane `quad` stores the eight channels 32*b + 8*quad .. +7: with kPair it holds them,
-              // else an exchange inside the quad brings them, the first four in the low bytes.
+              int8_t* q_piece = q_row + piece * 128 + half * 64;
+              // Lane `quad` stores the eight channels 32*b + 8*quad .. +7, which an exchange inside the
+              // quad brings, the first four in the low bytes.
 #pragma unroll
               for (int b = 0; b < 2; ++b) {
                 uint32_t w[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) w[i] = __byte_perm(code[b * 8 + 2 * i], code[b * 8 + 2 * i + 1], 0x0040);
-                uint2 packed;
-                if constexpr (kPair) {
-                  packed = make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
-                } else {
-                  quad_transpose(w, quad);
-                  const uint32_t front = __byte_perm(w[0], w[1], 0x5140);
-                  const uint32_t back = __byte_perm(w[2], w[3], 0x5140);
-                  packed = make_uint2(__byte_perm(front, back, 0x5410), __byte_perm(front, back, 0x7632));
-                }
+                quad_transpose(w, quad);
+                const uint32_t front = __byte_perm(w[0], w[1], 0x5140);
+                const uint32_t back = __byte_perm(w[2], w[3], 0x5140);
+                const uint2 packed =
+                    make_uint2(__byte_perm(front, back, 0x5410), __byte_perm(front, back, 0x7632));
                 if (row_stored) *reinterpret_cast<uint2*>(q_piece + b * 32 + 8 * quad) = packed;
               }
             }
-            if (row_stored && half == 0 && quad == 0 && (!kPair || sub == 0)) {
+            if (row_stored && half == 0 && quad == 0) {
               p.s[static_cast<long long>(row) * channel_groups + jg] = quantizer.scale;
             }
           }
         }
       }
       item_parity ^= 1u;
-      if (item_parity == 0) item_phase ^= 1u;
     }
   }
 
   tcgen05_fence_before();
   __syncthreads();
-  if constexpr (kPair) cluster_sync_all();   // no CTA leaves while its peer may still write here
   if (warp == 9) tmem_dealloc<1>(tmem_base, 512);
 }
 

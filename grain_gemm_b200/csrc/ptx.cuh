@@ -240,6 +240,11 @@ __device__ __forceinline__ void cp_async_f32x4(uint32_t smem_dst, const float* s
                : "memory");
 }
 
+// The same for 8 bytes, always read.
+__device__ __forceinline__ void cp_async_f32x2(uint32_t smem_dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+
 // One arrival on `bar` once all cp.async issued so far by this thread have landed (the
 // arrival is already part of the barrier's expected count).
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
@@ -313,6 +318,17 @@ __device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const CUtensorM
       "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(smem_u32(smem_dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(x), "r"(c1), "r"(0), "r"(c3)
+      : "memory");
+}
+
+// 5-D tiled load of Gate/Up weight rows by channel (see gate_up_channel_map).
+__device__ __forceinline__ void tma_load_channels_pair(void* smem_dst, const CUtensorMap* map, uint64_t* bar,
+                                                       int32_t x, int32_t row16) {
+  const uint32_t leader_bar = smem_u32(bar) & 0xFEFFFFFFu;
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %5, %5, %5, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(x), "r"(row16), "r"(0)
       : "memory");
 }
 

@@ -16,7 +16,7 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 static inline int encode_bytes(EncodeTiledFn encode, CUtensorMap* map, const void* base, int rank,
                                const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
   if (encode == nullptr) return static_cast<int>(cudaErrorNotSupported);
-  const cuuint32_t element_strides[4] = {1u, 1u, 1u, 1u};
+  const cuuint32_t element_strides[5] = {1u, 1u, 1u, 1u, 1u};
   const CUresult result = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, static_cast<cuuint32_t>(rank),
                                  const_cast<void*>(base), dims, strides, box, element_strides,
                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -84,6 +84,23 @@ static inline int gate_up_row_maps(EncodeTiledFn encode, CUtensorMap* gate, CUte
     status = weight_row_map(encode, gate, first, rows / 2, hidden, 2ll * hidden, 128, permuted);
   }
   return status;
+}
+
+// Map of Gate/Up weights by channel, for boxes of 128 channels (256 rows x 128 bytes): row 16u + 8j + r of
+// every 32 delivered ones is channel 2r + j of the next 16, gate (u = 0) or up (u = 1).  Coordinates
+// (x, 0, 0, 0, c): c counts steps of 16 channels, from 0 for the interleaved layout, in rows of
+// the whole weight for the split one.  Strides that are not multiples of one another, like the
+// permuted map above; there is no other order for the kernel that takes it.
+static inline int gate_up_channel_map(EncodeTiledFn encode, CUtensorMap* map, const void* weights, int experts,
+                                      int intermediate, int hidden, bool interleaved) {
+  const cuuint64_t step = static_cast<cuuint64_t>(hidden), inter = static_cast<cuuint64_t>(intermediate);
+  const cuuint64_t rows = 2ull * static_cast<cuuint64_t>(experts) * inter;
+  // The last coordinate ends with the last gate row, so that its up row is the weight's last row.
+  const cuuint64_t dims[5] = {step, 8, 2, 2, interleaved ? rows / 32 : (rows - inter) / 16};
+  const cuuint64_t split[4] = {2 * step, step, inter * step, 16 * step};
+  const cuuint64_t pairs[4] = {4 * step, 2 * step, step, 32 * step};
+  const cuuint32_t box[5] = {128u, 8u, 2u, 2u, 8u};
+  return encode_bytes(encode, map, weights, 5, dims, interleaved ? pairs : split, box);
 }
 
 }  // namespace gg
