@@ -48,6 +48,12 @@ _SIGNATURES = {
     "gg_moe_tile_capacity": (_INT, [_INT] * 3),
     "gg_moe_tiles": (_INT, [_VOID, _INT, _INT, _INT, _VOID, _VOID, _VOID]),
     "gg_moe_topk": (_INT, [_VOID, _INT, _INT, _INT, _INT, _VOID, _VOID, _INT, _VOID]),
+    "gg_moe_route_tiles": (_INT, [_VOID, _INT, _VOID, _INT, _INT, _INT] + [_VOID] * 7
+                           + [_SIZE, _INT, _INT, _VOID, _VOID, _VOID]),
+    "gg_moe_route_topk_tiles": (_INT, [_VOID, _INT, _VOID, _INT, _INT, _INT, _VOID, _VOID, _INT] + [_VOID] * 6
+                                + [_INT, _INT, _VOID, _VOID, _VOID]),
+    "gg_moe_gate_up_report": (_INT, [_VOID] * 8 + [_INT, _INT] + [_VOID] * 3 + [_INT] * 8
+                              + [_VOID, _INT, _VOID, _VOID]),
     "gg_moe_route_topk": (_INT, [_VOID, _INT, _VOID, _INT, _INT, _INT, _VOID, _VOID, _INT] + [_VOID] * 7),
     "gg_quantize_rows": (_INT, [_VOID, _INT, _LL, _INT, _INT, _VOID, _VOID, _VOID]),
     "gg_moe_silu_table": (_INT, [_VOID, _INT, _VOID]),

@@ -660,10 +660,14 @@ size_t gg_moe_route_workspace_bytes(int tokens, int top_k, int experts) {
   return static_cast<size_t>(chunks * (experts + 2)) * sizeof(int);
 }
 
-int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens, int top_k,
-                 int experts, void* effective_ids, void* order, void* inverse, void* counts,
-                 void* offsets, void* statistics, void* workspace, size_t workspace_bytes,
-                 void* stream_ptr) {
+int gg_moe_route_tiles(const void* ids, int ids_are_i64, const void* mask, int tokens, int top_k,
+                       int experts, void* effective_ids, void* order, void* inverse, void* counts,
+                       void* offsets, void* statistics, void* workspace, size_t workspace_bytes,
+                       int tile_rows, int tile_capacity, void* tile_expert, void* tile_row,
+                       void* stream_ptr) {
+  if (tile_expert && (!tile_row || tile_rows <= 0 || tile_capacity <= 0)) {
+    return static_cast<int>(cudaErrorInvalidValue);
+  }
   if (tokens < 0 || top_k <= 0 || experts <= 0 || !counts || !offsets || !statistics) {
     return static_cast<int>(cudaErrorInvalidValue);
   }
@@ -680,6 +684,7 @@ int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens,
   p.offsets = static_cast<int*>(offsets);
   p.statistics = static_cast<int*>(statistics);
   p.workspace = static_cast<int*>(workspace);
+  p.tiles = {static_cast<int*>(tile_expert), static_cast<int*>(tile_row), tile_rows, tile_capacity};
   const long long slots = static_cast<long long>(tokens) * top_k;
   const size_t smem = static_cast<size_t>(experts + 2) * sizeof(int);
   if (smem > 200 * 1024) return static_cast<int>(cudaErrorInvalidValue);
@@ -696,7 +701,7 @@ int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens,
     return gg::launch(gg::route_single_kernel, 1, gg::kRouteChunk, smem, stream, p);
   }
   if (slots <= gg::kRouteMediumSlots && experts + 1 <= gg::kRouteMediumKeys) {
-    const size_t medium = (static_cast<size_t>(33) * (experts + 1) + 33) * sizeof(int);
+    const size_t medium = (static_cast<size_t>(33) * (experts + 1) + 34) * sizeof(int);
     if (medium > 48 * 1024) {
       error = cudaFuncSetAttribute(gg::route_medium_kernel,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(medium));
@@ -721,6 +726,14 @@ int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens,
   if (!status) status = gg::launch(gg::route_scan_kernel, 1, 1024, smem, stream, p, chunks);
   if (!status) status = gg::launch(gg::route_place_kernel, chunks, gg::kRouteChunk, smem, stream, p);
   return status;
+}
+
+int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens, int top_k,
+                 int experts, void* effective_ids, void* order, void* inverse, void* counts,
+                 void* offsets, void* statistics, void* workspace, size_t workspace_bytes,
+                 void* stream) {
+  return gg_moe_route_tiles(ids, ids_are_i64, mask, tokens, top_k, experts, effective_ids, order, inverse, counts,
+                            offsets, statistics, workspace, workspace_bytes, 0, 0, nullptr, nullptr, stream);
 }
 
 // ---- routing without any allocation -----------------------------------------------------
@@ -781,9 +794,9 @@ int gg_moe_tiles(const void* offsets, int experts, int tile_rows, int capacity, 
   if (!offsets || !tile_expert || !tile_row || experts <= 0 || tile_rows <= 0 || capacity <= 0) {
     return static_cast<int>(cudaErrorInvalidValue);
   }
+  const gg::TileList list = {static_cast<int*>(tile_expert), static_cast<int*>(tile_row), tile_rows, capacity};
   return gg::launch(gg::moe_tiles_kernel, 1, 1024, 0, static_cast<cudaStream_t>(stream),
-                    static_cast<const int*>(offsets), experts, tile_rows, capacity,
-                    static_cast<int*>(tile_expert), static_cast<int*>(tile_row));
+                    static_cast<const int*>(offsets), experts, list);
 }
 
 size_t gg_moe_gate_up_scratch_bytes(int assignments, int hidden, int intermediate, int tile_rows,
@@ -808,12 +821,12 @@ int gg_moe_silu_table(void* table, int out_dtype, void* stream_ptr) {
                     static_cast<float*>(table), out_dtype == GG_OUT_FP16 ? 1 : 0);
 }
 
-int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const void* scale_w1,
-                   const void* order, const void* offsets, const void* tile_expert,
-                   const void* tile_row, int tile_capacity, int tile_rows, void* q, void* s,
-                   void* gate_up_scratch, int tokens, int top_k, int experts, int hidden,
-                   int intermediate, int interleaved, int out_dtype, int row_gather,
-                   void* stream_ptr) {
+int gg_moe_gate_up_report(const void* x, const void* scale_x, const void* w1, const void* scale_w1,
+                          const void* order, const void* offsets, const void* tile_expert,
+                          const void* tile_row, int tile_capacity, int tile_rows, void* q, void* s,
+                          void* gate_up_scratch, int tokens, int top_k, int experts, int hidden,
+                          int intermediate, int interleaved, int out_dtype, int row_gather,
+                          const void* values, int count, void* host_words, void* stream_ptr) {
   if (tokens <= 0 || top_k <= 0 || experts <= 0 || hidden <= 0 || intermediate <= 0 ||
       hidden % 256 || intermediate % 256 || tile_capacity <= 0 ||
       (out_dtype != GG_OUT_BF16 && out_dtype != GG_OUT_FP16) || !x || !scale_x || !w1 ||
@@ -822,6 +835,14 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
   const long long slots = static_cast<long long>(tokens) * top_k;
+  gg::HostReport report = {nullptr, nullptr, 0};
+  if (host_words) {
+    if (!values || count <= 0 || tile_rows != 128) return static_cast<int>(cudaErrorInvalidValue);
+    void* mapped = nullptr;
+    const cudaError_t error = cudaHostGetDevicePointer(&mapped, host_words, 0);
+    if (error != cudaSuccess) return gg::finished(error);
+    report = {static_cast<const int*>(values), static_cast<int*>(mapped), count};
+  }
   if (tile_rows == 128) {
     if (!gg::aligned16(x) || !gg::aligned16(w1) || !gg::aligned16(q) || !gate_up_scratch ||
         !gg::aligned16(gate_up_scratch)) {
@@ -830,8 +851,20 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     uint8_t* scratch = static_cast<uint8_t*>(gate_up_scratch);
     gg::GateUpParams p = {};
     CUtensorMap map_x, map_gate, map_up;
-    const void* x_rows = x;   // what map_x covers
-    int status;
+    int status = 0;
+    // Pairs need their weight rows by channel; without such a map the item stays on one CTA.
+    bool pairs = !row_gather && gg::gate_up_pairs(slots, experts, intermediate / 256) &&
+                 gg::gate_up_channel_map(gg::encode_tiled_fn(), &map_gate, w1, experts, intermediate, hidden,
+                                         interleaved != 0) == 0;
+    if (pairs) {
+      map_up = map_gate;
+    } else {
+      bool permuted = false;
+      status = gg::gate_up_row_maps(gg::encode_tiled_fn(), &map_gate, &map_up, w1,
+                                    static_cast<long long>(experts) * 2 * intermediate, hidden, interleaved != 0,
+                                    &permuted);
+      if (status) return status;
+    }
     if (row_gather) {
       p.silu_table = reinterpret_cast<float*>(scratch);
       p.row_scale = static_cast<const float*>(scale_x);
@@ -852,31 +885,11 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
           static_cast<const long long*>(order), static_cast<const int*>(offsets), experts, top_k,
           hidden, sorted_x, sorted_scale, const_cast<float*>(p.silu_table), out_dtype == GG_OUT_FP16 ? 1 : 0);
       if (status) return status;
-      x_rows = sorted_x;
-      status = gg::row_map(gg::encode_tiled_fn(), &map_x, sorted_x, slots, hidden, hidden, 128);
+      status = gg::row_map(gg::encode_tiled_fn(), &map_x, sorted_x, slots, hidden, hidden, pairs ? 16 : 128);
     }
     if (status) return status;
     if (row_gather) {
       status = gg_moe_silu_table(const_cast<float*>(p.silu_table), out_dtype, stream_ptr);
-      if (status) return status;
-    }
-    // Pairs need their weight rows by channel; without such a map the item stays on one CTA.
-    bool pairs = !row_gather && gg::gate_up_pairs(slots, experts, intermediate / 256);
-    if (pairs) {
-      CUtensorMap map_rows;
-      pairs = gg::gate_up_channel_map(gg::encode_tiled_fn(), &map_gate, w1, experts, intermediate, hidden,
-                                      interleaved != 0) == 0 &&
-              gg::row_map(gg::encode_tiled_fn(), &map_rows, x_rows, slots, hidden, hidden, 16) == 0;
-      if (pairs) {
-        map_x = map_rows;
-        map_up = map_gate;
-      }
-    }
-    if (!pairs) {
-      bool permuted = false;
-      status = gg::gate_up_row_maps(gg::encode_tiled_fn(), &map_gate, &map_up, w1,
-                                    static_cast<long long>(experts) * 2 * intermediate, hidden, interleaved != 0,
-                                    &permuted);
       if (status) return status;
     }
     p.order = static_cast<const long long*>(order);
@@ -890,6 +903,7 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
     p.hidden = hidden; p.intermediate = intermediate;
     p.max_tiles = tile_capacity; p.interleaved = interleaved;
     p.sw_vectors = gg::aligned16(scale_w1);
+    p.report = report;
     if (out_dtype == GG_OUT_BF16) {
       return gg::launch_gate_up_tc<__nv_bfloat16>(map_x, map_gate, map_up, p, slots, pairs, row_gather, stream);
     }
@@ -930,6 +944,17 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
         static_cast<int8_t*>(q), static_cast<float*>(s));
   }
   return static_cast<int>(cudaGetLastError());
+}
+
+int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const void* scale_w1,
+                   const void* order, const void* offsets, const void* tile_expert,
+                   const void* tile_row, int tile_capacity, int tile_rows, void* q, void* s,
+                   void* gate_up_scratch, int tokens, int top_k, int experts, int hidden,
+                   int intermediate, int interleaved, int out_dtype, int row_gather,
+                   void* stream) {
+  return gg_moe_gate_up_report(x, scale_x, w1, scale_w1, order, offsets, tile_expert, tile_row, tile_capacity,
+                               tile_rows, q, s, gate_up_scratch, tokens, top_k, experts, hidden, intermediate,
+                               interleaved, out_dtype, row_gather, nullptr, 0, nullptr, stream);
 }
 
 int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_w2,
@@ -1161,15 +1186,17 @@ int gg_moe_topk(const void* logits, int in_dtype, int tokens, int experts, int t
   return status;
 }
 
-int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int tokens, int experts,
-                      int top_k, void* weights, void* ids, int ids_are_i64, void* effective_ids,
-                      void* order, void* inverse, void* counts, void* offsets, void* statistics,
-                      void* stream_ptr) {
+int gg_moe_route_topk_tiles(const void* logits, int in_dtype, const void* mask, int tokens, int experts,
+                            int top_k, void* weights, void* ids, int ids_are_i64, void* effective_ids,
+                            void* order, void* inverse, void* counts, void* offsets, void* statistics,
+                            int tile_rows, int tile_capacity, void* tile_expert, void* tile_row,
+                            void* stream_ptr) {
   const long long slots = static_cast<long long>(tokens) * top_k;
   if (tokens <= 0 || experts <= 0 || experts > 1024 || top_k <= 0 || top_k > experts ||
       slots > gg::kRouteChunk ||
       (in_dtype != GG_OUT_FP32 && in_dtype != GG_OUT_BF16 && in_dtype != GG_OUT_FP16) || !logits ||
-      !weights || !ids || !effective_ids || !order || !inverse || !counts || !offsets || !statistics) {
+      !weights || !ids || !effective_ids || !order || !inverse || !counts || !offsets || !statistics ||
+      (tile_expert && (!tile_row || tile_rows <= 0 || tile_capacity <= 0))) {
     return static_cast<int>(cudaErrorInvalidValue);
   }
   cudaStream_t stream = static_cast<cudaStream_t>(stream_ptr);
@@ -1184,6 +1211,7 @@ int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int to
   p.counts = static_cast<int*>(counts);
   p.offsets = static_cast<int*>(offsets);
   p.statistics = static_cast<int*>(statistics);
+  p.tiles = {static_cast<int*>(tile_expert), static_cast<int*>(tile_row), tile_rows, tile_capacity};
   const size_t smem = static_cast<size_t>(experts + 2) * sizeof(int);
   float* w = static_cast<float*>(weights);
   int status;
@@ -1198,6 +1226,15 @@ int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int to
         static_cast<const __half*>(logits), w, p);
   }
   return status;
+}
+
+int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int tokens, int experts,
+                      int top_k, void* weights, void* ids, int ids_are_i64, void* effective_ids,
+                      void* order, void* inverse, void* counts, void* offsets, void* statistics,
+                      void* stream) {
+  return gg_moe_route_topk_tiles(logits, in_dtype, mask, tokens, experts, top_k, weights, ids, ids_are_i64,
+                                 effective_ids, order, inverse, counts, offsets, statistics, 0, 0, nullptr,
+                                 nullptr, stream);
 }
 
 int gg_quantize_rows(const void* x, int in_dtype, long long rows, int width, int group_size,

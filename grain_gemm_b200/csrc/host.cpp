@@ -17,7 +17,6 @@
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
-#include <ATen/cuda/CUDAEvent.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -44,16 +43,15 @@ struct Library {
   decltype(&gg_int8_gemm_ws) int8_gemm_ws;
   decltype(&gg_int8_gemm_workspace_bytes) int8_gemm_workspace_bytes;
   decltype(&gg_quantize_rows) quantize_rows;
-  decltype(&gg_moe_route_topk) moe_route_topk;
+  decltype(&gg_moe_topk) moe_topk;
+  decltype(&gg_moe_route_topk_tiles) moe_route_topk_tiles;
   decltype(&gg_moe_route_workspace_bytes) moe_route_workspace_bytes;
-  decltype(&gg_moe_route) moe_route;
+  decltype(&gg_moe_route_tiles) moe_route_tiles;
   decltype(&gg_moe_tile_capacity) moe_tile_capacity;
-  decltype(&gg_moe_tiles) moe_tiles;
   decltype(&gg_moe_gate_up_scratch_bytes) moe_gate_up_scratch_bytes;
-  decltype(&gg_moe_gate_up) moe_gate_up;
+  decltype(&gg_moe_gate_up_report) moe_gate_up_report;
   decltype(&gg_moe_down) moe_down;
   decltype(&gg_moe_combine) moe_combine;
-  decltype(&gg_report_to_host) report_to_host;
 };
 Library lib;
 
@@ -145,6 +143,32 @@ int64_t small_int(PyObject* object) {
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType type, const at::Device& device) {
   return at::empty(sizes, at::TensorOptions().dtype(type).device(device));
 }
+
+// Several small tensors in one allocation (each costs a call of the allocator 0.7 us of the host's time,
+// a decode step's routing has ten).  Sizes first, then the tensors: contiguous, 256-byte aligned.
+class Pieces {
+ public:
+  int64_t add(at::IntArrayRef sizes, at::ScalarType type) {
+    const int64_t at = bytes_;
+    int64_t count = 1;
+    for (const int64_t size : sizes) count *= size;
+    bytes_ += (count * static_cast<int64_t>(c10::elementSize(type)) + 255) / 256 * 256;
+    return at;
+  }
+  void allocate(const at::Device& device) { memory_ = empty({bytes_ > 0 ? bytes_ : 1}, at::kByte, device); }
+  at::Tensor get(int64_t at, at::IntArrayRef sizes, at::ScalarType type) const {
+    at::Tensor piece = at::detail::make_tensor<c10::TensorImpl>(
+        c10::Storage(memory_.storage()), memory_.key_set(), c10::scalarTypeToTypeMeta(type));
+    c10::TensorImpl* impl = piece.unsafeGetTensorImpl();
+    impl->set_sizes_contiguous(sizes);
+    impl->set_storage_offset(at / static_cast<int64_t>(c10::elementSize(type)));
+    return piece;
+  }
+
+ private:
+  int64_t bytes_ = 0;
+  at::Tensor memory_;
+};
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -270,9 +294,10 @@ struct Routing {
 };
 
 constexpr int kTileRows = 128;
+constexpr int64_t kFusedSlots = 1024;   // what gg_moe_route_topk_tiles takes
 
-// route_topk_routes(logits, top_k, token_mask or None, 64-bit ids?): the fused decode-sized call
-// with its row-tile list.  Returns (weights, ids, order, counts, offsets, inverse, effective_ids,
+// route_topk_routes(logits, top_k, token_mask or None, 64-bit ids?): selection, routing and row-tile list, one
+// kernel for decode-sized calls.  Returns (weights, ids, order, counts, offsets, inverse, effective_ids,
 // statistics, tile_expert, tile_row).
 PyObject* route_topk_routes(PyObject*, PyObject* const* args, Py_ssize_t count) {
   HANDLE_TH_ERRORS
@@ -283,8 +308,8 @@ PyObject* route_topk_routes(PyObject*, PyObject* const* args, Py_ssize_t count) 
   if (logits.dim() != 2 || !logits.is_contiguous()) Py_RETURN_NONE;
   const int64_t tokens = logits.size(0), experts = logits.size(1);
   const int in_dtype = out_code(logits.scalar_type());
-  if (in_dtype < 0 || top_k <= 0 || top_k > experts || experts > 1024 || tokens <= 0 || tokens > 1024 ||
-      tokens * top_k > 1024) {
+  if (in_dtype < 0 || top_k <= 0 || top_k > experts || experts > 1024 || tokens <= 0 ||
+      tokens * top_k > INT_MAX) {
     Py_RETURN_NONE;
   }
   const at::Tensor* mask = nullptr;
@@ -306,25 +331,46 @@ PyObject* route_topk_routes(PyObject*, PyObject* const* args, Py_ssize_t count) 
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(device.index());
     const int64_t slots = tokens * top_k;
     const at::ScalarType id_type = wide ? at::kLong : at::kInt;
-    weights = empty({tokens, top_k}, at::kFloat, device);
-    ids = empty({tokens, top_k}, id_type, device);
-    r.effective_ids = empty({slots}, id_type, device);
-    r.order = empty({slots}, at::kLong, device);
-    r.inverse = empty({slots}, at::kInt, device);
-    r.counts = empty({experts}, at::kInt, device);
-    r.offsets = empty({experts + 1}, at::kInt, device);
-    r.statistics = empty({3}, at::kInt, device);
     const int capacity = lib.moe_tile_capacity(slots, experts, kTileRows);
-    tile_expert = empty({capacity}, at::kInt, device);
-    tile_row = empty({capacity}, at::kInt, device);
-    if (!status.set(lib.moe_route_topk(logits.data_ptr(), in_dtype, mask ? mask->data_ptr() : nullptr, tokens,
-                                       experts, top_k, weights.data_ptr(), ids.data_ptr(), wide,
+    const bool fused = slots <= kFusedSlots;
+    const int64_t route_bytes = fused ? 0 : static_cast<int64_t>(lib.moe_route_workspace_bytes(tokens, top_k, experts));
+    Pieces pieces;
+    const int64_t at_weights = pieces.add({tokens, top_k}, at::kFloat), at_ids = pieces.add({tokens, top_k}, id_type),
+                  at_effective = pieces.add({slots}, id_type), at_order = pieces.add({slots}, at::kLong),
+                  at_inverse = pieces.add({slots}, at::kInt), at_counts = pieces.add({experts}, at::kInt),
+                  at_offsets = pieces.add({experts + 1}, at::kInt), at_statistics = pieces.add({3}, at::kInt),
+                  at_expert = pieces.add({capacity}, at::kInt), at_row = pieces.add({capacity}, at::kInt);
+    pieces.allocate(device);
+    weights = pieces.get(at_weights, {tokens, top_k}, at::kFloat);
+    ids = pieces.get(at_ids, {tokens, top_k}, id_type);
+    r.effective_ids = pieces.get(at_effective, {slots}, id_type);
+    r.order = pieces.get(at_order, {slots}, at::kLong);
+    r.inverse = pieces.get(at_inverse, {slots}, at::kInt);
+    r.counts = pieces.get(at_counts, {experts}, at::kInt);
+    r.offsets = pieces.get(at_offsets, {experts + 1}, at::kInt);
+    r.statistics = pieces.get(at_statistics, {3}, at::kInt);
+    tile_expert = pieces.get(at_expert, {capacity}, at::kInt);
+    tile_row = pieces.get(at_row, {capacity}, at::kInt);
+    const void* mask_data = mask ? mask->data_ptr() : nullptr;
+    if (fused) {
+      status.set(lib.moe_route_topk_tiles(logits.data_ptr(), in_dtype, mask_data, tokens, experts, top_k,
+                                          weights.data_ptr(), ids.data_ptr(), wide, r.effective_ids.data_ptr(),
+                                          r.order.data_ptr(), r.inverse.data_ptr(), r.counts.data_ptr(),
+                                          r.offsets.data_ptr(), r.statistics.data_ptr(), kTileRows, capacity,
+                                          tile_expert.data_ptr(), tile_row.data_ptr(), stream),
+                 "gg_moe_route_topk_tiles");
+    } else {
+      if (route_bytes) r.scratch = empty({route_bytes}, at::kByte, device);
+      if (!status.set(lib.moe_topk(logits.data_ptr(), in_dtype, tokens, experts, top_k, weights.data_ptr(),
+                                   ids.data_ptr(), wide, stream),
+                      "gg_moe_topk")) {
+        status.set(lib.moe_route_tiles(ids.data_ptr(), wide, mask_data, tokens, top_k, experts,
                                        r.effective_ids.data_ptr(), r.order.data_ptr(), r.inverse.data_ptr(),
-                                       r.counts.data_ptr(), r.offsets.data_ptr(), r.statistics.data_ptr(), stream),
-                    "gg_moe_route_topk")) {
-      status.set(lib.moe_tiles(r.offsets.data_ptr(), experts, kTileRows, capacity, tile_expert.data_ptr(),
-                               tile_row.data_ptr(), stream),
-                 "gg_moe_tiles");
+                                       r.counts.data_ptr(), r.offsets.data_ptr(), r.statistics.data_ptr(),
+                                       route_bytes ? r.scratch.data_ptr() : nullptr, route_bytes, kTileRows, capacity,
+                                       tile_expert.data_ptr(), tile_row.data_ptr(), stream),
+                   "gg_moe_route_tiles");
+      }
     }
   }
   if (status.code) return raise_status(status);
@@ -370,6 +416,23 @@ at::Tensor buffer(PyObject* workspace, const char* name, at::IntArrayRef sizes, 
   }
   Py_DECREF(wrapped);
   return fresh;
+}
+
+constexpr int kNotReported = -1;   // no count of ids is negative
+
+// Waits until a kernel of `stream` has stored the first word; an error of the stream ends the wait.
+int wait_for_report(const volatile int* word, cudaStream_t stream) {
+  for (unsigned spin = 1; *word == kNotReported; ++spin) {
+    if ((spin & 0xfffu) != 0) {
+      __builtin_ia32_pause();
+      continue;
+    }
+    const cudaError_t state = cudaStreamQuery(stream);
+    if (state == cudaErrorNotReady) continue;
+    if (state != cudaSuccess) return static_cast<int>(state);
+    if (*word == kNotReported) return static_cast<int>(cudaErrorUnknown);   // all done, nothing stored
+  }
+  return 0;
 }
 
 // moe_ffn(hidden_states, w_gate_up, w_down, topk_weights, topk_ids, scale_x, scale_gate_up,
@@ -467,6 +530,23 @@ PyObject* moe_ffn(PyObject*, PyObject* const* args, Py_ssize_t count) {
     r.statistics = tensor(PyTuple_GET_ITEM(given, 3));
     tile_expert = tensor(PyTuple_GET_ITEM(given, 4));
     tile_row = tensor(PyTuple_GET_ITEM(given, 5));
+  } else if (!workspace) {
+    route_bytes = lib.moe_route_workspace_bytes(tokens, top_k, experts);
+    const int64_t scratch = static_cast<int64_t>(route_bytes);
+    Pieces pieces;
+    const int64_t at_effective = pieces.add({slots}, ids.scalar_type()), at_order = pieces.add({slots}, at::kLong),
+                  at_inverse = pieces.add({slots}, at::kInt), at_counts = pieces.add({experts}, at::kInt),
+                  at_offsets = pieces.add({experts + 1}, at::kInt), at_statistics = pieces.add({3}, at::kInt),
+                  at_scratch = pieces.add({scratch}, at::kByte), at_tiles = pieces.add({2, capacity}, at::kInt);
+    pieces.allocate(device);
+    r.effective_ids = pieces.get(at_effective, {slots}, ids.scalar_type());
+    r.order = pieces.get(at_order, {slots}, at::kLong);
+    r.inverse = pieces.get(at_inverse, {slots}, at::kInt);
+    r.counts = pieces.get(at_counts, {experts}, at::kInt);
+    r.offsets = pieces.get(at_offsets, {experts + 1}, at::kInt);
+    r.statistics = pieces.get(at_statistics, {3}, at::kInt);
+    r.scratch = pieces.get(at_scratch, {scratch}, at::kByte);
+    r.tiles = pieces.get(at_tiles, {2, capacity}, at::kInt);
   } else {
     r.effective_ids = buffer(workspace, "effective_ids", {slots}, ids.scalar_type(), device);
     r.order = buffer(workspace, "order", {slots}, at::kLong, device);
@@ -506,31 +586,28 @@ PyObject* moe_ffn(PyObject*, PyObject* const* args, Py_ssize_t count) {
     const int* rows_of = given ? tile_row.data_ptr<int>() : r.tiles.data_ptr<int>() + capacity;
     const int tiles = given ? static_cast<int>(tile_expert.numel()) : capacity;
     if (!given) {
-      status.set(lib.moe_route(ids.data_ptr(), ids.scalar_type() == at::kLong, mask ? mask->data_ptr() : nullptr,
-                               tokens, top_k, experts, r.effective_ids.data_ptr(), r.order.data_ptr(),
-                               r.inverse.data_ptr(), r.counts.data_ptr(), r.offsets.data_ptr(),
-                               r.statistics.data_ptr(), route_bytes ? r.scratch.data_ptr() : nullptr,
-                               route_bytes, stream),
-                 "gg_moe_route");
-      if (!status.code) {
-        status.set(lib.moe_tiles(r.offsets.data_ptr(), experts, kTileRows, capacity, const_cast<int*>(experts_of),
-                                 const_cast<int*>(rows_of), stream),
-                   "gg_moe_tiles");
-      }
+      status.set(lib.moe_route_tiles(ids.data_ptr(), ids.scalar_type() == at::kLong, mask ? mask->data_ptr() : nullptr,
+                                     tokens, top_k, experts, r.effective_ids.data_ptr(), r.order.data_ptr(),
+                                     r.inverse.data_ptr(), r.counts.data_ptr(), r.offsets.data_ptr(),
+                                     r.statistics.data_ptr(), route_bytes ? r.scratch.data_ptr() : nullptr,
+                                     route_bytes, kTileRows, capacity, const_cast<int*>(experts_of),
+                                     const_cast<int*>(rows_of), stream),
+                 "gg_moe_route_tiles");
     }
-    // The check for unmasked ids outside [0, E): three integers are stored into page-locked host
-    // memory by a kernel and looked at after the remaining stages are in the stream.
-    at::cuda::CUDAEvent event;
+    // The check for unmasked ids outside [0, E): a warp of the Gate/Up kernel stores three integers into
+    // page-locked host memory, the count of such ids last, and they are looked at after the remaining
+    // stages are in the stream.
+    volatile int* const reported = words.data_ptr<int>();
+    bool reporting = false;
     if (!status.code) {
-      if (lib.report_to_host(r.statistics.data_ptr(), 3, words.data_ptr(), stream) != 0) {
-        words.copy_(r.statistics, /*non_blocking=*/true);
-      }
-      event.record(torch_stream);
-      status.set(lib.moe_gate_up(x.data_ptr(), scale_x.data_ptr(), w1.data_ptr(), scale_w1.data_ptr(),
+      *reported = kNotReported;
+      reporting = !status.set(
+          lib.moe_gate_up_report(x.data_ptr(), scale_x.data_ptr(), w1.data_ptr(), scale_w1.data_ptr(),
                                  r.order.data_ptr(), r.offsets.data_ptr(), experts_of, rows_of, tiles, kTileRows,
                                  qh.data_ptr(), sh.data_ptr(), scratch.data_ptr(), tokens, top_k, experts, hidden,
-                                 inter, interleaved, out_dtype, 0, stream),
-                 "gg_moe_gate_up");
+                                 inter, interleaved, out_dtype, 0, r.statistics.data_ptr(), 3, words.data_ptr(),
+                                 stream),
+          "gg_moe_gate_up");
     }
     if (!status.code) {
       status.set(lib.moe_down(qh.data_ptr(), sh.data_ptr(), w2.data_ptr(), scale_w2.data_ptr(), r.offsets.data_ptr(),
@@ -543,10 +620,10 @@ PyObject* moe_ffn(PyObject*, PyObject* const* args, Py_ssize_t count) {
                                  tokens, top_k, hidden, out_dtype, stream),
                  "gg_moe_combine");
     }
-    if (!status.code) {
-      event.synchronize();
-      invalid_ids = words.data_ptr<int>()[0] != 0;
-    }
+    // A refused launch leaves words that a kernel may still write, for the next call to mistake.
+    if (status.code) (void)cudaStreamSynchronize(stream);
+    else if (reporting) status.set(wait_for_report(reported, stream), "moe_ffn");
+    invalid_ids = !status.code && *reported != 0;
   }
   if (status.code) return raise_status(status);
   if (invalid_ids) {
@@ -580,16 +657,15 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t count) {
   entry("gg_int8_gemm_ws", fresh.int8_gemm_ws);
   entry("gg_int8_gemm_workspace_bytes", fresh.int8_gemm_workspace_bytes);
   entry("gg_quantize_rows", fresh.quantize_rows);
-  entry("gg_moe_route_topk", fresh.moe_route_topk);
+  entry("gg_moe_topk", fresh.moe_topk);
+  entry("gg_moe_route_topk_tiles", fresh.moe_route_topk_tiles);
   entry("gg_moe_route_workspace_bytes", fresh.moe_route_workspace_bytes);
-  entry("gg_moe_route", fresh.moe_route);
+  entry("gg_moe_route_tiles", fresh.moe_route_tiles);
   entry("gg_moe_tile_capacity", fresh.moe_tile_capacity);
-  entry("gg_moe_tiles", fresh.moe_tiles);
   entry("gg_moe_gate_up_scratch_bytes", fresh.moe_gate_up_scratch_bytes);
-  entry("gg_moe_gate_up", fresh.moe_gate_up);
+  entry("gg_moe_gate_up_report", fresh.moe_gate_up_report);
   entry("gg_moe_down", fresh.moe_down);
   entry("gg_moe_combine", fresh.moe_combine);
-  entry("gg_report_to_host", fresh.report_to_host);
   decltype(variant_table) table;
   PyObject *key, *rows;
   Py_ssize_t position = 0;

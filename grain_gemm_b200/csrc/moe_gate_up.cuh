@@ -9,6 +9,21 @@
 
 namespace gg {
 
+// A few integers for a host that polls: the first word arrives last.
+struct HostReport {
+  const int* values;
+  int* words;       // page-locked host memory; null: nothing to report
+  int count;
+};
+// By a warp that has nothing else to do: as a kernel of its own, or in front of other work of one, the
+// way over PCIe cost 1.5 us of a decode step.
+__device__ __forceinline__ void report_to_polling_host(const HostReport& report, int lane) {
+  if (report.words == nullptr || blockIdx.x != 0 || lane != 0) return;
+  for (int i = 1; i < report.count; ++i) report.words[i] = report.values[i];
+  __threadfence_system();
+  *const_cast<volatile int*>(report.words) = report.values[0];
+}
+
 struct GateUpParams {
   const float* row_scale;     // gathered: scale_x [T, H/256]; pre-sorted: [S, H/256] by sorted slot
   const long long* order;     // [S] sorted slot -> flattened assignment (gathered mode)
@@ -22,6 +37,7 @@ struct GateUpParams {
   float* s;                   // [S, I/256]
   int hidden, intermediate, max_tiles, interleaved;
   int sw_vectors;             // scale_w starts on a 16-byte boundary
+  HostReport report;          // routing statistics for a host that polls
 };
 
 // Work item -> (row tile, channel group).  Items of one expert are consecutive and ordered

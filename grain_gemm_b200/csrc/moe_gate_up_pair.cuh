@@ -13,6 +13,7 @@
 //   warp 9    MMA issuer of the leader CTA: two cta_group::2 MMAs a K step, each over one M tile (64 channels)
 //             of either CTA; a CTA holds half of the token rows.  Two TMEM buffers of 2 x 128 columns.
 //   warp 10   scale staging, as in the other kernels
+//   warp 11   hands routing statistics to the host where they are asked for
 //   warps 0-7 promotion: warp (quarter, half) holds lanes 32 * quarter.. of M tile `half` for all tokens;
 //             then SwiGLU, maxima, requantisation.
 //
@@ -498,6 +499,8 @@ __device__ __forceinline__ void gate_up_pair_body(const CUtensorMap& map_x, cons
         }
       }
       cp_async_wait_all();
+    } else {
+      report_to_polling_host(p.report, lane);
     }
   } else {
     setmaxnreg_inc<GG_PROMO_REGS>();

@@ -21,6 +21,7 @@
 //   warp 8    TMA producer: per stage the activation rows (one box, or 32 row gathers) and two weight boxes
 //   warp 9    MMA issuer (tcgen05.mma kind::i8, two TMEM buffers)
 //   warp 10   scale staging (cp.async of each K group's column and row scales into a shared-memory ring)
+//   warp 11   hands routing statistics to the host where they are asked for
 //   warps 0-7 promotion per K group, then SwiGLU (silu by table lookup); the first sub-tile's h
 //             is parked in shared memory until the second sub-tile supplies the other half of
 //             the row maximum.
@@ -155,7 +156,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
   if (warp != 9) {
     // ------------------------------------------------------------ TMA producer (warp 8)
     // Three boxes per stage: 128 sorted activation rows, 128 gate and 128 up weight rows.
-    // The warp walks the ring converged; one elected lane issues the tiled loads.  Warp 11 idles.
+    // The warp walks the ring converged; one elected lane issues the tiled loads.
     if (warp == 8) {
       const bool leader = elect_one();
       uint32_t stage = 0, phase = 0;
@@ -262,6 +263,8 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
       }
       cp_async_wait_all();
+    } else {
+      report_to_polling_host(p.report, lane);
     }
   } else {
     // ------------------------------------------------------------ MMA issuer

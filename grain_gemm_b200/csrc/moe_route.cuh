@@ -17,6 +17,33 @@ namespace gg {
 
 constexpr int kRouteChunk = 1024;
 
+// Row-tile list for the grouped kernels: every expert's sorted rows are cut into tiles of `rows`; the
+// lists have room for ceil(S / rows) + E entries, the used ones come first, the others get expert -1.
+struct TileList {
+  int* expert;      // null: no list is asked for
+  int* row;
+  int rows, capacity;
+};
+
+__device__ __forceinline__ int tiles_of(const TileList& list, int count) {
+  return list.expert != nullptr ? (count + list.rows - 1) / list.rows : 0;
+}
+// The tiles of one expert, whose rows start at `begin`, from entry `first` on.
+__device__ __forceinline__ void write_tiles(const TileList& list, int expert, int begin, int first, int tiles) {
+  for (int t = 0; t < tiles; ++t) {
+    list.expert[first + t] = expert;
+    list.row[first + t] = begin + t * list.rows;
+  }
+}
+// Entries behind the used ones, by the whole CTA.
+__device__ __forceinline__ void clear_unused_tiles(const TileList& list, int used) {
+  if (list.expert == nullptr) return;
+  for (int t = used + threadIdx.x; t < list.capacity; t += blockDim.x) {
+    list.expert[t] = -1;
+    list.row[t] = 0;
+  }
+}
+
 struct RouteParams {
   const void* ids;
   int ids_are_i64;
@@ -29,17 +56,26 @@ struct RouteParams {
   int* offsets;         // [E+1]
   int* statistics;      // [3]
   int* workspace;       // [chunks * (E + 1) + chunks] for the multi-chunk path
+  TileList tiles;
 };
 
-__device__ __forceinline__ int route_key(const RouteParams& p, long long s, bool& invalid) {
+__device__ __forceinline__ void store_effective_id(const RouteParams& p, long long s, int key) {
+  if (p.ids_are_i64) reinterpret_cast<long long*>(p.effective_ids)[s] = key;
+  else reinterpret_cast<int*>(p.effective_ids)[s] = key;
+}
+
+__device__ __forceinline__ int route_key_of(const RouteParams& p, long long s, bool& invalid) {
   const long long id = p.ids_are_i64 ? reinterpret_cast<const long long*>(p.ids)[s]
                                      : static_cast<long long>(reinterpret_cast<const int*>(p.ids)[s]);
   const bool enabled = p.mask == nullptr || p.mask[s / p.top_k] != 0;
   const bool in_range = id >= 0 && id < p.experts;
   invalid = enabled && !in_range;
-  const int key = (enabled && in_range) ? static_cast<int>(id) : p.experts;
-  if (p.ids_are_i64) reinterpret_cast<long long*>(p.effective_ids)[s] = key;
-  else reinterpret_cast<int*>(p.effective_ids)[s] = key;
+  return (enabled && in_range) ? static_cast<int>(id) : p.experts;
+}
+
+__device__ __forceinline__ int route_key(const RouteParams& p, long long s, bool& invalid) {
+  const int key = route_key_of(p, s, invalid);
+  store_effective_id(p, s, key);
   return key;
 }
 
@@ -72,19 +108,25 @@ __device__ __forceinline__ void route_place_chunk(const RouteParams& p, long lon
 }
 
 // Scan of the per-key totals held in bins[0..E]; leaves bins[key] = first slot of the key and
-// writes counts, offsets and statistics.  Called by one whole warp, 32 keys at a time (a single
-// thread took 2 us of a decode step for 128 experts).
-__device__ __forceinline__ void route_finish_totals(const RouteParams& p, int* bins, int invalid) {
+// writes counts, offsets, statistics and the used part of the tile list, whose length it returns
+// (in every lane).  Called by one whole warp, 32 keys at a time (a single thread took 2 us of a
+// decode step for 128 experts).
+__device__ __forceinline__ int route_finish_totals(const RouteParams& p, int* bins, int invalid) {
   const int lane = threadIdx.x & 31;
-  int running = 0, maximum = 0, valid = 0;
+  int running = 0, maximum = 0, valid = 0, used_tiles = 0;
   for (int base = 0; base <= p.experts; base += 32) {
     const int e = base + lane;
     const int count = e <= p.experts ? bins[e] : 0;
-    int inclusive = count;
+    const int tiles = e < p.experts ? tiles_of(p.tiles, count) : 0;
+    int inclusive = count, inclusive_tiles = tiles;
 #pragma unroll
     for (int offset = 1; offset < 32; offset <<= 1) {
       const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
-      if (lane >= offset) inclusive += other;
+      const int other_tiles = __shfl_up_sync(0xffffffffu, inclusive_tiles, offset);
+      if (lane >= offset) {
+        inclusive += other;
+        inclusive_tiles += other_tiles;
+      }
     }
     const int first = running + inclusive - count;
     if (e <= p.experts) bins[e] = first;
@@ -94,7 +136,9 @@ __device__ __forceinline__ void route_finish_totals(const RouteParams& p, int* b
       maximum = max(maximum, count);
       valid = first + count;
     }
+    write_tiles(p.tiles, e, first, used_tiles + inclusive_tiles - tiles, tiles);
     running += __shfl_sync(0xffffffffu, inclusive, 31);
+    used_tiles += __shfl_sync(0xffffffffu, inclusive_tiles, 31);
   }
 #pragma unroll
   for (int offset = 16; offset > 0; offset >>= 1) {
@@ -107,10 +151,12 @@ __device__ __forceinline__ void route_finish_totals(const RouteParams& p, int* b
     p.statistics[1] = maximum;
     p.statistics[2] = valid;
   }
+  return used_tiles;
 }
 
 // Whole routing problem in one CTA (S <= 1024): keys, histogram, scan and placement.
 __device__ __forceinline__ void route_single_body(const RouteParams& p, int* bins) {
+  __shared__ int used_tiles;
   const long long slots = static_cast<long long>(p.tokens) * p.top_k;
   for (int i = threadIdx.x; i < p.experts + 2; i += blockDim.x) bins[i] = 0;
   __syncthreads();
@@ -124,8 +170,12 @@ __device__ __forceinline__ void route_single_body(const RouteParams& p, int* bin
     if (invalid) atomicAdd(&bins[p.experts + 1], 1);
   }
   __syncthreads();
-  if (threadIdx.x < 32) route_finish_totals(p, bins, bins[p.experts + 1]);
+  if (threadIdx.x < 32) {
+    const int used = route_finish_totals(p, bins, bins[p.experts + 1]);
+    if (threadIdx.x == 0) used_tiles = used;
+  }
   __syncthreads();
+  clear_unused_tiles(p.tiles, used_tiles);
   route_place_chunk(p, s, present, key, bins, static_cast<int>((slots + 31) / 32));
 }
 
@@ -158,6 +208,7 @@ __global__ void __launch_bounds__(1024) route_medium_kernel(const RouteParams p)
   int* key_total = medium_smem + 32 * keys;        // [keys] totals, then first slots
   int* scan_scratch = key_total + keys;            // [32] warp totals of the block scan
   int* invalid_total = scan_scratch + 32;          // [1]
+  int* tile_total = invalid_total + 1;             // [1]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long slots = static_cast<long long>(p.tokens) * p.top_k;
   for (int i = threadIdx.x; i < 32 * keys; i += 1024) warp_bins[i] = 0;
@@ -169,16 +220,19 @@ __global__ void __launch_bounds__(1024) route_medium_kernel(const RouteParams p)
   int* bins = warp_bins + warp * keys;
   int key[kRouteMediumRounds];
   int invalid_count = 0;
+  // All keys are fetched before the first is counted: one memory latency instead of one per round.
 #pragma unroll
   for (int r = 0; r < kRouteMediumRounds; ++r) {
     const long long s = warp_begin + r * 32 + lane;
-    const bool present = r * 32 < per_warp && s < slots;
-    key[r] = -1;
-    if (present) {
-      bool invalid;
-      key[r] = route_key(p, s, invalid);
-      invalid_count += invalid ? 1 : 0;
-    }
+    bool invalid = false;
+    key[r] = r * 32 < per_warp && s < slots ? route_key_of(p, s, invalid) : -1;
+    invalid_count += invalid ? 1 : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < kRouteMediumRounds; ++r) {
+    const long long s = warp_begin + r * 32 + lane;
+    const bool present = key[r] >= 0;
+    if (present) store_effective_id(p, s, key[r]);
     const unsigned active = __ballot_sync(0xffffffffu, present);
     if (present) {
       const unsigned same = __match_any_sync(active, key[r]);
@@ -203,9 +257,12 @@ __global__ void __launch_bounds__(1024) route_medium_kernel(const RouteParams p)
     key_total[k] = running;
   }
   __syncthreads();
-  // Block-wide exclusive scan of key_total (keys <= 512: one value per thread of 16 warps).
-  int value = threadIdx.x < keys ? key_total[threadIdx.x] : 0;
-  int inclusive = value;
+  // Block-wide exclusive scan over the keys (at most 512: one per thread of 16 warps) of the totals, and in
+  // the upper half of the word of the tiles: at most 8192 of either.
+  const int value = threadIdx.x < keys ? key_total[threadIdx.x] : 0;
+  const int tiles = threadIdx.x < p.experts ? tiles_of(p.tiles, value) : 0;
+  const int packed = value | tiles << 16;
+  int inclusive = packed;
   for (int offset = 1; offset < 32; offset <<= 1) {
     const int other = __shfl_up_sync(0xffffffffu, inclusive, offset);
     if (lane >= offset) inclusive += other;
@@ -220,17 +277,21 @@ __global__ void __launch_bounds__(1024) route_medium_kernel(const RouteParams p)
       if (lane >= offset) scanned += other;
     }
     scan_scratch[lane] = scanned - total;
+    if (lane == 31) *tile_total = scanned >> 16;
   }
   __syncthreads();
-  const int first_slot = scan_scratch[warp] + inclusive - value;
+  const int before = scan_scratch[warp] + inclusive - packed;
+  const int first_slot = before & 0xffff;
   if (threadIdx.x < keys) {
     key_total[threadIdx.x] = first_slot;
     if (threadIdx.x < p.experts) {
       p.counts[threadIdx.x] = value;
       p.offsets[threadIdx.x + 1] = first_slot + value;
+      write_tiles(p.tiles, threadIdx.x, first_slot, before >> 16, tiles);
     }
     if (threadIdx.x == 0) p.offsets[0] = 0;
   }
+  clear_unused_tiles(p.tiles, *tile_total);
   // Largest expert count (statistics[1]).
   int largest = threadIdx.x < p.experts ? value : 0;
   for (int offset = 16; offset > 0; offset >>= 1) {
@@ -297,6 +358,7 @@ __global__ void __launch_bounds__(1024) route_scan_kernel(const RouteParams p, i
   dependents_may_launch();
   previous_kernel_done();
   extern __shared__ int bins[];  // [E + 1]
+  __shared__ int used_tiles;
   const int stride = p.experts + 1;
   for (int key = threadIdx.x; key <= p.experts; key += blockDim.x) {
     int total = 0;
@@ -312,9 +374,11 @@ __global__ void __launch_bounds__(1024) route_scan_kernel(const RouteParams p, i
     for (int offset = 16; offset > 0; offset >>= 1) {
       invalid += __shfl_xor_sync(0xffffffffu, invalid, offset);
     }
-    route_finish_totals(p, bins, invalid);
+    const int used = route_finish_totals(p, bins, invalid);
+    if (threadIdx.x == 0) used_tiles = used;
   }
   __syncthreads();
+  clear_unused_tiles(p.tiles, used_tiles);
   for (int key = threadIdx.x; key <= p.experts; key += blockDim.x) {
     int running = bins[key];
     for (int c = 0; c < chunks; ++c) {
@@ -357,13 +421,10 @@ report_to_host_kernel(const int* values, int count, int* host_words) {
   __threadfence_system();
 }
 
-// Row-tile list for the grouped kernels: every expert's sorted rows are cut into tiles of
-// `tile_rows`; tile_expert/tile_row have room for ceil(S / tile_rows) + E entries, unused
-// entries get expert -1.  One CTA: a block-wide exclusive scan of the experts' tile counts,
-// 1024 experts at a time.
+// Row-tile list of a routing that was made without one.  One CTA: a block-wide exclusive scan of the
+// experts' tile counts, 1024 experts at a time.
 __global__ void __launch_bounds__(1024)
-moe_tiles_kernel(const int* offsets, int experts, int tile_rows, int max_tiles, int* tile_expert,
-                 int* tile_row) {
+moe_tiles_kernel(const int* offsets, int experts, const TileList list) {
   dependents_may_launch();
   previous_kernel_done();
   __shared__ int warp_total[32];
@@ -376,7 +437,7 @@ moe_tiles_kernel(const int* offsets, int experts, int tile_rows, int max_tiles, 
     int begin = 0, tiles = 0;
     if (e < experts) {
       begin = offsets[e];
-      tiles = (offsets[e + 1] - begin + tile_rows - 1) / tile_rows;
+      tiles = tiles_of(list, offsets[e + 1] - begin);
     }
     int inclusive = tiles;
     for (int offset = 1; offset < 32; offset <<= 1) {
@@ -396,18 +457,12 @@ moe_tiles_kernel(const int* offsets, int experts, int tile_rows, int max_tiles, 
     }
     __syncthreads();
     const int first = carry + warp_total[warp] + inclusive - tiles;
-    for (int t = 0; t < tiles; ++t) {
-      tile_expert[first + t] = e;
-      tile_row[first + t] = begin + t * tile_rows;
-    }
+    write_tiles(list, e, begin, first, tiles);
     __syncthreads();
     if (threadIdx.x == 1023) carry = first + tiles;
     __syncthreads();
   }
-  for (int t = carry + threadIdx.x; t < max_tiles; t += blockDim.x) {
-    tile_expert[t] = -1;
-    tile_row[t] = 0;
-  }
+  clear_unused_tiles(list, carry);
 }
 
 // ------------------------------------------------------------------ SwiGLU + requantisation

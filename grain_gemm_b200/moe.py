@@ -5,7 +5,7 @@ Signature, validation and stage semantics follow the reference's ``src/grain_gem
 (``Routes`` :20-45, ``prepare_routes`` :222-291, ``swiglu_quantize`` :604-631, ``combine``
 :656-676).  The stages run as four hand-written sm_100a kernels behind the C ABI:
 
-1. route / stable sort                      (``gg_moe_route`` + ``gg_moe_tiles``)
+1. route / stable sort, row-tile list       (``gg_moe_route_tiles``)
 2. gathered Gate/Up + rounding + SwiGLU + G256 requantisation   (``gg_moe_gate_up``)
 3. grouped Down projection over the sorted slots                (``gg_moe_down``)
 4. top-k weighted combine                                       (``gg_moe_combine``)
@@ -181,6 +181,19 @@ class Routes:
     tile_expert: torch.Tensor | None = None
     tile_row: torch.Tensor | None = None
 
+    @classmethod
+    def of_parts(cls, parts, experts, tile_rows):
+        """From what the native host path returns; the frozen dataclass's own constructor sets the
+        fields one by one, 3 us of a decode step."""
+        _, ids, order, counts, offsets, inverse, effective_ids, statistics, expert, row = parts
+        tokens, top_k = ids.shape
+        routes = cls.__new__(cls)
+        routes.__dict__.update(order=order, counts=counts, offsets=offsets, inverse=inverse,
+                               effective_ids=effective_ids, statistics=statistics, tokens=tokens,
+                               top_k=top_k, experts=experts, tile_rows=tile_rows, tile_expert=expert,
+                               tile_row=row)
+        return routes
+
 
 def prepare_routes(topk_ids, num_experts, token_mask=None, tile_rows=TENSOR_CORE_TILE_ROWS,
                    workspace=None):
@@ -207,15 +220,19 @@ def prepare_routes(topk_ids, num_experts, token_mask=None, tile_rows=TENSOR_CORE
     scratch = (_buffer(workspace, "route_scratch", (workspace_bytes,), torch.uint8, device)
                if workspace_bytes else None)
     stream = _loader.stream_pointer(device)
-    _loader.check(lib.gg_moe_route(
+    capacity, tiles = 0, (None, None)
+    if tile_rows:
+        capacity = max(1, lib.gg_moe_tile_capacity(slots, num_experts, tile_rows))
+        tiles = _buffer(workspace, "tiles", (2, capacity), torch.int32, device)
+    _loader.check(lib.gg_moe_route_tiles(
         _loader.pointer(ids), int(ids.dtype == torch.int64), _loader.pointer(mask),
         tokens, top_k, num_experts, _loader.pointer(effective_ids), _loader.pointer(order),
         _loader.pointer(inverse), _loader.pointer(counts), _loader.pointer(offsets),
-        _loader.pointer(statistics), _loader.pointer(scratch), workspace_bytes, stream),
-        "gg_moe_route")
-    routes = Routes(order, counts, offsets, inverse, effective_ids, statistics,
-                    tokens, top_k, num_experts)
-    return prepare_tiles(routes, tile_rows, workspace) if tile_rows else routes
+        _loader.pointer(statistics), _loader.pointer(scratch), workspace_bytes, tile_rows, capacity,
+        _loader.pointer(tiles[0]), _loader.pointer(tiles[1]), stream),
+        "gg_moe_route_tiles")
+    return Routes(order, counts, offsets, inverse, effective_ids, statistics, tokens, top_k,
+                  num_experts, tile_rows, tiles[0], tiles[1])
 
 
 def prepare_tiles(routes, tile_rows, workspace=None):

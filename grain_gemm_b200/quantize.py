@@ -95,8 +95,8 @@ def route_topk_routes(logits, top_k, *, token_mask=None, ids_dtype=torch.int64, 
     """``route_topk`` and ``moe.prepare_routes`` together: ``(topk_weights, topk_ids, routes)``.
 
     For decode-sized problems (``T * top_k <= 1024``) both steps run in ONE kernel launch
-    (``gg_moe_route_topk``: the CTA that selects the experts sorts the assignments it has just
-    written); larger problems make the two calls.  Pass ``routes`` on to
+    (``gg_moe_route_topk_tiles``: the CTA that selects the experts sorts the assignments it has just
+    written and lists the row tiles); larger problems make the two calls.  Pass ``routes`` on to
     ``moe_ffn(..., routes=routes)`` to skip its own routing.  Results are identical either way.
     """
     from . import moe
@@ -104,9 +104,7 @@ def route_topk_routes(logits, top_k, *, token_mask=None, ids_dtype=torch.int64, 
             and (ids_dtype is torch.int64 or ids_dtype is torch.int32)):
         parts = _loader.host().route_topk_routes(logits, top_k, token_mask, ids_dtype is torch.int64)
         if parts is not None:
-            weights, ids, order, counts, offsets, inverse, effective_ids, statistics, expert, row = parts
-            return weights, ids, moe.Routes(order, counts, offsets, inverse, effective_ids, statistics,
-                                            *ids.shape, logits.shape[1], tile_rows, expert, row)
+            return parts[0], parts[1], moe.Routes.of_parts(parts, logits.shape[1], tile_rows)
     if not isinstance(logits, torch.Tensor) or logits.dim() != 2:
         raise ValueError("logits must be a [T, E] tensor")
     tokens, experts = logits.shape

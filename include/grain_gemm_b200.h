@@ -115,6 +115,16 @@ int gg_moe_route(const void* ids, int ids_are_i64, const void* mask, int tokens,
                  void* stream);
 
 /*
+ * gg_moe_route that also writes gg_moe_tiles' list, without a launch of its own (tile_expert NULL: no
+ * list).  tile_rows, tile_capacity, tile_expert and tile_row as for gg_moe_tiles.
+ */
+int gg_moe_route_tiles(const void* ids, int ids_are_i64, const void* mask, int tokens, int top_k,
+                       int experts, void* effective_ids, void* order, void* inverse, void* counts,
+                       void* offsets, void* statistics, void* workspace, size_t workspace_bytes,
+                       int tile_rows, int tile_capacity, void* tile_expert, void* tile_row,
+                       void* stream);
+
+/*
  * gg_moe_route for callers that cannot allocate device memory.  This entry point has no
  * counterpart in the reference.  Some hosts of this library are not allowed to call
  * cudaMalloc (or an allocator built on it) at the point where routing runs: an inference
@@ -178,6 +188,13 @@ int gg_moe_route_topk(const void* logits, int in_dtype, const void* mask, int to
                       void* order, void* inverse, void* counts, void* offsets, void* statistics,
                       void* stream);
 
+/* gg_moe_route_topk that also writes the row-tile list, as gg_moe_route_tiles does. */
+int gg_moe_route_topk_tiles(const void* logits, int in_dtype, const void* mask, int tokens, int experts,
+                            int top_k, void* weights, void* ids, int ids_are_i64, void* effective_ids,
+                            void* order, void* inverse, void* counts, void* offsets, void* statistics,
+                            int tile_rows, int tile_capacity, void* tile_expert, void* tile_row,
+                            void* stream);
+
 /*
  * Entry quantiser (the step before both paths): x[rows, width] of dtype in_dtype (GG_OUT_FP32,
  * GG_OUT_BF16 or GG_OUT_FP16 name the element type), contiguous, width a multiple of 256,
@@ -229,6 +246,18 @@ int gg_moe_gate_up(const void* x, const void* scale_x, const void* w1, const voi
                    const void* tile_row, int tile_capacity, int tile_rows, void* q, void* s,
                    void* gate_up_scratch, int tokens, int top_k, int experts, int hidden,
                    int intermediate, int interleaved, int out_dtype, int row_gather, void* stream);
+
+/*
+ * gg_moe_gate_up whose kernel also hands `count` integers at `values` (routing statistics) to the host, for a caller that polls: it stores a value that values[0] cannot have into host_words[0]
+ * (page-locked memory) before the call and waits until it changes; the other words are there by
+ * then.  tile_rows 128 only.
+ */
+int gg_moe_gate_up_report(const void* x, const void* scale_x, const void* w1, const void* scale_w1,
+                          const void* order, const void* offsets, const void* tile_expert,
+                          const void* tile_row, int tile_capacity, int tile_rows, void* q, void* s,
+                          void* gate_up_scratch, int tokens, int top_k, int experts, int hidden,
+                          int intermediate, int interleaved, int out_dtype, int row_gather,
+                          const void* values, int count, void* host_words, void* stream);
 
 /*
  * Down projection over the sorted slots: expert_out[S,H] (out_dtype) from q[S,I], s[S,I/256],
