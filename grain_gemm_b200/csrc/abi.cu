@@ -344,7 +344,7 @@ static int launch_tc_dtype(const CUtensorMap& map_a, const CUtensorMap& map_b, c
 static int weight_row_block(int bn, int out_dtype) {
   const int bytes = out_dtype == GG_OUT_FP32 ? 4 : 2;
   return bn == 256 ? GemmTcShape<1, 256, 4>::row_block(bytes)
-         : bn == 128 ? GemmTcShape<1, 128, 6>::row_block(bytes) : GemmTcShape<1, 64, 8>::row_block(bytes);
+         : bn == 128 ? GemmTcShape<1, 128, 3>::row_block(bytes) : GemmTcShape<1, 64, 4>::row_block(bytes);
 }
 
 static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
@@ -378,10 +378,10 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   p.c_vector_ok = aligned16(g.c) && (g.ldc * out_bytes) % 16 == 0;
   switch (variant) {
     case GG_VARIANT_TC_N256: return launch_tc_dtype<1, 256, 4, false>(map_a, map_b, p, g.out_dtype, stream);
-    case GG_VARIANT_TC_N128: return launch_tc_dtype<1, 128, 6, false>(map_a, map_b, p, g.out_dtype, stream);
-    case GG_VARIANT_TC_N64: return launch_tc_dtype<1, 64, 8, false>(map_a, map_b, p, g.out_dtype, stream);
+    case GG_VARIANT_TC_N128: return launch_tc_dtype<1, 128, 3, false>(map_a, map_b, p, g.out_dtype, stream);
+    case GG_VARIANT_TC_N64: return launch_tc_dtype<1, 64, 4, false>(map_a, map_b, p, g.out_dtype, stream);
     case GG_VARIANT_TC_PAIR_N256: return launch_tc_dtype<2, 256, 6, false>(map_a, map_b, p, g.out_dtype, stream);
-    case GG_VARIANT_TC_PAIR_N128: return launch_tc_dtype<2, 128, 8, false>(map_a, map_b, p, g.out_dtype, stream);
+    case GG_VARIANT_TC_PAIR_N128: return launch_tc_dtype<2, 128, 4, false>(map_a, map_b, p, g.out_dtype, stream);
     default: return static_cast<int>(cudaErrorInvalidValue);
   }
 }
@@ -1010,8 +1010,8 @@ int gg_moe_down(const void* q, const void* s, const void* w2, const void* scale_
     p.sb_expert_stride = static_cast<long long>(intermediate / 256) * hidden;
     p.row_destination = destinations;
     if (bn == 256) return gg::launch_tc_dtype<1, 256, 4, true>(map_a, map_b, p, out_dtype, stream);
-    if (bn == 128) return gg::launch_tc_dtype<1, 128, 6, true>(map_a, map_b, p, out_dtype, stream);
-    return gg::launch_tc_dtype<1, 64, 8, true>(map_a, map_b, p, out_dtype, stream);
+    if (bn == 128) return gg::launch_tc_dtype<1, 128, 3, true>(map_a, map_b, p, out_dtype, stream);
+    return gg::launch_tc_dtype<1, 64, 4, true>(map_a, map_b, p, out_dtype, stream);
   }
   if (tile_rows != gg::kSimtTile) return static_cast<int>(cudaErrorInvalidValue);
   gg::GemmSimtParams p = {};

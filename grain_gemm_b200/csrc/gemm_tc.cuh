@@ -8,8 +8,9 @@
 // to FP32 once, one fused multiply-add per group, one final cast.
 //
 // Kernel shape (persistent, warp specialised, 384 threads):
-//   producer    TMA warp: A tile [128 rows x 128 B of K] and B tile [BN/ctas rows x 128 B]
-//               per stage, 128-byte swizzle, kStages-deep ring guarded by full/empty mbarriers.
+//   producer    TMA warp: A tile [128 rows x 128 B of K] and B tile [BN/ctas rows x 128 B] per slab,
+//               one or two slabs a stage, 128-byte swizzle, kStages-deep ring guarded by full/empty
+//               mbarriers.
 //   warp 9      MMA issuer: tcgen05.mma kind::i8, K = 32 per instruction, INT32 accumulators in
 //               TMEM, two accumulator buffers of BN columns.  The first MMA of every K group
 //               overwrites the buffer, the last one commits it to the promotion warps.
@@ -109,7 +110,11 @@ constexpr int kScaleChunkGroups = 4;
 template <int kCtaGroup, int BN, int kStages, int kPromoWarps = 8, int kARows = 128>
 struct GemmTcShape {
   static constexpr int kBM = 128;                       // rows per CTA
-  static constexpr int kBK = 128;                       // bytes of K per stage
+  static constexpr int kBK = 128;                       // bytes of K per slab
+  // Slabs per stage.  Handing a stage from the producer to the MMA issuer and back takes each of them some
+  // 300 cycles a stage whatever its size; a slab of a tile of 64 or 128 columns is multiplied and
+  // promoted in less, so that tiles of these widths hand over two slabs at a time (one group of 256).
+  static constexpr int kSlabs = BN <= 128 ? 2 : 1;
   static constexpr int kBRows = BN / kCtaGroup;         // B rows loaded by each CTA
   // Rows of A actually fetched per stage.  Skinny problems (M <= kARows) fetch only that many:
   // the MMA still reads 128 rows, the rest being whatever follows in the stage (the B tile),
@@ -118,7 +123,8 @@ struct GemmTcShape {
   static_assert(kARows % 8 == 0 && kARows <= 128 && (kARows == 128 || kBRows >= 128),
                 "a short A tile needs the B tile behind it to cover the 128 rows the MMA reads");
   static constexpr int kBBytes = kBRows * kBK;
-  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kSlabBytes = kABytes + kBBytes;
+  static constexpr int kStageBytes = kSlabs * kSlabBytes;
   static constexpr int kTmemColumns = 2 * BN;
   // Ring of per-group scale vectors (the short-A shape is the split-K dump kernel, which
   // stages no scales and needs the room for its operand stages).
@@ -415,22 +421,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
       const int b_c1 = p.permuted_columns ? 0 : row_b;
       const int b_c3 = p.permuted_columns ? row_b / kRowBlock : 0;
-      for (int slab = 0, x = work.k_begin; slab < work.slabs; ++slab, x += Shape::kBK) {
+      for (int slab = 0; slab < work.slabs; slab += Shape::kSlabs) {
         if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1u, kSiteProducerEmpty, abort_flag)) {
           ok = false;
           break;
         }
+        const int in_stage = min(Shape::kSlabs, work.slabs - slab);
         if (leader) {
-          uint8_t* a_dst = stage_base + stage * Shape::kStageBytes;
-          uint8_t* b_dst = a_dst + Shape::kABytes;
-          if constexpr (kCtaGroup == 1) {
-            mbar_expect_tx(&full_bar[stage], Shape::kStageBytes);
-            tma_load_2d(a_dst, &map_a, &full_bar[stage], x, row_a);
-            tma_load_4d(b_dst, &map_b, &full_bar[stage], x, b_c1, b_c3);
-          } else {
-            if (cta_rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Shape::kStageBytes);
-            tma_load_2d_pair(a_dst, &map_a, &full_bar[stage], x, row_a);
-            tma_load_4d_pair(b_dst, &map_b, &full_bar[stage], x, b_c1, b_c3);
+          if (kCtaGroup == 1 || cta_rank == 0) {
+            mbar_expect_tx(&full_bar[stage], kCtaGroup * in_stage * Shape::kSlabBytes);
+          }
+#pragma unroll
+          for (int i = 0; i < Shape::kSlabs; ++i) {
+            if (i < in_stage) {
+              const int x = work.k_begin + (slab + i) * Shape::kBK;
+              uint8_t* a_dst = stage_base + stage * Shape::kStageBytes + i * Shape::kSlabBytes;
+              uint8_t* b_dst = a_dst + Shape::kABytes;
+              if constexpr (kCtaGroup == 1) {
+                tma_load_2d(a_dst, &map_a, &full_bar[stage], x, row_a);
+                tma_load_4d(b_dst, &map_b, &full_bar[stage], x, b_c1, b_c3);
+              } else {
+                tma_load_2d_pair(a_dst, &map_a, &full_bar[stage], x, row_a);
+                tma_load_4d_pair(b_dst, &map_b, &full_bar[stage], x, b_c1, b_c3);
+              }
+            }
           }
         }
         if (++stage == kStages) {
@@ -460,13 +474,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
         if (work.whole_g256) {
           // G = 256 with whole groups: two slabs per group, no per-MMA bookkeeping.
-          for (int slab = 0; slab < work.slabs; ++slab) {
+          for (int slab = 0; slab < work.slabs; slab += Shape::kSlabs) {
             if (!mbar_wait_warp(&full_bar[stage], phase, kSiteMmaFull, abort_flag)) {
               ok = false;
               break;
             }
             tcgen05_fence_after();
-            const bool group_start = (slab & 1) == 0;
+            const bool group_start = Shape::kSlabs == 2 || (slab & 1) == 0;
+            const bool group_end = Shape::kSlabs == 2 || !group_start;
             if (group_start) {
               if (!mbar_wait_warp(&tmem_empty_bar[buffer], empty_parity, kSiteMmaTmemEmpty,
                                   abort_flag)) {
@@ -476,21 +491,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               tcgen05_fence_after();
             }
             const uint32_t a_low = a_low_base + stage * (Shape::kStageBytes >> 4);
-            const uint32_t b_low = a_low + (Shape::kABytes >> 4);
             const uint32_t tmem_d = tmem_base + buffer * BN;
             if (leader) {
-              umma_i8<kCtaGroup>(tmem_d, a_low, b_low, idesc, group_start ? 0u : 1u);
-              umma_i8<kCtaGroup>(tmem_d, a_low + 2, b_low + 2, idesc, 1u);
-              umma_i8<kCtaGroup>(tmem_d, a_low + 4, b_low + 4, idesc, 1u);
-              umma_i8<kCtaGroup>(tmem_d, a_low + 6, b_low + 6, idesc, 1u);
+#pragma unroll
+              for (int i = 0; i < Shape::kSlabs; ++i) {
+                const uint32_t a_slab = a_low + i * (Shape::kSlabBytes >> 4);
+                const uint32_t b_slab = a_slab + (Shape::kABytes >> 4);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  umma_i8<kCtaGroup>(tmem_d, a_slab + 2 * j, b_slab + 2 * j, idesc,
+                                     group_start && i == 0 && j == 0 ? 0u : 1u);
+                }
+              }
               if constexpr (kCtaGroup == 1) umma_commit(&empty_bar[stage]);
               else umma_commit_pair(&empty_bar[stage], 3);
-              if (!group_start) {
+              if (group_end) {
                 if constexpr (kCtaGroup == 1) umma_commit(&tmem_full_bar[buffer]);
                 else umma_commit_pair(&tmem_full_bar[buffer], 3);
               }
             }
-            if (!group_start) {
+            if (group_end) {
               buffer ^= 1u;
               if (buffer == 0) empty_parity ^= 1u;
             }
@@ -502,16 +522,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           continue;
         }
         int remaining = work.ksteps;
-        for (int slab = 0; slab < work.slabs && ok; ++slab) {
+        for (int slab = 0; slab < work.slabs && ok; slab += Shape::kSlabs) {
           if (!mbar_wait_warp(&full_bar[stage], phase, kSiteMmaFull, abort_flag)) {
             ok = false;
             break;
           }
           tcgen05_fence_after();
           const uint32_t a_low = a_low_base + stage * (Shape::kStageBytes >> 4);
-          const uint32_t b_low = a_low + (Shape::kABytes >> 4);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
+          for (int j = 0; j < 4 * Shape::kSlabs; ++j) {
             if (remaining > 0) {
               if (step == 0) {
                 if (!mbar_wait_warp(&tmem_empty_bar[buffer], empty_parity, kSiteMmaTmemEmpty,
@@ -521,8 +540,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 tcgen05_fence_after();
               }
+              const uint32_t a_step = a_low + (j >> 2) * (Shape::kSlabBytes >> 4) + 2 * (j & 3);
               if (leader) {
-                umma_i8<kCtaGroup>(tmem_base + buffer * BN, a_low + 2 * j, b_low + 2 * j, idesc,
+                umma_i8<kCtaGroup>(tmem_base + buffer * BN, a_step, a_step + (Shape::kABytes >> 4), idesc,
                                    step != 0 ? 1u : 0u);
               }
               ++step;
