@@ -289,7 +289,7 @@ template <int kCtaGroup, int BN, int kStages, typename OutT, bool kGrouped, int 
           int kARows = 128>
 static int launch_tc_kernel(const CUtensorMap& map_a, const CUtensorMap& map_b,
                             const GemmTcParams& p, cudaStream_t stream) {
-  using Shape = GemmTcShape<kCtaGroup, BN, kStages, kPromoWarps, kARows>;
+  using Shape = GemmTcShape<kCtaGroup, BN, kStages, kPromoWarps, kARows, staged_stores<OutT>(BN, false)>;
   auto kernel = gemm_tc_kernel<kCtaGroup, BN, kStages, OutT, kGrouped, kPromoWarps, false, kARows>;
   cudaError_t error =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::kSmemBytes);
@@ -331,7 +331,11 @@ static int launch_tc_dtype(const CUtensorMap& map_a, const CUtensorMap& map_b, c
   switch (out_dtype) {
     case GG_OUT_FP32:
       if constexpr (kGrouped) return static_cast<int>(cudaErrorInvalidValue);
-      else return launch_tc_kernel<kCtaGroup, BN, kStages, float, kGrouped, kPromoWarps, kARows>(map_a, map_b, p, stream);
+      else {
+        // Staged stores take the room of some operand stages.
+        constexpr int kFp32Stages = !staged_stores<float>(BN, false) ? kStages : kCtaGroup == 2 ? 4 : 3;
+        return launch_tc_kernel<kCtaGroup, BN, kFp32Stages, float, kGrouped, kPromoWarps, kARows>(map_a, map_b, p, stream);
+      }
     case GG_OUT_BF16:
       return launch_tc_kernel<kCtaGroup, BN, kStages, __nv_bfloat16, kGrouped, kPromoWarps, kARows>(map_a, map_b, p, stream);
     case GG_OUT_FP16:

@@ -107,7 +107,7 @@ struct TileWork {
 // not once per group.
 constexpr int kScaleChunkGroups = 4;
 
-template <int kCtaGroup, int BN, int kStages, int kPromoWarps = 8, int kARows = 128>
+template <int kCtaGroup, int BN, int kStages, int kPromoWarps = 8, int kARows = 128, bool kStagedStores = false>
 struct GemmTcShape {
   static constexpr int kBM = 128;                       // rows per CTA
   static constexpr int kBK = 128;                       // bytes of K per slab
@@ -133,7 +133,12 @@ struct GemmTcShape {
   static constexpr int kScaleSlotFloats = BN + 128;     // scale_b columns, then scale_a rows
   static constexpr int kScaleBytes = kScaleSlots * kScaleSlotFloats * 4;
   static constexpr int kBarrierBytes = (2 * kStages + 4 + 2 * kScaleChunks) * 8 + 16;
-  static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleBytes + kBarrierBytes;
+  // Finished tiles that leave through shared memory: 32 rows of 256 bytes per promotion warp, 16 bytes
+  // apart beyond that (the lanes of a quarter warp write to different banks).
+  static constexpr int kOutPitch = 256 + 16;
+  static constexpr int kOutBytes = kStagedStores ? kPromoWarps * 32 * kOutPitch : 0;
+  static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleBytes + kOutBytes + kBarrierBytes;
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of a CTA");
   static constexpr int kThreads = (kPromoWarps + 4) * 32;   // + producer, MMA, two spares
   static constexpr int kColumnsPerThread = BN / (kPromoWarps / 4);
   // Weight rows come in blocks of this many for outputs of `bytes` bytes (see the drain layout below).
@@ -152,6 +157,11 @@ struct GemmTcShape {
   static_assert(kColumnsPerThread % kDrainWidth == 0, "tile too narrow for the warp count");
   static_assert(BN == 64 || BN == 128 || BN == 256, "unsupported tile width");
 };
+
+template <typename OutT>
+__host__ __device__ constexpr bool staged_stores(int bn, bool dump) {
+  return sizeof(OutT) == 4 && bn == 256 && !dump;
+}
 
 __device__ __forceinline__ void tile_coordinates(int tile, int tiles_m, int tiles_n, int& tm,
                                                  int& tn, int band_rows = 8) {
@@ -196,31 +206,36 @@ __device__ __forceinline__ TileWork decode_tile(const GemmTcParams& p, int tile,
 // with eight warps draining 128 lanes x 256 columns: 16x128b delivers 507 B/clk/SM, 32x32b 940,
 // and 16x256b, which would give adjacent column pairs, 256.
 //
-// A row leaves as 32-byte stores, four lanes covering 128 consecutive bytes (one cache line) of it:
-// thread q wants 16 consecutive 16-bit outputs, or eight FP32 ones.  So the tensor map permutes the
-// weight's rows on the way in, in blocks of 64 or 32 (weight_row_map in tensor_map.cuh): the block's
-// row 16q + 8b + k (FP32: 8q + k) comes to TMEM column 32b + 4k + q, accumulator pair j of the block's
-// half b holds the outputs 16q + 8b + 2j and + 1, and nothing is exchanged between lanes.
-// The stores are bound by the cache lines that a warp's instruction touches: with 16-byte stores (eight
-// half lines an instruction) the tile of 128 x 256 16-bit outputs took 3100 to 3700 cycles, as long as
-// two or three K groups; the grouped Down projection of 512 tokens over 128 experts (H = 2048, three groups
-// a tile) went from 50.7 to 41.8 us, 256 x 4096 x 4096 with FP32 outputs from 11.5 to 10.9 us.  Widths that are not a multiple of the block take the rows in their own order,
+// A thread leaves with 32 consecutive bytes of a row: 16 of 16-bit outputs, or eight FP32 ones.  So the
+// tensor map permutes the weight's rows on the way in, in blocks of 64 or 32 (weight_row_map in
+// tensor_map.cuh): the block's row 16q + 8b + k (FP32: 8q + k) comes to TMEM column 32b + 4k + q,
+// accumulator pair j of the block's half b holds the outputs 16q + 8b + 2j and + 1, and nothing is
+// exchanged between lanes.  Widths that are not a multiple of the block take the rows in their own order,
 // where pair j holds the columns 8j + q and 8j + 4 + q of 32 and a 4x4 exchange inside every quad
-// precedes 16-byte stores.
+// follows.
+// They leave as 32-byte stores, four lanes covering a cache line (with 16-byte stores, eight half lines an
+// instruction, the grouped Down projection of 512 tokens over 128 experts, H = 2048, three groups a
+// tile, took 50.7 us, with these 41.8).  All CTAs finish their tiles at about the same time, and the burst is
+// what memory takes 3000 cycles for (128 x 256 16-bit outputs, the promotion warps waiting; two K groups' worth).
+// FP32 tiles of 256 columns, 8400 cycles as 16-byte stores, go through shared memory and leave with one
+// bulk copy of 256 bytes a row, which the warps do not wait for: 2048 x 4096 x 4096 41.0 to 38.6 us, 3221 x 6848 x
+// 9728 198 to 188.  (As 32-byte stores they take 5000, but the accumulators, stored as they are, would have
+// to be eight consecutive registers in the promotion loop, too: 1760 cycles a K group instead of 1520.  16-bit
+// tiles gain nothing from the copies: the promotion loop of that kernel came out 6 % slower.)
 //
-// Byte offset in a scale slot of thread q's eight column scales, in accumulator-pair order, for the
-// 32-column block `block`, less q times column_quad_bytes: the order in which permuted rows' scales
-// lie in memory anyway.
-template <int kRowBlock>
-__host__ __device__ constexpr int column_block_bytes(int block) {
-  return kRowBlock == 64 ? (block >> 1) * 256 + (block & 1) * 32 : block * 128;
-}
-template <int kRowBlock>
-__host__ __device__ constexpr int column_quad_bytes() { return kRowBlock == 64 ? 64 : 32; }
-// Byte offset of column `c` (0..31) of a 32-column block from column_block_bytes, rows in their own order.
-template <int kRowBlock>
+// In a scale slot the eight column scales of thread q for a 32-column block are two 16-byte vectors at
+// 128 * block + 32 * q bytes, in accumulator-pair order: four lanes that read 32 bytes apart do not
+// conflict.  (With the scales of blocks of 64 rows left in memory order, 64 bytes apart, two of the four
+// shared their banks and a K group took 1610 cycles instead of 1540.)
+// Byte offset of column `c` (0..31) of a block for rows in their own order.
 __device__ __forceinline__ int ring_column_bytes(int c) {
-  return (c & 3) * column_quad_bytes<kRowBlock>() + 4 * ((c >> 3) * 2 + ((c >> 2) & 1));
+  return (c & 3) * 32 + 4 * ((c >> 3) * 2 + ((c >> 2) & 1));
+}
+// Byte offset of the permuted output `c` (0..31) of the first half of a row block: memory order for blocks of
+// 32; in blocks of 64 output 16q + 8b + k goes to block b, the second half's outputs 64 bytes behind the first's.
+template <int kRowBlock>
+__device__ __forceinline__ int ring_output_bytes(int c) {
+  return kRowBlock == 64 ? ((c >> 3) & 1) * 128 + (c >> 4) * 32 + (c & 7) * 4 : 4 * c;
 }
 // Position of row `r` (0..31 within its warp's 32 rows): the thread with row index
 // lane / 4 = r % 8 reads its four rows r % 8 + 8j as one 16-byte vector.
@@ -324,7 +339,8 @@ template <int kCtaGroup, int BN, int kStages, typename OutT, bool kGrouped, int 
 __global__ void __launch_bounds__((kPromoWarps + 4) * 32, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const GemmTcParams p) {
-  using Shape = GemmTcShape<kCtaGroup, BN, kStages, kPromoWarps, kARows>;
+  constexpr bool kStagedStores = staged_stores<OutT>(BN, kDump);
+  using Shape = GemmTcShape<kCtaGroup, BN, kStages, kPromoWarps, kARows, kStagedStores>;
   constexpr int kNC = Shape::kColumnsPerThread;   // columns owned by one promotion thread
   constexpr int kRowBlock = Shape::row_block(sizeof(OutT));
   constexpr int kProducerWarp = kPromoWarps, kMmaWarp = kPromoWarps + 1;
@@ -335,8 +351,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* stage_base = smem;
   float* scale_ring = reinterpret_cast<float*>(smem + kStages * Shape::kStageBytes);
+  [[maybe_unused]] const uint32_t out_base =
+      smem_u32(smem + kStages * Shape::kStageBytes + Shape::kScaleBytes);
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kStages * Shape::kStageBytes +
-                                                   Shape::kScaleBytes);
+                                                   Shape::kScaleBytes + Shape::kOutBytes);
   uint64_t* empty_bar = full_bar + kStages;
   uint64_t* tmem_full_bar = empty_bar + kStages;
   uint64_t* tmem_empty_bar = tmem_full_bar + 2;
@@ -580,10 +598,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // waiting for scales).
     constexpr int kColumnsPerLane = BN / 32;
     // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-    // (Rows in fragment order keep their scales in memory order, otherwise they go to where the
-    // promotion threads look for the columns they hold.)
-    const uint32_t column_position = p.permuted_columns ? 4 * lane : ring_column_bytes<kRowBlock>(lane);
-    const uint32_t odd_block = p.permuted_columns ? 128 : column_block_bytes<kRowBlock>(1);
+    const uint32_t column_position =
+        p.permuted_columns ? ring_output_bytes<kRowBlock>(lane) : ring_column_bytes(lane);
+    const uint32_t odd_block = p.permuted_columns && kRowBlock == 64 ? 64 : 128;
+    // Four consecutive outputs of a row block at a time (sb_vectors).
+    const uint32_t vector_position = kRowBlock == 64 ? (lane >> 4) * 256 + ((lane >> 3) & 1) * 64 +
+                                                           ring_output_bytes<kRowBlock>(4 * (lane & 7))
+                                                     : 16 * lane;
     const uint32_t row_position = 4 * ring_row_position(lane);
     const uint32_t ring_base = smem_u32(scale_ring);
     uint32_t chunk = 0, phase = 0;
@@ -628,7 +649,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
             for (int j = 0; j < (BN + 127) / 128; ++j, source += 128) {
               if (BN >= 128 || lane < BN / 4) {
-                cp_async_f32x4(destination + 512 * j + 16 * lane, source, n0 + 128 * j + 4 * lane < p.n);
+                cp_async_f32x4(destination + 512 * j + vector_position, source, n0 + 128 * j + 4 * lane < p.n);
               }
             }
             vector_source += p.sb_sg;
@@ -793,8 +814,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                               kSiteEpilogueTmemFull, abort_flag);
         }
         tcgen05_fence_after();
-        const uint32_t sb_columns =
-            smem_u32(scale_slot_base + col_base) + (lane & 3) * column_quad_bytes<kRowBlock>();
+        const uint32_t sb_columns = smem_u32(scale_slot_base + col_base + (lane & 3) * 8);
         const uint32_t taddr_low =
             tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buffer * BN + col_base;
         const uint32_t taddr_high = taddr_low + (16u << 16);
@@ -808,7 +828,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           for (int fragment = 0; fragment < 2 * kBlocks; ++fragment) {
             const int block = fragment >> 1;
             const int high_half = fragment & 1;
-            if (!high_half) load_column_scales(sb_columns + column_block_bytes<kRowBlock>(block), sb);
+            if (!high_half) load_column_scales(sb_columns + block * 128, sb);
             tmem_ld_wait();
             if (fragment + 1 < 2 * kBlocks) {
               const uint32_t next = ((fragment + 1) & 1 ? taddr_high : taddr_low) +
@@ -849,6 +869,38 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int quad = lane & 3;
         const int first_row = row - row_in_cta + quarter * 32 + fragment_row;
         const bool aligned = p.c_vector_ok != 0;
+        if constexpr (kStagedStores) {
+          static_assert(!kGrouped && kBlocks == 4, "two passes of two 32-column blocks");
+          if (aligned && !exchange) {
+            // The warp's rows go to shared memory, 64 FP32 columns at a time, and from there with one bulk copy
+            // of 256 bytes a row; the warp does not wait for memory to take them.
+            const uint32_t warp_base = out_base + warp * 32 * Shape::kOutPitch;
+            float* copied_to = reinterpret_cast<float*>(c) + static_cast<long long>(row) * p.ldc;   // this lane's row
+#pragma unroll
+            for (int pass = 0; pass < 2; ++pass) {
+              bulk_wait_read();
+              __syncwarp();                                    // the previous copies of all lanes have been read
+#pragma unroll
+              for (int r = 0; r < 4; ++r) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                  const float2* v = &acc[r][(2 * pass + i) * 4];
+                  const uint32_t at = warp_base + (fragment_row + 8 * r) * Shape::kOutPitch + 128 * i + 32 * quad;
+                  sts_f32x4(at, v[0], v[1]);
+                  sts_f32x4(at + 16, v[2], v[3]);
+                }
+              }
+              fence_shared_to_async();
+              __syncwarp();
+              const int col = n0 + col_base + 64 * pass;
+              if (row_ok && col < p.n) {
+                bulk_store(copied_to + col, warp_base + lane * Shape::kOutPitch, min(64, p.n - col) * 4);
+              }
+              bulk_commit();
+            }
+            continue;
+          }
+        }
         // Destination addresses of this thread's four rows, fetched in one batch before the first
         // store: a load issued between the stores would wait behind them (the compiler must assume
         // they alias), one round trip per row instead of one per tile.
@@ -940,9 +992,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
               }
               if (row_stored) {
-                if (wide) {
-                  if (col < p.n) store_global_32(c_row + col, w);
-                } else if (aligned && col + 8 <= p.n) {
+                if constexpr (!kStagedStores) {
+                  if (wide) {
+                    if (col < p.n) store_global_32(c_row + col, w);
+                    continue;
+                  }
+                }
+                if (aligned && col + 8 <= p.n) {
                   uint4* out = reinterpret_cast<uint4*>(c_row + col);
                   out[0] = make_uint4(w[0], w[1], w[2], w[3]);
                   out[1] = make_uint4(w[4], w[5], w[6], w[7]);
@@ -959,6 +1015,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
       }
     }
+    if constexpr (kStagedStores) bulk_wait_all();
     if constexpr (kGrouped) {
       // Rows stored into another GPU's memory are consumed there after a collective that
       // follows this kernel in the stream.

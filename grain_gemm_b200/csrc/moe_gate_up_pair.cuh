@@ -434,7 +434,7 @@ __device__ __forceinline__ void gate_up_pair_body(const CUtensorMap& map_x, cons
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
       const uint32_t ring_base = smem_u32(m.ring);
-      const uint32_t token_position = 1024 + ring_column_bytes<32>(lane);
+      const uint32_t token_position = 1024 + ring_column_bytes(lane);
       for (int item = first_item; item < total_items && ok; item += item_step) {
         int tile, jg, expert;
         if (!gate_up_item(p, item, channel_groups, tile, jg, expert)) continue;

@@ -210,7 +210,7 @@ moe_gate_up_tc_kernel(const __grid_constant__ CUtensorMap map_x,
       uint32_t chunk = 0, phase = 0;
       bool ok = true;
       // Byte offsets of this lane's column and row within a 32-float block of a ring slot.
-      const uint32_t column_position = ring_column_bytes<32>(lane);
+      const uint32_t column_position = ring_column_bytes(lane);
       const uint32_t row_position = 4 * ring_row_position(lane);
       const uint32_t ring_base = smem_u32(sb_ring);
       const int up_offset = p.interleaved ? 1 : p.intermediate;   // from a gate scale to its up scale

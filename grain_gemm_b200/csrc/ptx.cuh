@@ -224,6 +224,29 @@ __device__ __forceinline__ void store_global_32(void* address, const uint32_t (&
                : "memory");
 }
 
+// 16-byte shared-memory store by 32-bit shared address.
+__device__ __forceinline__ void sts_f32x4(uint32_t smem_address, float2 a, float2 b) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(smem_address), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y)
+               : "memory");
+}
+
+// ---------------------------------------------------------------- bulk copies to global memory
+
+// This thread's writes to shared memory become visible to copies that are started after it.
+__device__ __forceinline__ void fence_shared_to_async() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+// Shared -> global, both addresses and the size multiples of 16; part of this thread's open bulk group.
+__device__ __forceinline__ void bulk_store(void* destination, uint32_t smem_source, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(destination), "r"(smem_source),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// This thread's groups have left shared memory / are complete.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // ---------------------------------------------------------------- cp.async (scale staging)
 
 // Asynchronous 4-byte copy global -> shared; `valid == false` writes zero without reading.
