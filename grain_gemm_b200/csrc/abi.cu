@@ -95,14 +95,19 @@ struct GemmArgs {
 
 static bool valid_group(int g) { return g == 32 || g == 64 || g == 128 || g == 256; }
 
-// The automatic choice gives one row to the weight-streaming kernel whatever the weights' size,
-// two rows up to this many weight bytes (measured: beyond it split-K is faster for two rows).
-constexpr long long kGemvTwoRowBytes = 32ll << 20;
+// The automatic choice gives one row to the weight-streaming kernel up to this many weight bytes, two rows up to
+// the second number.  Beyond, the tensor-core tiles with short A are faster: one row, N x K = 4096 x 8192 11.4
+// against 14.0 us, 6144 x 6144 14.9 against 13.2, 8192 x 8192 19.2 against 17.7, 14080 x 8448 30.8 against 23.9; two
+// rows, 1024 x 4096 7.0 against 8.1, 4096 x 4096 9.1 against 8.7.
+constexpr long long kGemvOneRowBytes = 34ll << 20, kGemvTwoRowBytes = 8ll << 20;
 
 static bool tensor_core_layout(const GemmArgs& g) {
   return g.a_sk == 1 && g.b_sk == 1 && g.a_sm % 16 == 0 && g.b_sn % 16 == 0 && g.a_sm >= g.k &&
          g.b_sn >= g.k && aligned16(g.a) && aligned16(g.b);
 }
+
+// Up to this many rows the kernels for narrow tiles fetch as many rows of A instead of 128.
+constexpr int kSkinnyRows = 32;
 
 // Split-K plan for skinny M: N tiles of 256 columns times k_splits K ranges fill the SMs; the
 // INT32 group dots go through `workspace` and are folded in group order by a second kernel,
@@ -116,7 +121,7 @@ static SplitKPlan splitk_plan(int m, int n, int k, int group_size) {
   SplitKPlan plan = {1, 0, 0};
   const int groups = (k + group_size - 1) / group_size;
   const int unit = group_size >= 128 ? 1 : 128 / group_size;   // ranges start on 128-byte slabs
-  if (m > 32 || n <= 0 || groups < 2 * unit) return plan;
+  if (m > kSkinnyRows || n <= 0 || groups < 2 * unit) return plan;
   // Finest ranges: the kernel hands every group's INT32 dots to the fold anyway, so a work item
   // of one 128-byte-aligned range costs nothing extra, and tiles x ranges items spread evenly
   // over all SMs whatever N is (a skinny GEMM is bound by how many SMs pull weights at once).
@@ -217,16 +222,30 @@ static int launch_gemv(const GemmArgs& g, cudaStream_t stream) {
   return launch(kernel, grid, kGemvThreads, smem, stream, p);
 }
 
+// Whether a skinny problem (the tc_splitk variant) is one pass over narrow tiles rather than split.  A tile walks
+// its K groups one after the other, 0.29 us each, so splitting pays where the columns are few and the groups
+// many: measured, one pass against split, 8 rows: N = 1024, K = 4096 8.1 against 7.3 us, with G = 64 21.2 against 14.0;
+// N = 1024, K = 2048 5.1 against 6.4; N = 1536, K = 8192 13.3 against 14.7; N = 2048, K = 14336 21.1 against 24.3;
+// N = K = 4096 8.7 against 11.9; N = 14080, K = 8448 23.4 against 38.2 (32 rows: against 56).
+static int skinny_tile(int n) {
+  // One wave of tiles if 64 columns fill it: N = 8192 16.3 against 20.2 us with 128, 14080 29.2 against 23.4.
+  return (n + 63) / 64 <= sm_count() ? GG_VARIANT_TC_N64 : GG_VARIANT_TC_N128;
+}
+static bool skinny_in_one_pass(int n, int k, int group_size) {
+  const int groups = (k + group_size - 1) / group_size;
+  return n >= 1536 || groups <= 8;
+}
+
 static int select_variant(const GemmArgs& g) {
   if (!tensor_core_layout(g)) return GG_VARIANT_SIMT;
-  const bool gemv_rows_ok =
-      g.m == 1 || (g.m == 2 && static_cast<long long>(g.n) * g.k <= kGemvTwoRowBytes);
+  const long long weights = static_cast<long long>(g.n) * g.k;
+  const bool gemv_rows_ok = (g.m == 1 && weights <= kGemvOneRowBytes) || (g.m == 2 && weights <= kGemvTwoRowBytes);
   if (gemv_rows_ok && gemv_eligible(g)) return GG_VARIANT_GEMV;
   const int sms = sm_count();
   const long long tiles_256 = static_cast<long long>((g.m + 127) / 128) * ((g.n + 255) / 256);
   if (splitk_plan(g.m, g.n, g.k, g.group_size).splits >= 2) return GG_VARIANT_TC_SPLITK;
   if (g.m > 128 && tiles_256 >= sms) return GG_VARIANT_TC_PAIR_N256;
-  if (tiles_256 >= sms) return GG_VARIANT_TC_N256;
+  if (g.m > kSkinnyRows && tiles_256 >= sms) return GG_VARIANT_TC_N256;
   const long long tiles_128 = static_cast<long long>((g.m + 127) / 128) * ((g.n + 127) / 128);
   if (tiles_128 >= sms) return GG_VARIANT_TC_N128;
   // Narrow tiles only as long as they fit one wave: a tile of 128 columns takes 1.3 times as long
@@ -356,8 +375,9 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   const int bn = (variant == GG_VARIANT_TC_N256 || variant == GG_VARIANT_TC_PAIR_N256) ? 256
                  : (variant == GG_VARIANT_TC_N128 || variant == GG_VARIANT_TC_PAIR_N128) ? 128
                                                                                          : 64;
+  const bool skinny = g.m <= kSkinnyRows && !pair && bn <= 128;
   CUtensorMap map_a, map_b;
-  int status = row_map(encode_tiled_fn(), &map_a, g.a, g.m, g.k, g.a_sm, 128);
+  int status = row_map(encode_tiled_fn(), &map_a, g.a, g.m, g.k, g.a_sm, skinny ? kSkinnyRows : 128);
   if (status) return status;
   const int row_block = weight_row_block(bn, g.out_dtype);
   bool permuted = g.n % row_block == 0;
@@ -380,6 +400,10 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
   p.tiles_n = (g.n + bn - 1) / bn;
   const int out_bytes = g.out_dtype == GG_OUT_FP32 ? 4 : 2;
   p.c_vector_ok = aligned16(g.c) && (g.ldc * out_bytes) % 16 == 0;
+  if (skinny) {
+    if (bn == 64) return launch_tc_dtype<1, 64, 8, false, 8, kSkinnyRows>(map_a, map_b, p, g.out_dtype, stream);
+    return launch_tc_dtype<1, 128, 5, false, 8, kSkinnyRows>(map_a, map_b, p, g.out_dtype, stream);
+  }
   switch (variant) {
     case GG_VARIANT_TC_N256: return launch_tc_dtype<1, 256, 4, false>(map_a, map_b, p, g.out_dtype, stream);
     case GG_VARIANT_TC_N128: return launch_tc_dtype<1, 128, 3, false>(map_a, map_b, p, g.out_dtype, stream);
@@ -393,6 +417,9 @@ static int launch_gemm_tc(const GemmArgs& g, int variant, cudaStream_t stream) {
 static int launch_gemm_splitk(const GemmArgs& g, void* workspace, size_t workspace_bytes,
                               cudaStream_t stream) {
   const SplitKPlan plan = splitk_plan(g.m, g.n, g.k, g.group_size);
+  if (plan.splits >= 2 && skinny_in_one_pass(g.n, g.k, g.group_size)) {
+    return launch_gemm_tc(g, skinny_tile(g.n), stream);
+  }
   if (plan.splits < 2 || workspace == nullptr || workspace_bytes < plan.workspace_bytes ||
       !aligned16(workspace)) {
     return static_cast<int>(cudaErrorInvalidValue);
@@ -455,7 +482,7 @@ static int run_gemm(const GemmArgs& g, int variant, cudaStream_t stream, void* w
   if (variant == GG_VARIANT_AUTO) {
     variant = select_variant(g);
     // Without a workspace the skinny shapes stay on the single-pass kernels.
-    if (variant == GG_VARIANT_TC_SPLITK && workspace == nullptr) variant = GG_VARIANT_TC_N64;
+    if (variant == GG_VARIANT_TC_SPLITK && workspace == nullptr) variant = skinny_tile(g.n);
   }
   if (variant == GG_VARIANT_TC_SPLITK) {
     if (!tensor_core_layout(g)) return static_cast<int>(cudaErrorInvalidValue);
@@ -608,6 +635,7 @@ int gg_int8_gemm(const void* a, const void* b, const void* scale_a, const void* 
 
 size_t gg_int8_gemm_workspace_bytes(int m, int n, int k, int group_size) {
   if (m <= 0 || n <= 0 || k <= 0 || !gg::valid_group(group_size)) return 0;
+  if (gg::skinny_in_one_pass(n, k, group_size)) return 0;
   return gg::splitk_plan(m, n, k, group_size).workspace_bytes;
 }
 

@@ -116,19 +116,19 @@ struct GemmTcShape {
   // promoted in less, so that tiles of these widths hand over two slabs at a time (one group of 256).
   static constexpr int kSlabs = BN <= 128 ? 2 : 1;
   static constexpr int kBRows = BN / kCtaGroup;         // B rows loaded by each CTA
-  // Rows of A actually fetched per stage.  Skinny problems (M <= kARows) fetch only that many:
-  // the MMA still reads 128 rows, the rest being whatever follows in the stage (the B tile),
-  // which only feeds accumulator rows that are never stored.
+  // Rows of A actually fetched per slab.  Skinny problems (M <= kARows) fetch only that many, which leaves
+  // the room to weights: the MMA still reads 128 rows, the rest being whatever follows in shared
+  // memory (the B tile, the next slab, the scale ring), which only feeds accumulator rows that are
+  // never stored.
   static constexpr int kABytes = kARows * kBK;
-  static_assert(kARows % 8 == 0 && kARows <= 128 && (kARows == 128 || kBRows >= 128),
-                "a short A tile needs the B tile behind it to cover the 128 rows the MMA reads");
+  static_assert(kARows % 8 == 0 && kARows <= 128, "rows come in swizzle atoms of eight");
   static constexpr int kBBytes = kBRows * kBK;
   static constexpr int kSlabBytes = kABytes + kBBytes;
   static constexpr int kStageBytes = kSlabs * kSlabBytes;
   static constexpr int kTmemColumns = 2 * BN;
   // Ring of per-group scale vectors (the short-A shape is the split-K dump kernel, which
   // stages no scales and needs the room for its operand stages).
-  static constexpr int kScaleSlots = kARows == 128 ? 8 : 4;
+  static constexpr int kScaleSlots = kARows == 128 || BN < 256 ? 8 : 4;
   static constexpr int kScaleChunks = kScaleSlots / kScaleChunkGroups;
   static constexpr int kScaleSlotFloats = BN + 128;     // scale_b columns, then scale_a rows
   static constexpr int kScaleBytes = kScaleSlots * kScaleSlotFloats * 4;
@@ -139,6 +139,7 @@ struct GemmTcShape {
   static constexpr int kOutBytes = kStagedStores ? kPromoWarps * 32 * kOutPitch : 0;
   static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kScaleBytes + kOutBytes + kBarrierBytes;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory of a CTA");
+  static_assert(128 * kBK <= kSlabBytes + kScaleBytes, "the last slab's MMAs read inside the allocation");
   static constexpr int kThreads = (kPromoWarps + 4) * 32;   // + producer, MMA, two spares
   static constexpr int kColumnsPerThread = BN / (kPromoWarps / 4);
   // Weight rows come in blocks of this many for outputs of `bytes` bytes (see the drain layout below).

@@ -1,0 +1,36 @@
+"""Up to 32 rows: the narrow tiles that fetch 32 rows of A, and what the automatic choice makes of it, at the
+edges of the rule.  Bit for bit against the CUDA-core kernel.
+"""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 31, 32, 33])
+@pytest.mark.parametrize("n,k,g", [(1535, 2320, 256), (1536, 2320, 256), (77, 2048, 256), (77, 2064, 256), (9472, 272, 32),
+                                   (9536, 272, 128), (300, 16, 64)])
+def test_short_a_tiles_and_the_rule(n, k, g, m, dtype):
+    from grain_gemm_b200 import _loader, gemm, int8_gemm
+    gen = torch.Generator(device="cuda").manual_seed(n + m)
+
+    def draw(*shape):
+        return torch.randint(-127, 128, shape, dtype=torch.int8, device="cuda", generator=gen)
+
+    a, b = draw(m, k), draw(n, k).t()
+    groups = -(-k // g)
+    sa = torch.rand((m, groups), device="cuda", generator=gen)
+    sb = torch.rand((groups, n), device="cuda", generator=gen)
+    expected = gemm.launch(a, b, sa, sb, torch.empty((m, n), dtype=dtype, device="cuda"), g, "simt")
+    for variant in ("tc_n64", "tc_n128"):
+        assert torch.equal(gemm.launch(a, b, sa, sb, torch.empty_like(expected), g, variant), expected), variant
+    assert torch.equal(int8_gemm(a, b, sa, sb, group_size=g, output_dtype=dtype), expected)
+    # The C ABI's plain entry point has no workspace to split with.
+    out = torch.empty_like(expected)
+    status = _loader.library().gg_int8_gemm(
+        _loader.pointer(a), _loader.pointer(b), _loader.pointer(sa), _loader.pointer(sb), _loader.pointer(out), m, n, k,
+        k, 1, 1, k, groups, 1, n, 1, n, g, _loader.OUT_DTYPE[dtype], 0, _loader.stream_pointer(a.device))
+    assert status == 0 and torch.equal(out, expected)
+    assert _loader.device_status() == 0
