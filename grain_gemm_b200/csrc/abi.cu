@@ -95,12 +95,6 @@ struct GemmArgs {
 
 static bool valid_group(int g) { return g == 32 || g == 64 || g == 128 || g == 256; }
 
-// The automatic choice gives one row to the weight-streaming kernel up to this many weight bytes, two rows up to
-// the second number.  Beyond, the tensor-core tiles with short A are faster: one row, N x K = 4096 x 8192 11.4
-// against 14.0 us, 6144 x 6144 14.9 against 13.2, 8192 x 8192 19.2 against 17.7, 14080 x 8448 30.8 against 23.9; two
-// rows, 1024 x 4096 7.0 against 8.1, 4096 x 4096 9.1 against 8.7.
-constexpr long long kGemvOneRowBytes = 34ll << 20, kGemvTwoRowBytes = 8ll << 20;
-
 static bool tensor_core_layout(const GemmArgs& g) {
   return g.a_sk == 1 && g.b_sk == 1 && g.a_sm % 16 == 0 && g.b_sn % 16 == 0 && g.a_sm >= g.k &&
          g.b_sn >= g.k && aligned16(g.a) && aligned16(g.b);
@@ -225,7 +219,7 @@ static int launch_gemv(const GemmArgs& g, cudaStream_t stream) {
 // Whether a skinny problem (the tc_splitk variant) is one pass over narrow tiles rather than split.  A tile walks
 // its K groups one after the other, 0.29 us each, so splitting pays where the columns are few and the groups
 // many: measured, one pass against split, 8 rows: N = 1024, K = 4096 8.1 against 7.3 us, with G = 64 21.2 against 14.0;
-// N = 1024, K = 2048 5.1 against 6.4; N = 1536, K = 8192 13.3 against 14.7; N = 2048, K = 14336 21.1 against 24.3;
+// N = 1024, K = 2048 5.1 against 6.4; N = 1152, K = 3584 7.5 against 8.6; N = 1472, K = 7424 12.3 against 15.6; N = 2048, K = 14336 21.1 against 24.3;
 // N = K = 4096 8.7 against 11.9; N = 14080, K = 8448 23.4 against 38.2 (32 rows: against 56).
 static int skinny_tile(int n) {
   // One wave of tiles if 64 columns fill it: N = 8192 16.3 against 20.2 us with 128, 14080 29.2 against 23.4.
@@ -233,14 +227,30 @@ static int skinny_tile(int n) {
 }
 static bool skinny_in_one_pass(int n, int k, int group_size) {
   const int groups = (k + group_size - 1) / group_size;
-  return n >= 1536 || groups <= 8;
+  return groups <= 8 || n >= (group_size >= 128 ? 1152 : 1536);
+}
+
+// Whether the weight-streaming kernel is the faster one for up to eight rows, by estimates of both that follow
+// the measured times within 15 % or so (us, G = 256 unless said, estimate in brackets).  It reads 4.0 MB a us
+// and pays for every further row: one row, N x K = 4096 x 4096 7.4 [7.7], 8192 x 8192 19.2 [20.3]; two rows 9.1 [9.4],
+// 27 [27]; four 18 [16], 47 [54].  The narrow tiles read 5.6, but walk their K groups one after the other:
+// 4096 x 4096 8.7 [8.6], 8192 x 8192 16.3 [16.0], 4096 x 14336 with G = 128 37 [36], 1024 x 4096 with G = 64 split 14 [14].
+static bool streaming_is_faster(const GemmArgs& g) {
+  if (g.m > kGemvMaxRows || !gemv_eligible(g)) return false;
+  const double weights = static_cast<double>(g.n) * g.k;
+  const int groups = (g.k + g.group_size - 1) / g.group_size;
+  const double per_row[4] = {1.0, 1.4, 3.0, 5.0};
+  const double streaming = 3.5 + weights / 4.0e6 * per_row[g.m <= 2 ? g.m - 1 : g.m <= 4 ? 2 : 3];
+  const bool narrow = skinny_tile(g.n) == GG_VARIANT_TC_N64;
+  const double walk = groups * (g.group_size == 32 ? 0.17 : narrow ? 0.29 : 0.43);
+  const double tiles = skinny_in_one_pass(g.n, g.k, g.group_size)
+                           ? 4.0 + (weights / 5.6e6 > walk ? weights / 5.6e6 : walk) : 5.0 + 0.14 * groups;
+  return streaming < tiles;
 }
 
 static int select_variant(const GemmArgs& g) {
   if (!tensor_core_layout(g)) return GG_VARIANT_SIMT;
-  const long long weights = static_cast<long long>(g.n) * g.k;
-  const bool gemv_rows_ok = (g.m == 1 && weights <= kGemvOneRowBytes) || (g.m == 2 && weights <= kGemvTwoRowBytes);
-  if (gemv_rows_ok && gemv_eligible(g)) return GG_VARIANT_GEMV;
+  if (streaming_is_faster(g)) return GG_VARIANT_GEMV;
   const int sms = sm_count();
   const long long tiles_256 = static_cast<long long>((g.m + 127) / 128) * ((g.n + 255) / 256);
   if (splitk_plan(g.m, g.n, g.k, g.group_size).splits >= 2) return GG_VARIANT_TC_SPLITK;
