@@ -32,10 +32,10 @@
 // before they branch, the scale ring changes hands four groups at a time, no accumulator is
 // modified inside a branch, the probe of a wait carries no suspension limit, and the finished tile
 // needs no exchange between lanes.  That took a group of the G = 32 kernel, everything included, from
-// 1780 to 1500 cycles (M = 1024, N = K = 8192: 464 to 391 us, two waves of 256 groups) and 8192^3 at
-// G = 256 from 479 to 450 us in a short burst.  There a group takes 1710 to 1770 cycles at the 1.70
-// to 1.76 GHz that the part holds inside the launch: more than the loop's 1500, the rest is not
-// accounted for.
+// 1780 to 1430 cycles (M = 1024, N = K = 8192: 464 to 374 us, two waves of 256 groups) and 8192^3 at
+// G = 256 from 479 to 450 us in a short burst.  There a group takes 1540 cycles, and the tile's store
+// and set-up 3500 to 4000 of its 32 groups' time.  Narrow tiles are bound by latencies: a K group takes
+// 550 cycles with 64 columns and 820 with 128, whatever its size; the cause was not found.
 //
 // Any M and N (rows/columns beyond the edge are zero-filled by TMA and never stored), any
 // K that is a multiple of 16 (TMA row pitch), G in {32, 64, 128, 256}; a partial last group
